@@ -13,7 +13,7 @@
 //
 // A plan holds, for n problems (each with its own grid, views, detector and
 // scanner), a table of work tiles -- 32 detector columns x R rows of one
-// view for the thread walk, R columns x 32 rows for column warps (the walk
+// view for the thread walk, R columns x 64 rows for column warps (the walk
 // is fixed at plan time from NEFCT_TUNE_CB_WALK: column warps when both
 // directions use them) -- ordered longest rays first (problems sorted by
 // slab count, views and row bands inside).  The persistent kernel runs one CTA per resident
@@ -52,7 +52,8 @@ nefct_status zfold(const float *acc, float *vol, const nefct_grid &g, cudaStream
 struct BatchDesc {
     GridDev<float> g;
     RayGeom<float> rg;
-    int na, nb, nv, tiles_a, tiles_b, cubic;
+    int na, nb, nv, tiles_a, tiles_b;
+    int near;                            // pairs of neighbouring rows merge their reductions (col_rows_near)
     uint32_t flags;
     const float *cs, *sn, *off;          // per-view tables in the workspace
     const float *vol;
@@ -88,7 +89,6 @@ struct BatchPlan {
     std::vector<size_t> view_off, vol_off; // float offsets in the workspace sections
     uint32_t flags = 0;
     int rows = 4;
-    long long split = 0;                   // tiles of cubic-voxel problems come first
     size_t off_desc = 0, off_t0 = 0, off_views = 0, off_vols = 0, bytes = 0;
     unsigned char *ws = nullptr;           // bound workspace
     int grid_blocks = 0;
@@ -153,9 +153,8 @@ __global__ void __launch_bounds__(256) batch_zcopy_kernel(const __grid_constant_
     }
 }
 
-// One persistent launch serves tiles [begin, end) of problems that share
-// the DIV variant (cubic voxels or not).
-template <bool FWD, bool DIV>
+// One persistent launch serves the tiles [begin, end).
+template <bool FWD>
 __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ BatchArgs a)
 {
     __shared__ long long s_item;
@@ -178,22 +177,20 @@ __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ Batc
         cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib, r);
         const size_t id = ((size_t)iv * P.nb + ib) * P.na + ia;
         if (FWD) {
-            P.sino[id] = ray_forward<float, DIV>(P.g, r, P.flags, P.vol, P.volT);
+            P.sino[id] = ray_forward<float, false>(P.g, r, P.flags, P.vol, P.volT);
         } else {
             const float y = P.grad[id];
             if (y == 0.f) continue;
-            ray_backward<float, DIV>(P.g, r, P.flags, y, P.back, P.volT);
+            ray_backward<float, false>(P.g, r, P.flags, y, P.back, P.volT);
         }
     }
 }
 
-// Column-warp variant: a tile is blockDim.y columns x 32 rows of one view,
+// Column-warp variant: a tile is blockDim.y columns x 64 rows of one view,
 // one warp per column.  Bounded to 64 registers (4 CTAs of 256 threads per
 // SM) like the single-problem kernels: the dynamically indexed problem
-// descriptor then spills 100-260 bytes, and the kernel still runs faster
-// than at its unbounded 80-94 registers (96 small problems: 4.67 against
-// 5.26 ms per forward + transpose).
-template <bool FWD, bool DIV>
+// descriptor then spills up to 200 bytes outside the slab loops.
+template <bool FWD, bool REF>
 __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_constant__ BatchArgs a)
 {
     __shared__ long long s_item;
@@ -210,14 +207,33 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
         const long long rest = local / P.tiles_a;
         const int rt = (int)(rest % P.tiles_b);
         const int iv = (int)(rest / P.tiles_b);
-        const int ia = ct * blockDim.y + threadIdx.y, ib = rt * 32 + threadIdx.x;
+        const int ia = ct * blockDim.y + threadIdx.y;
         if (ia >= P.na) continue;         // uniform across the warp
-        const bool has = ib < P.nb;
-        const size_t id = ((size_t)iv * P.nb + (has ? ib : 0)) * P.na + ia;
-        float r[6];
-        cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has ? ib : 0, r);
-        if (FWD) colwarp_lane<DIV, true>(P.g, r, has, P.flags, P.volT, P.sino + id, 0.f, nullptr);
-        else colwarp_lane<DIV, false>(P.g, r, has, P.flags, nullptr, nullptr, has ? P.grad[id] : 0.f, P.volT);
+        if (FWD) {
+            auto row = [&](int i, float (&r)[6]) {
+                const int ib = col_row<2, false>(rt, threadIdx.x, i, false);
+                cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib < P.nb ? ib : 0, r);
+                return ib < P.nb;
+            };
+            auto store = [&](int i, float v) {
+                const int ib = col_row<2, false>(rt, threadIdx.x, i, false);
+                P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
+            };
+            colwarp_forward<2, REF>(P.g, P.flags, P.volT, row, store);
+        } else {
+            float r[2][6], y[2];
+            bool has[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int ib = P.near ? col_row<2, true>(rt, threadIdx.x, i, P.rg.db < 0.f)
+                                      : col_row<2, false>(rt, threadIdx.x, i, false);
+                has[i] = ib < P.nb;
+                y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
+                cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);
+            }
+            if (P.near) colwarp_backward<2, REF, true>(P.g, r, has, P.flags, y, P.volT);
+            else colwarp_backward<2, REF, false>(P.g, r, has, P.flags, y, P.volT);
+        }
     }
 }
 
@@ -294,28 +310,18 @@ static nefct_status batch_launch(BatchPlan *b, bool fwd, cudaStream_t s)
     const long long total = b->t0.back();
     const dim3 blk(32, b->rows);
     BatchArgs &a = *b->args;
-    if (b->split > 0) {
-        a.begin = 0; a.end = b->split; a.counter = counter;
-        if (b->colwarp) {
-            if (fwd) batch_colwarp_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
-            else batch_colwarp_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
-        } else {
-            if (fwd) batch_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
-            else batch_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
-        }
-        NEFCT_CHECK_LAUNCH("batch_kernel (cubic voxels)");
+    a.begin = 0; a.end = total; a.counter = counter;
+    if (b->colwarp) {
+        const bool ref = ref_rounding(b->flags);
+        if (fwd && ref) batch_colwarp_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
+        else if (fwd) batch_colwarp_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
+        else if (ref) batch_colwarp_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
+        else batch_colwarp_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
+    } else {
+        if (fwd) batch_kernel<true><<<b->grid_blocks, blk, 0, s>>>(a);
+        else batch_kernel<false><<<b->grid_blocks, blk, 0, s>>>(a);
     }
-    if (b->split < total) {
-        a.begin = b->split; a.end = total; a.counter = counter + 1;
-        if (b->colwarp) {
-            if (fwd) batch_colwarp_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
-            else batch_colwarp_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
-        } else {
-            if (fwd) batch_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
-            else batch_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
-        }
-        NEFCT_CHECK_LAUNCH("batch_kernel (other voxels)");
-    }
+    NEFCT_CHECK_LAUNCH("batch_kernel");
     if (!fwd && b->colwarp) {
         batch_zcopy_kernel<true><<<copy_blocks, dim3(32, 8), 0, s>>>(ca, copy_tiles);
         NEFCT_CHECK_LAUNCH("batch_zcopy_kernel (fold)");
@@ -375,17 +381,10 @@ nefct_status nefct_cb_batch_plan(const nefct_cb_problem *problems, int32_t n, ui
     for (int i = 0; i < n; ++i)
         b->colwarp = b->colwarp && cb_use_colwarp<float>(problems[i].geom.grid, flags, true) &&
                      cb_use_colwarp<float>(problems[i].geom.grid, flags, false);
-    // cubic-voxel problems first (one kernel variant each), longest rays
-    // first within each group: a tile's cost grows with its rays' slab count
-    auto cubic = [&](int i) {
-        const GridDev<float> g = make_grid_dev<float>(problems[i].geom.grid);
-        return g.dy == 1.f && g.dz == 1.f;
-    };
+    // longest rays first: a tile's cost grows with its rays' slab count
     b->order.resize(n);
     std::iota(b->order.begin(), b->order.end(), 0);
     std::stable_sort(b->order.begin(), b->order.end(), [&](int a, int c) {
-        const bool ca = cubic(a), cc = cubic(c);
-        if (ca != cc) return ca;
         const nefct_grid &ga = problems[a].geom.grid, &gc = problems[c].geom.grid;
         return std::max(ga.nx, ga.ny) > std::max(gc.nx, gc.ny);
     });
@@ -402,12 +401,11 @@ nefct_status nefct_cb_batch_plan(const nefct_cb_problem *problems, int32_t n, ui
         D.rg = make_ray_geom<float>(g);
         D.na = g.na; D.nb = g.nb; D.nv = g.nv;
         D.tiles_a = b->colwarp ? (g.na + b->rows - 1) / b->rows : (g.na + 31) / 32;
-        D.tiles_b = b->colwarp ? (g.nb + 31) / 32 : (g.nb + b->rows - 1) / b->rows;
-        D.cubic = D.g.dy == 1.f && D.g.dz == 1.f;
+        D.tiles_b = b->colwarp ? (g.nb + 63) / 64 : (g.nb + b->rows - 1) / b->rows;
+        D.near = col_rows_near(D.g, D.rg);
         D.flags = flags;
         b->t0[k + 1] = b->t0[k] + (long long)D.tiles_a * D.tiles_b * g.nv;
         b->c0[k + 1] = b->c0[k] + (long long)((g.grid.nx + 31) / 32) * ((g.grid.nz + 31) / 32) * g.grid.ny;
-        if (D.cubic) b->split = b->t0[k + 1];
         b->view_off[k] = views;
         views += 3 * (size_t)g.nv;
         b->vol_off[k] = vols;
@@ -463,11 +461,11 @@ nefct_status nefct_cb_batch_bind(nefct_cb_batch *b, void *workspace, size_t byte
     NEFCT_CHECK_CUDA(cudaGetDevice(&dev));
     NEFCT_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int lo = 1 << 30;
-    const void *kernels[4] = {(const void *)batch_kernel<true, false>, (const void *)batch_kernel<true, true>,
-                              (const void *)batch_kernel<false, false>, (const void *)batch_kernel<false, true>};
-    const void *colwarp_kernels[4] = {
-        (const void *)batch_colwarp_kernel<true, false>, (const void *)batch_colwarp_kernel<true, true>,
-        (const void *)batch_colwarp_kernel<false, false>, (const void *)batch_colwarp_kernel<false, true>};
+    const bool ref = ref_rounding(b->flags);
+    const void *kernels[2] = {(const void *)batch_kernel<true>, (const void *)batch_kernel<false>};
+    const void *colwarp_kernels[2] = {
+        ref ? (const void *)batch_colwarp_kernel<true, true> : (const void *)batch_colwarp_kernel<true, false>,
+        ref ? (const void *)batch_colwarp_kernel<false, true> : (const void *)batch_colwarp_kernel<false, false>};
     for (const void *k : b->colwarp ? colwarp_kernels : kernels) {
         NEFCT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * b->rows, 0));
         lo = std::min(lo, per_sm);

@@ -1,14 +1,47 @@
-// Instantiations of the cone-beam transpose (backprojection) kernels (one direction per
-// translation unit so the two compile in parallel).
+// Transpose cone-beam kernels (thread walk and column warps) for float and
+// double: see cb_kernels.cuh.
 #include "cb_kernels.cuh"
 
 namespace nefct {
+
+// Column warps: one warp per 32 R rows of column ia at view iv, into the
+// z-fastest accumulator p.outT.
+template <int R, bool REF, bool PAIR>
+__global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __grid_constant__ CBParams<float> p)
+{
+    const int ia = blockIdx.x * blockDim.y + threadIdx.y;
+    const int tile = p.band_major ? blockIdx.z : blockIdx.y;
+    const int iv = p.band_major ? blockIdx.y : blockIdx.z;
+    if (ia >= p.na) return;                       // uniform across the warp
+    float r[R][6], y[R];
+    bool has[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int ib = col_row<R, PAIR>(tile, threadIdx.x, i, p.rg.db < 0.f);
+        has[i] = ib < p.nb;
+        y[i] = has[i] ? cb_sino_value(p, ia, ib, iv) : 0.f;
+        cb_ray(p, ia, has[i] ? ib : 0, iv, r[i]);
+    }
+    colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, p.outT);
+}
+
+template <int R, bool PAIR>
+static cudaError_t launch_colwarp(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
+{
+    dim3 grid, block;
+    cb_colwarp_shape(p, na, nb, nvc, grid, block, R);
+    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, PAIR><<<grid, block, 0, s>>>(p);
+    else cb_colwarp_backward_kernel<R, false, PAIR><<<grid, block, 0, s>>>(p);
+    return cudaGetLastError();
+}
 
 template <typename T>
 cudaError_t cb_launch_backward(CBParams<T> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s, bool colwarp)
 {
     if constexpr (std::is_same<T, float>::value) {
-        if (colwarp) return cb_launch_colwarp<false>(p, na, nb, nvc, s);
+        if (colwarp)
+            return col_rows_near(p.g, p.rg) ? launch_colwarp<2, true>(p, na, nb, nvc, flags, s)
+                                            : launch_colwarp<1, false>(p, na, nb, nvc, flags, s);
     }
     return cb_launch<T, false>(p, na, nb, nvc, flags, s);
 }

@@ -7,15 +7,15 @@
 //    detector columns x blockDim.y rows per CTA, each warp 32 neighbouring
 //    columns of one row; volume x-fastest plus a y-fastest copy for x-driven
 //    rays;
-//  * column warps (cb_colwarp_kernel, FP32): each warp 32 consecutive rows
-//    of one column, blockDim.y columns per CTA, over a z-fastest copy of the
-//    volume (colwarp.cuh); the forward's cb_colwarp_rows_kernel gives each
-//    lane two rows (l and l + 32) of a 64-row tile.
+//  * column warps (colwarp_forward / colwarp_backward, FP32): each warp 32 R
+//    rows of one column, R per lane, blockDim.y columns per CTA, over a
+//    z-fastest copy of the volume (colwarp.cuh).
 // The grid runs (column tile, view, row band) with the row band slowest, or
 // (column tile, row band, view).  Per-view cos/sin/z-offset ride in the
 // kernel parameters.
 #pragma once
 
+#include <math.h>
 #include <type_traits>
 
 #include "colwarp.cuh"
@@ -67,6 +67,86 @@ template <typename T> __device__ __forceinline__ T cb_sino_value(const CBParams<
     return id < total ? p.sino[id] : (T)0;
 }
 
+// Whether a call's z splits follow the reference's rounding (colwarp.cuh, REF).
+__host__ __device__ __forceinline__ bool ref_rounding(uint32_t flags) { return (flags & NEFCT_TIE_GT) != 0; }
+
+// Sum of the volume along one ray again, without reading the voxels whose
+// share is exactly 0 (in the grid, next to a voxel the ray passes): taken when
+// a fast sum is not finite, so that an infinity or a NaN of a voxel the ray
+// does not pass cannot enter it.
+__device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1, float y1, float z1, float x2,
+                                               float y2, float z2, uint32_t flags, const float *vol, unsigned su,
+                                               unsigned sv, unsigned sw)
+{
+    const float r[6] = {x1, y1, z1, x2, y2, z2};
+    Walk<float> w;
+    if (!setup_walk(g, r, flags, w)) return 0.f;
+    GatherSink<true> f(vol, sw);
+    if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, sw, f);
+    else ray_walk<false>(g, w, su, sv, sw, f);
+    return f.whole * w.W;
+}
+
+// Strides of the thread walk along (u, v): x-driven rays use the y-fastest
+// copy when there is one.
+__device__ __forceinline__ void thread_strides(int nx, int ny, bool xdrive, bool copy, unsigned &su, unsigned &sv)
+{
+    su = !xdrive ? (unsigned)nx : copy ? (unsigned)ny : 1u;
+    sv = !xdrive || copy ? 1u : (unsigned)nx;
+}
+
+// Forward value of one ray: gathers x-driven rays from the y-fastest copy
+// volT when there is one, everything else from the x-fastest volume.  DIV
+// (double only): the voxels are not cubic.
+template <typename T, bool DIV, bool EXACT = false>
+__device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32_t flags, const T *vol, const T *volT)
+{
+    if (EXACT) return exact_forward(g, r, flags, vol, volT);
+    Walk<T> w;
+    if (!setup_walk(g, r, flags, w)) return (T)0;
+    const int sw = g.nx * g.ny;
+    if constexpr (std::is_same<T, float>::value) {
+        const float *const v = w.xdrive && volT ? volT : vol;
+        unsigned su, sv;
+        thread_strides(g.nx, g.ny, w.xdrive, volT != nullptr, su, sv);
+        GatherSink<> f(v, (unsigned)sw);
+        if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
+        else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
+        const float sum = f.whole;
+        if (!isfinite(sum)) return ray_resum(g, r[0], r[1], r[2], r[3], r[4], r[5], flags, v, su, sv, (unsigned)sw);
+        return sum * w.W;
+    } else {
+        if (!w.xdrive) return gather_walk<T, DIV, true, false>(w, g, vol, g.nx, 1, sw);
+        if (volT) return gather_walk<T, DIV, true, false>(w, g, volT, g.ny, 1, sw);
+        return gather_walk<T, DIV, false, false>(w, g, vol, 1, g.nx, sw);
+    }
+}
+
+// Transpose contribution of one ray with value y: x-driven rays reduce into
+// the y-fastest accumulator outT when there is one.
+template <typename T, bool DIV, bool EXACT = false>
+__device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, uint32_t flags, T y, T *out, T *outT)
+{
+    if (EXACT) {
+        exact_backward(g, r, flags, y, out, outT);
+        return;
+    }
+    Walk<T> w;
+    if (!setup_walk(g, r, flags, w)) return;
+    const int sw = g.nx * g.ny;
+    if constexpr (std::is_same<T, float>::value) {
+        unsigned su, sv;
+        thread_strides(g.nx, g.ny, w.xdrive, outT != nullptr, su, sv);
+        ScatterSink f{w.xdrive && outT ? outT : out, (unsigned)sw, y * w.W};
+        if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
+        else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
+    } else {
+        if (!w.xdrive) scatter_walk<T, DIV, true, false>(w, g, out, g.nx, 1, sw, y);
+        else if (outT) scatter_walk<T, DIV, true, false>(w, g, outT, g.ny, 1, sw, y);
+        else scatter_walk<T, DIV, false, false>(w, g, out, 1, g.nx, sw, y);
+    }
+}
+
 template <typename T, bool DIV, bool EXACT = false>
 __global__ void __launch_bounds__(256) cb_forward_kernel(const __grid_constant__ CBParams<T> p)
 {
@@ -92,217 +172,124 @@ __global__ void __launch_bounds__(256) cb_backward_kernel(const __grid_constant_
     ray_backward<T, DIV, EXACT>(p.g, r, p.flags, y, p.out, p.outT);
 }
 
-// One lane of a column warp (the whole warp calls it together).  has: the
-// lane has a ray r; FWD: gathers from the z-fastest copy volZ into *out;
-// otherwise reduces y times the ray's weights into the z-fastest accumulator
-// accZ, or (FIX) as 64-bit fixed-point integers (value * weight * scale,
-// rounded) into fixZ.  Rays without a contribution (outside the detector,
-// missing the grid, zero value) stay in the warp's walk with every slot
-// inactive.
-template <bool DIV, bool FWD, bool FIX = false>
-__device__ __forceinline__ void colwarp_lane(const GridDev<float> &g, const float *r, bool has, uint32_t flags,
-                                             const float *__restrict__ volZ, float *out, float y, float *accZ,
-                                             unsigned long long *fixZ = nullptr, float scale = 0.f)
+// Forward of R rows per lane of one detector column (the whole warp calls
+// it) over the z-fastest copy volZ.  row(i, r): the lane's i-th ray (false: it
+// has none); store(i, v): takes its value.
+template <int R, bool REF, class Row, class Store>
+__device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_t flags, const float *__restrict__ volZ,
+                                                Row row, Store store)
 {
-    Walk<float> w{};
-    const bool live = has && (FWD || y != 0.f) && setup_walk(g, r, flags, w);
-    if (!__any_sync(0xffffffffu, live)) {
-        if (FWD && has) *out = 0.f;
-        return;
-    }
-    ColShared c;
-    ColLane L;
-    int K0, K1, KI0, KI1;
-    if (!col_setup(g, w, live, c, L, K0, K1, KI0, KI1)) {
-        // rays of the column disagree on the shared parameters: walk alone
-        unsigned su, sv;
-        col_strides(g, w.xdrive, su, sv);
-        if (FWD) {
-            const float v = live ? gather_walk<float, DIV, false, false>(w, g, volZ, (int)su, (int)sv, 1) : 0.f;
-            if (has) *out = v;
-        } else if (live && FIX) {
-            scatter_walk_fixed<float, DIV, false>(w, g, fixZ, (int)su, (int)sv, 1, y, scale);
-        } else if (live) {
-            scatter_walk<float, DIV, false, false>(w, g, accZ, (int)su, (int)sv, 1, y);
+    ColRays<R> q;
+    unsigned has = 0;
+    {
+        float r[R][6];
+        bool h[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            h[i] = row(i, r[i]);
+            has |= (unsigned)h[i] << i;
         }
-        return;
+        if (!col_rays<R>(g, r, h, flags, q)) {
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (h[i]) store(i, 0.f);
+            return;
+        }
     }
-    if constexpr (FWD) {
-        float acc = 0.f;
-        // interior slabs load every slot unpredicated: an inactive slot has
-        // ratio 0 and a valid index (so a volume holding +-inf may give NaN
-        // where the reference gives +-inf); lanes without a ray are discarded
-        auto f = [&](const auto &s) {
-            float v[s.n];
+    GatherSink<> f[R];
 #pragma unroll
-            for (int i = 0; i < s.n; ++i) v[i] = (!s.checked || s.ok[i]) ? __ldg(volZ + s.idx[i]) : 0.f;
+    for (int i = 0; i < R; ++i) f[i] = GatherSink<>(volZ, 1u);
+    if (q.steep) {
 #pragma unroll
-            for (int i = 0; i < s.n; ++i) acc += v[i] * s.r[i];
-        };
-        col_walk_any<DIV, 0>(c, L, K0, K1, KI0, KI1, g, f);
-        if (has) *out = live ? acc * w.W : 0.f;
-    } else if constexpr (FIX) {
-        const float yw = y * w.W;
-        auto f = [&](const auto &s) {
-#pragma unroll
-            for (int i = 0; i < s.n; ++i)
-                if (s.ok[i]) atomicAdd(fixZ + s.idx[i], (unsigned long long)to_fixed((yw * s.r[i]) * scale));
-        };
-        col_walk_any<DIV, 1>(c, L, K0, K1, KI0, KI1, g, f);
+        for (int i = 0; i < R; ++i) col_each<REF>(q.c, q.K0, q.K1, q.z[i], q.zg, f[i]);
+    } else if (q.rising && q.falling) {
+        col_gather<R, REF, true>(q, volZ, f);
     } else {
-        const float yw = y * w.W;
-        auto f = [&](const auto &s) {
-            if constexpr (s.n == 2) {
-                // the two-slot split's weights are r and 1 - r: y w (1 - r) in one rounding
-                if (s.ok[0]) atomicAdd(accZ + s.idx[0], yw * s.r[0]);
-                if (s.ok[1]) atomicAdd(accZ + s.idx[1], fmaf(-yw, s.r[0], yw));
-            } else {
+        col_gather<R, REF, false>(q, volZ, f);
+    }
 #pragma unroll
-                for (int i = 0; i < s.n; ++i)
-                    if (s.ok[i]) atomicAdd(accZ + s.idx[i], yw * s.r[i]);
-            }
-        };
-        col_walk_any<DIV, 2>(c, L, K0, K1, KI0, KI1, g, f);
+    for (int i = 0; i < R; ++i) {
+        if (!(has >> i & 1u)) continue;
+        float v = f[i].whole;
+        if (!q.z[i].live) v = 0.f;
+        else if (isfinite(v)) v *= q.W[i];
+        else {
+            float r[6];
+            row(i, r);
+            v = ray_resum(g, r[0], r[1], r[2], r[3], r[4], r[5], flags, volZ, q.c.su, q.c.sv, 1u);
+        }
+        store(i, v);
     }
 }
 
-// R rays per lane (rows l, l + 32, ... of the column): the same walk and
-// arithmetic per ray as colwarp_lane, with the warp's slab table and split
-// decisions shared by all 32 R rays.  Float forward (FWD) and float
-// transpose only.
-template <bool DIV, bool FWD, int R>
-__device__ __forceinline__ void colwarp_rows(const GridDev<float> &g, const float (&r)[R][6], const bool (&has)[R],
-                                             uint32_t flags, const float *__restrict__ volZ, float *const (&out)[R],
-                                             const float (&y)[R], float *accZ)
+// Transpose of R rows per lane of one detector column: y[i] times the ray's
+// weights into the z-fastest accumulator accZ.  PAIR: rows 2i and 2i + 1 are
+// neighbours in z order and merge their reductions.
+template <int R, bool REF, bool PAIR>
+__device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const float (&r)[R][6], bool (&has)[R],
+                                                 uint32_t flags, const float (&y)[R], float *accZ)
 {
-    Walk<float> w[R];
-    bool live[R];
-    bool any = false;
+    ColRays<R> q;
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-        w[k] = Walk<float>{};
-        live[k] = has[k] && (FWD || y[k] != 0.f) && setup_walk(g, r[k], flags, w[k]);
-        any = any || live[k];
+    for (int i = 0; i < R; ++i) has[i] = has[i] && y[i] != 0.f;
+    if (!col_rays<R>(g, r, has, flags, q)) return;
+    float yw[R];
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        yw[i] = q.z[i].live ? y[i] * q.W[i] : 0.f;
+        finite = finite && isfinite(yw[i]);
     }
-    if (!__any_sync(0xffffffffu, any)) {
-        if (FWD) {
+    if (q.steep || !__all_sync(0xffffffffu, finite)) {
 #pragma unroll
-            for (int k = 0; k < R; ++k)
-                if (has[k]) *out[k] = 0.f;
+        for (int i = 0; i < R; ++i) {
+            ScatterSink f{accZ, 1u, yw[i]};
+            col_each<REF>(q.c, q.K0, q.K1, q.z[i], q.zg, f);
         }
         return;
     }
-    ColShared c;
-    ColLane L[R];
-    int K0, K1, KI0, KI1;
-    if (!col_setup_rows<R>(g, w, live, c, L, K0, K1, KI0, KI1)) {
-        // rays of the column disagree on the shared parameters: each walks alone
+    const bool mixed = q.rising && q.falling;
+    if constexpr (PAIR) {
+        // the gap between two rays is linear along the walk: in [0, 1) at both
+        // ends, by more than the positions' rounding, it is so in every slab
+        const float d0 = col_plane(q.c, q.K0), d1 = col_plane(q.c, q.K1 + 1);
+        bool near = true;
 #pragma unroll
-        for (int k = 0; k < R; ++k) {
-            unsigned su, sv;
-            col_strides(g, w[k].xdrive, su, sv);
-            if (FWD) {
-                const float v = live[k] ? gather_walk<float, DIV, false, false>(w[k], g, volZ, (int)su, (int)sv, 1) : 0.f;
-                if (has[k]) *out[k] = v;
-            } else if (live[k]) {
-                scatter_walk<float, DIV, false, false>(w[k], g, accZ, (int)su, (int)sv, 1, y[k]);
+        for (int i = 0; i < R; i += 2) {
+            ZRay &z0 = q.z[i], &z1 = q.z[i + 1];
+            if (z0.live && z1.live) {
+                const float dk = z1.kz - z0.kz, dz = z1.z0 - z0.z0;
+                const float g0 = fmaf(dk, d0, dz), g1 = fmaf(dk, d1, dz);
+                const float m = 1e-3f + 1e-6f * (fabsf(z0.z0) + fabsf(z0.kz) * (fabsf(q.c.pu) + fabsf(q.c.nu2)));
+                near = near && fminf(g0, g1) > m && fmaxf(g0, g1) < 1.f - m;
+            } else if (z0.live) {                  // one ray of the pair: the other walks along with value 0
+                z1 = z0;
+                z1.live = false;
+            } else if (z1.live) {
+                z0 = z1;
+                z0.live = false;
             }
         }
-        return;
-    }
-    if constexpr (FWD) {
-        float acc[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) acc[k] = 0.f;
-        auto f = [&](const auto &s, int k) {
-            float v[s.n];
-#pragma unroll
-            for (int i = 0; i < s.n; ++i) v[i] = (!s.checked || s.ok[i]) ? __ldg(volZ + s.idx[i]) : 0.f;
-#pragma unroll
-            for (int i = 0; i < s.n; ++i) acc[k] += v[i] * s.r[i];
-        };
-        col_walk_any_rows<DIV, 0, R>(c, L, K0, K1, KI0, KI1, g, f);
-#pragma unroll
-        for (int k = 0; k < R; ++k)
-            if (has[k]) *out[k] = live[k] ? acc[k] * w[k].W : 0.f;
+        if (!__all_sync(0xffffffffu, near)) {
+            col_scatter<R, REF, true, kAny>(q, accZ, yw);
+        } else if (mixed) {
+            col_scatter<R, REF, true, kNear>(q, accZ, yw);
+        } else {
+            col_scatter<R, REF, false, kNear>(q, accZ, yw);
+        }
     } else {
-        float yw[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) yw[k] = y[k] * w[k].W;
-        auto f = [&](const auto &s, int k) {
-            if constexpr (s.n == 2) {
-                if (s.ok[0]) atomicAdd(accZ + s.idx[0], yw[k] * s.r[0]);
-                if (s.ok[1]) atomicAdd(accZ + s.idx[1], fmaf(-yw[k], s.r[0], yw[k]));
-            } else {
-#pragma unroll
-                for (int i = 0; i < s.n; ++i)
-                    if (s.ok[i]) atomicAdd(accZ + s.idx[i], yw[k] * s.r[i]);
-            }
-        };
-        col_walk_any_rows<DIV, 2, R>(c, L, K0, K1, KI0, KI1, g, f);
+        if (mixed) col_scatter<R, REF, true, kSingle>(q, accZ, yw);
+        else col_scatter<R, REF, false, kSingle>(q, accZ, yw);
     }
 }
 
-// Column warps: warp = rows [32*tile, 32*tile + 32) of column ia at view iv,
-// over the z-fastest copy p.volT (forward, into p.out) or accumulator p.outT.
-// (at most 64 registers: 4 CTAs of 256 threads per SM; measured faster than
-// the unconstrained 70)
-template <bool DIV, bool FWD>
-__global__ void __launch_bounds__(256, 4) cb_colwarp_kernel(const __grid_constant__ CBParams<float> p)
+// Row i of lane `lane` in row tile `tile` of a column warp with R rows per
+// lane: rows 32 apart, or (PAIR) rows 2i and 2i + 1 neighbours, in z order
+// (rows fall in z when their pitch is negative).
+template <int R, bool PAIR> __device__ __forceinline__ int col_row(int tile, int lane, int i, bool falling)
 {
-    const int lane = threadIdx.x;
-    const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    int ib, iv;
-    if (p.band_major) { iv = blockIdx.y; ib = blockIdx.z * 32 + lane; }
-    else { ib = blockIdx.y * 32 + lane; iv = blockIdx.z; }
-    if (ia >= p.na) return;                       // uniform across the warp
-    const bool has = ib < p.nb;
-    float y = 0.f;
-    if (!FWD && has) y = cb_sino_value(p, ia, ib, iv);
-    float r[6];
-    cb_ray(p, ia, has ? ib : 0, iv, r);
-    float *const out = FWD ? p.out + (size_t)(p.v0 + iv) * p.na * p.nb + (size_t)ib * p.na + ia : nullptr;
-    colwarp_lane<DIV, FWD>(p.g, r, has, p.flags, p.volT, out, y, p.outT);
-}
-
-// Rays per lane of the float column-warp kernels, per direction.  Measured
-// (512^3, 180 of 720 views of 1024 x 768; 256^3, 360 views of 512 x 384):
-// two rays per lane take the forward from 79.6 to 77.7 ms and from 19.1 to
-// 18.8 ms (80 registers, 3 CTAs of 256 per SM; bit-identical output) but
-// the transpose from 97.8 to 100.2 ms, so the transpose keeps one.
-#ifndef NEFCT_COL_ROWS_FWD
-#define NEFCT_COL_ROWS_FWD 2
-#endif
-#ifndef NEFCT_COL_ROWS_BWD
-#define NEFCT_COL_ROWS_BWD 1
-#endif
-#ifndef NEFCT_COL_MINB
-#define NEFCT_COL_MINB 3
-#endif
-
-// Column warps with R rays per lane: warp = rows [32 R tile, 32 R (tile + 1))
-// of column ia at view iv (at most 80 registers: 3 CTAs of 256 per SM).
-template <bool DIV, bool FWD, int R>
-__global__ void __launch_bounds__(256, NEFCT_COL_MINB) cb_colwarp_rows_kernel(const __grid_constant__ CBParams<float> p)
-{
-    const int lane = threadIdx.x;
-    const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    const int tile = p.band_major ? blockIdx.z : blockIdx.y;
-    const int iv = p.band_major ? blockIdx.y : blockIdx.z;
-    if (ia >= p.na) return;                       // uniform across the warp
-    float r[R][6];
-    bool has[R];
-    float y[R];
-    float *out[R];
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-        const int ib = (tile * R + k) * 32 + lane;
-        has[k] = ib < p.nb;
-        y[k] = (!FWD && has[k]) ? cb_sino_value(p, ia, ib, iv) : 0.f;
-        cb_ray(p, ia, has[k] ? ib : 0, iv, r[k]);
-        out[k] = FWD ? p.out + (size_t)(p.v0 + iv) * p.na * p.nb + (size_t)ib * p.na + ia : nullptr;
-    }
-    colwarp_rows<DIV, FWD, R>(p.g, r, has, p.flags, p.volT, out, y, p.outT);
+    return PAIR ? tile * 32 * R + (i >> 1) * 64 + lane * 2 + (falling ? 1 - (i & 1) : (i & 1))
+                : (tile * R + i) * 32 + lane;
 }
 
 // Launch shape of the thread walk for nvc views (see cb_cell).
@@ -317,7 +304,7 @@ static inline void cb_shape(CBParams<T> &p, int na, int nb, int nvc, dim3 &grid,
 }
 
 // Launch shape of the column warps: NEFCT_TUNE_CB_ROWS columns (warps) per
-// CTA, 32 rows per warp.
+// CTA, 32 rays_per_lane rows per warp.
 template <typename T>
 static inline void cb_colwarp_shape(CBParams<T> &p, int na, int nb, int nvc, dim3 &grid, dim3 &block,
                                     int rays_per_lane = 1)
@@ -332,13 +319,25 @@ static inline void cb_colwarp_shape(CBParams<T> &p, int na, int nb, int nvc, dim
 // The walk skips its divisions when both transverse pitches equal the x pitch.
 template <typename T> static inline bool cubic(const GridDev<T> &g) { return g.dy == (T)1 && g.dz == (T)1; }
 
+// Whether neighbouring rows of a column are close enough, at the rotation
+// axis, for pairs of them to share reductions.  Rows further apart rarely meet
+// in a voxel, and 32 consecutive rows per warp then touch fewer sectors than
+// 32 pairs.  256^3, 24 views, pitch 0.7 / 0.85 / 0.95 / 1.1 voxels at the
+// axis: pairs 0.95 / 0.84 / 0.71 / 0.74 ms, single rows 1.27 / 0.91 / 0.67 /
+// 0.55 ms.
+static inline bool col_rows_near(const GridDev<float> &g, const RayGeom<float> &rg)
+{
+    return rg.src_iso > 0.f && rg.src_det > 0.f && fabsf(rg.db) * rg.src_iso / rg.src_det < 0.9f * g.dz * g.dx_;
+}
+
 // Column warps apply to FP32 slab walks with a workspace; the z-fastest
 // copy's transposes launch ny planes (grid z), and the packed v floors hold
-// n + 3 in 16 bits.
+// n + 3 in 16 bits.  (NEFCT_DETERMINISTIC changes nothing for the forward;
+// its transpose has kernels of its own.)
 template <typename T> static inline bool cb_use_colwarp(const nefct_grid &g, uint32_t flags, bool forward)
 {
     return sizeof(T) == sizeof(float) && (tune_get(NEFCT_TUNE_CB_WALK) & (forward ? 1 : 2)) != 0 &&
-           !(flags & (NEFCT_EXACT | NEFCT_NO_TRANSPOSE | NEFCT_DETERMINISTIC)) && g.ny <= 65535 &&
+           !(flags & (NEFCT_EXACT | NEFCT_NO_TRANSPOSE)) && (forward || !(flags & NEFCT_DETERMINISTIC)) && g.ny <= 65535 &&
            g.nx + 3 < 65536 && g.ny + 3 < 65536;
 }
 
@@ -349,32 +348,16 @@ static inline cudaError_t cb_launch(CBParams<T> &p, int na, int nb, int nvc, uin
 {
     dim3 grid, block;
     cb_shape(p, na, nb, nvc, grid, block);
-    const bool exact = (flags & NEFCT_EXACT) != 0, div = !cubic(p.g);
+    // (the float walk has no division path)
+    const bool exact = (flags & NEFCT_EXACT) != 0, div = sizeof(T) == 8 && !cubic(p.g);
     if constexpr (FWD) {
         if (exact) cb_forward_kernel<T, false, true><<<grid, block, 0, s>>>(p);
-        else if (div) cb_forward_kernel<T, true><<<grid, block, 0, s>>>(p);
+        else if (div) cb_forward_kernel<T, sizeof(T) == 8><<<grid, block, 0, s>>>(p);
         else cb_forward_kernel<T, false><<<grid, block, 0, s>>>(p);
     } else {
         if (exact) cb_backward_kernel<T, false, true><<<grid, block, 0, s>>>(p);
-        else if (div) cb_backward_kernel<T, true><<<grid, block, 0, s>>>(p);
+        else if (div) cb_backward_kernel<T, sizeof(T) == 8><<<grid, block, 0, s>>>(p);
         else cb_backward_kernel<T, false><<<grid, block, 0, s>>>(p);
-    }
-    return cudaGetLastError();
-}
-
-template <bool FWD>
-static inline cudaError_t cb_launch_colwarp(CBParams<float> &p, int na, int nb, int nvc, cudaStream_t s)
-{
-    dim3 grid, block;
-    constexpr int R = FWD ? NEFCT_COL_ROWS_FWD : NEFCT_COL_ROWS_BWD;
-    if constexpr (R > 1) {
-        cb_colwarp_shape(p, na, nb, nvc, grid, block, R);
-        if (cubic(p.g)) cb_colwarp_rows_kernel<false, FWD, R><<<grid, block, 0, s>>>(p);
-        else cb_colwarp_rows_kernel<true, FWD, R><<<grid, block, 0, s>>>(p);
-    } else {
-        cb_colwarp_shape(p, na, nb, nvc, grid, block);
-        if (cubic(p.g)) cb_colwarp_kernel<false, FWD><<<grid, block, 0, s>>>(p);
-        else cb_colwarp_kernel<true, FWD><<<grid, block, 0, s>>>(p);
     }
     return cudaGetLastError();
 }

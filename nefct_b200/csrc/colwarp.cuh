@@ -7,23 +7,35 @@
 // crossing ratio are bit-identical across the rows of a column; only the z
 // part (pw, kw, W) differs.
 //
-// One warp walks 32 consecutive rows of one column in lockstep over the
+// One warp walks 32 R rows of one column, R per lane, in lockstep over the
 // union of their slab ranges:
 //  * the v part of each slab is computed once per warp: lane j builds the
 //    entry of slab kc + j of a 32-slab chunk into the warp's table in shared
-//    memory, and every lane reads each slab's entry with one broadcast load;
-//    whether the slab crosses a v plane is the same for the whole warp, so
-//    the common case without a crossing takes a two-slot split without
-//    divergence;
-//  * each lane evaluates the z part and the three-voxel split of its own
-//    ray exactly as the single-ray walker does (same operations, same order);
+//    memory, and every lane reads each slab's entry with broadcast loads, once
+//    for its R rays; whether the slab crosses a v plane is the same for the
+//    whole warp;
 //  * the volume (forward) and the accumulator (transpose) are z-fastest
-//    copies [y][x][z]: the 32 rows of a warp sit at neighbouring z of the
-//    same (u, v) voxel column, so a warp's gather or reduction touches one or
-//    two 32-byte sectors instead of one per row band.
-// Slabs outside a ray's own range lie outside the grid for that ray and the
-// boundary checks reject them; the warp's check-free (interior) range is the
-// intersection of its rays' interior ranges.
+//    copies [y][x][z]: the rows of a warp sit at neighbouring z of the same
+//    (u, v) voxel column, and a ray's two z voxels are adjacent in memory.
+// A slab's v columns are in the grid or not for the whole warp, so the table
+// drops the ones that are not; the z voxels need range checks only in the
+// chunks of slabs where some ray of the warp can leave the grid in z (also
+// slabs before or after a ray's own range).
+//
+// The z split of a slab.  With q1, q2 the positions at the slab's lower and
+// upper plane (in z) and c = floor(q1) + 1, the share of the low voxel is
+// rw = min(1, (c - q1) / (q2 - q1)): 1 without a crossing, so no crossing test
+// is needed while |kz| (z voxels per slab) stays below 1; steeper rays take
+// the general split.
+//  * By default q1 = fma(kz, d, z0) and q2 - q1 = |kz| exactly: one fused
+//    multiply-add, a floor and one saturating multiply-add per ray and slab,
+//    with fewer roundings than the reference's (the error against FP64 is no
+//    larger), the same in the forward and its transpose.
+//  * REF (calls with NEFCT_TIE_GT, the switches of the reference's own
+//    backprojection): q1 and q2 with the reference's operations in its order.
+//    A nearly level ray (|kz| ~ 1e-3) divides rounding errors of ~1e-5 voxel
+//    by |kz|, and a voxel that few views reach shows them: there the result
+//    follows the reference's rounding.
 #pragma once
 
 #include <limits.h>
@@ -32,45 +44,51 @@
 
 namespace nefct {
 
-
-// v part of one slab: biased bases of the low/high v voxel columns (index of
-// (k, v, z) = b + floor bits of z), the clamped v floors for the boundary
-// checks, and the v crossing ratio.
-struct ColEntry {
-    unsigned b1, b2;    // k*su + c*sv - 0x4B400000 for the low/high v floor c
-    unsigned cv;        // (c1 + 2) | (c2 + 2) << 16, c clamped to [-2, nv + 1]
-    float rv;           // crossing ratio, 1 without a v crossing
-};
-
-// Warp's table of the slab entries of one 32-slab chunk: .x b1, .y b2,
-// .z rv (bits), .w the slab's exit plane offset t + 1 - pu (bits); the
-// packed v floors (cv) apart, read by boundary slabs only.
-struct ColTable {
-    uint4 e[32];
-    unsigned cv[32];
-};
-
-// Shared (warp-uniform) parameters of the column's walk.
-struct ColShared {
+// Transverse (v) part of a column's walk: the same for every row.
+struct ColWalk {
     float pu, pv, kv, dv, nv2, nu2;
     int nv;
     unsigned su, sv;
     bool vdiv;
 };
 
-// Entry of slab k: planes t = k - nu2 and t + 1, positions and floors as in
-// Walker::pos / Walker::next (same operations and order), so every value
-// equals the single-ray walker's.  Clamping a floor to [-2, nv + 1] keeps
-// every admission decision of the boundary checks.
-template <bool DIV> __device__ __forceinline__ ColEntry col_entry(const ColShared &c, int k)
+// v part of one slab: biased bases of the low/high v voxel columns (index of
+// (k, v, z) = b + sw * floor bits of z), the clamped v floors for the
+// boundary checks, and the v crossing ratio.
+struct ColEntry {
+    unsigned b1, b2;    // k*su + c*sv - sw*0x4B400000 for the low/high v floor c
+    unsigned cv;        // (c1 + 2) | (c2 + 2) << 16, c clamped to [-2, nv + 1]
+    float rv;           // crossing ratio, 1 without a v crossing
+};
+
+__device__ __forceinline__ ColWalk col_walk_of(const GridDev<float> &g, const Walk<float> &w, unsigned su, unsigned sv)
 {
-    const float ta = __fsub_rn((float)k, c.nu2), tb = __fadd_rn(ta, 1.f);
-    auto vpos = [&](float t) {
-        float q = __fadd_rn(c.pv, __fmul_rn(c.kv, __fsub_rn(t, c.pu)));
-        if (DIV && c.vdiv) q = __fdiv_rn(q, c.dv);
+    ColWalk c;
+    c.pu = w.pu; c.pv = w.pv; c.kv = w.kv;
+    c.dv = w.dv; c.vdiv = w.vdiv;
+    c.nv2 = w.nv2; c.nu2 = w.nu2; c.nv = w.nv;
+    c.su = su; c.sv = sv;
+    return c;
+}
+
+// Offset t - pu of plane k (t = k - nu2 is exact: nu2 is a multiple of 1/2
+// and |k| < 2^22).
+__device__ __forceinline__ float col_plane(const ColWalk &c, int k)
+{
+    return __fsub_rn(__fsub_rn((float)k, c.nu2), c.pu);
+}
+
+// Entry of slab k: planes t = k - nu2 and t + 1, positions and floors in the
+// reference's operations and order.  Clamping a floor to [-2, nv + 1] keeps
+// every admission decision of the boundary checks.  sw: z stride.
+__device__ __forceinline__ ColEntry col_entry(const ColWalk &c, int k, unsigned sw)
+{
+    auto vpos = [&](float d) {
+        float q = __fadd_rn(c.pv, __fmul_rn(c.kv, d));
+        if (c.vdiv) q = __fdiv_rn(q, c.dv);
         return __fadd_rn(q, c.nv2);
     };
-    const float qa = vpos(ta), qb = vpos(tb);
+    const float qa = vpos(col_plane(c, k)), qb = vpos(col_plane(c, k + 1));
     const float ma = magic_floor<true>(qa), mb = magic_floor<true>(qb);
     const float q1 = fminf(qa, qb), q2 = fmaxf(qa, qb);
     const float m1 = fminf(ma, mb), m2 = fmaxf(ma, mb);
@@ -78,365 +96,593 @@ template <bool DIV> __device__ __forceinline__ ColEntry col_entry(const ColShare
     e.rv = m1 != m2 ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1), __fadd_rn(q2, -q1)) : 1.f;
     const int c1 = min(max(__float_as_int(m1) - kFloorMagicBits, -2), c.nv + 1);
     const int c2 = min(max(__float_as_int(m2) - kFloorMagicBits, -2), c.nv + 1);
-    const unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits;
+    const unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * sw;
     e.b1 = base + (unsigned)c1 * c.sv;
     e.b2 = base + (unsigned)c2 * c.sv;
     e.cv = (unsigned)(c1 + 2) | ((unsigned)(c2 + 2) << 16);
     return e;
 }
 
-// Per-lane z state of the walk.
-struct ColLane {
-    float pw, kw, qaw, maw;
-    bool live, up;
+// z part of a ray, in voxel rows.
+struct ZRay {
+    float kz, z0, ikz;      // position kz * d + z0 at plane offset d; ikz = 1 / |kz| (at most 1e30)
+    float kw, pw;           // REF: position ((pw + kw * d) * rdz) + nz2
+    int down;               // kz < 0: the slab's lower z plane is its exit plane
+    bool live, steep;
 };
 
-// Contributions of one slab of a lane's ray: NS slots (voxel index, split
-// ratio, activity) in the reference's accumulation order.  In an interior
-// slab (CHK false) every slot's index is a voxel of the grid, also for an
-// inactive slot (whose ratio is 0: it repeats an active slot's voxel) and
-// for a lane without a ray (whose z plane stays at nz/2).
-template <int NS, bool CHK> struct ColSlots {
-    static constexpr int n = NS;
-    static constexpr bool checked = CHK;
-    unsigned idx[NS];
-    float r[NS];
-    bool ok[NS];
+// Rays from this slope on take the general split (below 1 by more than the
+// rounding of the positions).
+constexpr float kSteep = 0.999f;
+
+__device__ __forceinline__ ZRay z_ray(const Walk<float> &w, bool live)
+{
+    ZRay z;
+    z.live = live;
+    z.kz = live ? w.kz : 0.f;       // a lane without a ray walks row 0 (its indices stay in the grid)
+    z.z0 = live ? w.z0 : 0.5f;
+    z.kw = live ? w.kw : 0.f;
+    z.pw = live ? w.pw : 0.f;
+    z.ikz = fminf(__fdiv_rn(1.f, fabsf(z.kz)), 1e30f);
+    z.down = z.kz < 0.f;
+    z.steep = fabsf(z.kz) > kSteep;
+    return z;
+}
+
+// Grid constants of the z positions.
+struct ZGrid {
+    float rdz, nz2;         // 1 / dz, nz / 2
+    bool div;               // dz != 1
+    int nz;
+};
+__device__ __forceinline__ ZGrid z_grid(const GridDev<float> &g)
+{
+    return ZGrid{__fdiv_rn(1.f, g.dz), g.nz2, g.dz != 1.f, g.nz};
+}
+
+// Position at plane offset d in the reference's order of operations (its
+// division by dz as a multiplication by 1 / dz).
+__device__ __forceinline__ float z_pos(const ZRay &z, const ZGrid &zg, float d)
+{
+    float q = __fadd_rn(z.pw, __fmul_rn(z.kw, d));
+    if (zg.div) q = __fmul_rn(q, zg.rdz);
+    return __fadd_rn(q, zg.nz2);
+}
+
+// The z split of one slab: biased floors of its low and high voxel and the
+// share rw of the low one.  d, dh: offsets of the lower and upper plane.
+struct ZSplit {
+    unsigned i1, i2;
+    float rw;
 };
 
-// One slab of the lane's ray.  WUP: 1 every live ray has kw >= 0, 0 every
-// live ray has kw < 0, 2 mixed (per-lane choice).  The v crossing is shared
-// by the warp (b1 != b2): without one (VX false) the split has two slots,
-// (v1, w1) with ratio rw and (v1, w2) with 1 - rw, which is the general
-// three-slot split with rv = 1 (its third ratio, 1 - max(rv, rw), is 0 and
-// its slot inactive); with one, the general split.  SPLIT 0 takes the
-// general split for every slab (no branch: the forward's loads of
-// consecutive slabs interleave better); 1 the two-slot split; 2 the same
-// with the second slot always at w2 (it differs from the reference's pairing
-// only when the ratio rounds to 1 or above, where that slot's weight is a
-// rounding error; for the float transpose, whose atomic sums are not
-// reproducible anyway).  f(slots) consumes.  The slab's table entry (b1,
-// b2, exit plane offset d, v ratio rv, packed v floors cv) comes from the
-// caller; TWO: the two-slot split (the caller's SPLIT and no v crossing).
-template <bool DIV, bool CHECK, int WUP, int SPLIT, bool TWO, class Fn>
-__device__ __forceinline__ void col_lane_slab(ColLane &L, float dz, bool zdiv, float nz2, int nv, int nz,
-                                              unsigned b1, unsigned b2, float d, float rv, unsigned cv, Fn &f)
+template <bool REF>
+__device__ __forceinline__ ZSplit z_split(const ZRay &z, const ZGrid &zg, float d, float dh)
 {
-    float qbw = __fadd_rn(L.pw, __fmul_rn(L.kw, d));
-    if (DIV && zdiv) qbw = __fdiv_rn(qbw, dz);
-    qbw = __fadd_rn(qbw, nz2);
-    const float mbw = magic_floor<CHECK>(qbw);
-    const bool up = WUP == 2 ? L.up : WUP == 1;
-    const float q1w = up ? L.qaw : qbw, q2w = up ? qbw : L.qaw;
-    const float m1w = up ? L.maw : mbw, m2w = up ? mbw : L.maw;
-    L.qaw = qbw;
-    L.maw = mbw;
-    const bool wx = m1w != m2w;
-    const float rw = wx ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2w, -kFloorMagic), -q1w), __fadd_rn(q2w, -q1w)) : 1.f;
-    const unsigned i1 = (unsigned)__float_as_int(m1w), i2 = (unsigned)__float_as_int(m2w);
-    const int cv1 = CHECK ? (int)(cv & 0xffffu) - 2 : 0, cv2 = CHECK ? (int)(cv >> 16) - 2 : 0;
-    const int cw1 = (int)i1 - kFloorMagicBits, cw2 = (int)i2 - kFloorMagicBits;
-    if constexpr (TWO) {
-        // no v crossing (uniform across the warp)
-        const bool vfirst = 1.f > rw;
-        ColSlots<2, CHECK> s;
-        s.r[0] = rw;                            // min(1, rw)
-        s.r[1] = __fsub_rn(1.f, rw);            // |1 - rw|
-        s.idx[0] = b1 + i1;
-        s.idx[1] = b1 + ((SPLIT == 2 || vfirst) ? i2 : i1);
-        if (CHECK) {
-            const bool adm = L.live && (unsigned)cv1 < (unsigned)nv && (unsigned)(cw1 + (int)wx) < (unsigned)(nz + (int)wx);
-            const int mw = (SPLIT == 2 || vfirst) ? cw2 : cw1;     // the slot's own voxel
-            s.ok[0] = adm && cw1 >= 0;
-            s.ok[1] = adm && wx && (unsigned)mw < (unsigned)nz;
-        } else {
-            s.ok[0] = L.live;
-            s.ok[1] = L.live && wx;
-        }
-        f(s);
+    ZSplit s;
+    float q = REF ? z_pos(z, zg, d) : __fmaf_rn(z.kz, d, z.z0);
+    const float m = magic_floor<true>(q);
+    q = fminf(fmaxf(q, -kFloorClamp), kFloorClamp);
+    s.i1 = (unsigned)__float_as_int(m);
+    s.i2 = s.i1 + 1u;
+    if (REF || z.steep) {
+        float qh = REF ? z_pos(z, zg, dh) : __fmaf_rn(z.kz, dh, z.z0);
+        const float mh = magic_floor<true>(qh);
+        qh = fminf(fmaxf(qh, -kFloorClamp), kFloorClamp);
+        const float den = REF ? rcp_approx(__fadd_rn(qh, -q)) : z.ikz;
+        s.rw = mh != m ? __fmul_rn(__fadd_rn(__fadd_rn(mh, -kFloorMagic), -q), den) : 1.f;
+        if (REF || mh != m) s.i2 = (unsigned)__float_as_int(mh);
     } else {
-        const bool vx = SPLIT || b1 != b2;
-        const bool vfirst = rv > rw;
-        ColSlots<3, CHECK> s;
-        s.r[0] = fminf(rv, rw);
-        s.r[1] = fabsf(__fsub_rn(rv, rw));
-        s.r[2] = __fsub_rn(1.f, fmaxf(rv, rw));
-        s.idx[0] = b1 + i1;
-        s.idx[1] = vfirst ? b1 + i2 : b2 + i1;
-        s.idx[2] = b2 + i2;
-        if (CHECK) {
-            // slab admission (reference siddon.cu.cc :80, :92, :112, :116, :132)
-            const bool adm = L.live && (unsigned)(cv1 + (int)vx) < (unsigned)(nv + (int)vx) &&
-                             (unsigned)(cw1 + (int)wx) < (unsigned)(nz + (int)wx);
-            const int mv = vfirst ? cv1 : cv2, mw = vfirst ? cw2 : cw1;
-            s.ok[0] = adm && (cv1 | cw1) >= 0;
-            s.ok[1] = adm && (vx || wx) && (unsigned)mv < (unsigned)nv && (unsigned)mw < (unsigned)nz;
-            s.ok[2] = adm && vx && wx && cv2 < nv && cw2 < nz;
-        } else {
-            s.ok[0] = L.live;
-            s.ok[1] = L.live && (vx || wx);
-            s.ok[2] = L.live && vx && wx;
-        }
-        f(s);
+        s.rw = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
     }
+    return s;
 }
 
-// One slab of the lane's one ray, its entry read from the warp's table.
-template <bool DIV, bool CHECK, int WUP, int SPLIT, class Fn>
-__device__ __forceinline__ void col_slab(ColLane &L, float dz, bool zdiv, float nz2, int nv, int nz,
-                                         const ColTable &tab, int j, Fn &f)
+// Shares of a slab with a v crossing: the overlap of the ray's v intervals
+// [0, rv], [rv, 1] and z intervals [0, rw], [rw, 1] (the reference's pairing,
+// Q1): (v1, w1), (v1, w2), (v2, w1), (v2, w2); one of the middle two is 0.
+struct Shares {
+    float w11, w12, w21, w22;
+};
+__device__ __forceinline__ Shares slab_shares(float rv, float rw)
 {
-    const uint4 te = tab.e[j];          // same address for every lane: one broadcast
-    const unsigned cv = CHECK ? tab.cv[j] : 0u;
-    if (SPLIT && te.x == te.y)
-        col_lane_slab<DIV, CHECK, WUP, SPLIT, true>(L, dz, zdiv, nz2, nv, nz, te.x, te.y, __uint_as_float(te.w),
-                                                    __uint_as_float(te.z), cv, f);
-    else
-        col_lane_slab<DIV, CHECK, WUP, SPLIT, false>(L, dz, zdiv, nz2, nv, nz, te.x, te.y, __uint_as_float(te.w),
-                                                     __uint_as_float(te.z), cv, f);
+    Shares s;
+    s.w11 = fminf(rv, rw);
+    s.w12 = __fsub_rn(rv, s.w11);
+    s.w21 = __fsub_rn(rw, s.w11);
+    s.w22 = __fsub_rn(__fsub_rn(1.f, rv), s.w21);
+    return s;
 }
 
-// The same slab for the R rays of a lane (rows l, l + 32, ... of the
-// column): one table read and one split decision for all of them;
-// f(slots, r) consumes ray r's slots.
-template <bool DIV, bool CHECK, int WUP, int SPLIT, int R, class Fn>
-__device__ __forceinline__ void col_slab_rows(ColLane (&L)[R], float dz, bool zdiv, float nz2, int nv, int nz,
-                                              const ColTable &tab, int j, Fn &f)
+// Which of a slab's v columns are in the grid (bits v1, v2), with the
+// reference's slab admission (siddon.cu.cc:80, :92, :112, :116, :132).
+__device__ __forceinline__ unsigned v_columns(bool vx, unsigned cv, int nv)
 {
-    const uint4 te = tab.e[j];
-    const unsigned cv = CHECK ? tab.cv[j] : 0u;
-    const float d = __uint_as_float(te.w), rv = __uint_as_float(te.z);
-    if (SPLIT && te.x == te.y) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            auto fr = [&](const auto &s) { f(s, r); };
-            col_lane_slab<DIV, CHECK, WUP, SPLIT, true>(L[r], dz, zdiv, nz2, nv, nz, te.x, te.y, d, rv, cv, fr);
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            auto fr = [&](const auto &s) { f(s, r); };
-            col_lane_slab<DIV, CHECK, WUP, SPLIT, false>(L[r], dz, zdiv, nz2, nv, nz, te.x, te.y, d, rv, cv, fr);
-        }
+    const int cv1 = (int)(cv & 0xffffu) - 2, cv2 = (int)(cv >> 16) - 2;
+    const bool adm = (unsigned)(cv1 + (int)vx) < (unsigned)(nv + (int)vx);
+    return (unsigned)(adm && cv1 >= 0) | (unsigned)(adm && cv2 < nv) << 1;
+}
+
+// Which of a slab's voxels are in the grid: bits v1w1, v1w2, v2w1, v2w2.
+__device__ __forceinline__ unsigned slab_inside(const ZRay &z, const ZSplit &s, bool vx, unsigned cv, int nv, int nz)
+{
+    const int cw1 = (int)s.i1 - kFloorMagicBits, cw2 = (int)s.i2 - kFloorMagicBits;
+    bool adm = z.live;
+    if (z.steep) {
+        const bool wx = s.i1 != s.i2;
+        adm = adm && (unsigned)(cw1 + (int)wx) < (unsigned)(nz + (int)wx);
     }
+    const unsigned w = (unsigned)(adm && (unsigned)cw1 < (unsigned)nz) | (unsigned)(adm && (unsigned)cw2 < (unsigned)nz) << 1;
+    const unsigned v = v_columns(vx, cv, nv);
+    return (v & 1u ? w : 0u) | (v & 2u ? w << 2 : 0u);
 }
 
-// Walks slabs [a, b] (inside the current 32-slab chunk starting at kc) in
-// one check mode.
-template <bool DIV, bool CHECK, int WUP, int SPLIT, class Fn>
-__device__ __forceinline__ void col_range(int a, int b, int kc, const ColShared &c, ColLane &L,
-                                          const ColTable &tab, const GridDev<float> &g, Fn &f)
-{
-    const bool zdiv = g.dz != 1.f;
-#pragma unroll 4
-    for (int k = a; k <= b; ++k)
-        col_slab<DIV, CHECK, WUP, SPLIT>(L, g.dz, zdiv, g.nz2, c.nv, g.nz, tab, k - kc, f);
-}
-
-// Slabs [K0, K1] of the warp in 32-slab chunks (lane j builds the entry of
-// slab kc + j into the warp's table); boundary slabs outside [KI0, KI1] with
-// range checks.  The slab planes k - nu2 and k + 1 - nu2 are exact (nu2 is a
-// multiple of 1/2 and |k| < 2^22), so the table's exit plane offset equals
-// the one a walk carrying t += 1 evaluates.
-template <bool DIV, int WUP, int SPLIT, class Fn>
-__device__ __forceinline__ void col_walk(const ColShared &c, ColLane &L, int K0, int K1, int KI0, int KI1,
-                                         const GridDev<float> &g, ColTable &tab, Fn &f)
-{
-    // plane K0 - nu2 (entry plane of the first slab)
-    const float t = __fsub_rn((float)K0, c.nu2);
-    float q = __fadd_rn(L.pw, __fmul_rn(L.kw, __fsub_rn(t, c.pu)));
-    if (DIV && g.dz != 1.f) q = __fdiv_rn(q, g.dz);
-    L.qaw = __fadd_rn(q, g.nz2);
-    L.maw = magic_floor<true>(L.qaw);
-    const int lane = threadIdx.x & 31;
-    if (KI0 > KI1) { KI0 = K1 + 1; KI1 = K1; }      // no interior: everything checked
-    for (int kc = K0; kc <= K1; kc += 32) {
-        const ColEntry e = col_entry<DIV>(c, kc + lane);
-        const float d = __fsub_rn(__fadd_rn(__fsub_rn((float)(kc + lane), c.nu2), 1.f), c.pu);
-        __syncwarp();                   // the previous chunk's reads are done
-        tab.e[lane] = make_uint4(e.b1, e.b2, __float_as_uint(e.rv), __float_as_uint(d));
-        tab.cv[lane] = e.cv;
-        __syncwarp();
-        const int ke = min(K1, kc + 31);
-        col_range<DIV, true, WUP, SPLIT>(kc, min(ke, KI0 - 1), kc, c, L, tab, g, f);
-        col_range<DIV, false, WUP, SPLIT>(max(kc, KI0), min(ke, KI1), kc, c, L, tab, g, f);
-        col_range<DIV, true, WUP, SPLIT>(max(kc, KI1 + 1), ke, kc, c, L, tab, g, f);
-    }
-}
-
-template <bool DIV, int SPLIT, class Fn>
-__device__ __forceinline__ void col_walk_any(const ColShared &c, ColLane &L, int K0, int K1, int KI0, int KI1,
-                                             const GridDev<float> &g, Fn &f)
-{
-    // one table per warp; column-warp blocks are 32 x (at most 8) threads
-    __shared__ ColTable tables[8];
-    ColTable &tab = tables[threadIdx.y];
-    const bool all_up = __all_sync(0xffffffffu, L.up || !L.live);
-    const bool all_down = __all_sync(0xffffffffu, !L.up || !L.live);
-    if (all_up) col_walk<DIV, 1, SPLIT>(c, L, K0, K1, KI0, KI1, g, tab, f);
-    else if (all_down) col_walk<DIV, 0, SPLIT>(c, L, K0, K1, KI0, KI1, g, tab, f);
-    else col_walk<DIV, 2, SPLIT>(c, L, K0, K1, KI0, KI1, g, tab, f);
-}
-
-// Strides of the z-fastest layout [y][x][z] along (u, v) of the drive axis.
-__device__ __forceinline__ void col_strides(const GridDev<float> &g, bool xdrive, unsigned &su, unsigned &sv)
-{
-    const unsigned xs = (unsigned)g.nz, ys = (unsigned)g.nx * (unsigned)g.nz;
-    su = xdrive ? xs : ys;
-    sv = xdrive ? ys : xs;
-}
-
-// Sets up the warp: shared parameters from the first live lane, the warp's
-// slab and interior ranges.  Returns false when the rays do not share their
-// v parameters bit for bit (each lane then walks alone).
-__device__ __forceinline__ bool col_setup(const GridDev<float> &g, const Walk<float> &w, bool live, ColShared &c,
-                                          ColLane &L, int &K0, int &K1, int &KI0, int &KI1)
-{
-    const unsigned lm = __ballot_sync(0xffffffffu, live);
-    const int src = __ffs(lm) - 1;
-    c.pu = __shfl_sync(0xffffffffu, w.pu, src);
-    c.pv = __shfl_sync(0xffffffffu, w.pv, src);
-    c.kv = __shfl_sync(0xffffffffu, w.kv, src);
-    const bool xdrive = __shfl_sync(0xffffffffu, (int)w.xdrive, src) != 0;
-    const bool same = !live || (__float_as_int(w.pu) == __float_as_int(c.pu) &&
-                                __float_as_int(w.pv) == __float_as_int(c.pv) &&
-                                __float_as_int(w.kv) == __float_as_int(c.kv) && w.xdrive == xdrive);
-    if (!__all_sync(0xffffffffu, same)) return false;
-    c.dv = xdrive ? g.dy : 1.f;
-    c.vdiv = xdrive && g.dy != 1.f;
-    c.nv2 = xdrive ? g.ny2 : g.nx2;
-    c.nu2 = xdrive ? g.nx2 : g.ny2;
-    c.nv = xdrive ? g.ny : g.nx;
-    col_strides(g, xdrive, c.su, c.sv);
-    K0 = __reduce_min_sync(0xffffffffu, live ? w.k0 : INT_MAX);
-    K1 = __reduce_max_sync(0xffffffffu, live ? w.k1 : INT_MIN);
-    KI0 = __reduce_max_sync(0xffffffffu, live ? w.ki0 : INT_MIN);
-    KI1 = __reduce_min_sync(0xffffffffu, live ? w.ki1 : INT_MAX);
-    // a lane without a ray walks the plane z = nz/2 (indices stay in the grid)
-    L.pw = live ? w.pw : 0.f;
-    L.kw = live ? w.kw : 0.f;
-    L.live = live;
-    L.up = w.kw >= 0.f;
-    return true;
-}
-
-// ---- R rays per lane: rows l, l + 32, ..., l + 32 (R - 1) of the column ----
+// ---- sinks: what one ray does with a slab's voxels ----
 //
-// The warp's table serves 32 R rays: each slab's entry is read and its split
-// decided once per lane for all of them.  Each ray's own arithmetic is the
-// one-ray walk's.
+// f.pair(kind, b, s, ok, wl, wh): voxels (v, w1) with share wl and (v, w2)
+// with share wh of the voxel column at b; ok: bit 0 and 1, whether they are in
+// the grid.
 
-template <bool DIV, bool CHECK, int WUP, int SPLIT, int R, class Fn>
-__device__ __forceinline__ void col_range_rows(int a, int b, int kc, const ColShared &c, ColLane (&L)[R],
-                                               const ColTable &tab, const GridDev<float> &g, Fn &f)
+// Slabs without a v crossing; with one and both columns in the grid; with one
+// and a single column in the grid.
+enum SlabKind { kPlain, kCross, kHalf };
+
+// Forward: sums of value * share, by kind of slab and by aligned block of 32
+// slabs (close() ends a block), so that the total does not depend on which
+// rays walk together; sums of partial sums also round less than one running
+// sum.  SKIP0: voxels of share 0 are not read.
+template <bool SKIP0 = false> struct GatherSink {
+    const float *__restrict__ vol;
+    unsigned sw;
+    float sum[3], whole;
+
+    __device__ __forceinline__ GatherSink() {}
+    __device__ __forceinline__ GatherSink(const float *v, unsigned sw_) : vol(v), sw(sw_), sum{0.f, 0.f, 0.f}, whole(0.f) {}
+    __device__ __forceinline__ void pair(SlabKind kind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh)
+    {
+        const float lo = (ok & 1u) && (!SKIP0 || wl != 0.f) ? __ldg(vol + (b + s.i1 * sw)) : 0.f;
+        const float hi = (ok & 2u) && (!SKIP0 || wh != 0.f) ? __ldg(vol + (b + s.i2 * sw)) : 0.f;
+        const float acc = kind == kPlain ? sum[0] : kind == kCross ? sum[1] : sum[2];
+        const float v = __fmaf_rn(hi, wh, __fmaf_rn(lo, wl, acc));
+        if (kind == kPlain) sum[0] = v;
+        else if (kind == kCross) sum[1] = v;
+        else sum[2] = v;
+    }
+    __device__ __forceinline__ void close()
+    {
+        whole = __fadd_rn(whole, __fadd_rn(__fadd_rn(sum[0], sum[1]), sum[2]));
+        sum[0] = sum[1] = sum[2] = 0.f;
+    }
+};
+
+// Transpose: one reduction of yw * share per voxel with a share.
+struct ScatterSink {
+    float *acc;
+    unsigned sw;
+    float yw;
+
+    __device__ __forceinline__ void pair(SlabKind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh) const
+    {
+        if ((ok & 1u) && wl != 0.f) atomicAdd(acc + (b + s.i1 * sw), yw * wl);
+        if ((ok & 2u) && wh != 0.f) atomicAdd(acc + (b + s.i2 * sw), yw * wh);
+    }
+    __device__ __forceinline__ void close() const {}
+};
+
+// Deterministic transpose: each contribution yw * share, scaled by a power of
+// two (exact) and rounded to a 64-bit integer (siddon.cuh, to_fixed).
+struct FixedSink {
+    unsigned long long *acc;
+    unsigned sw;
+    float yw, scale;
+
+    __device__ __forceinline__ void pair(SlabKind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh) const
+    {
+        if ((ok & 1u) && wl != 0.f) atomicAdd(acc + (b + s.i1 * sw), (unsigned long long)to_fixed((yw * wl) * scale));
+        if ((ok & 2u) && wh != 0.f) atomicAdd(acc + (b + s.i2 * sw), (unsigned long long)to_fixed((yw * wh) * scale));
+    }
+    __device__ __forceinline__ void close() const {}
+};
+
+// One slab of one ray, range checked (also right for interior slabs).
+template <bool REF, class Sink>
+__device__ __forceinline__ void ray_slab(const ZRay &z, const ZGrid &zg, float d, float dh, unsigned b1, unsigned b2,
+                                         float rv, unsigned cv, int nv, Sink &f)
 {
-    const bool zdiv = g.dz != 1.f;
-#pragma unroll 2
-    for (int k = a; k <= b; ++k)
-        col_slab_rows<DIV, CHECK, WUP, SPLIT, R>(L, g.dz, zdiv, g.nz2, c.nv, g.nz, tab, k - kc, f);
+    const ZSplit s = z_split<REF>(z, zg, d, dh);
+    const bool four = b1 != b2;
+    const unsigned ok = slab_inside(z, s, four, cv, nv, zg.nz);
+    if (!four) {
+        f.pair(kPlain, b1, s, ok, s.rw, __fsub_rn(1.f, s.rw));
+    } else {
+        const Shares h = slab_shares(rv, s.rw);
+        const SlabKind kind = v_columns(true, cv, nv) == 3u ? kCross : kHalf;
+        if (ok & 3u) f.pair(kind, b1, s, ok, h.w11, h.w12);
+        if (ok & 12u) f.pair(kind, b2, s, ok >> 2, h.w21, h.w22);
+    }
 }
 
-template <bool DIV, int WUP, int SPLIT, int R, class Fn>
-__device__ __forceinline__ void col_walk_rows(const ColShared &c, ColLane (&L)[R], int K0, int K1, int KI0, int KI1,
-                                              const GridDev<float> &g, ColTable &tab, Fn &f)
+// One ray alone (any strides): every slab's v part evaluated by the thread,
+// with a column warp's operations per slab, so with its bits.
+template <bool REF, class Sink>
+__device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<float> &w, unsigned su, unsigned sv,
+                                         unsigned sw, Sink &f)
 {
-    const float t = __fsub_rn((float)K0, c.nu2);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        float q = __fadd_rn(L[r].pw, __fmul_rn(L[r].kw, __fsub_rn(t, c.pu)));
-        if (DIV && g.dz != 1.f) q = __fdiv_rn(q, g.dz);
-        L[r].qaw = __fadd_rn(q, g.nz2);
-        L[r].maw = magic_floor<true>(L[r].qaw);
-    }
-    const int lane = threadIdx.x & 31;
-    if (KI0 > KI1) { KI0 = K1 + 1; KI1 = K1; }
-    for (int kc = K0; kc <= K1; kc += 32) {
-        const ColEntry e = col_entry<DIV>(c, kc + lane);
-        const float d = __fsub_rn(__fadd_rn(__fsub_rn((float)(kc + lane), c.nu2), 1.f), c.pu);
-        __syncwarp();
-        tab.e[lane] = make_uint4(e.b1, e.b2, __float_as_uint(e.rv), __float_as_uint(d));
-        tab.cv[lane] = e.cv;
-        __syncwarp();
-        const int ke = min(K1, kc + 31);
-        col_range_rows<DIV, true, WUP, SPLIT, R>(kc, min(ke, KI0 - 1), kc, c, L, tab, g, f);
-        col_range_rows<DIV, false, WUP, SPLIT, R>(max(kc, KI0), min(ke, KI1), kc, c, L, tab, g, f);
-        col_range_rows<DIV, true, WUP, SPLIT, R>(max(kc, KI1 + 1), ke, kc, c, L, tab, g, f);
+    const ColWalk c = col_walk_of(g, w, su, sv);
+    const ZRay z = z_ray(w, true);
+    const ZGrid zg = z_grid(g);
+    for (int k = w.k0; k <= w.k1; ++k) {
+        const ColEntry e = col_entry(c, k, sw);
+        const float a = col_plane(c, k), b = col_plane(c, k + 1);
+        ray_slab<REF>(z, zg, z.down ? b : a, z.down ? a : b, e.b1, e.b2, e.rv, e.cv, c.nv, f);
+        if ((k & 31) == 31 || k == w.k1) f.close();
     }
 }
 
-template <bool DIV, int SPLIT, int R, class Fn>
-__device__ __forceinline__ void col_walk_any_rows(const ColShared &c, ColLane (&L)[R], int K0, int K1, int KI0,
-                                                  int KI1, const GridDev<float> &g, Fn &f)
-{
-    __shared__ ColTable tables[8];
-    ColTable &tab = tables[threadIdx.y];
-    bool up = true, down = true;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        up = up && (L[r].up || !L[r].live);
-        down = down && (!L[r].up || !L[r].live);
-    }
-    const bool all_up = __all_sync(0xffffffffu, up), all_down = __all_sync(0xffffffffu, down);
-    if (all_up) col_walk_rows<DIV, 1, SPLIT, R>(c, L, K0, K1, KI0, KI1, g, tab, f);
-    else if (all_down) col_walk_rows<DIV, 0, SPLIT, R>(c, L, K0, K1, KI0, KI1, g, tab, f);
-    else col_walk_rows<DIV, 2, SPLIT, R>(c, L, K0, K1, KI0, KI1, g, tab, f);
-}
+// ---- column warps ----
 
-// col_setup for R rays per lane (all in one detector column).
+// A column's walk for one warp: the shared v part, the R rays of the lane and
+// the warp's slab ranges.
+template <int R> struct ColRays {
+    ColWalk c;
+    ZGrid zg;
+    ZRay z[R];
+    float W[R];
+    int K0, K1;                     // slabs that some ray of the warp can touch
+    int ZI0, ZI1;                   // slabs where no ray of the warp needs a z range check
+    bool rising, falling, steep;    // the warp has rays of this kind
+};
+
+// Rays r (the whole warp calls it; has: the lane has the ray and it takes
+// part); false when no ray of the warp contributes.
 template <int R>
-__device__ __forceinline__ bool col_setup_rows(const GridDev<float> &g, const Walk<float> (&w)[R],
-                                               const bool (&live)[R], ColShared &c, ColLane (&L)[R], int &K0,
-                                               int &K1, int &KI0, int &KI1)
+__device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&r)[R][6], const bool (&has)[R],
+                                         uint32_t flags, ColRays<R> &q)
 {
-    bool any = false;
-    int first = 0;
+    int k0 = INT_MAX, k1 = INT_MIN, zi0 = INT_MIN, zi1 = INT_MAX;
+    bool any = false, up = false, down = false, steep = false;
+    q.zg = z_grid(g);
 #pragma unroll
-    for (int r = R - 1; r >= 0; --r)
-        if (live[r]) { any = true; first = r; }
-    float pu = w[0].pu, pv = w[0].pv, kv = w[0].kv;
-    bool xd = w[0].xdrive;
-#pragma unroll
-    for (int r = 1; r < R; ++r)
-        if (first == r) { pu = w[r].pu; pv = w[r].pv; kv = w[r].kv; xd = w[r].xdrive; }
-    const unsigned lm = __ballot_sync(0xffffffffu, any);
-    const int src = __ffs(lm) - 1;
-    c.pu = __shfl_sync(0xffffffffu, pu, src);
-    c.pv = __shfl_sync(0xffffffffu, pv, src);
-    c.kv = __shfl_sync(0xffffffffu, kv, src);
-    const bool xdrive = __shfl_sync(0xffffffffu, (int)xd, src) != 0;
-    bool same = true;
-    int k0 = INT_MAX, k1 = INT_MIN, ki0 = INT_MIN, ki1 = INT_MAX;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        same = same && (!live[r] || (__float_as_int(w[r].pu) == __float_as_int(c.pu) &&
-                                     __float_as_int(w[r].pv) == __float_as_int(c.pv) &&
-                                     __float_as_int(w[r].kv) == __float_as_int(c.kv) && w[r].xdrive == xdrive));
-        if (live[r]) {
-            k0 = min(k0, w[r].k0);
-            k1 = max(k1, w[r].k1);
-            ki0 = max(ki0, w[r].ki0);
-            ki1 = min(ki1, w[r].ki1);
+    for (int i = 0; i < R; ++i) {
+        Walk<float> w;
+        const bool live = setup_walk(g, r[i], flags, w) && has[i];
+        if (i == 0) {
+            // x and y do not depend on the row: every lane has the same v part
+            const unsigned xs = (unsigned)g.nz, ys = (unsigned)g.nx * (unsigned)g.nz;
+            q.c = col_walk_of(g, w, w.xdrive ? xs : ys, w.xdrive ? ys : xs);
+        }
+        q.z[i] = z_ray(w, live);
+        q.W[i] = w.W;
+        if (live) {
+            any = true;
+            k0 = min(k0, w.k0);
+            k1 = max(k1, w.k1);
+            zi0 = max(zi0, w.zi0);
+            zi1 = min(zi1, w.zi1);
+            up = up || !q.z[i].down;
+            down = down || q.z[i].down;
+            steep = steep || q.z[i].steep;
         }
     }
-    if (!__all_sync(0xffffffffu, same)) return false;
-    c.dv = xdrive ? g.dy : 1.f;
-    c.vdiv = xdrive && g.dy != 1.f;
-    c.nv2 = xdrive ? g.ny2 : g.nx2;
-    c.nu2 = xdrive ? g.nx2 : g.ny2;
-    c.nv = xdrive ? g.ny : g.nx;
-    col_strides(g, xdrive, c.su, c.sv);
-    K0 = __reduce_min_sync(0xffffffffu, k0);
-    K1 = __reduce_max_sync(0xffffffffu, k1);
-    KI0 = __reduce_max_sync(0xffffffffu, ki0);
-    KI1 = __reduce_min_sync(0xffffffffu, ki1);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        L[r].pw = live[r] ? w[r].pw : 0.f;
-        L[r].kw = live[r] ? w[r].kw : 0.f;
-        L[r].live = live[r];
-        L[r].up = w[r].kw >= 0.f;
-    }
+    if (!__any_sync(0xffffffffu, any)) return false;
+    q.K0 = __reduce_min_sync(0xffffffffu, k0);
+    q.K1 = __reduce_max_sync(0xffffffffu, k1);
+    q.ZI0 = __reduce_max_sync(0xffffffffu, zi0);
+    q.ZI1 = __reduce_min_sync(0xffffffffu, zi1);
+    q.rising = __any_sync(0xffffffffu, up);
+    q.falling = __any_sync(0xffffffffu, down);
+    q.steep = __any_sync(0xffffffffu, steep);
     return true;
+}
+
+// Warp's table of one 32-slab chunk, its slabs grouped by kind (slabs without
+// a v column in the grid are dropped): rows [0, cross) plain, [cross, half)
+// cross, [half, n) half.  a = (address of the low v column -- of the one
+// column in the grid for a half slab -- less 4 bytes per floor bias, offsets
+// of the lower and the upper z plane), c = (address of the high v column, or
+// 1 in c.x when a half slab's column is the high one; rv; 1 - rv).  d: the
+// offsets of the slab's entry and exit planes.
+struct ColTable {
+    uint4 a[32], c[32];
+    float2 d[32];
+};
+
+struct ColChunk {
+    int cross, half, n;
+};
+
+// Column warps are blocks of 32 x (at most 8) threads: one table per warp.
+__device__ __forceinline__ ColTable &col_table()
+{
+    __shared__ ColTable tables[8];
+    return tables[threadIdx.y];
+}
+
+// Lane j evaluates slab kc + j, if it is one of K0..K1.
+__device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0, int K1, bool falling, const float *vol,
+                                              ColTable &tab)
+{
+    const int lane = threadIdx.x & 31, k = kc + lane;
+    const ColEntry e = col_entry(cw, k, 1u);
+    const float da = col_plane(cw, k), db = col_plane(cw, k + 1);
+    const bool vx = e.b1 != e.b2;
+    const unsigned in = k >= K0 && k <= K1 ? v_columns(vx, e.cv, cw.nv) : 0u;
+    const bool is_plain = !vx && in != 0u, is_cross = vx && in == 3u, is_half = vx && (in == 1u || in == 2u);
+    const unsigned plain = __ballot_sync(0xffffffffu, is_plain), cross = __ballot_sync(0xffffffffu, is_cross);
+    const unsigned half = __ballot_sync(0xffffffffu, is_half), below = (1u << lane) - 1u;
+    ColChunk h;
+    h.cross = __popc(plain);
+    h.half = h.cross + __popc(cross);
+    h.n = h.half + __popc(half);
+    const int row = is_plain ? __popc(plain & below) : is_cross ? h.cross + __popc(cross & below)
+                                                                 : h.half + __popc(half & below);
+    __syncwarp();                       // the previous chunk's reads are done
+    if (is_plain || is_cross || is_half) {
+        const char *const base = reinterpret_cast<const char *>(vol) - 4ull * (unsigned)kFloorMagicBits;
+        const unsigned i1 = is_half && in == 2u ? e.b2 : e.b1;
+        const unsigned long long p1 = (unsigned long long)(base + 4ull * (i1 + (unsigned)kFloorMagicBits));
+        const unsigned long long p2 = (unsigned long long)(base + 4ull * (e.b2 + (unsigned)kFloorMagicBits));
+        tab.a[row] = make_uint4((unsigned)p1, (unsigned)(p1 >> 32), __float_as_uint(falling ? db : da),
+                                __float_as_uint(falling ? da : db));
+        tab.c[row] = make_uint4(is_half ? in - 1u : (unsigned)p2, (unsigned)(p2 >> 32), __float_as_uint(e.rv),
+                                __float_as_uint(__fsub_rn(1.f, e.rv)));
+        tab.d[row] = make_float2(da, db);
+    }
+    __syncwarp();
+    return h;
+}
+
+// Every slab of one ray per lane, range checked: warps that the walks below
+// do not take (steep rays), and the deterministic transpose.
+template <bool REF, class Sink>
+__device__ __forceinline__ void col_each(const ColWalk &cw, int K0, int K1, const ZRay &z, const ZGrid &zg, Sink &f)
+{
+    ColTable &tab = col_table();
+    const int lane = threadIdx.x & 31;
+    for (int kc = K0 & ~31; kc <= K1; kc += 32) {
+        const ColEntry e = col_entry(cw, kc + lane, 1u);
+        __syncwarp();
+        tab.a[lane] = make_uint4(e.b1, e.b2, __float_as_uint(e.rv), e.cv);
+        tab.d[lane] = make_float2(col_plane(cw, kc + lane), col_plane(cw, kc + lane + 1));
+        __syncwarp();
+        const int n = min(K1 - kc + 1, 32);
+#pragma unroll 1
+        for (int j = max(K0 - kc, 0); j < n; ++j) {
+            const uint4 te = tab.a[j];
+            const float2 d = tab.d[j];
+            ray_slab<REF>(z, zg, z.down ? d.y : d.x, z.down ? d.x : d.y, te.x, te.y, __uint_as_float(te.z), te.w, cw.nv,
+                          f);
+        }
+        f.close();
+    }
+}
+
+// Voxel of biased floor m in the column at the table's address (lo, hi).
+__device__ __forceinline__ float *col_voxel(unsigned lo, unsigned hi, float m)
+{
+    return reinterpret_cast<float *>(((unsigned long long)hi << 32 | lo) + 4ull * (unsigned)__float_as_int(m));
+}
+
+// Whether the voxel of biased floor m, and the one above it, are in the grid.
+struct ZInside {
+    float lo, hi;           // biased floors 0 and nz
+    __device__ __forceinline__ ZInside(int nz) : lo(kFloorMagic), hi(kFloorMagic + (float)nz) {}
+    __device__ __forceinline__ bool low(float m) const { return m >= lo && m < hi; }
+    __device__ __forceinline__ bool high(float m) const { return m >= lo - 1.f && m < hi - 1.f; }
+};
+
+// A reduction that does not return the old value, for v != 0 (the address is
+// global: a plain atomicAdd on an address rebuilt from integers compiles to a
+// generic atomic, half as fast).
+__device__ __forceinline__ void red_add(float *p, float v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.neu.f32 p, %1, 0f00000000;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p),
+                 "f"(v)
+                 : "memory");
+}
+
+// Plane offsets of ray z at a table row: the warp's, or (MIXED: the warp has
+// rising and falling rays) the ray's own.
+template <bool MIXED>
+__device__ __forceinline__ void col_planes(const ColTable &tab, int j, const uint4 &te, const ZRay &z, float &lo, float &hi)
+{
+    if (MIXED) {
+        const float2 d = tab.d[j];
+        lo = z.down ? d.y : d.x;
+        hi = z.down ? d.x : d.y;
+    } else {
+        lo = __uint_as_float(te.z);
+        hi = __uint_as_float(te.w);
+    }
+}
+
+// z split of a slab of a ray that is not steep: biased floor and low share.
+// (The grid has at most 2^20 rows and slabs, and such a ray moves at most one
+// row per slab: positions stay below 2^22, no clamp is needed for the floor.)
+template <bool REF>
+__device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &r)
+{
+    const float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
+    m = __fadd_rd(q, kFloorMagic);
+    if (REF) {
+        const float c = __fadd_rn(m, 1.f - kFloorMagic);
+        r = __saturatef(__fmul_rn(__fadd_rn(c, -q), rcp_approx(__fadd_rn(z_pos(z, zg, hi), -q))));
+    } else {
+        r = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
+    }
+}
+
+// Forward of one chunk's table rows.  Each kind of slab is walked in a loop of
+// its own: no branch stands between the loads of consecutive slabs, so they
+// overlap.  ZCHK: z range checks.
+template <int R, bool REF, bool MIXED, bool ZCHK>
+__device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
+                                                GatherSink<> (&f)[R])
+{
+    const ZInside in(q.zg.nz);
+    auto load = [&](const float *p, float m, float &a, float &b) {
+        a = !ZCHK || in.low(m) ? __ldg(p) : 0.f;
+        b = !ZCHK || in.high(m) ? __ldg(p + 1) : 0.f;
+    };
+#pragma unroll 4
+    for (int j = 0; j < h.cross; ++j) {
+        const uint4 te = tab.a[j];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float lo, hi, m, r, a, b;
+            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
+            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
+            load(col_voxel(te.x, te.y, m), m, a, b);
+            f[i].sum[0] = __fmaf_rn(b, __fsub_rn(1.f, r), __fmaf_rn(a, r, f[i].sum[0]));
+        }
+    }
+#pragma unroll 2
+    for (int j = h.cross; j < h.half; ++j) {
+        const uint4 te = tab.a[j], tc = tab.c[j];
+        const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float lo, hi, m, r, a, b, c, d;
+            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
+            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
+            load(col_voxel(te.x, te.y, m), m, a, b);
+            load(col_voxel(tc.x, tc.y, m), m, c, d);
+            const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11);
+            const float acc = __fmaf_rn(b, __fsub_rn(rv, w11), __fmaf_rn(a, w11, f[i].sum[1]));
+            f[i].sum[1] = __fmaf_rn(d, __fsub_rn(ov, w21), __fmaf_rn(c, w21, acc));
+        }
+    }
+#pragma unroll 1
+    for (int j = h.half; j < h.n; ++j) {
+        const uint4 te = tab.a[j], tc = tab.c[j];
+        const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float lo, hi, m, r, a, b;
+            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
+            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
+            load(col_voxel(te.x, te.y, m), m, a, b);
+            const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11);
+            const float wl = tc.x ? w21 : w11, wh = tc.x ? __fsub_rn(ov, w21) : __fsub_rn(rv, w11);
+            f[i].sum[2] = __fmaf_rn(b, wh, __fmaf_rn(a, wl, f[i].sum[2]));
+        }
+    }
+}
+
+// Forward of the lane's R rays (not steep): sums into f.
+template <int R, bool REF, bool MIXED>
+__device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__restrict__ vol, GatherSink<> (&f)[R])
+{
+    ColTable &tab = col_table();
+    for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
+        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, vol, tab);
+        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1) col_gather_rows<R, REF, MIXED, false>(q, tab, h, f);
+        else col_gather_rows<R, REF, MIXED, true>(q, tab, h, f);
+#pragma unroll
+        for (int i = 0; i < R; ++i) f[i].close();
+    }
+}
+
+// How the transpose's rays 2i and 2i + 1 share reductions: not at all; as
+// neighbours, the second 0 to 1 voxel above the first in every slab; as
+// neighbours at any distance.
+enum Merge { kSingle, kNear, kAny };
+
+// Transpose of one chunk's table rows.  Two neighbouring rays' shares of a
+// voxel column are summed in registers over the voxels w, w + 1, w + 2 of the
+// first one's low voxel w, so a slab takes at most three reductions per column
+// instead of four, and the lanes of a warp, two rows apart, rarely hit the
+// same voxel.
+template <int R, bool REF, bool MIXED, Merge MERGE, bool ZCHK>
+__device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
+                                                 const float (&y)[R])
+{
+    const ZInside in(q.zg.nz);
+    // values l, u of the low and high voxels of rays i.. in one voxel column
+    constexpr int S = MERGE == kSingle ? 1 : 2;
+    auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], float (&l)[S], float (&u)[S]) {
+        if (ZCHK) {
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                if (!in.low(m[k])) l[k] = 0.f;
+                if (!in.high(m[k])) u[k] = 0.f;
+            }
+        }
+        float *const p = col_voxel(lo, hi, m[0]);
+        if constexpr (MERGE == kNear) {
+            const bool same = m[0] == m[1];
+            if (same) l[0] += l[1];
+            u[0] += same ? u[1] : l[1];
+            if (!same) red_add(p + 2, u[1]);
+        } else if constexpr (MERGE == kAny) {
+            const bool same = m[0] == m[1], next = m[1] == m[0] + 1.f;
+            float *const s = col_voxel(lo, hi, m[1]);
+            l[0] += same ? l[1] : 0.f;
+            u[0] += same ? u[1] : next ? l[1] : 0.f;
+            if (!same && !next) red_add(s, l[1]);
+            if (!same) red_add(s + 1, u[1]);
+        }
+        red_add(p, l[0]);
+        red_add(p + 1, u[0]);
+    };
+#pragma unroll 1
+    for (int j = h.cross; j < h.n; ++j) {
+        const uint4 te = tab.a[j], tc = tab.c[j];
+        const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
+#pragma unroll
+        for (int i = 0; i < R; i += S) {
+            float lo, hi, m[S], l1[S], u1[S], l2[S], u2[S];
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                float r;
+                col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
+                z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
+                const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11), yk = y[i + k];
+                l1[k] = yk * w11;
+                u1[k] = yk * __fsub_rn(rv, w11);
+                l2[k] = yk * w21;
+                u2[k] = yk * __fsub_rn(ov, w21);
+            }
+            if (j < h.half) {
+                reduce(te.x, te.y, m, l1, u1);
+                reduce(tc.x, tc.y, m, l2, u2);
+            } else if (tc.x == 0u) {
+                reduce(te.x, te.y, m, l1, u1);
+            } else {
+                reduce(te.x, te.y, m, l2, u2);
+            }
+        }
+    }
+#pragma unroll 2
+    for (int j = 0; j < h.cross; ++j) {
+        const uint4 te = tab.a[j];
+#pragma unroll
+        for (int i = 0; i < R; i += S) {
+            float lo, hi, m[S], l[S], u[S];
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                float r;
+                col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
+                z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
+                l[k] = y[i + k] * r;
+                u[k] = __fmaf_rn(-y[i + k], r, y[i + k]);
+            }
+            reduce(te.x, te.y, m, l, u);
+        }
+    }
+}
+
+// Transpose of the lane's R rays (not steep; y finite, 0 for a ray that takes
+// no part).
+template <int R, bool REF, bool MIXED, Merge MERGE>
+__device__ __forceinline__ void col_scatter(const ColRays<R> &q, float *acc, const float (&y)[R])
+{
+    ColTable &tab = col_table();
+    for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
+        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, acc, tab);
+        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1) col_scatter_rows<R, REF, MIXED, MERGE, false>(q, tab, h, y);
+        else col_scatter_rows<R, REF, MIXED, MERGE, true>(q, tab, h, y);
+    }
 }
 
 }  // namespace nefct

@@ -36,7 +36,6 @@ __global__ void __launch_bounds__(256) cb_count_kernel(const __grid_constant__ C
 
 // ---------------- deterministic transpose (fixed point) ----------------
 
-template <bool DIV>
 __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_constant__ CBParams<float> p)
 {
     int ia, ib, iv;
@@ -48,30 +47,33 @@ __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_con
     cb_ray(p, ia, ib, iv, r);
     Walk<float> w;
     if (!setup_walk(p.g, r, p.flags, w)) return;
-    const float scale = *p.fix_scale;
-    const int sw = p.g.nx * p.g.ny;
-    if (!w.xdrive) scatter_walk_fixed<float, DIV, true>(w, p.g, p.fix, p.g.nx, 1, sw, y, scale);
-    else if (p.fixT) scatter_walk_fixed<float, DIV, true>(w, p.g, p.fixT, p.g.ny, 1, sw, y, scale);
-    else scatter_walk_fixed<float, DIV, false>(w, p.g, p.fix, 1, p.g.nx, sw, y, scale);
+    const unsigned sw = (unsigned)(p.g.nx * p.g.ny);
+    unsigned su, sv;
+    thread_strides(p.g.nx, p.g.ny, w.xdrive, p.fixT != nullptr, su, sv);
+    FixedSink f{w.xdrive && p.fixT ? p.fixT : p.fix, sw, y * w.W, *p.fix_scale};
+    if (ref_rounding(p.flags)) ray_walk<true>(p.g, w, su, sv, sw, f);
+    else ray_walk<false>(p.g, w, su, sv, sw, f);
 }
 
 // Column-warp variant: 64-bit fixed-point reductions into a z-fastest
 // accumulator (the same per-contribution integers as the thread walk, so the
 // integer sums and the result are bitwise the same).
-template <bool DIV>
 __global__ void __launch_bounds__(256) cb_colwarp_fixed_kernel(const __grid_constant__ CBParams<float> p)
 {
-    const int lane = threadIdx.x;
     const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    int ib, iv;
-    if (p.band_major) { iv = blockIdx.y; ib = blockIdx.z * 32 + lane; }
-    else { ib = blockIdx.y * 32 + lane; iv = blockIdx.z; }
+    const int tile = p.band_major ? blockIdx.z : blockIdx.y;
+    const int iv = p.band_major ? blockIdx.y : blockIdx.z;
     if (ia >= p.na) return;                       // uniform across the warp
-    const bool has = ib < p.nb;
-    const float y = has ? cb_sino_value(p, ia, ib, iv) : 0.f;
-    float r[6];
-    cb_ray(p, ia, has ? ib : 0, iv, r);
-    colwarp_lane<DIV, false, true>(p.g, r, has, p.flags, nullptr, nullptr, y, nullptr, p.fix, *p.fix_scale);
+    const int ib = tile * 32 + threadIdx.x;
+    float r[1][6];
+    const float y = ib < p.nb ? cb_sino_value(p, ia, ib, iv) : 0.f;
+    const bool has[1] = {ib < p.nb && y != 0.f};
+    cb_ray(p, ia, ib < p.nb ? ib : 0, iv, r[0]);
+    ColRays<1> q;
+    if (!col_rays<1>(p.g, r, has, p.flags, q)) return;
+    FixedSink f{p.fix, 1u, q.z[0].live ? y * q.W[0] : 0.f, *p.fix_scale};
+    if (ref_rounding(p.flags)) col_each<true>(q.c, q.K0, q.K1, q.z[0], q.zg, f);
+    else col_each<false>(q.c, q.K0, q.K1, q.z[0], q.zg, f);
 }
 
 // vol[z][y][x] = accZ[y][x][z] / scale (the integer sums of the column warps)
@@ -507,14 +509,12 @@ static nefct_status cb_backward_fixed_impl(const nefct_cb_geom *g, const float *
         dim3 grid, block;
         if (cw) {
             cb_colwarp_shape(p, g->na, g->nb, nvc, grid, block);
-            if (cubic(p.g)) cb_colwarp_fixed_kernel<false><<<grid, block, 0, s>>>(p);
-            else cb_colwarp_fixed_kernel<true><<<grid, block, 0, s>>>(p);
+            cb_colwarp_fixed_kernel<<<grid, block, 0, s>>>(p);
             NEFCT_CHECK_LAUNCH("cb_colwarp_fixed_kernel");
             continue;
         }
         cb_shape(p, g->na, g->nb, nvc, grid, block);
-        if (cubic(p.g)) cb_backward_fixed_kernel<false><<<grid, block, 0, s>>>(p);
-        else cb_backward_fixed_kernel<true><<<grid, block, 0, s>>>(p);
+        cb_backward_fixed_kernel<<<grid, block, 0, s>>>(p);
         NEFCT_CHECK_LAUNCH("cb_backward_fixed_kernel");
     }
     if (cw) {

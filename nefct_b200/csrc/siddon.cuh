@@ -15,9 +15,9 @@
 //  * the per-contribution weight is r * W with W = S*dx/L^2 hoisted per ray
 //    (the reference re-evaluates r*S*dx/L/L per contribution; the results
 //    differ by rounding only);
-//  * the slab range is clipped in FP64 to the slabs where the ray can touch
-//    the volume (with a one-voxel margin); slabs outside contribute nothing,
-//    so the clip changes no result, only the trip count;
+//  * the slab range is clipped to the slabs where the ray can touch the volume
+//    (with a margin for rounding); slabs outside contribute nothing, so the
+//    clip changes no result, only the trip count;
 //  * the three-way case split is written as one predicated sequence of at
 //    most three (voxel, weight) slots, in the reference's accumulation order;
 //  * the crossing ratios use the approximate reciprocal (<= 2 ulp) in FP32:
@@ -26,6 +26,8 @@
 //    (rounding-level difference from the per-contribution products);
 //  * slabs whose candidate voxels are all inside the grid skip the range
 //    checks (interior range computed with the clip).
+// This walk serves the double builds, the LOR pair and the intersection
+// count; the float cone-beam kernels split slabs as colwarp.cuh does.
 #pragma once
 
 #include "common.cuh"
@@ -99,43 +101,46 @@ __device__ __forceinline__ void cb_ray(const RayGeom<T> &p, T cs, T sn, T off, i
 template <typename T> struct Walk {
     T pu, pv, pw;        // source in voxel units along (drive, other transverse, z)
     T kv, kw;            // slopes d(v)/d(u), d(z)/d(u)
+    T kz, z0;            // z position in rows at plane offset d = t - pu: kz * d + z0
     T dv, nu2, nv2;
     T W, Wmid;           // contribution weights (Wmid: three-voxel middle slot, Q5)
     int nu, nv, k0, k1;  // slab count, transverse extent, inclusive slab range
     int ki0, ki1;        // interior slabs: every candidate voxel is inside the grid
+    int zi0, zi1;        // slabs whose low z voxel and its upper neighbour are inside the grid
     bool xdrive, vdiv;
 };
 
-// Slab ranges of the driving axis (FP64).  Slab k lies between planes
-// t = k - nu2 and t + 1, and the transverse position is p(t) = A + B t.
-// [k0, k1]: slabs whose positions reach [-1 - m, n + 1 + m], i.e. that can
-// touch the grid.  [ki0, ki1]: slabs whose positions at both planes lie in
-// [m, n - m], so the floors of both planes are valid indices and no range
-// check is needed.  m covers the difference between these FP64 positions and
-// the FP32 ones the walk evaluates: 1/64 voxel plus 1e-5 of the largest
-// magnitude entering them (a few hundred FP32 ulps).
-__device__ __forceinline__ void clip_axis(double A, double B, int n, double nu2, int nu, double mag, int &k0,
-                                          int &k1, int &ki0, int &ki1)
+// Slab ranges of the driving axis.  Slab k lies between planes t = k - nu2
+// and t + 1, and the transverse position is p(t) = A + B (t - pu).
+// [k0, k1]: slabs whose positions reach [-m, n + m], i.e. that can touch the
+// grid.  [ki0, ki1]: slabs whose positions at both planes lie in [m, top - m],
+// so the voxels they touch need no range check.  m covers the rounding of
+// these positions and of the walk's own: 1/64 voxel plus 1e-5 of the
+// magnitudes entering them (a hundred float ulps).  The ranges decide only
+// which slabs are checked, so float suffices for the float walks (the double
+// build evaluates them in double).
+template <typename T>
+__device__ __forceinline__ void clip_axis(T A, T B, int n, int top, T pu, T nu2, int nu, int &k0, int &k1, int &ki0,
+                                          int &ki1)
 {
-    const double m = 1.0 / 64.0 + 1e-5 * mag;
-    if (B == 0.0) {
-        if (A < -1.0 - m || A > (double)n + 1.0 + m) { k0 = 1; k1 = 0; }
-        if (A < m || A > (double)n - m) { ki0 = 1; ki1 = 0; }
+    const T aB = B > (T)0 ? B : -B, aA = A > (T)0 ? A : -A, apu = pu > (T)0 ? pu : -pu;
+    const T m = (T)(1.0 / 64.0) + (T)1e-5 * (aA + aB * (apu + (T)nu) + (T)n);
+    const T hi = (T)n + m, ih = (T)top - m;
+    if (!(aB > (T)1e-30)) {
+        if (A < -m || A > hi) { k0 = 1; k1 = 0; }
+        if (A < m || A > ih) { ki0 = 1; ki1 = 0; }
         return;
     }
-    auto span = [&](double lo, double hi, double &t0, double &t1) {
-        t0 = (lo - A) / B;
-        t1 = (hi - A) / B;
-        if (t0 > t1) { const double s = t0; t0 = t1; t1 = s; }
-    };
-    auto clampk = [&](double v) { return (int)fmin(fmax(v, -2.0), (double)nu + 1.0); };
-    double t0, t1;
-    span(-1.0 - m, (double)n + 1.0 + m, t0, t1);
-    k0 = max(k0, clampk(ceil(t0 + nu2 - 1.0)));
-    k1 = min(k1, clampk(floor(t1 + nu2)));
-    span(m, (double)n - m, t0, t1);
-    ki0 = max(ki0, clampk(ceil(t0 + nu2)));
-    ki1 = min(ki1, clampk(floor(t1 + nu2) - 1.0));
+    const T iB = (T)1 / B, t = pu + nu2;
+    auto clampk = [&](T v) { return (int)fmin(fmax(v, (T)-2), (T)nu + (T)1); };
+    T a = (-m - A) * iB + t, b = (hi - A) * iB + t;
+    k0 = max(k0, clampk(ceil(fmin(a, b) - (T)1)));
+    k1 = min(k1, clampk(floor(fmax(a, b))));
+    a = (m - A) * iB + t;
+    b = (ih - A) * iB + t;
+    if (m > ih) { ki0 = 1; ki1 = 0; return; }
+    ki0 = max(ki0, clampk(ceil(fmin(a, b))));
+    ki1 = min(ki1, clampk(floor(fmax(a, b)) - (T)1));
 }
 
 // Per-ray setup of project_device / backproject_device (reference :19-44,
@@ -149,9 +154,6 @@ __device__ __forceinline__ bool setup_walk(const GridDev<T> &g, const T *r, uint
     const T z1 = F::div(F::sub(r[2], g.cz), g.dx_), z2 = F::div(F::sub(r[5], g.cz), g.dx_);
     const T xd = F::sub(x2, x1), yd = F::sub(y2, y1), zd = F::sub(z2, z1);
     const T xy2 = F::add(F::mul(xd, xd), F::mul(yd, yd));
-    if ((flags & NEFCT_SKIP_SHORT) && F::sqrt(xy2) < (T)10) return false;   // Q4
-    // a ray along z has 0/0 slopes in the reference (undefined); it contributes 0 here
-    if (xy2 == (T)0) return false;
     const T L = F::sqrt(F::add(xy2, F::mul(zd, zd)));
     const T axd = xd > (T)0 ? xd : -xd, ayd = yd > (T)0 ? yd : -yd;
     w.xdrive = (flags & NEFCT_TIE_GT) ? (axd > ayd) : (axd >= ayd);
@@ -166,6 +168,8 @@ __device__ __forceinline__ bool setup_walk(const GridDev<T> &g, const T *r, uint
         w.dv = (T)1; w.vdiv = false; w.nu2 = g.ny2; w.nv2 = g.nx2;
     }
     w.pw = z1;
+    w.kz = g.dz != (T)1 ? F::div(w.kw, g.dz) : w.kw;
+    w.z0 = F::add(g.dz != (T)1 ? F::div(z1, g.dz) : z1, g.nz2);
     const T S = F::sqrt(F::add(F::add((T)1, F::mul(w.kv, w.kv)), F::mul(w.kw, w.kw)));
     T W = F::mul(S, g.dx_);
     if (!(flags & NEFCT_NO_INV_L2)) W = F::div(F::div(W, L), L);
@@ -174,17 +178,18 @@ __device__ __forceinline__ bool setup_walk(const GridDev<T> &g, const T *r, uint
 
     w.k0 = 0; w.k1 = w.nu - 1;
     w.ki0 = 0; w.ki1 = w.nu - 1;
-    const double pu = (double)w.pu, kv = (double)w.kv, kw = (double)w.kw;
-    const double dv = (double)w.dv, dz = (double)g.dz;
-    const double mag = fabs(pu) + fabs((double)w.pv) + fabs((double)w.pw) + (double)(w.nu + w.nv + g.nz);
-    clip_axis(((double)w.pv - kv * pu) / dv + (double)w.nv2, kv / dv, w.nv, (double)w.nu2, w.nu, mag, w.k0, w.k1,
-              w.ki0, w.ki1);
-    clip_axis(((double)w.pw - kw * pu) / dz + (double)g.nz2, kw / dz, g.nz, (double)w.nu2, w.nu, mag, w.k0, w.k1,
-              w.ki0, w.ki1);
+    const T kvv = w.vdiv ? w.kv / w.dv : w.kv, v0 = (w.vdiv ? w.pv / w.dv : w.pv) + w.nv2;
+    clip_axis<T>(v0, kvv, w.nv, w.nv, w.pu, w.nu2, w.nu, w.k0, w.k1, w.ki0, w.ki1);
+    // (top row nz - 1: such a slab reads its low voxel's upper neighbour too)
+    w.zi0 = 0; w.zi1 = w.nu - 1;
+    clip_axis<T>(w.z0, w.kz, g.nz, g.nz - 1, w.pu, w.nu2, w.nu, w.k0, w.k1, w.zi0, w.zi1);
     w.k0 = max(w.k0, 0);
     w.k1 = min(w.k1, w.nu - 1);
-    w.ki0 = max(w.ki0, w.k0);
-    w.ki1 = min(w.ki1, w.k1);
+    w.ki0 = max(max(w.ki0, w.zi0), w.k0);
+    w.ki1 = min(min(w.ki1, w.zi1), w.k1);
+    if ((flags & NEFCT_SKIP_SHORT) && F::sqrt(xy2) < (T)10) return false;   // Q4
+    // a ray along z has 0/0 slopes in the reference (undefined); it contributes 0 here
+    if (xy2 == (T)0) return false;
     return w.k0 <= w.k1;
 }
 
@@ -441,20 +446,6 @@ __device__ __forceinline__ void scatter_walk(const Walk<T> &w, const GridDev<T> 
 // not depend on the order of the reductions, so the result is bitwise
 // reproducible.  The caller picks the scale so that no sum can overflow.
 __device__ __forceinline__ long long to_fixed(float v) { return __float2ll_rn(v); }
-__device__ __forceinline__ long long to_fixed(double v) { return __double2ll_rn(v); }
-
-template <typename T, bool DIV, bool SV1>
-__device__ __forceinline__ void scatter_walk_fixed(const Walk<T> &w, const GridDev<T> &g, unsigned long long *base,
-                                                   int su, int sv, int sw, T value, T scale)
-{
-    const T yw = value * w.W;
-    auto f = [&](const SlabSlots<T> &s) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            if (s.ok[j]) atomicAdd(base + s.idx[j], (unsigned long long)to_fixed((yw * s.r[j]) * scale));
-    };
-    with_walker<T, DIV, SV1>(w, g, su, sv, sw, [&](auto &it) { walk_all(it, w.k0, w.k1, w.ki0, w.ki1, f); });
-}
 
 // Number of contributions of the ray (the throughput unit).  Uses the
 // reference's exact ratio division, so near-equal crossing ratios order the
@@ -601,37 +592,6 @@ __device__ __forceinline__ void exact_backward(const GridDev<T> &g, const T *r, 
     if (e.xdom && outT) exact_walk(g, e, g.ny, 1, sw, f);
     else if (e.xdom) exact_walk(g, e, 1, g.nx, sw, f);
     else exact_walk(g, e, g.nx, 1, sw, f);
-}
-
-// Forward value of one ray: gathers x-driven rays from the y-fastest copy
-// volT when there is one, everything else from the x-fastest volume.
-template <typename T, bool DIV, bool EXACT = false>
-__device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32_t flags, const T *vol, const T *volT)
-{
-    if (EXACT) return exact_forward(g, r, flags, vol, volT);
-    Walk<T> w;
-    if (!setup_walk(g, r, flags, w)) return (T)0;
-    const int sw = g.nx * g.ny;
-    if (!w.xdrive) return gather_walk<T, DIV, true, false>(w, g, vol, g.nx, 1, sw);
-    if (volT) return gather_walk<T, DIV, true, false>(w, g, volT, g.ny, 1, sw);
-    return gather_walk<T, DIV, false, false>(w, g, vol, 1, g.nx, sw);
-}
-
-// Transpose contribution of one ray with value y: x-driven rays reduce into
-// the y-fastest accumulator outT when there is one.
-template <typename T, bool DIV, bool EXACT = false>
-__device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, uint32_t flags, T y, T *out, T *outT)
-{
-    if (EXACT) {
-        exact_backward(g, r, flags, y, out, outT);
-        return;
-    }
-    Walk<T> w;
-    if (!setup_walk(g, r, flags, w)) return;
-    const int sw = g.nx * g.ny;
-    if (!w.xdrive) scatter_walk<T, DIV, true, false>(w, g, out, g.nx, 1, sw, y);
-    else if (outT) scatter_walk<T, DIV, true, false>(w, g, outT, g.ny, 1, sw, y);
-    else scatter_walk<T, DIV, false, false>(w, g, out, 1, g.nx, sw, y);
 }
 
 // out[z][x][y] = in[z][y][x] (32x32 tiles through shared memory)

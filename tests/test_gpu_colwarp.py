@@ -1,0 +1,105 @@
+"""GPU: the column-warp kernels at the edges of their row tiles and dispatch
+rules -- row counts around the tiles of one, two and three rows per lane, row
+pitches on both sides of the rule for merged reductions (and pairs that drift
+more than a voxel apart inside it), rows falling in z, warps with rising and
+falling rays, cone angles beyond 45 degrees, voxels that are not cubic,
+rounding rules, infinities -- against the CPU restatement, and against the
+thread walk, whose forward has the same bits.
+
+Tolerance: the parity bar of the other tests (rel-L2 1e-5, max-abs 1e-4 x max).
+The walk's z positions differ from the restatement's by at most two roundings
+of about 1e-6 voxel on these grids, i.e. ~1e-6 of a result.
+"""
+import numpy as np
+import pytest
+import torch
+
+import nefct_b200 as nb
+from nefct_b200 import _lib, autotune, ops
+from tests.test_gpu_siddon import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+ANGLES = np.array([0.1, 0.7, np.pi / 2, 2.2, 3.6, 5.3], np.float32)
+
+# rows; row pitch (detector, magnification 2); z voxel; z offset of the views
+CASES = [
+    (1, 1.2, 1.0, 0.0), (31, 1.2, 1.0, 0.0), (32, 1.0, 1.0, 0.4), (33, 1.2, 1.0, 0.0), (63, 0.6, 1.0, 0.0),
+    (64, 1.2, 1.0, -6.0), (65, 1.2, 1.0, 6.0), (96, 0.7, 1.0, 0.0), (97, 0.7, 1.0, 0.0), (129, 0.4, 1.0, 3.0),
+    (45, -1.1, 1.0, 0.0),                   # rows falling in z
+    (40, 1.75, 1.0, 0.0),                   # pairs under the rule at the axis, over a voxel apart behind it
+    (40, 1.9, 1.0, 0.0), (40, 3.1, 1.0, 0.0),          # single rows
+    (50, 1.2, 0.7, 0.0), (50, 1.2, 1.6, 1.0),          # voxels that are not cubic
+]
+
+
+def _geom(rows, pitch, vz, off, src_iso=70.0):
+    shape = (26, 22, 24)
+    return nb.ConeBeam(shape, ANGLES, src_iso, 2 * src_iso, 37, 1.5, rows, pitch, size=(26.0, 24.2, 24.0 * vz),
+                       center=(0.3, -0.2, 0.1), z_offsets=np.linspace(off - 0.5, off + 0.5, ANGLES.size))
+
+
+def _oracle(oracle_lib, g, vol, y, flags):
+    og = oracle_lib.grid(g.shape, g.center, g.size)
+    args = (g.angles, g.src_iso, g.src_det, g.na, g.da, 0.5, g.nb, g.db, 0.5)
+    of = (0 if flags & _lib.TIE_GT else oracle_lib.TIE_GE) | (0 if flags & _lib.NO_INV_L2 else oracle_lib.INV_L2)
+    of |= oracle_lib.SKIP_SHORT if flags & _lib.SKIP_SHORT else 0
+    fwd = oracle_lib.cb_forward(og, vol, *args, off=g.z_offsets, flags=of)[0]
+    return fwd, oracle_lib.cb_backward(og, y, *args, off=g.z_offsets, flags=of)
+
+
+def _both(g, vol, y, flags, walk):
+    saved = autotune.current()
+    try:
+        autotune.apply(saved["rows"], saved["order"], walk)
+        return ops.cb_forward(vol, g, flags), ops.cb_backward(y, g, flags)
+    finally:
+        autotune.apply(saved["rows"], saved["order"], saved["walk"])
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("case", CASES, ids=[f"{c[0]}x{c[1]}-dz{c[2]}-off{c[3]}" for c in CASES])
+def test_row_tiles_and_dispatch(cuda, oracle_lib, case, flags):
+    g = _geom(*case)
+    rng = np.random.default_rng(case[0])
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    y[1, : case[0] // 3] = 0                       # rays that take no part
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    f, b = _both(g, v, s, flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(b.cpu().numpy(), ref_b)
+    ft, bt = _both(g, v, s, flags, 0)
+    assert torch.equal(f, ft)
+    assert_parity(b.cpu().numpy(), bt.cpu().numpy(), rel=1e-6, mabs=1e-5)
+    det = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC) for _ in range(2)]
+    assert torch.equal(det[0], det[1])
+    assert_parity(det[0].cpu().numpy(), b.cpu().numpy(), rel=1e-6, mabs=1e-5)
+
+
+def test_deterministic_flag_leaves_the_forward_alone(cuda):
+    g = _geom(65, 1.2, 1.0, 0.0)
+    vol = torch.rand(g.vol_shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(1))
+    assert torch.equal(ops.cb_forward(vol, g, _lib.DETERMINISTIC), ops.cb_forward(vol, g, 0))
+
+
+@pytest.mark.parametrize("pitch", [1.2, 3.0], ids=["pairs", "single-rows"])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_values_that_are_not_finite_stay_on_their_rays(cuda, oracle_lib, value, pitch):
+    """A voxel that is not finite reaches the rays that pass it and no other;
+    a sinogram value that is not finite the voxels on its ray."""
+    g = _geom(45, pitch, 1.0, 0.0)
+    rng = np.random.default_rng(7)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    vol[11, 9, 14] = value
+    y[2, 21, 17] = value
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, 0)
+    f, b = (t.cpu().numpy() for t in _both(g, torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda), 0, 3))
+    for out, ref in ((f, ref_f), (b, ref_b)):
+        fine = np.isfinite(ref)
+        assert 0 < (~fine).sum() < ref.size // 10
+        np.testing.assert_array_equal(np.isfinite(out), fine)
+        np.testing.assert_array_equal(np.isnan(out), np.isnan(ref))
+        assert_parity(np.where(fine, out, 0), np.where(fine, ref, 0))
