@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
                 y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
                 cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);
             }
-            if (P.near) colwarp_backward<2, REF, true>(P.g, r, has, P.flags, y, P.volT);
-            else colwarp_backward<2, REF, false>(P.g, r, has, P.flags, y, P.volT);
+            if (P.near) colwarp_backward<2, REF, true>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
+            else colwarp_backward<2, REF, false>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
         }
     }
 }

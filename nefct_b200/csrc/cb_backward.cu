@@ -5,8 +5,9 @@
 namespace nefct {
 
 // Column warps: one warp per 32 R rows of column ia at view iv, into the
-// z-fastest accumulator p.outT.
-template <int R, bool REF, bool PAIR>
+// z-fastest accumulator p.outT (FIXED: the deterministic transpose's integers
+// p.fix).
+template <int R, bool REF, bool PAIR, bool FIXED>
 __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __grid_constant__ CBParams<float> p)
 {
     const int ia = blockIdx.x * blockDim.y + threadIdx.y;
@@ -22,26 +23,37 @@ __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __gri
         y[i] = has[i] ? cb_sino_value(p, ia, ib, iv) : 0.f;
         cb_ray(p, ia, has[i] ? ib : 0, iv, r[i]);
     }
-    colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, p.outT);
+    if constexpr (FIXED) colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, FixedAcc{p.fix, *p.fix_scale});
+    else colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, FloatAcc{p.outT});
 }
 
-template <int R, bool PAIR>
+template <int R, bool PAIR, bool FIXED>
 static cudaError_t launch_colwarp(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
 {
     dim3 grid, block;
     cb_colwarp_shape(p, na, nb, nvc, grid, block, R);
-    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, PAIR><<<grid, block, 0, s>>>(p);
-    else cb_colwarp_backward_kernel<R, false, PAIR><<<grid, block, 0, s>>>(p);
+    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, PAIR, FIXED><<<grid, block, 0, s>>>(p);
+    else cb_colwarp_backward_kernel<R, false, PAIR, FIXED><<<grid, block, 0, s>>>(p);
     return cudaGetLastError();
+}
+
+template <bool FIXED>
+static cudaError_t launch_rows(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
+{
+    return col_rows_near(p.g, p.rg) ? launch_colwarp<2, true, FIXED>(p, na, nb, nvc, flags, s)
+                                    : launch_colwarp<1, false, FIXED>(p, na, nb, nvc, flags, s);
+}
+
+cudaError_t cb_launch_backward_fixed(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
+{
+    return launch_rows<true>(p, na, nb, nvc, flags, s);
 }
 
 template <typename T>
 cudaError_t cb_launch_backward(CBParams<T> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s, bool colwarp)
 {
     if constexpr (std::is_same<T, float>::value) {
-        if (colwarp)
-            return col_rows_near(p.g, p.rg) ? launch_colwarp<2, true>(p, na, nb, nvc, flags, s)
-                                            : launch_colwarp<1, false>(p, na, nb, nvc, flags, s);
+        if (colwarp) return launch_rows<false>(p, na, nb, nvc, flags, s);
     }
     return cb_launch<T, false>(p, na, nb, nvc, flags, s);
 }

@@ -222,12 +222,15 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
     }
 }
 
+__device__ __forceinline__ ScatterSink ray_sink(const FloatAcc &a, float yw) { return ScatterSink{a.vol, 1u, yw}; }
+__device__ __forceinline__ FixedSink ray_sink(const FixedAcc &a, float yw) { return FixedSink{a.vol, 1u, yw, a.scale}; }
+
 // Transpose of R rows per lane of one detector column: y[i] times the ray's
-// weights into the z-fastest accumulator accZ.  PAIR: rows 2i and 2i + 1 are
+// weights into the z-fastest accumulator acc.  PAIR: rows 2i and 2i + 1 are
 // neighbours in z order and merge their reductions.
-template <int R, bool REF, bool PAIR>
+template <int R, bool REF, bool PAIR, class Acc>
 __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const float (&r)[R][6], bool (&has)[R],
-                                                 uint32_t flags, const float (&y)[R], float *accZ)
+                                                 uint32_t flags, const float (&y)[R], const Acc &acc)
 {
     ColRays<R> q;
 #pragma unroll
@@ -243,7 +246,7 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
     if (q.steep || !__all_sync(0xffffffffu, finite)) {
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            ScatterSink f{accZ, 1u, yw[i]};
+            auto f = ray_sink(acc, yw[i]);
             col_each<REF>(q.c, q.K0, q.K1, q.z[i], q.zg, f);
         }
         return;
@@ -270,16 +273,12 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
                 z0.live = false;
             }
         }
-        if (!__all_sync(0xffffffffu, near)) {
-            col_scatter<R, REF, true, kAny>(q, accZ, yw);
-        } else if (mixed) {
-            col_scatter<R, REF, true, kNear>(q, accZ, yw);
-        } else {
-            col_scatter<R, REF, false, kNear>(q, accZ, yw);
-        }
+        if (!__all_sync(0xffffffffu, near)) col_scatter<R, REF, true, kAny>(q, acc, yw);
+        else if (mixed) col_scatter<R, REF, true, kNear>(q, acc, yw);
+        else col_scatter<R, REF, false, kNear>(q, acc, yw);
     } else {
-        if (mixed) col_scatter<R, REF, true, kSingle>(q, accZ, yw);
-        else col_scatter<R, REF, false, kSingle>(q, accZ, yw);
+        if (mixed) col_scatter<R, REF, true, kSingle>(q, acc, yw);
+        else col_scatter<R, REF, false, kSingle>(q, acc, yw);
     }
 }
 
@@ -372,5 +371,8 @@ cudaError_t cb_launch_forward(CBParams<T> &p, int na, int nb, int nvc, uint32_t 
 template <typename T>
 cudaError_t cb_launch_backward(CBParams<T> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s,
                                bool colwarp = false);
+
+// The deterministic transpose's column warps (p.fix: z-fastest accumulator).
+cudaError_t cb_launch_backward_fixed(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s);
 
 }  // namespace nefct

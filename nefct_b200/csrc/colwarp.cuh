@@ -156,25 +156,43 @@ struct ZSplit {
     float rw;
 };
 
+// z split of a slab of a ray that is not steep: biased floor and low share.
+// (The grid has at most 2^20 rows and slabs, and such a ray moves at most one
+// row per slab: positions stay below 2^22, no clamp is needed for the floor.)
+template <bool REF>
+__device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &r)
+{
+    const float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
+    m = __fadd_rd(q, kFloorMagic);
+    if (REF) {
+        const float c = __fadd_rn(m, 1.f - kFloorMagic);
+        r = __saturatef(__fmul_rn(__fadd_rn(c, -q), rcp_approx(__fadd_rn(z_pos(z, zg, hi), -q))));
+    } else {
+        r = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
+    }
+}
+
 template <bool REF>
 __device__ __forceinline__ ZSplit z_split(const ZRay &z, const ZGrid &zg, float d, float dh)
 {
     ZSplit s;
-    float q = REF ? z_pos(z, zg, d) : __fmaf_rn(z.kz, d, z.z0);
-    const float m = magic_floor<true>(q);
-    q = fminf(fmaxf(q, -kFloorClamp), kFloorClamp);
-    s.i1 = (unsigned)__float_as_int(m);
-    s.i2 = s.i1 + 1u;
-    if (REF || z.steep) {
-        float qh = REF ? z_pos(z, zg, dh) : __fmaf_rn(z.kz, dh, z.z0);
-        const float mh = magic_floor<true>(qh);
-        qh = fminf(fmaxf(qh, -kFloorClamp), kFloorClamp);
-        const float den = REF ? rcp_approx(__fadd_rn(qh, -q)) : z.ikz;
-        s.rw = mh != m ? __fmul_rn(__fadd_rn(__fadd_rn(mh, -kFloorMagic), -q), den) : 1.f;
-        if (REF || mh != m) s.i2 = (unsigned)__float_as_int(mh);
-    } else {
-        s.rw = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
+    float m;
+    if (!z.steep) {
+        z_inner<REF>(z, zg, d, dh, m, s.rw);
+        s.i1 = (unsigned)__float_as_int(m);
+        s.i2 = s.i1 + 1u;
+        return s;
     }
+    float q = REF ? z_pos(z, zg, d) : __fmaf_rn(z.kz, d, z.z0);
+    float qh = REF ? z_pos(z, zg, dh) : __fmaf_rn(z.kz, dh, z.z0);
+    m = magic_floor<true>(q);
+    const float mh = magic_floor<true>(qh);
+    q = fminf(fmaxf(q, -kFloorClamp), kFloorClamp);
+    qh = fminf(fmaxf(qh, -kFloorClamp), kFloorClamp);
+    const float iden = REF ? rcp_approx(__fadd_rn(qh, -q)) : z.ikz;
+    s.rw = mh != m ? __fmul_rn(__fadd_rn(__fadd_rn(mh, -kFloorMagic), -q), iden) : 1.f;
+    s.i1 = (unsigned)__float_as_int(m);
+    s.i2 = (unsigned)__float_as_int(mh);
     return s;
 }
 
@@ -378,8 +396,8 @@ __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&
 // Warp's table of one 32-slab chunk, its slabs grouped by kind (slabs without
 // a v column in the grid are dropped): rows [0, cross) plain, [cross, half)
 // cross, [half, n) half.  a = (address of the low v column -- of the one
-// column in the grid for a half slab -- less 4 bytes per floor bias, offsets
-// of the lower and the upper z plane), c = (address of the high v column, or
+// column in the grid for a half slab -- less one element per floor bias,
+// offsets of the lower and the upper z plane), c = (address of the high v column, or
 // 1 in c.x when a half slab's column is the high one; rv; 1 - rv).  d: the
 // offsets of the slab's entry and exit planes.
 struct ColTable {
@@ -398,8 +416,9 @@ __device__ __forceinline__ ColTable &col_table()
     return tables[threadIdx.y];
 }
 
-// Lane j evaluates slab kc + j, if it is one of K0..K1.
-__device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0, int K1, bool falling, const float *vol,
+// Lane j evaluates slab kc + j, if it is one of K0..K1.  T: the volume's elements.
+template <typename T>
+__device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0, int K1, bool falling, const T *vol,
                                               ColTable &tab)
 {
     const int lane = threadIdx.x & 31, k = kc + lane;
@@ -418,10 +437,10 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
                                                                  : h.half + __popc(half & below);
     __syncwarp();                       // the previous chunk's reads are done
     if (is_plain || is_cross || is_half) {
-        const char *const base = reinterpret_cast<const char *>(vol) - 4ull * (unsigned)kFloorMagicBits;
+        const char *const base = reinterpret_cast<const char *>(vol) - sizeof(T) * (unsigned)kFloorMagicBits;
         const unsigned i1 = is_half && in == 2u ? e.b2 : e.b1;
-        const unsigned long long p1 = (unsigned long long)(base + 4ull * (i1 + (unsigned)kFloorMagicBits));
-        const unsigned long long p2 = (unsigned long long)(base + 4ull * (e.b2 + (unsigned)kFloorMagicBits));
+        const unsigned long long p1 = (unsigned long long)(base + sizeof(T) * (i1 + (unsigned)kFloorMagicBits));
+        const unsigned long long p2 = (unsigned long long)(base + sizeof(T) * (e.b2 + (unsigned)kFloorMagicBits));
         tab.a[row] = make_uint4((unsigned)p1, (unsigned)(p1 >> 32), __float_as_uint(falling ? db : da),
                                 __float_as_uint(falling ? da : db));
         tab.c[row] = make_uint4(is_half ? in - 1u : (unsigned)p2, (unsigned)(p2 >> 32), __float_as_uint(e.rv),
@@ -458,9 +477,9 @@ __device__ __forceinline__ void col_each(const ColWalk &cw, int K0, int K1, cons
 }
 
 // Voxel of biased floor m in the column at the table's address (lo, hi).
-__device__ __forceinline__ float *col_voxel(unsigned lo, unsigned hi, float m)
+template <typename T = float> __device__ __forceinline__ T *col_voxel(unsigned lo, unsigned hi, float m)
 {
-    return reinterpret_cast<float *>(((unsigned long long)hi << 32 | lo) + 4ull * (unsigned)__float_as_int(m));
+    return reinterpret_cast<T *>(((unsigned long long)hi << 32 | lo) + sizeof(T) * (unsigned)__float_as_int(m));
 }
 
 // Whether the voxel of biased floor m, and the one above it, are in the grid.
@@ -471,15 +490,36 @@ struct ZInside {
     __device__ __forceinline__ bool high(float m) const { return m >= lo - 1.f && m < hi - 1.f; }
 };
 
-// A reduction that does not return the old value, for v != 0 (the address is
-// global: a plain atomicAdd on an address rebuilt from integers compiles to a
-// generic atomic, half as fast).
-__device__ __forceinline__ void red_add(float *p, float v)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.neu.f32 p, %1, 0f00000000;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p),
-                 "f"(v)
-                 : "memory");
-}
+// The transpose's accumulators: floats, or 64-bit integers of yw * share times
+// a power of two (exact), rounded (the deterministic transpose: integer sums
+// do not depend on the order of the reductions).  red() reduces v != 0 without
+// returning the old value (the address is global: a plain atomicAdd on an
+// address rebuilt from integers compiles to a generic atomic, half as fast).
+struct FloatAcc {
+    using T = float;
+    float *vol;
+    __device__ __forceinline__ float value(float v) const { return v; }
+    // y times the share 1 - r, rounded once
+    __device__ __forceinline__ float rest(float y, float r) const { return __fmaf_rn(-y, r, y); }
+    static __device__ __forceinline__ void red(float *p, float v)
+    {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.neu.f32 p, %1, 0f00000000;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p),
+                     "f"(v)
+                     : "memory");
+    }
+};
+struct FixedAcc {
+    using T = long long;
+    unsigned long long *vol;
+    float scale;
+    __device__ __forceinline__ long long value(float v) const { return to_fixed(v * scale); }
+    __device__ __forceinline__ long long rest(float y, float r) const { return value(y * __fsub_rn(1.f, r)); }
+    static __device__ __forceinline__ void red(long long *p, long long v)
+    {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s64 p, %1, 0;\n\t@p red.global.add.u64 [%0], %1;\n\t}" ::"l"(p), "l"(v)
+                     : "memory");
+    }
+};
 
 // Plane offsets of ray z at a table row: the warp's, or (MIXED: the warp has
 // rising and falling rays) the ray's own.
@@ -493,22 +533,6 @@ __device__ __forceinline__ void col_planes(const ColTable &tab, int j, const uin
     } else {
         lo = __uint_as_float(te.z);
         hi = __uint_as_float(te.w);
-    }
-}
-
-// z split of a slab of a ray that is not steep: biased floor and low share.
-// (The grid has at most 2^20 rows and slabs, and such a ray moves at most one
-// row per slab: positions stay below 2^22, no clamp is needed for the floor.)
-template <bool REF>
-__device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &r)
-{
-    const float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
-    m = __fadd_rd(q, kFloorMagic);
-    if (REF) {
-        const float c = __fadd_rn(m, 1.f - kFloorMagic);
-        r = __saturatef(__fmul_rn(__fadd_rn(c, -q), rcp_approx(__fadd_rn(z_pos(z, zg, hi), -q))));
-    } else {
-        r = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
     }
 }
 
@@ -593,37 +617,38 @@ enum Merge { kSingle, kNear, kAny };
 // first one's low voxel w, so a slab takes at most three reductions per column
 // instead of four, and the lanes of a warp, two rows apart, rarely hit the
 // same voxel.
-template <int R, bool REF, bool MIXED, Merge MERGE, bool ZCHK>
+template <int R, bool REF, bool MIXED, Merge MERGE, bool ZCHK, class Acc>
 __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
-                                                 const float (&y)[R])
+                                                 const Acc &acc, const float (&y)[R])
 {
+    using T = typename Acc::T;
     const ZInside in(q.zg.nz);
     // values l, u of the low and high voxels of rays i.. in one voxel column
     constexpr int S = MERGE == kSingle ? 1 : 2;
-    auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], float (&l)[S], float (&u)[S]) {
+    auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], T (&l)[S], T (&u)[S]) {
         if (ZCHK) {
 #pragma unroll
             for (int k = 0; k < S; ++k) {
-                if (!in.low(m[k])) l[k] = 0.f;
-                if (!in.high(m[k])) u[k] = 0.f;
+                if (!in.low(m[k])) l[k] = (T)0;
+                if (!in.high(m[k])) u[k] = (T)0;
             }
         }
-        float *const p = col_voxel(lo, hi, m[0]);
+        T *const p = col_voxel<T>(lo, hi, m[0]);
         if constexpr (MERGE == kNear) {
             const bool same = m[0] == m[1];
             if (same) l[0] += l[1];
             u[0] += same ? u[1] : l[1];
-            if (!same) red_add(p + 2, u[1]);
+            if (!same) Acc::red(p + 2, u[1]);
         } else if constexpr (MERGE == kAny) {
             const bool same = m[0] == m[1], next = m[1] == m[0] + 1.f;
-            float *const s = col_voxel(lo, hi, m[1]);
-            l[0] += same ? l[1] : 0.f;
-            u[0] += same ? u[1] : next ? l[1] : 0.f;
-            if (!same && !next) red_add(s, l[1]);
-            if (!same) red_add(s + 1, u[1]);
+            T *const s = col_voxel<T>(lo, hi, m[1]);
+            l[0] += same ? l[1] : (T)0;
+            u[0] += same ? u[1] : next ? l[1] : (T)0;
+            if (!same && !next) Acc::red(s, l[1]);
+            if (!same) Acc::red(s + 1, u[1]);
         }
-        red_add(p, l[0]);
-        red_add(p + 1, u[0]);
+        Acc::red(p, l[0]);
+        Acc::red(p + 1, u[0]);
     };
 #pragma unroll 1
     for (int j = h.cross; j < h.n; ++j) {
@@ -631,17 +656,18 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
 #pragma unroll
         for (int i = 0; i < R; i += S) {
-            float lo, hi, m[S], l1[S], u1[S], l2[S], u2[S];
+            float lo, hi, m[S];
+            T l1[S], u1[S], l2[S], u2[S];
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 float r;
                 col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
                 z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
                 const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11), yk = y[i + k];
-                l1[k] = yk * w11;
-                u1[k] = yk * __fsub_rn(rv, w11);
-                l2[k] = yk * w21;
-                u2[k] = yk * __fsub_rn(ov, w21);
+                l1[k] = acc.value(yk * w11);
+                u1[k] = acc.value(yk * __fsub_rn(rv, w11));
+                l2[k] = acc.value(yk * w21);
+                u2[k] = acc.value(yk * __fsub_rn(ov, w21));
             }
             if (j < h.half) {
                 reduce(te.x, te.y, m, l1, u1);
@@ -658,14 +684,15 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         const uint4 te = tab.a[j];
 #pragma unroll
         for (int i = 0; i < R; i += S) {
-            float lo, hi, m[S], l[S], u[S];
+            float lo, hi, m[S];
+            T l[S], u[S];
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 float r;
                 col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
                 z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
-                l[k] = y[i + k] * r;
-                u[k] = __fmaf_rn(-y[i + k], r, y[i + k]);
+                l[k] = acc.value(y[i + k] * r);
+                u[k] = acc.rest(y[i + k], r);
             }
             reduce(te.x, te.y, m, l, u);
         }
@@ -674,14 +701,16 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
 
 // Transpose of the lane's R rays (not steep; y finite, 0 for a ray that takes
 // no part).
-template <int R, bool REF, bool MIXED, Merge MERGE>
-__device__ __forceinline__ void col_scatter(const ColRays<R> &q, float *acc, const float (&y)[R])
+template <int R, bool REF, bool MIXED, Merge MERGE, class Acc>
+__device__ __forceinline__ void col_scatter(const ColRays<R> &q, const Acc &acc, const float (&y)[R])
 {
     ColTable &tab = col_table();
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
-        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, acc, tab);
-        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1) col_scatter_rows<R, REF, MIXED, MERGE, false>(q, tab, h, y);
-        else col_scatter_rows<R, REF, MIXED, MERGE, true>(q, tab, h, y);
+        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, acc.vol, tab);
+        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1)
+            col_scatter_rows<R, REF, MIXED, MERGE, false>(q, tab, h, acc, y);
+        else
+            col_scatter_rows<R, REF, MIXED, MERGE, true>(q, tab, h, acc, y);
     }
 }
 

@@ -55,27 +55,6 @@ __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_con
     else ray_walk<false>(p.g, w, su, sv, sw, f);
 }
 
-// Column-warp variant: 64-bit fixed-point reductions into a z-fastest
-// accumulator (the same per-contribution integers as the thread walk, so the
-// integer sums and the result are bitwise the same).
-__global__ void __launch_bounds__(256) cb_colwarp_fixed_kernel(const __grid_constant__ CBParams<float> p)
-{
-    const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    const int tile = p.band_major ? blockIdx.z : blockIdx.y;
-    const int iv = p.band_major ? blockIdx.y : blockIdx.z;
-    if (ia >= p.na) return;                       // uniform across the warp
-    const int ib = tile * 32 + threadIdx.x;
-    float r[1][6];
-    const float y = ib < p.nb ? cb_sino_value(p, ia, ib, iv) : 0.f;
-    const bool has[1] = {ib < p.nb && y != 0.f};
-    cb_ray(p, ia, ib < p.nb ? ib : 0, iv, r[0]);
-    ColRays<1> q;
-    if (!col_rays<1>(p.g, r, has, p.flags, q)) return;
-    FixedSink f{p.fix, 1u, q.z[0].live ? y * q.W[0] : 0.f, *p.fix_scale};
-    if (ref_rounding(p.flags)) col_each<true>(q.c, q.K0, q.K1, q.z[0], q.zg, f);
-    else col_each<false>(q.c, q.K0, q.K1, q.z[0], q.zg, f);
-}
-
 // vol[z][y][x] = accZ[y][x][z] / scale (the integer sums of the column warps)
 __global__ void __launch_bounds__(256) fixed_zfold_kernel(const unsigned long long *__restrict__ acc, int nx, int ny,
                                                           int nz, const float *scale, float *__restrict__ vol)
@@ -489,7 +468,9 @@ static nefct_status cb_backward_fixed_impl(const nefct_cb_geom *g, const float *
     float *scale = (float *)(w + 16);
     unsigned long long *accN = (unsigned long long *)(w + 256);
     unsigned long long *accT = tr ? accN + nvox : nullptr;
-    NEFCT_CHECK_CUDA(cudaMemsetAsync(w, 0, need, s));
+    // column warps reduce everything into accN in z-fastest order
+    const bool cw = tr && cb_use_colwarp<float>(g->grid, flags & ~NEFCT_DETERMINISTIC, false);
+    NEFCT_CHECK_CUDA(cudaMemsetAsync(w, 0, cw ? 256 + nvox * sizeof(unsigned long long) : need, s));
     const size_t ns = (size_t)g->na * g->nb * g->nv;
     maxabs_kernel<<<(unsigned)std::min<size_t>((ns + 255) / 256, 148 * 16), 256, 0, s>>>(sino, ns, maxbits);
     NEFCT_CHECK_LAUNCH("maxabs_kernel");
@@ -501,18 +482,17 @@ static nefct_status cb_backward_fixed_impl(const nefct_cb_geom *g, const float *
     p.fix = accN;
     p.fixT = accT;
     p.fix_scale = scale;
-    // column warps reduce everything into accN in z-fastest order
-    const bool cw = tr && cb_use_colwarp<float>(g->grid, flags & ~NEFCT_DETERMINISTIC, false);
     for (int v0 = 0; v0 < g->nv; v0 += ViewTable<float>::kMax) {
         const int nvc = std::min(ViewTable<float>::kMax, g->nv - v0);
         fill_views(p, g, v0, nvc);
-        dim3 grid, block;
         if (cw) {
-            cb_colwarp_shape(p, g->na, g->nb, nvc, grid, block);
-            cb_colwarp_fixed_kernel<<<grid, block, 0, s>>>(p);
-            NEFCT_CHECK_LAUNCH("cb_colwarp_fixed_kernel");
+            // the same per-contribution integers as the thread walk's, so the
+            // sums and the result are bitwise the same
+            const cudaError_t e = cb_launch_backward_fixed(p, g->na, g->nb, nvc, flags, s);
+            if (e != cudaSuccess) return cuda_fail(e, "cb_colwarp_backward_kernel (fixed)");
             continue;
         }
+        dim3 grid, block;
         cb_shape(p, g->na, g->nb, nvc, grid, block);
         cb_backward_fixed_kernel<<<grid, block, 0, s>>>(p);
         NEFCT_CHECK_LAUNCH("cb_backward_fixed_kernel");
