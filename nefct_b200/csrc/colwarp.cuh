@@ -636,16 +636,16 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         T *const p = col_voxel<T>(lo, hi, m[0]);
         if constexpr (MERGE == kNear) {
             const bool same = m[0] == m[1];
-            if (same) l[0] += l[1];
+            l[0] += same ? l[1] : (T)0;
             u[0] += same ? u[1] : l[1];
-            if (!same) Acc::red(p + 2, u[1]);
+            Acc::red(p + 2, same ? (T)0 : u[1]);
         } else if constexpr (MERGE == kAny) {
             const bool same = m[0] == m[1], next = m[1] == m[0] + 1.f;
             T *const s = col_voxel<T>(lo, hi, m[1]);
             l[0] += same ? l[1] : (T)0;
             u[0] += same ? u[1] : next ? l[1] : (T)0;
-            if (!same && !next) Acc::red(s, l[1]);
-            if (!same) Acc::red(s + 1, u[1]);
+            Acc::red(s, same || next ? (T)0 : l[1]);
+            Acc::red(s + 1, same ? (T)0 : u[1]);
         }
         Acc::red(p, l[0]);
         Acc::red(p + 1, u[0]);

@@ -288,9 +288,9 @@ __device__ __forceinline__ void dd_rows(const DDTable &tab, int single, int n, i
                 if constexpr (MODE == kInner || MODE == kChecked) {
                     // row 1's lowest voxel is row 0's or the one above
                     const bool same = m[0] == m[1];
-                    if (same) v[0][0] += v[1][0];
+                    v[0][0] += same ? v[1][0] : 0.f;
                     v[0][1] += same ? v[1][1] : v[1][0];
-                    if (!same) FloatAcc::red(p + 2, v[1][1]);
+                    FloatAcc::red(p + 2, same ? 0.f : v[1][1]);
                 } else {
                     float *const q = col_voxel(lo, hi, m[1]);
 #pragma unroll

@@ -123,54 +123,164 @@ __global__ void __launch_bounds__(256) fixed_fold_kernel(const unsigned long lon
 
 // ---------------- LOR projector pair (cpp/siddon) ----------------
 
-template <typename T> struct LorParams {
-    GridDev<T> g;
-    const T *lors;
+struct LorParams {
+    GridDev<float> g;
+    const float *lors;
     long long n;
     uint32_t flags;
-    const T *vol;
-    const T *vals;
-    T *out;
+    const float *vol;
+    const float *vals;
+    float *out;
     const int32_t *order;     // walk order (a permutation of 0..n-1), or nullptr
 };
+
+// A line's walk: the general walk's operations (siddon.cuh) with the slope
+// signs as run-time selects instead of template variants, which keeps the
+// kernels under 64 registers and a warp's lines of different signs together
+// (the variants took 100 to 116 registers, so half the warps to hide the
+// gathers' latency with, and ran one after the other).  256^3, 4 Mi ring lines
+// in walk order: forward 4.11 -> 2.99 ms, bound by the gathers' requests (12
+// sectors each), backward 4.64 -> 4.68 ms, by the L2's rate of scattered
+// reductions (1.9e11/s); in list order 22.8 -> 2.95 and 15.8 -> 4.47 ms.  A
+// y-fastest copy for one of the driving axes, either way round, is slower:
+// 3.5 and 7 to 9 ms (neighbouring lines then reduce into the same sectors).
+// Index of voxel (k, v, z): base + k su + v sv + z sw, floors biased.
+struct LineWalk {
+    float pv, kv, dv, nv2, pw, kw, dz, nz2, pu, t, qv, mv, qz, mz;
+    unsigned su, sv, sw, base;
+    int nv, nz;
+    bool vdown, zdown, vdiv, zdiv;
+
+    __device__ __forceinline__ void plane(float tt, float &v, float &z) const
+    {
+        const float d = __fsub_rn(tt, pu);
+        v = __fadd_rn(pv, __fmul_rn(kv, d));
+        z = __fadd_rn(pw, __fmul_rn(kw, d));
+        if (vdiv) v = __fdiv_rn(v, dv);
+        if (zdiv) z = __fdiv_rn(z, dz);
+        v = __fadd_rn(v, nv2);
+        z = __fadd_rn(z, nz2);
+    }
+
+    __device__ __forceinline__ LineWalk(const GridDev<float> &g, const Walk<float> &w)
+        : pv(w.pv), kv(w.kv), dv(w.dv), nv2(w.nv2), pw(w.pw), kw(w.kw), dz(g.dz), nz2(g.nz2), pu(w.pu),
+          su(w.xdrive ? 1u : (unsigned)g.nx), sv(w.xdrive ? (unsigned)g.nx : 1u), sw((unsigned)g.nx * (unsigned)g.ny), nv(w.nv), nz(g.nz), vdown(w.kv < 0.f), zdown(w.kw < 0.f), vdiv(w.vdiv),
+          zdiv(g.dz != 1.f)
+    {
+        t = __fsub_rn((float)w.k0, w.nu2);
+        base = (unsigned)w.k0 * su - (unsigned)kFloorMagicBits * (sv + sw);
+        plane(t, qv, qz);
+        mv = magic_floor<true>(qv);
+        mz = magic_floor<true>(qz);
+    }
+
+    template <bool CHECK> __device__ __forceinline__ SlabSlots<float> next()
+    {
+        t = __fadd_rn(t, 1.f);
+        float bv, bz;
+        plane(t, bv, bz);
+        const float nv_ = magic_floor<CHECK>(bv), nz_ = magic_floor<CHECK>(bz);
+        const float q1v = vdown ? bv : qv, q2v = vdown ? qv : bv, m1v = vdown ? nv_ : mv, m2v = vdown ? mv : nv_;
+        const float q1z = zdown ? bz : qz, q2z = zdown ? qz : bz, m1z = zdown ? nz_ : mz, m2z = zdown ? mz : nz_;
+        qv = bv; qz = bz; mv = nv_; mz = nz_;
+        const bool vx = m1v != m2v, wx = m1z != m2z;
+        const float rv = vx ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2v, -kFloorMagic), -q1v), __fadd_rn(q2v, -q1v)) : 1.f;
+        const float rw = wx ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2z, -kFloorMagic), -q1z), __fadd_rn(q2z, -q1z)) : 1.f;
+        const bool vfirst = rv > rw;
+        const unsigned i1 = base + (unsigned)__float_as_int(m1v) * sv, i2 = base + (unsigned)__float_as_int(m2v) * sv;
+        const unsigned j1 = (unsigned)__float_as_int(m1z) * sw, j2 = (unsigned)__float_as_int(m2z) * sw;
+        base += su;
+        SlabSlots<float> s;
+        s.r[0] = fminf(rv, rw);
+        s.r[1] = fabsf(__fsub_rn(rv, rw));
+        s.r[2] = __fsub_rn(1.f, fmaxf(rv, rw));
+        s.idx[0] = i1 + j1;
+        s.idx[1] = vfirst ? i1 + j2 : i2 + j1;
+        s.idx[2] = i2 + j2;
+        s.mid3 = vx && wx;
+        s.ok[0] = true;
+        s.ok[1] = vx || wx;
+        s.ok[2] = vx && wx;
+        if (CHECK) {
+            const int cv1 = __float_as_int(m1v) - kFloorMagicBits, cv2 = __float_as_int(m2v) - kFloorMagicBits;
+            const int cw1 = __float_as_int(m1z) - kFloorMagicBits, cw2 = __float_as_int(m2z) - kFloorMagicBits;
+            const bool adm = (unsigned)(cv1 + (int)vx) < (unsigned)(nv + (int)vx) &&
+                             (unsigned)(cw1 + (int)wx) < (unsigned)(nz + (int)wx);
+            const int v = vfirst ? cv1 : cv2, z = vfirst ? cw2 : cw1;
+            s.ok[0] = adm && (cv1 | cw1) >= 0;
+            s.ok[1] = adm && s.ok[1] && (unsigned)v < (unsigned)nv && (unsigned)z < (unsigned)nz;
+            s.ok[2] = adm && s.ok[2] && cv2 < nv && cw2 < nz;
+        }
+        return s;
+    }
+};
+
+// Calls f(slots) for the slabs k0..k1 of the line, those outside [ki0, ki1]
+// range checked.
+template <class Fn> __device__ __forceinline__ void line_walk(LineWalk &l, const Walk<float> &w, Fn &f)
+{
+    const int a = w.ki0 <= w.ki1 ? w.ki0 : w.k1 + 1, b = w.ki0 <= w.ki1 ? w.ki1 : w.k1;
+    int k = w.k0;
+#pragma unroll 1
+    for (; k < a; ++k) f(l.next<true>());
+#pragma unroll 2
+    for (; k <= b; ++k) f(l.next<false>());
+#pragma unroll 1
+    for (; k <= w.k1; ++k) f(l.next<true>());
+}
 
 // The walk visits lines in `order` so that a warp's 32 lines are nearly
 // parallel neighbours (similar trip counts, nearby voxels); results stay at
 // each line's own index.
-template <typename T, bool DIV, bool Q5>
-__global__ void __launch_bounds__(256) lor_forward_kernel(const __grid_constant__ LorParams<T> p)
+template <bool Q5>
+__global__ void __launch_bounds__(256, 4) lor_forward_kernel(const __grid_constant__ LorParams p)
 {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < p.n;
          t += (long long)gridDim.x * blockDim.x) {
         const long long i = p.order ? (long long)p.order[t] : t;
-        T r[6];
+        float r[6];
         for (int j = 0; j < 6; ++j) r[j] = p.lors[j * p.n + i];
-        Walk<T> w;
-        T acc = (T)0;
+        Walk<float> w;
+        float sum = 0.f;
         if (setup_walk(p.g, r, p.flags, w)) {
-            const int sw = p.g.nx * p.g.ny;
-            acc = w.xdrive ? gather_walk<T, DIV, false, Q5>(w, p.g, p.vol, 1, p.g.nx, sw)
-                           : gather_walk<T, DIV, true, Q5>(w, p.g, p.vol, p.g.nx, 1, sw);
+            LineWalk l(p.g, w);
+            float acc = 0.f, mid = 0.f;
+            auto f = [&](const SlabSlots<float> &s) {
+                const float v0 = s.ok[0] ? __ldg(p.vol + s.idx[0]) : 0.f;
+                const float v1 = s.ok[1] ? __ldg(p.vol + s.idx[1]) : 0.f;
+                const float v2 = s.ok[2] ? __ldg(p.vol + s.idx[2]) : 0.f;
+                acc += v0 * s.r[0];
+                if (Q5 && s.mid3) mid += v1 * s.r[1];
+                else acc += v1 * s.r[1];
+                acc += v2 * s.r[2];
+            };
+            line_walk(l, w, f);
+            sum = Q5 ? acc * w.W + mid * w.Wmid : acc * w.W;
         }
-        p.out[i] = acc;
+        p.out[i] = sum;
     }
 }
 
-template <typename T, bool DIV, bool Q5>
-__global__ void __launch_bounds__(256) lor_backward_kernel(const __grid_constant__ LorParams<T> p)
+template <bool Q5>
+__global__ void __launch_bounds__(256, 4) lor_backward_kernel(const __grid_constant__ LorParams p)
 {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < p.n;
          t += (long long)gridDim.x * blockDim.x) {
         const long long i = p.order ? (long long)p.order[t] : t;
-        const T y = p.vals[i];
-        if (y == (T)0) continue;
-        T r[6];
+        const float y = p.vals[i];
+        if (y == 0.f) continue;
+        float r[6];
         for (int j = 0; j < 6; ++j) r[j] = p.lors[j * p.n + i];
-        Walk<T> w;
+        Walk<float> w;
         if (!setup_walk(p.g, r, p.flags, w)) continue;
-        const int sw = p.g.nx * p.g.ny;
-        if (w.xdrive) scatter_walk<T, DIV, false, Q5>(w, p.g, p.out, 1, p.g.nx, sw, y);
-        else scatter_walk<T, DIV, true, Q5>(w, p.g, p.out, p.g.nx, 1, sw, y);
+        LineWalk l(p.g, w);
+        const float yw = y * w.W, ym = y * w.Wmid;
+        auto f = [&](const SlabSlots<float> &s) {
+            if (s.ok[0]) atomicAdd(p.out + s.idx[0], yw * s.r[0]);
+            if (s.ok[1]) atomicAdd(p.out + s.idx[1], ((Q5 && s.mid3) ? ym : yw) * s.r[1]);
+            if (s.ok[2]) atomicAdd(p.out + s.idx[2], yw * s.r[2]);
+        };
+        line_walk(l, w, f);
     }
 }
 
@@ -178,7 +288,7 @@ __global__ void __launch_bounds__(256) lor_backward_kernel(const __grid_constant
 // direction folded to [0, pi), signed distance of the in-plane line from the
 // grid centre, z where the line passes the centre, and z slope.  Lines with
 // equal keys are nearly parallel neighbours.
-__global__ void __launch_bounds__(256) lor_key_kernel(const __grid_constant__ LorParams<float> p, int32_t *keys)
+__global__ void __launch_bounds__(256) lor_key_kernel(const __grid_constant__ LorParams p, int32_t *keys)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -556,8 +666,7 @@ static nefct_status cb_backward_impl(const nefct_cb_geom *g, const T *sino, T *v
     return NEFCT_OK;
 }
 
-template <typename T>
-static nefct_status lor_impl(const nefct_grid *grid, const T *lors, int64_t n, const T *src, T *dst,
+static nefct_status lor_impl(const nefct_grid *grid, const float *lors, int64_t n, const float *src, float *dst,
                              uint32_t flags, cudaStream_t s, bool forward, const int32_t *order = nullptr)
 {
     if (!grid) return fail(NEFCT_ERR_INVALID, "grid is NULL");
@@ -570,34 +679,28 @@ static nefct_status lor_impl(const nefct_grid *grid, const T *lors, int64_t n, c
     if (flags & ~kWalkFlags) return fail(NEFCT_ERR_INVALID, "unknown flag bits 0x%x", flags & ~kWalkFlags);
     if (forward && n == 0) return NEFCT_OK;          // no lines: nothing to write
     if (!dst) return fail(NEFCT_ERR_INVALID, "NULL output");
-    LorParams<T> p;
-    p.g = make_grid_dev<T>(*grid);
+    const size_t bytes = (size_t)grid->nx * grid->ny * grid->nz * sizeof(float);
+    LorParams p{};
+    p.g = make_grid_dev<float>(*grid);
     p.lors = lors; p.n = n; p.flags = flags; p.order = order;
     if (n >= (1ll << 31) && order) return fail(NEFCT_ERR_INVALID, "ordered walks take fewer than 2^31 lines");
+    p.out = dst;
     if (!forward) {
-        const size_t nvox = (size_t)grid->nx * grid->ny * grid->nz;
-        NEFCT_CHECK_CUDA(cudaMemsetAsync(dst, 0, nvox * sizeof(T), s));
-        p.vals = src; p.out = dst; p.vol = nullptr;
+        NEFCT_CHECK_CUDA(cudaMemsetAsync(dst, 0, bytes, s));
+        p.vals = src;
     } else {
-        p.vol = src; p.out = dst; p.vals = nullptr;
+        p.vol = src;
     }
     if (n == 0) return NEFCT_OK;
-    const long long blocks = std::min<long long>((n + 255) / 256, 148ll * 64);
-    const bool q5 = (flags & NEFCT_Q5) != 0, cub = cubic(p.g);
-#define NEFCT_LOR_LAUNCH(K)                                                              \
-    do {                                                                                 \
-        if (cub && !q5) K<T, false, false><<<(unsigned)blocks, 256, 0, s>>>(p);          \
-        else if (cub) K<T, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);             \
-        else if (!q5) K<T, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);             \
-        else K<T, true, true><<<(unsigned)blocks, 256, 0, s>>>(p);                       \
-    } while (0)
-    if (forward) NEFCT_LOR_LAUNCH(lor_forward_kernel);
-    else NEFCT_LOR_LAUNCH(lor_backward_kernel);
-#undef NEFCT_LOR_LAUNCH
+    const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148ll * 64);
+    const bool q5 = (flags & NEFCT_Q5) != 0;
+    if (forward && q5) lor_forward_kernel<true><<<blocks, 256, 0, s>>>(p);
+    else if (forward) lor_forward_kernel<false><<<blocks, 256, 0, s>>>(p);
+    else if (q5) lor_backward_kernel<true><<<blocks, 256, 0, s>>>(p);
+    else lor_backward_kernel<false><<<blocks, 256, 0, s>>>(p);
     NEFCT_CHECK_LAUNCH(forward ? "lor_forward_kernel" : "lor_backward_kernel");
     return NEFCT_OK;
 }
-
 
 // ---------------- forward projection for callers that cannot allocate ----------------
 //
@@ -798,13 +901,13 @@ nefct_status nefct_cb_count_intersections(const nefct_cb_geom *g, uint32_t flags
 nefct_status nefct_lor_forward(const nefct_grid *grid, const float *lors, int64_t n, const float *vol,
                                float *out, uint32_t flags, void *stream)
 {
-    return lor_impl<float>(grid, lors, n, vol, out, flags, (cudaStream_t)stream, true);
+    return lor_impl(grid, lors, n, vol, out, flags, (cudaStream_t)stream, true);
 }
 
 nefct_status nefct_lor_backward(const nefct_grid *grid, const float *lors, int64_t n, const float *vals,
                                 float *vol, uint32_t flags, void *stream)
 {
-    return lor_impl<float>(grid, lors, n, vals, vol, flags, (cudaStream_t)stream, false);
+    return lor_impl(grid, lors, n, vals, vol, flags, (cudaStream_t)stream, false);
 }
 
 nefct_status nefct_lor_order_keys(const nefct_grid *grid, const float *lors, int64_t n, int32_t *keys, void *stream)
@@ -815,7 +918,7 @@ nefct_status nefct_lor_order_keys(const nefct_grid *grid, const float *lors, int
     if (n < 0 || n >= (1ll << 31)) return fail(NEFCT_ERR_INVALID, "line count must be in [0, 2^31)");
     if (n == 0) return NEFCT_OK;
     if (!lors || !keys) return fail(NEFCT_ERR_INVALID, "NULL buffer");
-    LorParams<float> p{};
+    LorParams p{};
     p.g = make_grid_dev<float>(*grid);
     p.lors = lors;
     p.n = n;
@@ -829,14 +932,14 @@ nefct_status nefct_lor_forward_ordered(const nefct_grid *grid, const float *lors
                                        const float *vol, float *out, uint32_t flags, void *stream)
 {
     if (!order && n > 0) return fail(NEFCT_ERR_INVALID, "order is NULL");
-    return lor_impl<float>(grid, lors, n, vol, out, flags, (cudaStream_t)stream, true, order);
+    return lor_impl(grid, lors, n, vol, out, flags, (cudaStream_t)stream, true, order);
 }
 
 nefct_status nefct_lor_backward_ordered(const nefct_grid *grid, const float *lors, int64_t n, const int32_t *order,
                                         const float *vals, float *vol, uint32_t flags, void *stream)
 {
     if (!order && n > 0) return fail(NEFCT_ERR_INVALID, "order is NULL");
-    return lor_impl<float>(grid, lors, n, vals, vol, flags, (cudaStream_t)stream, false, order);
+    return lor_impl(grid, lors, n, vals, vol, flags, (cudaStream_t)stream, false, order);
 }
 
 // See cb_forward_static_impl: the same kernels and result as
