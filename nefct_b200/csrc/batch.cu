@@ -53,7 +53,7 @@ struct BatchDesc {
     GridDev<float> g;
     RayGeom<float> rg;
     int na, nb, nv, tiles_a, tiles_b;
-    int near;                            // pairs of neighbouring rows merge their reductions (col_rows_near)
+    int near;                            // pairs of neighbouring rows merge their reductions (col_rows_next)
     uint32_t flags;
     const float *cs, *sn, *off;          // per-view tables in the workspace
     const float *vol;
@@ -402,7 +402,7 @@ nefct_status nefct_cb_batch_plan(const nefct_cb_problem *problems, int32_t n, ui
         D.na = g.na; D.nb = g.nb; D.nv = g.nv;
         D.tiles_a = b->colwarp ? (g.na + b->rows - 1) / b->rows : (g.na + 31) / 32;
         D.tiles_b = b->colwarp ? (g.nb + 63) / 64 : (g.nb + b->rows - 1) / b->rows;
-        D.near = col_rows_near(D.g, D.rg);
+        D.near = col_rows_next(D.g, D.rg, D.nb) > 1;
         D.flags = flags;
         b->t0[k + 1] = b->t0[k] + (long long)D.tiles_a * D.tiles_b * g.nv;
         b->c0[k + 1] = b->c0[k] + (long long)((g.grid.nx + 31) / 32) * ((g.grid.nz + 31) / 32) * g.grid.ny;

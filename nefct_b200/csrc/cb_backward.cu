@@ -7,7 +7,7 @@ namespace nefct {
 // Column warps: one warp per 32 R rows of column ia at view iv, into the
 // z-fastest accumulator p.outT (FIXED: the deterministic transpose's integers
 // p.fix).
-template <int R, bool REF, bool PAIR, bool FIXED>
+template <int R, bool REF, bool NEXT, bool FIXED>
 __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __grid_constant__ CBParams<float> p)
 {
     const int ia = blockIdx.x * blockDim.y + threadIdx.y;
@@ -18,30 +18,34 @@ __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __gri
     bool has[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        const int ib = col_row<R, PAIR>(tile, threadIdx.x, i, p.rg.db < 0.f);
+        const int ib = col_row<R, NEXT>(tile, threadIdx.x, i, p.rg.db < 0.f);
         has[i] = ib < p.nb;
         y[i] = has[i] ? cb_sino_value(p, ia, ib, iv) : 0.f;
         cb_ray(p, ia, has[i] ? ib : 0, iv, r[i]);
     }
-    if constexpr (FIXED) colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, FixedAcc{p.fix, *p.fix_scale});
-    else colwarp_backward<R, REF, PAIR>(p.g, r, has, p.flags, y, FloatAcc{p.outT});
+    if constexpr (FIXED) colwarp_backward<R, REF, NEXT>(p.g, r, has, p.flags, y, FixedAcc{p.fix, *p.fix_scale});
+    else colwarp_backward<R, REF, NEXT>(p.g, r, has, p.flags, y, FloatAcc{p.outT});
 }
 
-template <int R, bool PAIR, bool FIXED>
+template <int R, bool FIXED>
 static cudaError_t launch_colwarp(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
 {
     dim3 grid, block;
     cb_colwarp_shape(p, na, nb, nvc, grid, block, R);
-    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, PAIR, FIXED><<<grid, block, 0, s>>>(p);
-    else cb_colwarp_backward_kernel<R, false, PAIR, FIXED><<<grid, block, 0, s>>>(p);
+    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, (R > 1), FIXED><<<grid, block, 0, s>>>(p);
+    else cb_colwarp_backward_kernel<R, false, (R > 1), FIXED><<<grid, block, 0, s>>>(p);
     return cudaGetLastError();
 }
 
 template <bool FIXED>
 static cudaError_t launch_rows(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
 {
-    return col_rows_near(p.g, p.rg) ? launch_colwarp<2, true, FIXED>(p, na, nb, nvc, flags, s)
-                                    : launch_colwarp<1, false, FIXED>(p, na, nb, nvc, flags, s);
+    switch (col_rows_next(p.g, p.rg, nb)) {
+    case 1: return launch_colwarp<1, FIXED>(p, na, nb, nvc, flags, s);
+    case 2: return launch_colwarp<2, FIXED>(p, na, nb, nvc, flags, s);
+    case 3: return launch_colwarp<3, FIXED>(p, na, nb, nvc, flags, s);
+    default: return launch_colwarp<4, FIXED>(p, na, nb, nvc, flags, s);
+    }
 }
 
 cudaError_t cb_launch_backward_fixed(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)

@@ -16,6 +16,7 @@
 #pragma once
 
 #include <math.h>
+#include <algorithm>
 #include <type_traits>
 
 #include "colwarp.cuh"
@@ -226,9 +227,9 @@ __device__ __forceinline__ ScatterSink ray_sink(const FloatAcc &a, float yw) { r
 __device__ __forceinline__ FixedSink ray_sink(const FixedAcc &a, float yw) { return FixedSink{a.vol, 1u, yw, a.scale}; }
 
 // Transpose of R rows per lane of one detector column: y[i] times the ray's
-// weights into the z-fastest accumulator acc.  PAIR: rows 2i and 2i + 1 are
-// neighbours in z order and merge their reductions.
-template <int R, bool REF, bool PAIR, class Acc>
+// weights into the z-fastest accumulator acc.  NEXT: the rows are neighbours
+// in z order and merge their reductions.
+template <int R, bool REF, bool NEXT, class Acc>
 __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const float (&r)[R][6], bool (&has)[R],
                                                  uint32_t flags, const float (&y)[R], const Acc &acc)
 {
@@ -252,28 +253,39 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
         return;
     }
     const bool mixed = q.rising && q.falling;
-    if constexpr (PAIR) {
-        // the gap between two rays is linear along the walk: in [0, 1) at both
-        // ends, by more than the positions' rounding, it is so in every slab
-        const float d0 = col_plane(q.c, q.K0), d1 = col_plane(q.c, q.K1 + 1);
-        bool near = true;
+    if constexpr (NEXT) {
+        // a row that takes no part walks along with a neighbour, with value 0
+        bool copy[R];
 #pragma unroll
-        for (int i = 0; i < R; i += 2) {
-            ZRay &z0 = q.z[i], &z1 = q.z[i + 1];
-            if (z0.live && z1.live) {
-                const float dk = z1.kz - z0.kz, dz = z1.z0 - z0.z0;
-                const float g0 = fmaf(dk, d0, dz), g1 = fmaf(dk, d1, dz);
-                const float m = 1e-3f + 1e-6f * (fabsf(z0.z0) + fabsf(z0.kz) * (fabsf(q.c.pu) + fabsf(q.c.nu2)));
-                near = near && fminf(g0, g1) > m && fmaxf(g0, g1) < 1.f - m;
-            } else if (z0.live) {                  // one ray of the pair: the other walks along with value 0
-                z1 = z0;
-                z1.live = false;
-            } else if (z1.live) {
-                z0 = z1;
-                z0.live = false;
+        for (int i = 0; i < R; ++i) {
+            copy[i] = !q.z[i].live;
+            if (i > 0 && copy[i]) {
+                q.z[i] = q.z[i - 1];
+                q.z[i].live = false;
             }
         }
-        if (!__all_sync(0xffffffffu, near)) col_scatter<R, REF, true, kAny>(q, acc, yw);
+#pragma unroll
+        for (int i = R - 2; i >= 0; --i)
+            if (copy[i] && (i == 0 || copy[i - 1])) {
+                q.z[i] = q.z[i + 1];
+                q.z[i].live = false;
+            }
+        // the gap between two rays is linear along the walk: in order, and
+        // within a voxel of the first ray, at both ends, by more than the
+        // positions' rounding, it is so in every slab
+        const float d0 = col_plane(q.c, q.K0), d1 = col_plane(q.c, q.K1 + 1);
+        const float m = 1e-3f + 1e-6f * (fabsf(q.z[0].z0) + fabsf(q.z[0].kz) * (fabsf(q.c.pu) + fabsf(q.c.nu2)));
+        bool near = true;
+#pragma unroll
+        for (int i = 1; i < R; ++i) {
+            const float a = fmaf(q.z[i].kz - q.z[i - 1].kz, d0, q.z[i].z0 - q.z[i - 1].z0);
+            const float b = fmaf(q.z[i].kz - q.z[i - 1].kz, d1, q.z[i].z0 - q.z[i - 1].z0);
+            near = near && (copy[i] || copy[i - 1] ? fminf(a, b) >= 0.f : fminf(a, b) > m);
+        }
+        const float a = fmaf(q.z[R - 1].kz - q.z[0].kz, d0, q.z[R - 1].z0 - q.z[0].z0);
+        const float b = fmaf(q.z[R - 1].kz - q.z[0].kz, d1, q.z[R - 1].z0 - q.z[0].z0);
+        near = near && fmaxf(a, b) < 1.f - m;
+        if (!__all_sync(0xffffffffu, near)) col_scatter<R, REF, true, R == 2 ? kAny : kSingle>(q, acc, yw);
         else if (mixed) col_scatter<R, REF, true, kNear>(q, acc, yw);
         else col_scatter<R, REF, false, kNear>(q, acc, yw);
     } else {
@@ -283,12 +295,11 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
 }
 
 // Row i of lane `lane` in row tile `tile` of a column warp with R rows per
-// lane: rows 32 apart, or (PAIR) rows 2i and 2i + 1 neighbours, in z order
-// (rows fall in z when their pitch is negative).
-template <int R, bool PAIR> __device__ __forceinline__ int col_row(int tile, int lane, int i, bool falling)
+// lane: rows 32 apart, or (NEXT) neighbours, in z order (rows fall in z when
+// the row pitch is negative).
+template <int R, bool NEXT> __device__ __forceinline__ int col_row(int tile, int lane, int i, bool falling)
 {
-    return PAIR ? tile * 32 * R + (i >> 1) * 64 + lane * 2 + (falling ? 1 - (i & 1) : (i & 1))
-                : (tile * R + i) * 32 + lane;
+    return NEXT ? (tile * 32 + lane) * R + (falling ? R - 1 - i : i) : (tile * R + i) * 32 + lane;
 }
 
 // Launch shape of the thread walk for nvc views (see cb_cell).
@@ -318,15 +329,29 @@ static inline void cb_colwarp_shape(CBParams<T> &p, int na, int nb, int nvc, dim
 // The walk skips its divisions when both transverse pitches equal the x pitch.
 template <typename T> static inline bool cubic(const GridDev<T> &g) { return g.dy == (T)1 && g.dz == (T)1; }
 
-// Whether neighbouring rows of a column are close enough, at the rotation
-// axis, for pairs of them to share reductions.  Rows further apart rarely meet
-// in a voxel, and 32 consecutive rows per warp then touch fewer sectors than
-// 32 pairs.  256^3, 24 views, pitch 0.7 / 0.85 / 0.95 / 1.1 voxels at the
-// axis: pairs 0.95 / 0.84 / 0.71 / 0.74 ms, single rows 1.27 / 0.91 / 0.67 /
-// 0.55 ms.
-static inline bool col_rows_near(const GridDev<float> &g, const RayGeom<float> &rg)
+// Neighbouring rows per lane that share the transpose's reductions.
+//  * 1 while the row pitch at the rotation axis is 0.9 voxel or more: rows that
+//    far apart rarely meet in a voxel, and 32 consecutive rows per warp then
+//    touch fewer sectors than 32 pairs (256^3, 24 views, pitch 0.7 / 0.85 /
+//    0.95 / 1.1 voxels: pairs 0.95 / 0.84 / 0.71 / 0.74 ms, single rows 1.27 /
+//    0.91 / 0.67 / 0.55 ms);
+//  * else two, or up to four if so many stay within a voxel at the far side of
+//    the grid (thick slices), whichever covers the nb rows with the fewest slab
+//    steps: a warp of 32 R rows takes about 1 / 1.45 / 1.85 times as long with R
+//    = 2 / 3 / 4 (200 x 200 x 44 voxels of 2.5 mm, 60 views: 77 rows 0.50 / 0.38
+//    / - ms, 120 rows 0.50 / 0.65 / 0.46 ms).
+static inline int col_rows_next(const GridDev<float> &g, const RayGeom<float> &rg, int nb)
 {
-    return rg.src_iso > 0.f && rg.src_det > 0.f && fabsf(rg.db) * rg.src_iso / rg.src_det < 0.9f * g.dz * g.dx_;
+    if (!(rg.src_iso > 0.f && rg.src_det > 0.f)) return 1;
+    const double rad = 0.5 * sqrt((double)g.nx * g.nx + (double)g.ny * g.dy * g.ny * g.dy) * g.dx_;
+    const double pitch = fabs((double)rg.db) / rg.src_det / ((double)g.dz * g.dx_);       // voxels per unit distance
+    if (pitch * rg.src_iso >= 0.9) return 1;
+    const int most = std::min(4.0, 1.0 + 0.98 / (pitch * (rg.src_iso + rad)));
+    const int cost[5] = {0, 0, 100, 145, 185};
+    int best = 2;
+    for (int r = 3; r <= most; ++r)
+        if ((nb + 32 * r - 1) / (32 * r) * cost[r] < (nb + 32 * best - 1) / (32 * best) * cost[best]) best = r;
+    return best;
 }
 
 // Column warps apply to FP32 slab walks with a workspace; the z-fastest

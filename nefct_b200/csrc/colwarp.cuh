@@ -607,16 +607,16 @@ __device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__r
     }
 }
 
-// How the transpose's rays 2i and 2i + 1 share reductions: not at all; as
-// neighbours, the second 0 to 1 voxel above the first in every slab; as
-// neighbours at any distance.
+// How the transpose's R rays of a lane share reductions: not at all; as
+// neighbours, in z order and all within less than a voxel of the first one in
+// every slab; as two neighbours at any distance.
 enum Merge { kSingle, kNear, kAny };
 
-// Transpose of one chunk's table rows.  Two neighbouring rays' shares of a
-// voxel column are summed in registers over the voxels w, w + 1, w + 2 of the
-// first one's low voxel w, so a slab takes at most three reductions per column
-// instead of four, and the lanes of a warp, two rows apart, rarely hit the
-// same voxel.
+// Transpose of one chunk's table rows.  Neighbouring rays' shares of a voxel
+// column are summed in registers over the voxels w, w + 1, w + 2 of the first
+// one's low voxel w, so a slab takes at most three reductions per column
+// instead of two per ray, and the lanes of a warp, R rows apart, rarely hit
+// the same voxel.
 template <int R, bool REF, bool MIXED, Merge MERGE, bool ZCHK, class Acc>
 __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
                                                  const Acc &acc, const float (&y)[R])
@@ -624,7 +624,7 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
     using T = typename Acc::T;
     const ZInside in(q.zg.nz);
     // values l, u of the low and high voxels of rays i.. in one voxel column
-    constexpr int S = MERGE == kSingle ? 1 : 2;
+    constexpr int S = MERGE == kSingle ? 1 : R;
     auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], T (&l)[S], T (&u)[S]) {
         if (ZCHK) {
 #pragma unroll
@@ -635,10 +635,15 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         }
         T *const p = col_voxel<T>(lo, hi, m[0]);
         if constexpr (MERGE == kNear) {
-            const bool same = m[0] == m[1];
-            l[0] += same ? l[1] : (T)0;
-            u[0] += same ? u[1] : l[1];
-            Acc::red(p + 2, same ? (T)0 : u[1]);
+            T top = (T)0;
+#pragma unroll
+            for (int k = 1; k < S; ++k) {
+                const bool same = m[0] == m[k];
+                l[0] += same ? l[k] : (T)0;
+                u[0] += same ? u[k] : l[k];
+                top += same ? (T)0 : u[k];
+            }
+            Acc::red(p + 2, top);
         } else if constexpr (MERGE == kAny) {
             const bool same = m[0] == m[1], next = m[1] == m[0] + 1.f;
             T *const s = col_voxel<T>(lo, hi, m[1]);

@@ -30,6 +30,10 @@ CASES = [
     (40, 1.75, 1.0, 0.0),                   # pairs under the rule at the axis, over a voxel apart behind it
     (40, 1.9, 1.0, 0.0), (40, 3.1, 1.0, 0.0),          # single rows
     (50, 1.2, 0.7, 0.0), (50, 1.2, 1.6, 1.0),          # voxels that are not cubic
+    # three and four rows per lane (thick slices), full and partial groups, rows
+    # falling in z, and groups that drift over a voxel
+    (77, 0.7, 1.0, 0.0), (96, 0.7, 1.0, 2.0), (70, -0.7, 1.0, -3.0), (127, 0.5, 1.0, 0.0), (128, 0.45, 1.0, 5.0),
+    (101, -0.5, 1.0, 0.0), (90, 1.3, 2.5, 0.0), (91, 0.88, 1.0, 0.0),
 ]
 
 
