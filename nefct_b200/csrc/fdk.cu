@@ -384,8 +384,8 @@ static cudaError_t launch_filter(const FilterParams &p, const float *sino, float
 
 // Voxels along z per thread: the column part of a view is computed once per
 // kZ voxels (measured at 256^3 x 360 views: 2 -> 11.1 ms, 4 -> 8.68 ms,
-// 8 -> 8.27 ms, 12 -> 8.47 ms, 16 -> 10.4 ms; 8 holds 61-66 registers
-// without spills, more shrink the resident warps).
+// 8 -> 8.27 ms, 12 -> 8.47 ms, 16 -> 10.4 ms; 8 fits the 64 registers that
+// eight CTAs per SM leave, more spill or shrink the resident warps).
 #ifndef NEFCT_FDK_KZ
 #define NEFCT_FDK_KZ 8
 #endif
@@ -426,6 +426,8 @@ __global__ void __launch_bounds__(256) fdk_quad_kernel(const float *__restrict__
 // voxels project onto fewer detector columns than a 32 x 1 row (whose
 // detector footprint reaches ~50 columns), so its gathers touch fewer
 // sectors (measured 7 % faster than 32 x 1 and 16 x 2, 1 % than 4 x 8).
+// Eight lanes, which a 16-byte load serves at a time, own a 2 x 4 block of it
+// (an 8 x 1 row: 6.29 against 6.06 ms at 256^3 x 360 views).
 static constexpr int kTW = 8;
 
 // Voxel centres held in the kernel parameters (x, then y, then z) when the
@@ -443,6 +445,12 @@ struct BpParams {
     float ctr[kCtrMax];
 };
 
+// What bounds it: the L1's data path (91 % of its wavefronts, eight per
+// 16-byte gather of a warp instead of the four its bytes fill).  256^3, 360
+// views of 512 x 384: 6.06 ms with the repacks and the edge pass, against
+// 6.98 ms with the row test and the clamped row on every voxel and no bound on
+// the registers.  Two 8-byte tap pairs in place of the quads: 6.10 ms.
+//
 // Per view the column part (rotation, magnification m, detector column a,
 // its bilinear weights, the distance weight) follows the reference's
 // operations with its divisions replaced by one approximate reciprocal of
@@ -545,12 +553,13 @@ __device__ __forceinline__ bool bp_tap(const BpParams &p, const float *pv, const
 }
 
 template <bool QUAD>
-__global__ void __launch_bounds__(128) fdk_bp_kernel(const __grid_constant__ BpParams p,
-                                                     const float *__restrict__ sino, const float4 *__restrict__ quad,
-                                                     float *__restrict__ vol)
+__global__ void __launch_bounds__(128, 8) fdk_bp_kernel(const __grid_constant__ BpParams p,
+                                                        const float *__restrict__ sino,
+                                                        const float4 *__restrict__ quad, float *__restrict__ vol)
 {
-    const int ix = blockIdx.x * kTW + (threadIdx.x % kTW);
-    const int iy = (blockIdx.y * 4 + threadIdx.y) * (32 / kTW) + threadIdx.x / kTW;
+    const int lane = threadIdx.x;
+    const int ix = blockIdx.x * kTW + (lane & 1) + (lane >> 3) * 2;
+    const int iy = (blockIdx.y * 4 + threadIdx.y) * (32 / kTW) + ((lane >> 1) & 3);
     const int z0 = blockIdx.z * kZ;
     if (ix >= p.nx || iy >= p.ny) return;
     const float xc = bp_cx(p, ix);
@@ -567,7 +576,8 @@ __global__ void __launch_bounds__(128) fdk_bp_kernel(const __grid_constant__ BpP
     float zabs = 0.f;
 #pragma unroll
     for (int k = 0; k < kZ; ++k) zabs = fmaxf(zabs, fabsf(zc[k]));
-    const float bhi = (float)(p.nb + 1);
+    const float bhi = (float)(p.nb + 1), brow = (float)(p.nb - 1);
+    const unsigned pitch = (unsigned)p.na * (unsigned)(QUAD ? sizeof(float4) : sizeof(float));   // bytes per row
     for (int v = 0; v < p.nvc; ++v) {
         BpColumn c;
         bp_column(p, p.cs[v], p.sn[v], xc, yc, c);
@@ -577,6 +587,31 @@ __global__ void __launch_bounds__(128) fdk_bp_kernel(const __grid_constant__ BpP
         const float4 *pq = QUAD ? quad + (size_t)v * p.na * p.nb + c.ia : nullptr;
         float r0, r1, wb, wb2;
         if (fabsf(c.bm) * zabs + fabsf(p.cb) < 2097152.f) {
+            // rows are monotone in z: with the first and last voxel's row inside
+            // the detector none is dropped
+            const float b0 = __fmaf_rn(c.bm, zc[0], p.cb), b1 = __fmaf_rn(c.bm, zc[kZ - 1], p.cb);
+            if (fminf(b0, b1) >= 0.f && fmaxf(b0, b1) < brow) {
+                const char *const base = (QUAD ? (const char *)pq : (const char *)pv) - (size_t)0x4B400000u * pitch;
+#pragma unroll
+                for (int k = 0; k < kZ; ++k) {
+                    const float b = __fmaf_rn(c.bm, zc[k], p.cb);
+                    const float mb = __fadd_rd(b, 12582912.0f);
+                    const float w2 = __fsub_rn(b, __fsub_rn(mb, 12582912.0f)), w1 = __fsub_rn(1.f, w2);
+                    const char *const q = base + (unsigned long long)(unsigned)__float_as_int(mb) * pitch;
+                    float t00, t01, t10, t11;
+                    if (QUAD) {
+                        const float4 q4 = __ldg((const float4 *)q);
+                        t00 = q4.x; t01 = q4.y; t10 = q4.z; t11 = q4.w;
+                    } else {
+                        const float *const f = (const float *)q;
+                        t00 = __ldg(f); t01 = __ldg(f + 1); t10 = __ldg(f + p.na); t11 = __ldg(f + p.na + 1);
+                    }
+                    const float a0 = __fmaf_rn(t01, c.wa2u, __fmul_rn(t00, c.wau));
+                    const float a1 = __fmaf_rn(t11, c.wa2u, __fmul_rn(t10, c.wau));
+                    acc[k] = __fmaf_rn(a1, w2, __fmaf_rn(a0, w1, acc[k]));
+                }
+                continue;
+            }
 #pragma unroll
             for (int k = 0; k < kZ; ++k) {
                 // branch-free: a dropped row (Q11) reads row nb - 2's taps with

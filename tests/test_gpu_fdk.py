@@ -187,3 +187,24 @@ def test_tap_quad_backprojection_is_bitwise_equal(cuda, weight, cyl):
     torch.cuda.synchronize()
     assert torch.equal(quad, plain)
     assert float(plain.abs().max()) > 0
+
+
+@pytest.mark.parametrize("nb_,b_shift", [(2, 0.0), (9, 1.5), (40, 0.0), (40, -30.0)])
+@pytest.mark.parametrize("nz", [1, 8, 21])
+def test_rows_inside_and_across_the_detector_edge_bitwise(cuda, nb_, b_shift, nz):
+    """A voxel column whose rows all lie inside the detector and one whose
+    rows leave it give a voxel the same bits: every slice backprojected as a
+    grid of its own (all rows of its blocks equal) against the whole grid
+    (blocks inside, across and outside the detector's first and last rows)."""
+    ang = np.linspace(0, 2 * np.pi, 20, endpoint=False)
+
+    def geom(n, cz):
+        return nb.ConeBeam((13, 11, n), ang, 128.0, 256.0, 40, 1.0, nb_, 1.0, b_shift=b_shift, center=(0.0, 0.0, cz),
+                           size=(13.0, 11.0, float(n)))
+    g = geom(nz, 0.0)
+    sino = torch.rand(g.sino_shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(5))
+    whole = ops.fdk_backproject(sino, g)
+    for iz in range(nz):
+        # slice centres are multiples of 1/2, exact in float32
+        one = ops.fdk_backproject(sino, geom(1, iz + 0.5 - nz / 2))
+        assert torch.equal(whole[iz], one[0])
