@@ -211,12 +211,12 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
         if (ia >= P.na) continue;         // uniform across the warp
         if (FWD) {
             auto row = [&](int i, float (&r)[6]) {
-                const int ib = col_row<2, false>(rt, threadIdx.x, i, false);
+                const int ib = col_row<2, false>(rt * 64, threadIdx.x, i, false);
                 cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib < P.nb ? ib : 0, r);
                 return ib < P.nb;
             };
             auto store = [&](int i, float v) {
-                const int ib = col_row<2, false>(rt, threadIdx.x, i, false);
+                const int ib = col_row<2, false>(rt * 64, threadIdx.x, i, false);
                 P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
             };
             colwarp_forward<2, REF>(P.g, P.flags, P.volT, row, store);
@@ -225,8 +225,8 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
             bool has[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int ib = P.near ? col_row<2, true>(rt, threadIdx.x, i, P.rg.db < 0.f)
-                                      : col_row<2, false>(rt, threadIdx.x, i, false);
+                const int ib = P.near ? col_row<2, true>(rt * 64, threadIdx.x, i, P.rg.db < 0.f)
+                                      : col_row<2, false>(rt * 64, threadIdx.x, i, false);
                 has[i] = ib < P.nb;
                 y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
                 cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);

@@ -4,21 +4,21 @@
 
 namespace nefct {
 
-// Column warps: one warp per 32 R rows of column ia at view iv, into the
-// z-fastest accumulator p.outT (FIXED: the deterministic transpose's integers
-// p.fix).
+// Column warps: one warp per 32 R rows of column ia at view iv, from row
+// p.row0 on, into the z-fastest accumulator p.outT (FIXED: the deterministic
+// transpose's integers p.fix).
 template <int R, bool REF, bool NEXT, bool FIXED>
 __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __grid_constant__ CBParams<float> p)
 {
     const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    const int tile = p.band_major ? blockIdx.z : blockIdx.y;
+    const int first = p.row0 + (int)(p.band_major ? blockIdx.z : blockIdx.y) * 32 * R;
     const int iv = p.band_major ? blockIdx.y : blockIdx.z;
     if (ia >= p.na) return;                       // uniform across the warp
     float r[R][6], y[R];
     bool has[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        const int ib = col_row<R, NEXT>(tile, threadIdx.x, i, p.rg.db < 0.f);
+        const int ib = col_row<R, NEXT>(first, threadIdx.x, i, p.rg.db < 0.f);
         has[i] = ib < p.nb;
         y[i] = has[i] ? cb_sino_value(p, ia, ib, iv) : 0.f;
         cb_ray(p, ia, has[i] ? ib : 0, iv, r[i]);
@@ -27,25 +27,26 @@ __global__ void __launch_bounds__(256, 4) cb_colwarp_backward_kernel(const __gri
     else colwarp_backward<R, REF, NEXT>(p.g, r, has, p.flags, y, FloatAcc{p.outT});
 }
 
-template <int R, bool FIXED>
-static cudaError_t launch_colwarp(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
+template <bool REF, bool FIXED>
+static cudaError_t launch_colwarp(CBParams<float> &p, int na, int rows, int nvc, int R, cudaStream_t s)
 {
     dim3 grid, block;
-    cb_colwarp_shape(p, na, nb, nvc, grid, block, R);
-    if (ref_rounding(flags)) cb_colwarp_backward_kernel<R, true, (R > 1), FIXED><<<grid, block, 0, s>>>(p);
-    else cb_colwarp_backward_kernel<R, false, (R > 1), FIXED><<<grid, block, 0, s>>>(p);
+    cb_colwarp_shape(p, na, rows, nvc, grid, block, R);
+    if (R == 1) cb_colwarp_backward_kernel<1, REF, false, FIXED><<<grid, block, 0, s>>>(p);
+    else if (R == 2) cb_colwarp_backward_kernel<2, REF, true, FIXED><<<grid, block, 0, s>>>(p);
+    else if (R == 3) cb_colwarp_backward_kernel<3, REF, true, FIXED><<<grid, block, 0, s>>>(p);
+    else cb_colwarp_backward_kernel<4, REF, true, FIXED><<<grid, block, 0, s>>>(p);
     return cudaGetLastError();
 }
 
 template <bool FIXED>
 static cudaError_t launch_rows(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)
 {
-    switch (col_rows_next(p.g, p.rg, nb)) {
-    case 1: return launch_colwarp<1, FIXED>(p, na, nb, nvc, flags, s);
-    case 2: return launch_colwarp<2, FIXED>(p, na, nb, nvc, flags, s);
-    case 3: return launch_colwarp<3, FIXED>(p, na, nb, nvc, flags, s);
-    default: return launch_colwarp<4, FIXED>(p, na, nb, nvc, flags, s);
-    }
+    const bool ref = ref_rounding(flags);
+    return cb_row_launches(p, nb, col_rows_next(p.g, p.rg, nb), [&](int rows, int R) {
+        return ref ? launch_colwarp<true, FIXED>(p, na, rows, nvc, R, s)
+                   : launch_colwarp<false, FIXED>(p, na, rows, nvc, R, s);
+    });
 }
 
 cudaError_t cb_launch_backward_fixed(CBParams<float> &p, int na, int nb, int nvc, uint32_t flags, cudaStream_t s)

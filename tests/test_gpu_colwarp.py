@@ -34,6 +34,9 @@ CASES = [
     # falling in z, and groups that drift over a voxel
     (77, 0.7, 1.0, 0.0), (96, 0.7, 1.0, 2.0), (70, -0.7, 1.0, -3.0), (127, 0.5, 1.0, 0.0), (128, 0.45, 1.0, 5.0),
     (101, -0.5, 1.0, 0.0), (90, 1.3, 2.5, 0.0), (91, 0.88, 1.0, 0.0),
+    # last rows in a launch of their own: three and four rows per lane, then one
+    # and three
+    (193, 0.4, 1.0, 2.0),
 ]
 
 
