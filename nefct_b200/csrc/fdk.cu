@@ -9,9 +9,11 @@
 // filtered rows come back as the real and imaginary parts of the inverse
 // transform), forward transform, multiply by H/L, inverse transform as the
 // conjugate of a forward transform of the conjugate.  The transforms are
-// Stockham autosort FFTs (radix 4, plus one radix-2 stage when log2 L is
-// odd) in shared memory; the first stage reads the weighted rows from
-// global memory and the last writes the filtered rows.  H is built on the
+// Stockham autosort FFTs of 16 elements per thread: two or three passes of
+// radix 16 (the first of the forward and the last of the inverse of radix 2
+// to 16, whichever makes up L) in registers, with the elements exchanged
+// through shared memory between passes; the first pass reads the weighted rows
+// from global memory and the last writes the filtered rows.  H is built on the
 // host in FP64 (radix-2 FFT below) with the MATLAB scale folded in.
 //
 // Backprojection (nefct/cc/pixel_3d/pixel.cu.cc:12-146 geometry and index
@@ -110,7 +112,6 @@ static std::vector<float> ramp_response(int na, int window, double scale)
 
 static constexpr int kMaxCols = 2048;            // detector columns the filter supports
 static constexpr int kMaxL = 4096;               // ramp_length(kMaxCols)
-static constexpr int kFftThreads = 256;
 
 struct FilterParams {
     int na, nb, nv, L, log2L, pairs_per_view, pairs;
@@ -121,30 +122,6 @@ struct FilterParams {
     double fanang;                              // ParkerWeight's fanang (half the fan angle), degrees
     float h[kMaxL / 2 + 1];                     // H[k] * scale / L, k = 0..L/2
 };
-
-// Shared-memory index of element e of a transform buffer: C float2 of
-// padding per 16 elements.  A stage writes its output with the padding that
-// keeps its strided stores free of bank conflicts (fft_cpad) and the next
-// stage reads with the same padding; loads of 16 consecutive elements are
-// conflict-free under any padding.
-template <int C> __host__ __device__ __forceinline__ int fpad(int e) { return e + C * (e >> 4); }
-
-// Padding of the output of the stage with Ns points per finished
-// sub-transform: a half-warp writes elements 4j + r (Ns = 1), 8m + k + 2r
-// (Ns = 2), 16m + k + 4r (Ns = 4) or 32m + k + 8r (Ns = 8), which C = 1, 2, 4, 4
-// spread over 16 distinct 8-byte bank pairs; for Ns >= 16 the half-warp's
-// elements are consecutive.
-__host__ __device__ constexpr int fft_cpad(int Ns) { return Ns == 1 ? 1 : Ns == 2 ? 2 : Ns <= 8 ? 4 : 1; }
-
-// Shared memory: two padded L-point complex buffers (ping-pong), the
-// twiddle tables of the radix-4 stages (stage with Ns points per finished
-// sub-transform: W^(r k L/(4 Ns)) at [Ns - 1 or Ns - 2 + (r - 1) Ns + k],
-// 3 Ns entries, fewer than L in all) and H[0..L/2].
-static constexpr int fft_buf(int L) { return L + L / 4; }   // fpad<4>(L) bound
-static inline size_t filt_smem_bytes(int L)
-{
-    return (size_t)(2 * fft_buf(L) + L) * sizeof(float2) + (size_t)(L / 2 + 4) * sizeof(float);
-}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
@@ -191,193 +168,310 @@ __device__ __forceinline__ float parker_weight(const FilterParams &p, int iv, in
     return (float)pk;
 }
 
-// One Stockham stage of radix R (2 or 4) of a length-2^LOG2L transform with
-// Ns = 2^LNS points per finished sub-transform: butterfly j (< L/R) reads
-// elements j + r L/R, multiplies them by W^(r k L/(R Ns)) (k = j mod Ns;
-// radix 4 only, from the stage's table tws), transforms them and writes
-// them to (j - k) R + k + r Ns.  load(e, i) gives element e (i = fpad(e),
-// its shared-memory index); store(e, i, value) takes output element e.  The
-// sizes are compile-time, so the index arithmetic folds into constants.
-// ZIN: the inputs r >= R/2 are known zero (elements >= L/2 of the padded
-// rows in the first stage); LOW: only the outputs r < R/2 are wanted
-// (elements < L/2, the cropped rows, in the last stage).
-template <int R, int LOG2L, int LNS, int CIN, bool ZIN = false, bool LOW = false, class Load, class Store>
-__device__ __forceinline__ void fft_stage(const float2 *tws, Load load, Store store)
+// exp(-2 pi i n / 16), n = 0..9 (the powers that the radix-16 butterfly uses).
+static __constant__ float2 kRoot16[10] = {
+    {1.f, 0.f}, {0.923879532511286756f, -0.382683432365089772f}, {0.707106781186547524f, -0.707106781186547524f},
+    {0.382683432365089772f, -0.923879532511286756f}, {0.f, -1.f}, {-0.382683432365089772f, -0.923879532511286756f},
+    {-0.707106781186547524f, -0.707106781186547524f}, {-0.923879532511286756f, -0.382683432365089772f}, {-1.f, 0.f},
+    {-0.923879532511286756f, 0.382683432365089772f}};
+
+template <int N> __device__ __forceinline__ float2 mul_root16(float2 a)
 {
-    constexpr int lR = R == 2 ? 1 : 2;
-    constexpr int LR = 1 << (LOG2L - lR), Ns = 1 << LNS;
-    constexpr int COUT = fft_cpad(Ns);
-    constexpr int PLR = LR + CIN * (LR / 16);          // fpad(j + r LR) = fpad(j) + r PLR (LR % 16 == 0)
-    constexpr int ITER = (LR + kFftThreads - 1) / kFftThreads;
-#pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-        const int j = threadIdx.x + it * kFftThreads;
-        if (LR % kFftThreads != 0 && j >= LR) break;
-        const int k = j & (Ns - 1);
-        const int pj = fpad<CIN>(j);
-        float2 a[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) a[r] = (ZIN && r >= R / 2) ? make_float2(0.f, 0.f) : load(j + r * LR, pj + r * PLR);
-        const int o = ((j - k) << lR) + k;
-        auto out = [&](int r, float2 v) {
-            if constexpr (Ns >= 16) store(o + r * Ns, fpad<COUT>(o) + r * (Ns + COUT * (Ns / 16)), v);
-            else store(o + r * Ns, fpad<COUT>(o + r * Ns), v);
-        };
-        if constexpr (R == 2) {
-            if constexpr (ZIN) {                 // the radix-2 stage is the first (Ns = 1)
-                out(0, a[0]);
-                out(1, a[0]);
-            } else {
-                out(0, cadd(a[0], a[1]));
-                out(1, csub(a[0], a[1]));
-            }
-        } else {
-            if constexpr (Ns > 1) {
-#pragma unroll
-                for (int r = 1; r < 4; ++r)
-                    if (!(ZIN && r >= 2)) a[r] = cmul(a[r], tws[(r - 1) * Ns + k]);
-            }
-            const float2 t0 = ZIN ? a[0] : cadd(a[0], a[2]), t1 = ZIN ? a[0] : csub(a[0], a[2]);
-            const float2 t2 = ZIN ? a[1] : cadd(a[1], a[3]), t3 = cmul_mi(ZIN ? a[1] : csub(a[1], a[3]));
-            out(0, cadd(t0, t2));
-            out(1, cadd(t1, t3));
-            if constexpr (!LOW) {
-                out(2, csub(t0, t2));
-                out(3, csub(t1, t3));
-            }
-        }
+    constexpr float h = 0.707106781186547524f;
+    if constexpr (N == 0) return a;
+    else if constexpr (N == 2) return make_float2((a.x + a.y) * h, (a.y - a.x) * h);
+    else if constexpr (N == 4) return cmul_mi(a);
+    else if constexpr (N == 6) return make_float2((a.y - a.x) * h, (a.x + a.y) * -h);
+    else return cmul(a, kRoot16[N]);
+}
+
+// DFT of four values in place.  ZIN: c and d are zero; LOW: only the outputs a
+// and b are wanted.
+template <bool ZIN, bool LOW> __device__ __forceinline__ void dft4(float2 &a, float2 &b, float2 &c, float2 &d)
+{
+    const float2 t0 = ZIN ? a : cadd(a, c), t1 = ZIN ? a : csub(a, c);
+    const float2 t2 = ZIN ? b : cadd(b, d), t3 = cmul_mi(ZIN ? b : csub(b, d));
+    a = cadd(t0, t2);
+    b = cadd(t1, t3);
+    if (!LOW) {
+        c = csub(t0, t2);
+        d = csub(t1, t3);
     }
 }
 
-// Stages of a length-2^log2L transform: one radix-2 stage first when
-// log2L is odd, radix 4 after.
-__host__ __device__ constexpr int fft_stages(int log2L) { return (log2L & 1) ? 1 + (log2L - 1) / 2 : log2L / 2; }
-
-// Offset of the twiddle table of the radix-4 stage with Ns points per
-// finished sub-transform (Ns = 4^i, or 2 * 4^i after a radix-2 stage).
-__host__ __device__ constexpr int tw_offset(int Ns, bool odd) { return odd ? Ns - 2 : Ns - 1; }
-
-// Radix-4 stages from Ns = 2^LNS on: the stages before the last read src
-// and write dst in shared memory (swapping them after each stage), the
-// last (Ns = L/4) writes through last.
-template <int LOG2L, int LNS, bool LOW, class Last>
-__device__ __forceinline__ void fft_tail(const float2 *tw, const float2 *src, float2 *dst, Last last)
+// DFT of the R values x[m] = a[I + m S], S = 16 / R, in place.  ZIN: the upper
+// half of the inputs is zero; LOW: only the lower half of the outputs is wanted.
+template <int R, int I, bool ZIN, bool LOW> __device__ __forceinline__ void dft(float2 (&a)[16])
 {
-    constexpr bool odd = LOG2L & 1;
-    constexpr int CIN = fft_cpad(1 << (LNS - (LNS == 1 ? 1 : 2)));   // the previous stage's output padding
-    const float2 *tws = tw + tw_offset(1 << LNS, odd);
-    auto ld = [src](int, int i) { return src[i]; };
-    if constexpr (LNS + 2 == LOG2L) {
-        fft_stage<4, LOG2L, LNS, CIN, false, LOW>(tws, ld, last);
-        __syncthreads();
+    constexpr int S = 16 / R;
+    if constexpr (R == 2) {
+        const float2 x = a[I], y = a[I + S];
+        a[I] = ZIN ? x : cadd(x, y);
+        if (!LOW) a[I + S] = ZIN ? x : csub(x, y);
+    } else if constexpr (R == 4) {
+        dft4<ZIN, LOW>(a[I], a[I + S], a[I + 2 * S], a[I + 3 * S]);
+    } else if constexpr (R == 8) {
+        // x[q + 2 s]: radix 4 over s, then radix 2 over q; output k1 + 4 k2
+        dft4<ZIN, false>(a[I], a[I + 2 * S], a[I + 4 * S], a[I + 6 * S]);
+        dft4<ZIN, false>(a[I + S], a[I + 3 * S], a[I + 5 * S], a[I + 7 * S]);
+        const float2 y[4] = {a[I], a[I + 2 * S], a[I + 4 * S], a[I + 6 * S]};
+        const float2 z[4] = {a[I + S], mul_root16<2>(a[I + 3 * S]), mul_root16<4>(a[I + 5 * S]),
+                             mul_root16<6>(a[I + 7 * S])};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[I + k * S] = cadd(y[k], z[k]);
+            if (!LOW) a[I + (k + 4) * S] = csub(y[k], z[k]);
+        }
     } else {
-        fft_stage<4, LOG2L, LNS, CIN>(tws, ld, [dst](int, int i, float2 v) { dst[i] = v; });
-        __syncthreads();
-        fft_tail<LOG2L, LNS + 2, LOW>(tw, dst, const_cast<float2 *>(src), last);
+        // x[q + 4 s]: radix 4 over s, then radix 4 over q; output k1 + 4 k2
+        dft4<ZIN, false>(a[0], a[4], a[8], a[12]);
+        dft4<ZIN, false>(a[1], a[5], a[9], a[13]);
+        dft4<ZIN, false>(a[2], a[6], a[10], a[14]);
+        dft4<ZIN, false>(a[3], a[7], a[11], a[15]);
+        a[5] = mul_root16<1>(a[5]);
+        a[9] = mul_root16<2>(a[9]);
+        a[13] = mul_root16<3>(a[13]);
+        a[6] = mul_root16<2>(a[6]);
+        a[10] = mul_root16<4>(a[10]);
+        a[14] = mul_root16<6>(a[14]);
+        a[7] = mul_root16<3>(a[7]);
+        a[11] = mul_root16<6>(a[11]);
+        a[15] = mul_root16<9>(a[15]);
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) dft4<false, LOW>(a[k], a[k + 1], a[k + 2], a[k + 3]);
+        // a[4 k1 + k2] is output k1 + 4 k2
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+            for (int k2 = k1 + 1; k2 < 4; ++k2) {
+                const float2 t = a[4 * k1 + k2];
+                a[4 * k1 + k2] = a[4 * k2 + k1];
+                a[4 * k2 + k1] = t;
+            }
     }
 }
 
-// Forward FFT of length 2^LOG2L: the first stage reads through first(e, i)
-// (ZIN: inputs e >= L/2 are zero), the last writes through last(e, i, value)
-// (LOW: outputs e < L/2 only), the stages between ping-pong in shared
-// memory (padded indices): stage 0 writes b1, stage 1 b0, ...
-template <int LOG2L, bool ZIN, bool LOW, class First, class Last>
-__device__ __forceinline__ void fft_run(const float2 *tw, float2 *b0, float2 *b1, First first, Last last)
+// Every radix-R butterfly of a thread's 16 elements.
+template <int R, bool ZIN, bool LOW, int I = 0> __device__ __forceinline__ void dft_all(float2 (&a)[16])
 {
-    constexpr bool odd = LOG2L & 1;
-    auto to_b1 = [b1](int, int i, float2 v) { b1[i] = v; };
-    // the first stage's input index is that of the spectrum buffer (written
-    // by a last stage, Ns = L/4 >= 16: padding 1) when it is read from there
-    if constexpr (odd) fft_stage<2, LOG2L, 0, 1, ZIN>(tw, first, to_b1);
-    else fft_stage<4, LOG2L, 0, 1, ZIN>(tw, first, to_b1);
-    __syncthreads();
-    fft_tail<LOG2L, odd ? 1 : 2, LOW>(tw, b1, b0, last);
+    dft<R, I, ZIN, LOW>(a);
+    if constexpr (I + 1 < 16 / R) dft_all<R, ZIN, LOW, I + 1>(a);
 }
 
-// Persistent CTAs over row pairs (view iv, rows b and b + 1); transform
-// length 2^LOG2L.
-template <int LOG2L>
-__global__ void __launch_bounds__(kFftThreads) fdk_filter_kernel(const __grid_constant__ FilterParams p,
-                                                                 const float *__restrict__ sino,
-                                                                 float *__restrict__ out)
+// Twiddle factors of a radix-R pass with Ns points per finished sub-transform:
+// W^(r k), W = exp(-2 pi i / (R Ns)), at [(r - 1) Ns + k], r = 1..R - 1, k < Ns.
+// (Products of the powers 1, 2, 3, 4, 8 and 12 in place of the others took the
+// same time, with 10 % more rounding error.)
+template <int R, int Ns> __device__ __forceinline__ void tw_fill(float2 *tw)
 {
-    constexpr int L = 1 << LOG2L;
-    constexpr bool odd = LOG2L & 1;
-    extern __shared__ __align__(16) float2 fsm[];
-    const int na = p.na;
-    float2 *b0 = fsm, *b1 = fsm + fft_buf(L), *tw = fsm + 2 * fft_buf(L);
-    float *hs = reinterpret_cast<float *>(tw + L);
-    // twiddle tables of the radix-4 stages: W^(r k L/(4 Ns)) = exp(-2 pi i r k / (4 Ns))
-    for (int Ns = odd ? 2 : 1; Ns <= L / 4; Ns *= 4) {
-        const int off = tw_offset(Ns, odd);
-        for (int i = threadIdx.x; i < 3 * Ns; i += blockDim.x) {
-            const int r = 1 + i / Ns, k = i - (r - 1) * Ns;
-            float sn, cs;
-            sincospif((float)(r * k) / (float)(2 * Ns), &sn, &cs);   // exact argument (power-of-two denominator)
-            tw[off + i] = make_float2(cs, -sn);
+    for (int i = threadIdx.x; i < (R - 1) * Ns; i += blockDim.x) {
+        const int row = i / Ns, k = i - row * Ns;
+        float sn, cs;
+        sincospif((float)((row + 1) * k) / (float)(R * Ns / 2), &sn, &cs);    // exact argument (power-of-two denominator)
+        tw[i] = make_float2(cs, -sn);
+    }
+}
+
+// a[i + r S] (element j + r L / R, S = 16 / R, j = t + i T) times W^(r k),
+// k = j mod Ns.
+template <int R, int Ns, int T> __device__ __forceinline__ void tw_apply(const float2 *tw, int t, float2 (&a)[16])
+{
+    constexpr int S = 16 / R;
+#pragma unroll
+    for (int i = 0; i < S; ++i) {
+        const int k = (t + i * T) & (Ns - 1);
+#pragma unroll
+        for (int r = 1; r < R; ++r) a[i + r * S] = cmul(a[i + r * S], tw[(r - 1) * Ns + k]);
+    }
+}
+
+// The transforms of length L = 2^LOG2L: T threads of 16 elements each, thread t
+// holding elements t + m T (m = 0..15) before and after every pass.  The
+// forward's passes have the radices C, 16 (, 16), the inverse's 16 (, 16), C.
+template <int LOG2L> struct Fft {
+    static constexpr int L = 1 << LOG2L, T = L / 16;
+    static constexpr bool three = LOG2L > 8;
+    static constexpr int C = three ? L / 256 : L / 16;
+    static constexpr int threads = 256, groups = threads / T;
+    // one element of padding per 16: the strided writes of an exchange (16
+    // elements 2 to 16 apart, or rows of Ns consecutive ones 16 Ns apart) and the
+    // consecutive reads are free of bank conflicts
+    static constexpr int buffer = L + L / 16;
+    // twiddle tables: forward's second and third pass, inverse's second and third
+    static constexpr int f2 = 0, f3 = f2 + 15 * C, i2 = three ? f3 + 15 * 16 * C : f3;
+    static constexpr int i3 = three ? i2 + 15 * 16 : i2, tables = i3 + (C - 1) * (L / C);
+    static constexpr size_t smem = (size_t)(groups * buffer + tables) * sizeof(float2) + (L / 2 + 4) * sizeof(float);
+
+    static __device__ __forceinline__ int pad(int e) { return e + (e >> 4); }
+
+    // Barrier of the T threads of a transform (T < 32: within a warp).
+    static __device__ __forceinline__ void sync(int group)
+    {
+        if constexpr (T <= 32) __syncwarp();
+        else if constexpr (T == threads) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(T) : "memory");
+    }
+
+    // Writes the outputs of a radix-R pass with Ns points per finished
+    // sub-transform and reads the next pass's inputs.
+    template <int R, int Ns> static __device__ __forceinline__ void exchange(float2 *buf, int t, int group, float2 (&a)[16])
+    {
+        constexpr int S = 16 / R;
+        sync(group);                          // the last exchange's reads are done
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            const int j = t + i * T, k = j & (Ns - 1), o = (j - k) * R + k;
+#pragma unroll
+            for (int r = 0; r < R; ++r) buf[pad(o + r * Ns)] = a[i + r * S];
+        }
+        sync(group);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) a[m] = buf[pad(t + m * T)];
+    }
+
+    // Elements m >= 8 are zero on entry.
+    static __device__ __forceinline__ void forward(float2 *buf, const float2 *tw, int t, int group, float2 (&a)[16])
+    {
+        dft_all<C, true, false>(a);
+        exchange<C, 1>(buf, t, group, a);
+        tw_apply<16, C, T>(tw + f2, t, a);
+        dft_all<16, false, false>(a);
+        if constexpr (three) {
+            exchange<16, C>(buf, t, group, a);
+            tw_apply<16, 16 * C, T>(tw + f3, t, a);
+            dft_all<16, false, false>(a);
         }
     }
-    for (int k = threadIdx.x; k <= L / 2; k += blockDim.x) hs[k] = p.h[k];
+
+    // A forward transform too; only the elements m < 8 are wanted.
+    static __device__ __forceinline__ void inverse(float2 *buf, const float2 *tw, int t, int group, float2 (&a)[16])
+    {
+        dft_all<16, false, false>(a);
+        exchange<16, 1>(buf, t, group, a);
+        if constexpr (three) {
+            tw_apply<16, 16, T>(tw + i2, t, a);
+            dft_all<16, false, false>(a);
+            exchange<16, 16>(buf, t, group, a);
+        }
+        tw_apply<C, L / C, T>(tw + i3, t, a);
+        dft_all<C, false, true>(a);
+    }
+};
+
+// Persistent CTAs; T threads take consecutive row pairs (view iv, rows b and
+// b + 1), so the Parker weights of a thread's columns, FP64 with an arc tangent
+// and a sine or cosine each, are evaluated once per view it meets instead of
+// once per pair.
+//
+// What bounds it: the shared-memory pipe (about 70 % of its wavefronts: four
+// exchanges and three passes of twiddle factors per pair; a radix-4 FFT exchanges
+// nine times at L = 1024).  300 views of 500 x 300: 327 -> 195 us (the rows cross
+// memory in 55); 200 views of 1000 x 300: 512 -> 270 us; 100 views of 2048 x 300:
+// 1009 -> 312 us; 1000 views of 120 x 200: 323 -> 77 us; 211 views of 389 x 283
+// with Parker weights: 275 -> 140 us.  At most 85 registers, three CTAs per SM:
+// 0.304 ms for 360 views of 512 x 384, against 0.322 with two; CTAs of 64 or 128
+// threads as fast.
+template <int LOG2L, bool PARKER>
+__global__ void __launch_bounds__(256, LOG2L < 12 ? 3 : 2) fdk_filter_kernel(const __grid_constant__ FilterParams p,
+                                                            const float *__restrict__ sino, float *__restrict__ out)
+{
+    using F = Fft<LOG2L>;
+    extern __shared__ __align__(16) float2 fsm[];
+    float2 *const tw = fsm + F::groups * F::buffer;
+    float *const hs = reinterpret_cast<float *>(tw + F::tables);
+    tw_fill<16, F::C>(tw + F::f2);
+    if constexpr (F::three) {
+        tw_fill<16, 16 * F::C>(tw + F::f3);
+        tw_fill<16, 16>(tw + F::i2);
+    }
+    tw_fill<F::C, F::L / F::C>(tw + F::i3);
+    for (int k = threadIdx.x; k <= F::L / 2; k += blockDim.x) hs[k] = p.h[k];
     __syncthreads();
-    // the last stage of the forward transform would write b1 after an odd
-    // number of stages, b0 after an even number: keep the spectrum there
-    float2 *const z = (fft_stages(LOG2L) & 1) ? b1 : b0;
-    float2 *const zf = z == b0 ? b1 : b0;
-    for (int pr = blockIdx.x; pr < p.pairs; pr += gridDim.x) {
+    const int na = p.na, group = threadIdx.x / F::T, t = threadIdx.x % F::T;
+    float2 *const buf = fsm + group * F::buffer;
+    const int gid = blockIdx.x * F::groups + group, ngroups = gridDim.x * F::groups;
+    // every group takes as many steps as the longest (barriers): the last ones of some do nothing
+    const int per = (p.pairs + ngroups - 1) / ngroups;
+    float pk[PARKER ? 8 : 1];
+    int pk_view = -1;
+    for (int s = 0; s < per; ++s) {
+        const long long pair = (long long)gid * per + s;
+        const bool has = pair < p.pairs;
+        const int pr = has ? (int)pair : 0;
         const int iv = pr / p.pairs_per_view;
         const int row = 2 * (pr - iv * p.pairs_per_view);
         const bool two = row + 1 < p.nb;
-        const float *x0 = sino + ((size_t)iv * p.nb + row) * na;
-        const float *x1 = x0 + na;
-        // forward transform of the weighted pair, zero beyond na
-        const float c0 = cos_row(p, row), c1 = cos_row(p, row + 1);
-        auto first = [&](int e, int) {
-            if (e >= na) return make_float2(0.f, 0.f);
-            const float pk = p.parker ? parker_weight(p, iv, e) : 1.f;
-            const float a = x0[e] * (cos_weight(p, c0, e) * pk);
-            const float b = two ? x1[e] * (cos_weight(p, c1, e) * pk) : 0.f;
-            return make_float2(a, b);
-        };
-        // (rows occupy at most L/2 elements: the upper half of the input is zero)
-        fft_run<LOG2L, true, false>(tw, b0, b1, first, [z](int, int i, float2 v) { z[i] = v; });
-        // inverse: conj(FFT(conj(Z H / L))); its real and imaginary parts are
-        // the filtered rows.  Stage 0 reads z and writes the other buffer,
-        // so the second run starts from (z, zf) as (b0, b1).
-        auto first2 = [&](int e, int i) {
-            const float hk = hs[e <= L / 2 ? e : L - e];
-            const float2 v = z[i];
-            return make_float2(v.x * hk, -(v.y * hk));
-        };
-        float *const y0 = out + ((size_t)iv * p.nb + row) * na;
-        float *const y1 = y0 + na;
-        auto last2 = [&](int e, int, float2 v) {
-            if (e < na) {
-                y0[e] = v.x;
-                if (two) y1[e] = -v.y;
+        const float *const x0 = sino + ((size_t)iv * p.nb + row) * na, *const x1 = x0 + na;
+        // the weighted pair, zero beyond na (na <= L/2: m < 8)
+        float2 a[16];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int e = t + m * F::T;
+            const bool in = has && e < na;
+            a[m] = make_float2(in ? __ldg(x0 + e) : 0.f, in && two ? __ldg(x1 + e) : 0.f);
+        }
+        if (PARKER && iv != pk_view) {
+            pk_view = iv;
+#pragma unroll 1
+            for (int m = 0; m < 8; ++m) {
+                const float w = parker_weight(p, iv, t + m * F::T);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i == m) pk[PARKER ? i : 0] = w;
             }
-        };
-        // (only the first na <= L/2 outputs are kept)
-        fft_run<LOG2L, false, true>(tw, z, zf, first2, last2);
+        }
+        const float c0 = cos_row(p, row), c1 = cos_row(p, row + 1);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int e = t + m * F::T;
+            const float w0 = cos_weight(p, c0, e), w1 = cos_weight(p, c1, e);
+            a[m].x *= PARKER ? w0 * pk[PARKER ? m : 0] : w0;
+            a[m].y *= PARKER ? w1 * pk[PARKER ? m : 0] : w1;
+        }
+        F::forward(buf, tw, t, group, a);
+        // conj(Z H / L): the real and imaginary parts of the conjugate of its
+        // forward transform are the filtered rows
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            const int e = t + m * F::T;
+            const float h = hs[m < 8 ? e : F::L - e];
+            a[m] = make_float2(a[m].x * h, -(a[m].y * h));
+        }
+        F::inverse(buf, tw, t, group, a);
+        float *const y0 = out + ((size_t)iv * p.nb + row) * na, *const y1 = y0 + na;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int e = t + m * F::T;
+            if (!has || e >= na) continue;
+            y0[e] = a[m].x;
+            if (two) y1[e] = -a[m].y;
+        }
     }
 }
 
 // Launches the filter for transform length 2^LOG2L.
-template <int LOG2L>
+template <int LOG2L, bool PARKER>
 static cudaError_t launch_filter(const FilterParams &p, const float *sino, float *out, cudaStream_t s)
 {
-    const size_t smem = filt_smem_bytes(1 << LOG2L);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(fdk_filter_kernel<LOG2L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+    using F = Fft<LOG2L>;
+    const auto kernel = fdk_filter_kernel<LOG2L, PARKER>;
+    if (F::smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem);
         if (e != cudaSuccess) return e;
     }
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fdk_filter_kernel<LOG2L>, kFftThreads, smem);
-    const int blocks = std::min(p.pairs, sms * std::max(per_sm, 1));
-    fdk_filter_kernel<LOG2L><<<blocks, kFftThreads, smem, s>>>(p, sino, out);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, F::threads, F::smem);
+    const int blocks = std::min((p.pairs + F::groups - 1) / F::groups, sms * std::max(per_sm, 1));
+    kernel<<<blocks, F::threads, F::smem, s>>>(p, sino, out);
     return cudaGetLastError();
+}
+
+template <int LOG2L>
+static cudaError_t launch_filter(const FilterParams &p, const float *sino, float *out, cudaStream_t s)
+{
+    return p.parker ? launch_filter<LOG2L, true>(p, sino, out, s) : launch_filter<LOG2L, false>(p, sino, out, s);
 }
 
 // ---------------- device: voxel-driven backprojection ----------------

@@ -208,3 +208,18 @@ def test_rows_inside_and_across_the_detector_edge_bitwise(cuda, nb_, b_shift, nz
         # slice centres are multiples of 1/2, exact in float32
         one = ops.fdk_backproject(sino, geom(1, iz + 0.5 - nz / 2))
         assert torch.equal(whole[iz], one[0])
+
+
+@pytest.mark.parametrize("parker", [0, 1, -1])
+@pytest.mark.parametrize("na,nb_,nv", [(32, 2, 3), (64, 7, 3), (65, 1, 4), (128, 5, 3), (256, 4, 3), (257, 9, 3),
+                                       (512, 6, 3), (513, 3, 3), (1024, 1, 3), (1025, 2, 3), (2047, 3, 2),
+                                       (300, 51, 130)])
+def test_filter_transform_lengths_vs_restatement(cuda, na, nb_, nv, parker):
+    """Every transform length at both ends of its range of columns, odd and even
+    row counts, and (last) enough row pairs that a thread walks several views."""
+    ang = np.deg2rad(np.arange(nv) * (220.0 / nv)).astype(np.float32)
+    g = nb.ConeBeam((8, 8, 8), ang, 300.0, 600.0, na, 400.0 / na, nb_, 1.1)
+    sino = np.random.default_rng(na).random((nv, nb_, na), dtype=np.float32)
+    out = ops.fdk_filter(torch.from_numpy(sino).to(cuda), g, "hann", parker).cpu().numpy()
+    ref = ofdk.fdk_filter(sino, 600.0, 300.0, 400.0 / na, 1.1, window="hann", parker=parker, angles=ang)
+    assert_parity(out, ref)
