@@ -91,29 +91,86 @@ __global__ void __launch_bounds__(256) warp_forward_kernel(const T *__restrict__
     }
 }
 
+// Reduces v[j] into the corners j (x, y) at flat index base (valid).  The whole
+// warp calls it: where the next lane's corners start one voxel further in x, it
+// takes this lane's upper two over, so a row of lanes reduces each voxel once.
+template <typename T>
+__device__ __forceinline__ void warp_reduce(T *gimg, bool valid, int base, T (&v)[4], int sy)
+{
+    const int lane = threadIdx.x & 31, at = valid ? base : -2;
+    const int before = __shfl_up_sync(0xffffffffu, at, 1), after = __shfl_down_sync(0xffffffffu, at, 1);
+    const T p1 = __shfl_up_sync(0xffffffffu, v[1], 1), p3 = __shfl_up_sync(0xffffffffu, v[3], 1);
+    if (!valid) return;
+    if (lane > 0 && before == at - 1) {
+        v[0] += p1;
+        v[2] += p3;
+    }
+    T *const b = gimg + base;
+    atomicAdd(b, v[0]);
+    atomicAdd(b + sy, v[2]);
+    if (lane == 31 || after != at + 1) {
+        atomicAdd(b + 1, v[1]);
+        atomicAdd(b + 1 + sy, v[3]);
+    }
+}
+
+// Voxels along z per thread of the adjoint (2 is 5 % slower on smooth fields and
+// 2 % faster on white noise, 8 the reverse).
+static constexpr int kWarpZ = 4;
+
+// What bounds it: the reductions, which the L2 takes sector by sector (1.9e11/s).
+// Where the field is smooth, neighbours in z have base corners one above the
+// other and neighbours in x one beside the other: a thread adds the upper four
+// taps of a voxel to the lower four of the next, and a lane takes over its
+// neighbour's (warp_reduce), which leaves 2 to 3 reductions of a voxel's 8.
+// 192^3 / 512^3, smooth field: 71 / 1160 -> 46 / 668 us; white noise of +-3 voxels,
+// where nothing is shared: 237 / 4420 -> 250 / 4570 us.
 template <typename T>
 __global__ void __launch_bounds__(256) warp_adjoint_kernel(const T *__restrict__ gout, const T *__restrict__ mx,
                                                            const T *__restrict__ my, const T *__restrict__ mz,
                                                            int nx, int ny, int nz, T *__restrict__ gimg)
 {
-    const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, iz = blockIdx.z;
-    if (ix >= nx || iy >= ny) return;
-    const int id = ix + iy * nx + iz * nx * ny;
-    const T g = gout[id];
-    if (g == (T)0) return;
-    const Tap<T> t = warp_tap<T>(ix, iy, iz, mx[id], my[id], mz[id], nx, ny, nz);
-    if (!t.ok) return;
+    const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y, z0 = blockIdx.z * kWarpZ;
+    if (iy >= ny) return;                               // uniform across the warp
     const int sy = nx, sz = nx * ny;
-    const T wx2 = t.fx, wx = (T)1 - wx2, wy2 = t.fy, wy = (T)1 - wy2, wz2 = t.fz, wz = (T)1 - wz2;
-    T *b = gimg + t.base;
-    atomicAdd(b, g * (wx * wy * wz));
-    atomicAdd(b + sz, g * (wx * wy * wz2));
-    atomicAdd(b + sy, g * (wx * wy2 * wz));
-    atomicAdd(b + sy + sz, g * (wx * wy2 * wz2));
-    atomicAdd(b + 1, g * (wx2 * wy * wz));
-    atomicAdd(b + 1 + sz, g * (wx2 * wy * wz2));
-    atomicAdd(b + 1 + sy, g * (wx2 * wy2 * wz));
-    atomicAdd(b + 1 + sy + sz, g * (wx2 * wy2 * wz2));
+    const bool in = ix < nx;
+    T g[kWarpZ], m[kWarpZ][3];
+#pragma unroll
+    for (int k = 0; k < kWarpZ; ++k) {
+        const bool has = in && z0 + k < nz;
+        const int id = has ? ix + iy * nx + (z0 + k) * sz : 0;
+        g[k] = has ? gout[id] : (T)0;
+        m[k][0] = has ? mx[id] : (T)0;
+        m[k][1] = has ? my[id] : (T)0;
+        m[k][2] = has ? mz[id] : (T)0;
+    }
+    bool held = false;                                  // up: the upper plane of the voxel before
+    int at = 0;
+    T up[4];
+#pragma unroll
+    for (int k = 0; k < kWarpZ; ++k) {
+        const Tap<T> t = warp_tap<T>(ix, iy, z0 + k, m[k][0], m[k][1], m[k][2], nx, ny, nz);
+        const bool ok = t.ok && g[k] != (T)0;
+        const T wx2 = t.fx, wx = (T)1 - wx2, wy2 = t.fy, wy = (T)1 - wy2, wz2 = t.fz, wz = (T)1 - wz2;
+        T low[4] = {g[k] * (wx * wy * wz), g[k] * (wx2 * wy * wz), g[k] * (wx * wy2 * wz), g[k] * (wx2 * wy2 * wz)};
+        if (held) {
+            if (ok && t.base == at) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) low[j] += up[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) atomicAdd(gimg + at + (j & 1) + (j >> 1) * sy, up[j]);
+            }
+        }
+        warp_reduce<T>(gimg, ok, t.base, low, sy);
+        held = ok;
+        at = t.base + sz;
+        up[0] = g[k] * (wx * wy * wz2);
+        up[1] = g[k] * (wx2 * wy * wz2);
+        up[2] = g[k] * (wx * wy2 * wz2);
+        up[3] = g[k] * (wx2 * wy2 * wz2);
+    }
+    warp_reduce<T>(gimg, held, at, up, sy);
 }
 
 template <typename T>
@@ -224,7 +281,8 @@ static nefct_status warp_adjoint_impl(const T *gout, const T *mx, const T *my, c
     if (st) return st;
     if (!gout || !mx || !my || !mz || !gimg) return fail(NEFCT_ERR_INVALID, "NULL buffer");
     NEFCT_CHECK_CUDA(cudaMemsetAsync(gimg, 0, (size_t)nx * ny * nz * sizeof(T), s));
-    warp_adjoint_kernel<T><<<dim3((nx + 31) / 32, (ny + 7) / 8, nz), dim3(32, 8), 0, s>>>(gout, mx, my, mz, nx, ny, nz, gimg);
+    const dim3 grid((nx + 31) / 32, (ny + 7) / 8, (nz + kWarpZ - 1) / kWarpZ);
+    warp_adjoint_kernel<T><<<grid, dim3(32, 8), 0, s>>>(gout, mx, my, mz, nx, ny, nz, gimg);
     NEFCT_CHECK_LAUNCH("warp_adjoint_kernel");
     return NEFCT_OK;
 }

@@ -126,3 +126,57 @@ def test_warp_invert_vs_reference_texture_kernel(cuda, oracle_lib, case):
         assert float(r.abs().max()) > 0.3 * float(f.abs().max())       # a real inverse, not zeros
         assert float(d.max()) <= 0.015, float(d.max())
         assert float(d.mean()) <= 0.002, float(d.mean())
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["zero", "smooth", "rough", "steps"])
+@pytest.mark.parametrize("shape", [(3, 5, 4), (4, 8, 32), (5, 9, 33), (18, 7, 70)])
+def test_warp_and_derivatives_share_corners(cuda, shape, kind, dtype):
+    """The warp, its adjoint and its field gradient against sums over the eight
+    corners in double precision, where neighbouring samples share corners
+    (zero, smooth), do not (rough) and do so here and there (steps), for
+    partial z groups and row tails; zeros in the cotangent take no part.
+
+    Tolerance: a float32 result is a sum of rounded products of up to a few
+    dozen terms, 2e-6 of the largest."""
+    rng = np.random.default_rng(shape[0])
+    nz, ny, nx = shape
+    z, y, x = np.meshgrid(*[np.arange(n) for n in shape], indexing="ij")
+    if kind == "rough":
+        m = [rng.uniform(-2.5, 2.5, shape) for _ in range(3)]
+    elif kind == "steps":
+        m = [rng.integers(-1, 2, shape) * (rng.random(shape) < 0.3) + 0.25 for _ in range(3)]
+    else:
+        amp = 0.0 if kind == "zero" else 1.3
+        m = [amp * np.sin(0.21 * x + 0.17 * y + 0.4 * z + i) for i in range(3)]
+    m = [a.astype(dtype) for a in m]
+    img, g = rng.random(shape).astype(dtype), rng.standard_normal(shape).astype(dtype)
+    g[rng.random(shape) < 0.1] = 0
+    p = [(c.astype(dtype) + a) for c, a in zip((x, y, z), m)]
+    f = [np.floor(a) for a in p]
+    ok = np.ones(shape, bool)
+    for a, n in zip(f, (nx, ny, nz)):
+        ok &= (a > 0) & (a + 1 < n)
+    w = [(a - b).astype(np.float64)[ok] for a, b in zip(p, f)]
+    i = [a.astype(int)[ok] for a in f]
+    out, adj = np.zeros(shape), np.zeros(shape)
+    grad = [np.zeros(shape) for _ in range(3)]
+    g64, acc, dacc = g.astype(np.float64)[ok], np.zeros(ok.sum()), [np.zeros(ok.sum()) for _ in range(3)]
+    for c in range(8):
+        b = [c & 1, c >> 1 & 1, c >> 2]
+        at = (i[2] + b[2], i[1] + b[1], i[0] + b[0])
+        part = [u if s else 1 - u for u, s in zip(w, b)]
+        v = img[at].astype(np.float64)
+        acc += v * part[0] * part[1] * part[2]
+        np.add.at(adj, at, g64 * part[0] * part[1] * part[2])
+        for k in range(3):
+            o = [part[j] for j in range(3) if j != k]
+            dacc[k] += (1 if b[k] else -1) * v * o[0] * o[1]
+    out[ok] = acc
+    for k in range(3):
+        grad[k][ok] = dacc[k] * g64
+    t = [torch.from_numpy(np.ascontiguousarray(a)).to(cuda) for a in (img, *m, g)]
+    tol = 2e-6 if dtype == np.float32 else 1e-13
+    for got, ref in ((ops.warp_forward(*t[:4]), out), (ops.warp_adjoint(t[4], *t[1:4]), adj),
+                     *zip(ops.warp_grad_dvf(*t), grad)):
+        np.testing.assert_allclose(got.cpu().numpy(), ref, rtol=0, atol=tol * max(np.abs(ref).max(), 1.0))
