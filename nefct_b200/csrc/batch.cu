@@ -186,6 +186,37 @@ __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ Batc
     }
 }
 
+// One warp's rows of column ia at view iv, from row `first` on: R rows per lane.
+template <bool FWD, bool REF, int R>
+__device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first, int iv)
+{
+    if (FWD) {
+        auto row = [&](int i, float (&r)[6]) {
+            const int ib = col_row<R, false>(first, threadIdx.x, i, false);
+            cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib < P.nb ? ib : 0, r);
+            return ib < P.nb;
+        };
+        auto store = [&](int i, float v) {
+            const int ib = col_row<R, false>(first, threadIdx.x, i, false);
+            P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
+        };
+        colwarp_forward<R, REF>(P.g, P.flags, P.volT, row, store);
+    } else {
+        float r[R][6], y[R];
+        bool has[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int ib = R > 1 && P.near ? col_row<R, true>(first, threadIdx.x, i, P.rg.db < 0.f)
+                                           : col_row<R, false>(first, threadIdx.x, i, false);
+            has[i] = ib < P.nb;
+            y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
+            cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);
+        }
+        if (R > 1 && P.near) colwarp_backward<R, REF, (R > 1)>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
+        else colwarp_backward<R, REF, false>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
+    }
+}
+
 // Column-warp variant: a tile is blockDim.y columns x 64 rows of one view,
 // one warp per column.  Bounded to 64 registers (4 CTAs of 256 threads per
 // SM) like the single-problem kernels: the dynamically indexed problem
@@ -209,31 +240,10 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
         const int iv = (int)(rest / P.tiles_b);
         const int ia = ct * blockDim.y + threadIdx.y;
         if (ia >= P.na) continue;         // uniform across the warp
-        if (FWD) {
-            auto row = [&](int i, float (&r)[6]) {
-                const int ib = col_row<2, false>(rt * 64, threadIdx.x, i, false);
-                cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib < P.nb ? ib : 0, r);
-                return ib < P.nb;
-            };
-            auto store = [&](int i, float v) {
-                const int ib = col_row<2, false>(rt * 64, threadIdx.x, i, false);
-                P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
-            };
-            colwarp_forward<2, REF>(P.g, P.flags, P.volT, row, store);
-        } else {
-            float r[2][6], y[2];
-            bool has[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int ib = P.near ? col_row<2, true>(rt * 64, threadIdx.x, i, P.rg.db < 0.f)
-                                      : col_row<2, false>(rt * 64, threadIdx.x, i, false);
-                has[i] = ib < P.nb;
-                y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
-                cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);
-            }
-            if (P.near) colwarp_backward<2, REF, true>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
-            else colwarp_backward<2, REF, false>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
-        }
+        // 32 rows or fewer left: one row per lane (28 problems of 16^3 to 64^3 with 24
+        // to 128 rows, both directions: 0.837 -> 0.796 ms)
+        if (P.nb - rt * 64 > 32) batch_rows<FWD, REF, 2>(P, ia, rt * 64, iv);
+        else batch_rows<FWD, REF, 1>(P, ia, rt * 64, iv);
     }
 }
 

@@ -168,3 +168,24 @@ def test_batch_tile_shape_autotuning(cuda):
     for g, v, gr, s, b in zip(geoms, vols, grads, bp.sinos, bp.backs):
         assert torch.equal(s, ops.cb_forward(v, g))
         assert_parity(b.cpu().numpy(), ops.cb_backward(gr, g).cpu().numpy())
+
+
+@pytest.mark.parametrize("flags", [0, nb._lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("pitch", [0.9, 2.2, -0.9], ids=["pairs", "single-rows", "falling"])
+def test_batch_row_tiles(cuda, flags, pitch):
+    """Row counts around the tiles of 64 and of 32 rows: the same walk as the
+    single-problem kernels, whose forward gives the same bits."""
+    rows = (1, 31, 32, 33, 64, 65, 96, 97)
+    geoms = [nb.ConeBeam((20, 18, 22), np.linspace(0, 2 * np.pi, 7), 70.0, 140.0, 21, 2.0, r, pitch,
+                         size=(20.0, 18.0, 22.0)) for r in rows]
+    rng = np.random.default_rng(1)
+    vols = [torch.from_numpy(rng.random(g.vol_shape, dtype=np.float32)).to(cuda) for g in geoms]
+    grads = [torch.from_numpy(rng.random(g.sino_shape, dtype=np.float32)).to(cuda) for g in geoms]
+    with _walk(3):
+        bp = BatchProjector(geoms, vols, grads=grads, flags=flags, strategy="persistent")
+        bp.step()
+        torch.cuda.synchronize()
+        for g, v, y, s, b in zip(geoms, vols, grads, bp.sinos, bp.backs):
+            assert torch.equal(s, ops.cb_forward(v, g, flags))
+            # the same shares in another order of addition
+            assert_parity(b.cpu().numpy(), ops.cb_backward(y, g, flags).cpu().numpy(), rel=1e-6, mabs=1e-5)
