@@ -51,8 +51,8 @@ const char *nefct_last_error(void);
  *   NEFCT_TUNE_CB_ORDER  0: row bands outermost (default; keeps the volume
  *                        slab of the rows in flight in L2), 1: views outermost
  *   NEFCT_TUNE_CB_WALK   bit 0 forward, bit 1 transpose: column warps (FP32
- *                        slab walk with a workspace) -- each warp walks 32
- *                        rows of one detector column, which share their
+ *                        slab walk with a workspace) -- each warp walks up to
+ *                        128 rows of one detector column, which share their
  *                        transverse walk, over a z-fastest copy of the volume,
  *                        and NEFCT_TUNE_CB_ROWS counts columns per CTA; a
  *                        clear bit: one thread per ray.  Default 3 */

@@ -2,7 +2,7 @@
 
 For a geometry signature (grid, views, detector, kind, flags) it times the
 equivalent launch variants of include/nefct_b200.h's tuning table -- the walk
-(one thread per ray, or one warp per 32 rows of a detector column), rows or
+(one thread per ray, or warps that walk rows of a detector column), rows or
 columns per CTA and the grid order -- on the current device with CUDA
 events (forward + transpose, after a warm-up), applies the fastest with
 nefct_tune_set and caches the choice in a JSON file

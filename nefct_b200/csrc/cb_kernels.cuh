@@ -84,8 +84,11 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     Walk<float> w;
     if (!setup_walk(g, r, flags, w)) return 0.f;
     GatherSink<true> f(vol, sw);
-    if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, sw, f);
-    else ray_walk<false>(g, w, su, sv, sw, f);
+    const ColWalk c = col_walk_of(g, w, su, sv);
+    const ZRay z = z_ray(w, true);
+    if (ref_rounding(flags)) ray_each<true>(c, z, z_grid(g), sw, f, w.k0, w.k1);
+    else ray_each<false>(c, z, z_grid(g), sw, f, w.k0, w.k1);
+    f.close();
     return f.whole * w.W;
 }
 
@@ -150,7 +153,7 @@ __device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, ui
 }
 
 template <typename T, bool DIV, bool EXACT = false>
-__global__ void __launch_bounds__(256) cb_forward_kernel(const __grid_constant__ CBParams<T> p)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && !EXACT ? 4 : 1) cb_forward_kernel(const __grid_constant__ CBParams<T> p)
 {
     int ia, ib, iv;
     cb_cell(p, ia, ib, iv);
