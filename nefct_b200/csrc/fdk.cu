@@ -553,9 +553,10 @@ struct BpParams {
 
 // What bounds it: the L1's data path (91 % of its wavefronts, eight per
 // 16-byte gather of a warp instead of the four its bytes fill).  256^3, 360
-// views of 512 x 384: 6.06 ms with the repacks and the edge pass, against
-// 6.98 ms with the row test and the clamped row on every voxel and no bound on
-// the registers.  Two 8-byte tap pairs in place of the quads: 6.10 ms.
+// views of 512 x 384: 5.93 ms with the repacks and the edge pass (6.06 with the
+// repacks at two thirds of their present rate), against 6.98 ms with the row test
+// and the clamped row on every voxel and no bound on the registers.  Two 8-byte
+// tap pairs in place of the quads: 6.10 against 6.06 ms.
 //
 // Per view the column part (rotation, magnification m, detector column a,
 // its bilinear weights, the distance weight) follows the reference's
