@@ -390,8 +390,11 @@ __device__ __forceinline__ void ray_inner(const ColWalk &c, const ZRay &z, const
             float m, r;
             z_inner<REF>(z, zg, z.down ? db : da, z.down ? da : db, m, r);
             const float both = fminf(rv, r), over = __fsub_rn(r, both);      // r's share in the high column
-            const unsigned p0 = base + (unsigned)__float_as_int(m1) * c.sv + (unsigned)__float_as_int(m) * sw;
-            f.inner(vx, p0, p0 + (rv > r ? sw : c.sv), p0 + (c.sv + sw), both, fabsf(__fsub_rn(rv, r)),
+            // (the high column is the one at the slab's far plane: where dv < 1 it
+            // need not be the low one's neighbour)
+            const unsigned row = base + (unsigned)__float_as_int(m) * sw;
+            const unsigned p0 = row + (unsigned)__float_as_int(m1) * c.sv, ph = row + (unsigned)__float_as_int(m2) * c.sv;
+            f.inner(vx, p0, rv > r ? p0 + sw : ph, ph + sw, both, fabsf(__fsub_rn(rv, r)),
                     __fsub_rn(__fsub_rn(1.f, rv), over));
             base += c.su;
             da = db;

@@ -110,3 +110,31 @@ def test_values_that_are_not_finite_stay_on_their_rays(cuda, oracle_lib, value, 
         np.testing.assert_array_equal(np.isfinite(out), fine)
         np.testing.assert_array_equal(np.isnan(out), np.isnan(ref))
         assert_parity(np.where(fine, out, 0), np.where(fine, ref, 0))
+
+
+def _thread_walk(g, vol, y, flags):
+    """The thread walk with and without its y-fastest copy."""
+    return _both(g, vol, y, flags, 0), _both(g, vol, y, flags | _lib.NO_TRANSPOSE, 3)
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("ratio", [0.91, 0.5, 0.25])
+def test_rows_thinner_than_columns(cuda, oracle_lib, ratio, flags):
+    """Grids whose y pitch is below the x pitch: a slab of an x-driven ray moves
+    over a voxel in y, so its high column is not the one above its low column."""
+    g = nb.ConeBeam((26, 22, 24), ANGLES, 70.0, 140.0, 37, 1.5, 65, 1.2, size=(26.0, 22.0 * ratio, 24.0),
+                    center=(0.3, -0.2, 0.1), z_offsets=np.linspace(-0.5, 0.5, ANGLES.size))
+    rng = np.random.default_rng(11)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    f, b = _both(g, v, s, flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(b.cpu().numpy(), ref_b)
+    for ft, bt in _thread_walk(g, v, s, flags):
+        assert torch.equal(f, ft)
+        assert_parity(bt.cpu().numpy(), ref_b)
+    fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
+    assert torch.equal(*fixed)
+    assert_parity(fixed[0].cpu().numpy(), ref_b)
