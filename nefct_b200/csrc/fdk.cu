@@ -1037,6 +1037,13 @@ nefct_status nefct_fdk_backproject_ws(const nefct_cb_geom *g, const float *filte
     if (quad && ws_bytes < nefct_fdk_workspace_bytes(g))
         return fail(NEFCT_ERR_WORKSPACE, "needs %zu workspace bytes, got %zu", nefct_fdk_workspace_bytes(g), ws_bytes);
     if (quad && ((uintptr_t)ws & 15)) return fail(NEFCT_ERR_INVALID, "workspace must be 16-byte aligned");
+    // a detector of one row or column has no cell with four taps (Q11): every
+    // voxel is dropped
+    if (g->na < 2 || g->nb < 2) {
+        const size_t voxels = (size_t)g->grid.nx * g->grid.ny * g->grid.nz;
+        NEFCT_CHECK_CUDA(cudaMemsetAsync(vol, 0, voxels * sizeof(float), (cudaStream_t)stream));
+        return NEFCT_OK;
+    }
     BpParams *p = new BpParams();
     p->nx = g->grid.nx; p->ny = g->grid.ny; p->nz = g->grid.nz;
     p->na = g->na; p->nb = g->nb;

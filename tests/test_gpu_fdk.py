@@ -243,3 +243,18 @@ def test_tap_quads_at_tile_edges_are_bitwise_equal(cuda, na, nb_):
     _lib.check(lib.nefct_fdk_backproject_ws(C.byref(s), sino.data_ptr(), quad.data_ptr(), 0, ws.data_ptr(), wn, stream))
     torch.cuda.synchronize()
     assert torch.equal(quad, plain) and float(plain.abs().max()) > 0
+
+
+@pytest.mark.parametrize("na,nb_", [(40, 1), (1, 24), (1, 1)])
+def test_detectors_of_one_row_or_column_give_zeros(cuda, na, nb_):
+    """No cell has four taps, so every voxel is dropped (and no tap is read)."""
+    import ctypes as C
+    from nefct_b200 import _lib
+    g = nb.ConeBeam((24, 20, 12), np.linspace(0, 2 * np.pi, 5, endpoint=False), 90.0, 180.0, na, 1.5, nb_, 1.5)
+    sino = torch.ones(g.sino_shape, device=cuda)
+    plain = torch.full(g.vol_shape, np.nan, device=cuda)
+    s = g.struct()
+    _lib.check(_lib.load().nefct_fdk_backproject(C.byref(s), sino.data_ptr(), plain.data_ptr(), 0,
+                                                 torch.cuda.current_stream(cuda).cuda_stream))
+    for vol in (plain, ops.fdk_backproject(sino, g), ops.fdk_backproject(sino, g, weight=False)):
+        assert vol.shape == g.vol_shape and not vol.any()
