@@ -683,8 +683,10 @@ __global__ void __launch_bounds__(128, 8) fdk_bp_kernel(const __grid_constant__ 
     float zabs = 0.f;
 #pragma unroll
     for (int k = 0; k < kZ; ++k) zabs = fmaxf(zabs, fabsf(zc[k]));
-    const float bhi = (float)(p.nb + 1), brow = (float)(p.nb - 1);
+    // (the rows inside the detector are addressed with 32-bit row pitches; longer
+    // rows take the path with the row test)
     const unsigned pitch = (unsigned)p.na * (unsigned)(QUAD ? sizeof(float4) : sizeof(float));   // bytes per row
+    const float bhi = (float)(p.nb + 1), brow = p.na < 1 << 28 ? (float)(p.nb - 1) : 0.f;
     for (int v = 0; v < p.nvc; ++v) {
         BpColumn c;
         bp_column(p, p.cs[v], p.sn[v], xc, yc, c);

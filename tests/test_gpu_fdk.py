@@ -258,3 +258,22 @@ def test_detectors_of_one_row_or_column_give_zeros(cuda, na, nb_):
                                                  torch.cuda.current_stream(cuda).cuda_stream))
     for vol in (plain, ops.fdk_backproject(sino, g), ops.fdk_backproject(sino, g, weight=False)):
         assert vol.shape == g.vol_shape and not vol.any()
+
+
+def test_rows_longer_than_32_bit_pitches(cuda):
+    """2^28 + 1 columns: a row of tap quads takes more than 2^32 bytes (16 GB
+    on the device in all)."""
+    import ctypes as C
+    from nefct_b200 import _lib
+    na = (1 << 28) + 1
+    # one view, whose voxels see the middle of the detector: 2^20 columns per unit
+    g = nb.ConeBeam((6, 5, 4), np.zeros(1), 90.0, 180.0, na, 2.0 ** -20, 3, 4.0, center=(0.0, 0.0, 1.0))
+    sino = torch.arange(na, dtype=torch.int32, device=cuda).bitwise_and(1023).float().add(torch.tensor(
+        [[[1.0], [5000.0], [30000.0]]], device=cuda))
+    plain = torch.empty(g.vol_shape, device=cuda)
+    s = g.struct()
+    _lib.check(_lib.load().nefct_fdk_backproject(C.byref(s), sino.data_ptr(), plain.data_ptr(), 0,
+                                                 torch.cuda.current_stream(cuda).cuda_stream))
+    quad = ops.fdk_backproject(sino, g)
+    # every row position lies in (0.2, 1.8): taps of rows 0 | 1 and 1 | 2
+    assert torch.equal(quad, plain) and float(plain.max()) > 1.5 * 5000 > float(plain.min()) > 0
