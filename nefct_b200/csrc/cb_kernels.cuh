@@ -85,9 +85,10 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     if (!setup_walk(g, r, flags, w)) return 0.f;
     GatherSink<true> f(vol, sw);
     const ColWalk c = col_walk_of(g, w, su, sv);
-    const ZRay z = z_ray(w, true);
-    if (ref_rounding(flags)) ray_each<true>(c, z, z_grid(g), sw, f, w.k0, w.k1);
-    else ray_each<false>(c, z, z_grid(g), sw, f, w.k0, w.k1);
+    const ZGrid zg = z_grid(g);
+    const ZRay z = z_ray(w, zg, true);
+    if (ref_rounding(flags)) ray_each<true>(c, z, zg, sw, f, w.k0, w.k1);
+    else ray_each<false>(c, z, zg, sw, f, w.k0, w.k1);
     f.close();
     return f.whole * w.W;
 }

@@ -115,29 +115,31 @@ struct ZRay {
 // rounding of the positions).
 constexpr float kSteep = 0.999f;
 
-__device__ __forceinline__ ZRay z_ray(const Walk<float> &w, bool live)
-{
-    ZRay z;
-    z.live = live;
-    z.kz = live ? w.kz : 0.f;       // a lane without a ray walks row 0 (its indices stay in the grid)
-    z.z0 = live ? w.z0 : 0.5f;
-    z.kw = live ? w.kw : 0.f;
-    z.pw = live ? w.pw : 0.f;
-    z.ikz = fminf(__fdiv_rn(1.f, fabsf(z.kz)), 1e30f);
-    z.down = z.kz < 0.f;
-    z.steep = fabsf(z.kz) > kSteep;
-    return z;
-}
-
 // Grid constants of the z positions.
 struct ZGrid {
-    float rdz, nz2;         // 1 / dz, nz / 2
+    float dz, rdz, nz2;     // dz, 1 / dz, nz / 2
     bool div;               // dz != 1
     int nz;
 };
 __device__ __forceinline__ ZGrid z_grid(const GridDev<float> &g)
 {
-    return ZGrid{__fdiv_rn(1.f, g.dz), g.nz2, g.dz != 1.f, g.nz};
+    return ZGrid{g.dz, __fdiv_rn(1.f, g.dz), g.nz2, g.dz != 1.f, g.nz};
+}
+
+// (a lane without a ray walks row 0 under either rounding: its indices stay in
+// the grid)
+__device__ __forceinline__ ZRay z_ray(const Walk<float> &w, const ZGrid &zg, bool live)
+{
+    ZRay z;
+    z.live = live;
+    z.kz = live ? w.kz : 0.f;
+    z.z0 = live ? w.z0 : 0.5f;
+    z.kw = live ? w.kw : 0.f;
+    z.pw = live ? w.pw : __fmul_rn(__fsub_rn(0.5f, zg.nz2), zg.dz);
+    z.ikz = fminf(__fdiv_rn(1.f, fabsf(z.kz)), 1e30f);
+    z.down = z.kz < 0.f;
+    z.steep = fabsf(z.kz) > kSteep;
+    return z;
 }
 
 // Position at plane offset d in the reference's order of operations (its
@@ -411,8 +413,8 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
                                          unsigned sw, Sink &f)
 {
     const ColWalk c = col_walk_of(g, w, su, sv);
-    const ZRay z = z_ray(w, true);
     const ZGrid zg = z_grid(g);
+    const ZRay z = z_ray(w, zg, true);
     const bool interior = !z.steep && w.ki0 <= w.ki1;
     ray_each<REF>(c, z, zg, sw, f, w.k0, interior ? w.ki0 - 1 : w.k1);
     if (interior) {
@@ -455,7 +457,7 @@ __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&
             const unsigned xs = (unsigned)g.nz, ys = (unsigned)g.nx * (unsigned)g.nz;
             q.c = col_walk_of(g, w, w.xdrive ? xs : ys, w.xdrive ? ys : xs);
         }
-        q.z[i] = z_ray(w, live);
+        q.z[i] = z_ray(w, q.zg, live);
         q.W[i] = w.W;
         if (live) {
             any = true;

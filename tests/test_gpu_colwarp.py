@@ -138,3 +138,19 @@ def test_rows_thinner_than_columns(cuda, oracle_lib, ratio, flags):
     fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
     assert torch.equal(*fixed)
     assert_parity(fixed[0].cpu().numpy(), ref_b)
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("rows", [20, 33, 70])
+def test_two_slices_and_lanes_without_a_ray(cuda, oracle_lib, rows, flags):
+    """nz = 2, rays that stay in the lower slice (slabs without range checks) and
+    warps with lanes past the last row, which walk row 0."""
+    g = nb.ConeBeam((26, 22, 2), ANGLES, 70.0, 140.0, 37, 1.5, rows, 0.02, size=(26.0, 22.0, 8.0),
+                    center=(0.3, -0.2, 2.0), z_offsets=np.linspace(-0.1, 0.1, ANGLES.size))
+    rng = np.random.default_rng(rows)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    f, b = _both(g, torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda), flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(b.cpu().numpy(), ref_b)
