@@ -83,12 +83,12 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     const float r[6] = {x1, y1, z1, x2, y2, z2};
     Walk<float> w;
     if (!setup_walk(g, r, flags, w)) return 0.f;
-    GatherSink<true> f(vol, sw);
+    GatherSink f(vol);
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
     const ZRay z = z_ray(w, zg, true);
-    if (ref_rounding(flags)) ray_each<true>(c, z, zg, sw, f, w.k0, w.k1);
-    else ray_each<false>(c, z, zg, sw, f, w.k0, w.k1);
+    if (ref_rounding(flags)) ray_slabs<true, true, false, -1>(c, z, zg, w.k0, w.k1, sw, f);
+    else ray_slabs<false, true, false, -1>(c, z, zg, w.k0, w.k1, sw, f);
     f.close();
     return f.whole * w.W;
 }
@@ -115,7 +115,7 @@ __device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32
         const float *const v = w.xdrive && volT ? volT : vol;
         unsigned su, sv;
         thread_strides(g.nx, g.ny, w.xdrive, volT != nullptr, su, sv);
-        GatherSink<> f(v, (unsigned)sw);
+        GatherSink f(v);
         if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
         else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
         const float sum = f.whole;
@@ -143,7 +143,7 @@ __device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, ui
     if constexpr (std::is_same<T, float>::value) {
         unsigned su, sv;
         thread_strides(g.nx, g.ny, w.xdrive, outT != nullptr, su, sv);
-        ScatterSink f{w.xdrive && outT ? outT : out, (unsigned)sw, y * w.W};
+        ScatterSink f{w.xdrive && outT ? outT : out, y * w.W};
         if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
         else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
     } else {
@@ -202,9 +202,9 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
             return;
         }
     }
-    GatherSink<> f[R];
+    GatherSink f[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) f[i] = GatherSink<>(volZ, 1u);
+    for (int i = 0; i < R; ++i) f[i] = GatherSink(volZ);
     if (q.steep) {
 #pragma unroll
         for (int i = 0; i < R; ++i) col_each<REF>(q.c, q.K0, q.K1, q.z[i], q.zg, f[i]);
@@ -228,8 +228,8 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
     }
 }
 
-__device__ __forceinline__ ScatterSink ray_sink(const FloatAcc &a, float yw) { return ScatterSink{a.vol, 1u, yw}; }
-__device__ __forceinline__ FixedSink ray_sink(const FixedAcc &a, float yw) { return FixedSink{a.vol, 1u, yw, a.scale}; }
+__device__ __forceinline__ ScatterSink ray_sink(const FloatAcc &a, float yw) { return ScatterSink{a.vol, yw}; }
+__device__ __forceinline__ FixedSink ray_sink(const FixedAcc &a, float yw) { return FixedSink{a.vol, yw, a.scale}; }
 
 // Transpose of R rows per lane of one detector column: y[i] times the ray's
 // weights into the z-fastest accumulator acc.  NEXT: the rows are neighbours
@@ -392,14 +392,14 @@ static inline int col_rows_next(const GridDev<float> &g, const RayGeom<float> &r
 }
 
 // Column warps apply to FP32 slab walks with a workspace; the z-fastest
-// copy's transposes launch ny planes (grid z), and the packed v floors hold
-// n + 3 in 16 bits.  (NEFCT_DETERMINISTIC changes nothing for the forward;
-// its transpose has kernels of its own.)
+// copy's transposes launch ny planes (grid z: at most 65535); grids as wide keep
+// the thread walk too, the only one run at that width.  (NEFCT_DETERMINISTIC
+// changes nothing for the forward; its transpose has kernels of its own.)
 template <typename T> static inline bool cb_use_colwarp(const nefct_grid &g, uint32_t flags, bool forward)
 {
     return sizeof(T) == sizeof(float) && (tune_get(NEFCT_TUNE_CB_WALK) & (forward ? 1 : 2)) != 0 &&
-           !(flags & (NEFCT_EXACT | NEFCT_NO_TRANSPOSE)) && (forward || !(flags & NEFCT_DETERMINISTIC)) && g.ny <= 65535 &&
-           g.nx + 3 < 65536 && g.ny + 3 < 65536;
+           !(flags & (NEFCT_EXACT | NEFCT_NO_TRANSPOSE)) && (forward || !(flags & NEFCT_DETERMINISTIC)) &&
+           g.nx < 65533 && g.ny < 65533;
 }
 
 // Launches the thread-walk forward (FWD) or transpose kernel for the views

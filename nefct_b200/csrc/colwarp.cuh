@@ -52,13 +52,14 @@ struct ColWalk {
     bool vdiv;
 };
 
-// v part of one slab: biased bases of the low/high v voxel columns (index of
-// (k, v, z) = b + sw * floor bits of z), the clamped v floors for the
-// boundary checks, and the v crossing ratio.
+// v part of one slab of a column warp: biased bases of the low/high v voxel
+// columns (index of (k, v, z) = b + floor bits of z), which of them are in the
+// grid, and the v crossing ratio.
 struct ColEntry {
-    unsigned b1, b2;    // k*su + c*sv - sw*0x4B400000 for the low/high v floor c
-    unsigned cv;        // (c1 + 2) | (c2 + 2) << 16, c clamped to [-2, nv + 1]
+    unsigned b1, b2;    // k*su + c*sv - 0x4B400000 for the low/high v floor c
+    unsigned in;        // bit 0, 1: the low, high column is in the grid
     float rv;           // crossing ratio, 1 without a v crossing
+    bool vx;            // the slab crosses a v plane
 };
 
 __device__ __forceinline__ ColWalk col_walk_of(const GridDev<float> &g, const Walk<float> &w, unsigned su, unsigned sv)
@@ -78,28 +79,46 @@ __device__ __forceinline__ float col_plane(const ColWalk &c, int k)
     return __fsub_rn(__fsub_rn((float)k, c.nu2), c.pu);
 }
 
-// Entry of slab k: planes t = k - nu2 and t + 1, positions and floors in the
-// reference's operations and order.  Clamping a floor to [-2, nv + 1] keeps
-// every admission decision of the boundary checks.  sw: z stride.
-__device__ __forceinline__ ColEntry col_entry(const ColWalk &c, int k, unsigned sw)
+// v position at plane offset d in the reference's operations and order.
+// DIV: 1 (0) divides by dv (not); -1: as c says.
+template <int DIV = -1> __device__ __forceinline__ float col_vpos(const ColWalk &c, float d)
 {
-    auto vpos = [&](float d) {
-        float q = __fadd_rn(c.pv, __fmul_rn(c.kv, d));
-        if (c.vdiv) q = __fdiv_rn(q, c.dv);
-        return __fadd_rn(q, c.nv2);
-    };
-    const float qa = vpos(col_plane(c, k)), qb = vpos(col_plane(c, k + 1));
+    float q = __fadd_rn(c.pv, __fmul_rn(c.kv, d));
+    if (DIV < 0 ? c.vdiv : DIV != 0) q = __fdiv_rn(q, c.dv);
+    return __fadd_rn(q, c.nv2);
+}
+
+// Crossing ratio of a slab with v positions q1 <= q2 and biased floors m1, m2.
+__device__ __forceinline__ float col_ratio(float q1, float q2, float m1, float m2)
+{
+    return m1 != m2 ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1), __fadd_rn(q2, -q1)) : 1.f;
+}
+
+// Whether a voxel of biased floor m, and the one above it, are among n.
+struct Inside {
+    float lo, hi;           // biased floors 0 and n
+    __device__ __forceinline__ Inside(int n) : lo(kFloorMagic), hi(kFloorMagic + (float)n) {}
+    __device__ __forceinline__ bool low(float m) const { return m >= lo && m < hi; }
+    __device__ __forceinline__ bool high(float m) const { return m >= lo - 1.f && m < hi - 1.f; }
+    // the high one of a slab with floors m < mh, admitted from m = -1 on
+    // (the reference's slab admission, siddon.cu.cc:80, :92, :112, :116, :132)
+    __device__ __forceinline__ bool far(float m, float mh) const { return m >= lo - 1.f && mh >= lo && mh < hi; }
+};
+
+// Entry of slab k: planes t = k - nu2 and t + 1.
+__device__ __forceinline__ ColEntry col_entry(const ColWalk &c, int k)
+{
+    const float qa = col_vpos(c, col_plane(c, k)), qb = col_vpos(c, col_plane(c, k + 1));
     const float ma = magic_floor<true>(qa), mb = magic_floor<true>(qb);
-    const float q1 = fminf(qa, qb), q2 = fmaxf(qa, qb);
     const float m1 = fminf(ma, mb), m2 = fmaxf(ma, mb);
+    const Inside in(c.nv);
     ColEntry e;
-    e.rv = m1 != m2 ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1), __fadd_rn(q2, -q1)) : 1.f;
-    const int c1 = min(max(__float_as_int(m1) - kFloorMagicBits, -2), c.nv + 1);
-    const int c2 = min(max(__float_as_int(m2) - kFloorMagicBits, -2), c.nv + 1);
-    const unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * sw;
-    e.b1 = base + (unsigned)c1 * c.sv;
-    e.b2 = base + (unsigned)c2 * c.sv;
-    e.cv = (unsigned)(c1 + 2) | ((unsigned)(c2 + 2) << 16);
+    e.rv = col_ratio(fminf(qa, qb), fmaxf(qa, qb), m1, m2);
+    e.vx = m1 != m2;
+    e.in = (unsigned)in.low(m1) | (unsigned)(e.vx && in.far(m1, m2)) << 1;
+    const unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + 1u);
+    e.b1 = base + (unsigned)__float_as_int(m1) * c.sv;
+    e.b2 = base + (unsigned)__float_as_int(m2) * c.sv;
     return e;
 }
 
@@ -151,13 +170,6 @@ __device__ __forceinline__ float z_pos(const ZRay &z, const ZGrid &zg, float d)
     return __fadd_rn(q, zg.nz2);
 }
 
-// The z split of one slab: biased floors of its low and high voxel and the
-// share rw of the low one.  d, dh: offsets of the lower and upper plane.
-struct ZSplit {
-    unsigned i1, i2;
-    float rw;
-};
-
 // z split of a slab of a ray that is not steep: biased floor and low share.
 // (The grid has at most 2^20 rows and slabs, and such a ray moves at most one
 // row per slab: positions stay below 2^22, no clamp is needed for the floor.)
@@ -174,74 +186,33 @@ __device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo
     }
 }
 
+// z split of any ray's slab: biased floors of its low and high voxel and the low
+// share.  lo, hi: offsets of the lower and upper plane.
 template <bool REF>
-__device__ __forceinline__ ZSplit z_split(const ZRay &z, const ZGrid &zg, float d, float dh)
+__device__ __forceinline__ void z_split(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &mh, float &r)
 {
-    ZSplit s;
-    float m;
     if (!z.steep) {
-        z_inner<REF>(z, zg, d, dh, m, s.rw);
-        s.i1 = (unsigned)__float_as_int(m);
-        s.i2 = s.i1 + 1u;
-        return s;
+        z_inner<REF>(z, zg, lo, hi, m, r);
+        mh = __fadd_rn(m, 1.f);
+        return;
     }
-    float q = REF ? z_pos(z, zg, d) : __fmaf_rn(z.kz, d, z.z0);
-    float qh = REF ? z_pos(z, zg, dh) : __fmaf_rn(z.kz, dh, z.z0);
+    float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
+    float qh = REF ? z_pos(z, zg, hi) : __fmaf_rn(z.kz, hi, z.z0);
     m = magic_floor<true>(q);
-    const float mh = magic_floor<true>(qh);
+    mh = magic_floor<true>(qh);
     q = fminf(fmaxf(q, -kFloorClamp), kFloorClamp);
     qh = fminf(fmaxf(qh, -kFloorClamp), kFloorClamp);
     const float iden = REF ? rcp_approx(__fadd_rn(qh, -q)) : z.ikz;
-    s.rw = mh != m ? __fmul_rn(__fadd_rn(__fadd_rn(mh, -kFloorMagic), -q), iden) : 1.f;
-    s.i1 = (unsigned)__float_as_int(m);
-    s.i2 = (unsigned)__float_as_int(mh);
-    return s;
-}
-
-// Shares of a slab with a v crossing: the overlap of the ray's v intervals
-// [0, rv], [rv, 1] and z intervals [0, rw], [rw, 1] (the reference's pairing,
-// Q1): (v1, w1), (v1, w2), (v2, w1), (v2, w2); one of the middle two is 0.
-struct Shares {
-    float w11, w12, w21, w22;
-};
-__device__ __forceinline__ Shares slab_shares(float rv, float rw)
-{
-    Shares s;
-    s.w11 = fminf(rv, rw);
-    s.w12 = __fsub_rn(rv, s.w11);
-    s.w21 = __fsub_rn(rw, s.w11);
-    s.w22 = __fsub_rn(__fsub_rn(1.f, rv), s.w21);
-    return s;
-}
-
-// Which of a slab's v columns are in the grid (bits v1, v2), with the
-// reference's slab admission (siddon.cu.cc:80, :92, :112, :116, :132).
-__device__ __forceinline__ unsigned v_columns(bool vx, unsigned cv, int nv)
-{
-    const int cv1 = (int)(cv & 0xffffu) - 2, cv2 = (int)(cv >> 16) - 2;
-    const bool adm = (unsigned)(cv1 + (int)vx) < (unsigned)(nv + (int)vx);
-    return (unsigned)(adm && cv1 >= 0) | (unsigned)(adm && cv2 < nv) << 1;
-}
-
-// Which of a slab's voxels are in the grid: bits v1w1, v1w2, v2w1, v2w2.
-__device__ __forceinline__ unsigned slab_inside(const ZRay &z, const ZSplit &s, bool vx, unsigned cv, int nv, int nz)
-{
-    const int cw1 = (int)s.i1 - kFloorMagicBits, cw2 = (int)s.i2 - kFloorMagicBits;
-    bool adm = z.live;
-    if (z.steep) {
-        const bool wx = s.i1 != s.i2;
-        adm = adm && (unsigned)(cw1 + (int)wx) < (unsigned)(nz + (int)wx);
-    }
-    const unsigned w = (unsigned)(adm && (unsigned)cw1 < (unsigned)nz) | (unsigned)(adm && (unsigned)cw2 < (unsigned)nz) << 1;
-    const unsigned v = v_columns(vx, cv, nv);
-    return (v & 1u ? w : 0u) | (v & 2u ? w << 2 : 0u);
+    r = mh != m ? __fmul_rn(__fadd_rn(__fadd_rn(mh, -kFloorMagic), -q), iden) : 1.f;
 }
 
 // ---- sinks: what one ray does with a slab's voxels ----
 //
-// f.pair(kind, b, s, ok, wl, wh): voxels (v, w1) with share wl and (v, w2)
-// with share wh of the voxel column at b; ok: bit 0 and 1, whether they are in
-// the grid.
+// The shares of a slab are the overlaps of the ray's v intervals [0, rv], [rv,
+// 1] and z intervals [0, r], [r, 1] (the reference's pairing, Q1): (v1, z1),
+// (v1, z2) or (v2, z1), (v2, z2).  f.inner(vx, p, w): these three voxels, all in
+// the grid; f.edge(kind, p, ok, w): bit i of ok: voxel i is in the grid (a
+// voxel without a share is not touched).
 
 // Slabs without a v crossing; with one and both columns in the grid; with one
 // and a single column in the grid.
@@ -250,32 +221,32 @@ enum SlabKind { kPlain, kCross, kHalf };
 // Forward: sums of value * share, by kind of slab and by aligned block of 32
 // slabs (close() ends a block), so that the total does not depend on which
 // rays walk together; sums of partial sums also round less than one running
-// sum.  SKIP0: voxels of share 0 are not read.
-template <bool SKIP0 = false> struct GatherSink {
+// sum.
+struct GatherSink {
     const float *__restrict__ vol;
-    unsigned sw;
     float sum[3], whole;
 
     __device__ __forceinline__ GatherSink() {}
-    __device__ __forceinline__ GatherSink(const float *v, unsigned sw_) : vol(v), sw(sw_), sum{0.f, 0.f, 0.f}, whole(0.f) {}
-    __device__ __forceinline__ void pair(SlabKind kind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh)
+    __device__ __forceinline__ GatherSink(const float *v) : vol(v), sum{0.f, 0.f, 0.f}, whole(0.f) {}
+    __device__ __forceinline__ void edge(SlabKind kind, const unsigned (&p)[3], unsigned ok, const float (&w)[3])
     {
-        const float lo = (ok & 1u) && (!SKIP0 || wl != 0.f) ? __ldg(vol + (b + s.i1 * sw)) : 0.f;
-        const float hi = (ok & 2u) && (!SKIP0 || wh != 0.f) ? __ldg(vol + (b + s.i2 * sw)) : 0.f;
-        const float acc = kind == kPlain ? sum[0] : kind == kCross ? sum[1] : sum[2];
-        const float v = __fmaf_rn(hi, wh, __fmaf_rn(lo, wl, acc));
-        if (kind == kPlain) sum[0] = v;
-        else if (kind == kCross) sum[1] = v;
-        else sum[2] = v;
+        float s = kind == kPlain ? sum[0] : kind == kCross ? sum[1] : sum[2];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float v = (ok >> i & 1u) && w[i] != 0.f ? __ldg(vol + p[i]) : 0.f;
+            s = __fmaf_rn(v, w[i], s);
+        }
+        if (kind == kPlain) sum[0] = s;
+        else if (kind == kCross) sum[1] = s;
+        else sum[2] = s;
     }
-    // Interior slab: voxels p0, pm and p2 with their shares (of the last two,
-    // those without a share, most of them, are not read).
-    __device__ __forceinline__ void inner(bool vx, unsigned p0, unsigned pm, unsigned p2, float w0, float wm, float w2)
+    // (of the last two, those without a share, most of them, are not read)
+    __device__ __forceinline__ void inner(bool vx, const unsigned (&p)[3], const float (&w)[3])
     {
-        const float v0 = __ldg(vol + p0);
-        const float vm = wm != 0.f ? __ldg(vol + pm) : 0.f;
-        const float v2 = w2 != 0.f ? __ldg(vol + p2) : 0.f;
-        const float v = __fmaf_rn(v2, w2, __fmaf_rn(vm, wm, __fmaf_rn(v0, w0, vx ? sum[1] : sum[0])));
+        const float v0 = __ldg(vol + p[0]);
+        const float v1 = w[1] != 0.f ? __ldg(vol + p[1]) : 0.f;
+        const float v2 = w[2] != 0.f ? __ldg(vol + p[2]) : 0.f;
+        const float v = __fmaf_rn(v2, w[2], __fmaf_rn(v1, w[1], __fmaf_rn(v0, w[0], vx ? sum[1] : sum[0])));
         if (vx) sum[1] = v;
         else sum[0] = v;
     }
@@ -289,19 +260,17 @@ template <bool SKIP0 = false> struct GatherSink {
 // Transpose: one reduction of yw * share per voxel with a share.
 struct ScatterSink {
     float *acc;
-    unsigned sw;
     float yw;
 
-    __device__ __forceinline__ void pair(SlabKind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh) const
+    __device__ __forceinline__ void edge(SlabKind, const unsigned (&p)[3], unsigned ok, const float (&w)[3]) const
     {
-        if ((ok & 1u) && wl != 0.f) atomicAdd(acc + (b + s.i1 * sw), yw * wl);
-        if ((ok & 2u) && wh != 0.f) atomicAdd(acc + (b + s.i2 * sw), yw * wh);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if ((ok >> i & 1u) && w[i] != 0.f) atomicAdd(acc + p[i], yw * w[i]);
     }
-    __device__ __forceinline__ void inner(bool, unsigned p0, unsigned pm, unsigned p2, float w0, float wm, float w2) const
+    __device__ __forceinline__ void inner(bool, const unsigned (&p)[3], const float (&w)[3]) const
     {
-        if (w0 != 0.f) atomicAdd(acc + p0, yw * w0);
-        if (wm != 0.f) atomicAdd(acc + pm, yw * wm);
-        if (w2 != 0.f) atomicAdd(acc + p2, yw * w2);
+        edge(kPlain, p, 7u, w);
     }
     __device__ __forceinline__ void close() const {}
 };
@@ -310,104 +279,81 @@ struct ScatterSink {
 // two (exact) and rounded to a 64-bit integer (siddon.cuh, to_fixed).
 struct FixedSink {
     unsigned long long *acc;
-    unsigned sw;
     float yw, scale;
 
-    __device__ __forceinline__ void pair(SlabKind, unsigned b, const ZSplit &s, unsigned ok, float wl, float wh) const
+    __device__ __forceinline__ void edge(SlabKind, const unsigned (&p)[3], unsigned ok, const float (&w)[3]) const
     {
-        if ((ok & 1u) && wl != 0.f) atomicAdd(acc + (b + s.i1 * sw), (unsigned long long)to_fixed((yw * wl) * scale));
-        if ((ok & 2u) && wh != 0.f) atomicAdd(acc + (b + s.i2 * sw), (unsigned long long)to_fixed((yw * wh) * scale));
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if ((ok >> i & 1u) && w[i] != 0.f)
+                atomicAdd(acc + p[i], (unsigned long long)to_fixed((yw * w[i]) * scale));
     }
-    __device__ __forceinline__ void inner(bool, unsigned p0, unsigned pm, unsigned p2, float w0, float wm, float w2) const
+    __device__ __forceinline__ void inner(bool, const unsigned (&p)[3], const float (&w)[3]) const
     {
-        if (w0 != 0.f) atomicAdd(acc + p0, (unsigned long long)to_fixed((yw * w0) * scale));
-        if (wm != 0.f) atomicAdd(acc + pm, (unsigned long long)to_fixed((yw * wm) * scale));
-        if (w2 != 0.f) atomicAdd(acc + p2, (unsigned long long)to_fixed((yw * w2) * scale));
+        edge(kPlain, p, 7u, w);
     }
     __device__ __forceinline__ void close() const {}
 };
 
-// One slab of one ray, range checked (also right for interior slabs).
-template <bool REF, class Sink>
-__device__ __forceinline__ void ray_slab(const ZRay &z, const ZGrid &zg, float d, float dh, unsigned b1, unsigned b2,
-                                         float rv, unsigned cv, int nv, Sink &f)
-{
-    const ZSplit s = z_split<REF>(z, zg, d, dh);
-    const bool four = b1 != b2;
-    const unsigned ok = slab_inside(z, s, four, cv, nv, zg.nz);
-    if (!four) {
-        f.pair(kPlain, b1, s, ok, s.rw, __fsub_rn(1.f, s.rw));
-    } else {
-        const Shares h = slab_shares(rv, s.rw);
-        const SlabKind kind = v_columns(true, cv, nv) == 3u ? kCross : kHalf;
-        if (ok & 3u) f.pair(kind, b1, s, ok, h.w11, h.w12);
-        if (ok & 12u) f.pair(kind, b2, s, ok >> 2, h.w21, h.w22);
-    }
-}
-
-// Slabs k..end of one ray alone (any strides): every slab's v part evaluated by
-// the thread, with a column warp's operations per slab, so with its bits.
-template <bool REF, class Sink>
-__device__ __forceinline__ void ray_each(const ColWalk &c, const ZRay &z, const ZGrid &zg, unsigned sw, Sink &f, int k,
-                                         int end)
-{
-#pragma unroll 1
-    for (; k <= end; ++k) {
-        const ColEntry e = col_entry(c, k, sw);
-        const float a = col_plane(c, k), b = col_plane(c, k + 1);
-        ray_slab<REF>(z, zg, z.down ? b : a, z.down ? a : b, e.b1, e.b2, e.rv, e.cv, c.nv, f);
-        if ((k & 31) == 31) f.close();
-    }
-}
-
-// The thread walk's interior slabs (ki0..ki1): no range checks, v positions and
-// floors carried from plane to plane, a slab without a v crossing taken as one
-// with rv = 1 (its third voxel has no share).  DOWN: v falls along the walk.
-// Bound by issue and the gathers' latency; 256^3, 72 views of 512 x 384: forward
-// 6.2 ms with the y-fastest copy and 7.5 without, transpose 6.6 and 12.3 (every
-// slab range checked and evaluated anew: 17.0, 17.5, 15.2 and 15.1; the walk that
-// evaluates the z position as the reference does, and sums in one pass: 5.6,
-// 6.5, 8.1 and 12.1, with other bits than the column warps).
-template <bool REF, bool DOWN, class Sink>
-__device__ __forceinline__ void ray_inner(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
+// Slabs k..end of one ray alone (any strides), with a column warp's operations
+// per slab, so with its bits; v positions and floors are carried from plane to
+// plane.  CHECK: range checks, any slope; else every voxel is in the grid and
+// the ray is not steep, DOWN: v falls along the walk.  A slab without a v
+// crossing is taken as one with rv = 1 (its third voxel has no share).  The
+// high column is the one at the slab's far plane: where dv < 1 it need not be
+// the low one's neighbour.
+template <bool REF, bool CHECK, bool DOWN, int DIV, class Sink>
+__device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
                                           Sink &f)
 {
-    auto vpos = [&](float d) {
-        float q = __fadd_rn(c.pv, __fmul_rn(c.kv, d));
-        if (c.vdiv) q = __fdiv_rn(q, c.dv);
-        return __fadd_rn(q, c.nv2);
-    };
+    const Inside vin(c.nv), zin(zg.nz);
     float t = __fsub_rn((float)k, c.nu2), da = __fsub_rn(t, c.pu);
-    float qa = vpos(da), ma = magic_floor<false>(qa);
+    float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa);
     unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + sw);
+    auto slab = [&]() {
+        t = __fadd_rn(t, 1.f);
+        const float db = __fsub_rn(t, c.pu), qb = col_vpos<DIV>(c, db), mb = magic_floor<CHECK>(qb);
+        const float q1 = CHECK ? fminf(qa, qb) : DOWN ? qb : qa, q2 = CHECK ? fmaxf(qa, qb) : DOWN ? qa : qb;
+        const float m1 = CHECK ? fminf(ma, mb) : DOWN ? mb : ma, m2 = CHECK ? fmaxf(ma, mb) : DOWN ? ma : mb;
+        const bool vx = m1 != m2;
+        const float rv = col_ratio(q1, q2, m1, m2);
+        const float lo = z.down ? db : da, hi = z.down ? da : db;
+        float m, mh, r;
+        if constexpr (CHECK) z_split<REF>(z, zg, lo, hi, m, mh, r);
+        else z_inner<REF>(z, zg, lo, hi, m, r);
+        const unsigned z1 = base + (unsigned)__float_as_int(m) * sw;
+        const unsigned up = CHECK ? (unsigned)(__float_as_int(mh) - __float_as_int(m)) * sw : sw;
+        const unsigned v1 = z1 + (unsigned)__float_as_int(m1) * c.sv, v2 = z1 + (unsigned)__float_as_int(m2) * c.sv;
+        const bool vfirst = rv > r;             // the middle voxel is (v1, z2), else (v2, z1)
+        const unsigned p[3] = {v1, vfirst ? v1 + up : v2, v2 + up};
+        const float both = fminf(rv, r), over = __fsub_rn(r, both);      // r's share in the high column
+        const float w[3] = {both, fabsf(__fsub_rn(rv, r)), __fsub_rn(__fsub_rn(1.f, rv), over)};
+        if constexpr (CHECK) {
+            const bool a = vin.low(m1), b = vx && vin.far(m1, m2), l = zin.low(m), h = zin.far(m, mh);
+            f.edge(!vx ? kPlain : a && b ? kCross : kHalf, p,
+                   (unsigned)(a && l) | (unsigned)(vfirst ? a && h : b && l) << 1 | (unsigned)(b && h) << 2, w);
+        } else {
+            f.inner(vx, p, w);
+        }
+        base += c.su;
+        da = db;
+        qa = qb;
+        ma = mb;
+    };
     while (k <= end) {
         const int last = min(k | 31, end);
+        if constexpr (CHECK) {
+#pragma unroll 1
+            for (; k <= last; ++k) slab();
+        } else {
 #pragma unroll 4
-        for (; k <= last; ++k) {
-            t = __fadd_rn(t, 1.f);
-            const float db = __fsub_rn(t, c.pu), qb = vpos(db), mb = magic_floor<false>(qb);
-            const float q1 = DOWN ? qb : qa, q2 = DOWN ? qa : qb, m1 = DOWN ? mb : ma, m2 = DOWN ? ma : mb;
-            const bool vx = m1 != m2;
-            const float rv = vx ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1), __fadd_rn(q2, -q1)) : 1.f;
-            float m, r;
-            z_inner<REF>(z, zg, z.down ? db : da, z.down ? da : db, m, r);
-            const float both = fminf(rv, r), over = __fsub_rn(r, both);      // r's share in the high column
-            // (the high column is the one at the slab's far plane: where dv < 1 it
-            // need not be the low one's neighbour)
-            const unsigned row = base + (unsigned)__float_as_int(m) * sw;
-            const unsigned p0 = row + (unsigned)__float_as_int(m1) * c.sv, ph = row + (unsigned)__float_as_int(m2) * c.sv;
-            f.inner(vx, p0, rv > r ? p0 + sw : ph, ph + sw, both, fabsf(__fsub_rn(rv, r)),
-                    __fsub_rn(__fsub_rn(1.f, rv), over));
-            base += c.su;
-            da = db;
-            qa = qb;
-            ma = mb;
+            for (; k <= last; ++k) slab();
         }
         if ((last & 31) == 31) f.close();
     }
 }
 
-// The thread walk.
+// The thread walk: the slabs k0..k1 of a ray, of them ki0..ki1 without range checks.
 template <bool REF, class Sink>
 __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<float> &w, unsigned su, unsigned sv,
                                          unsigned sw, Sink &f)
@@ -416,11 +362,21 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
     const ZGrid zg = z_grid(g);
     const ZRay z = z_ray(w, zg, true);
     const bool interior = !z.steep && w.ki0 <= w.ki1;
-    ray_each<REF>(c, z, zg, sw, f, w.k0, interior ? w.ki0 - 1 : w.k1);
-    if (interior) {
-        if (c.kv < 0.f) ray_inner<REF, true>(c, z, zg, w.ki0, w.ki1, sw, f);
-        else ray_inner<REF, false>(c, z, zg, w.ki0, w.ki1, sw, f);
-        ray_each<REF>(c, z, zg, sw, f, w.ki1 + 1, w.k1);
+    int k = w.k0, end = interior ? w.ki0 - 1 : w.k1;
+#pragma unroll 1
+    for (;;) {
+        ray_slabs<REF, true, false, -1>(c, z, zg, k, end, sw, f);
+        if (end == w.k1) break;
+        if (c.vdiv) {
+            if (c.kv < 0.f) ray_slabs<REF, false, true, 1>(c, z, zg, w.ki0, w.ki1, sw, f);
+            else ray_slabs<REF, false, false, 1>(c, z, zg, w.ki0, w.ki1, sw, f);
+        } else {
+            if (c.kv < 0.f) ray_slabs<REF, false, true, 0>(c, z, zg, w.ki0, w.ki1, sw, f);
+            else ray_slabs<REF, false, false, 0>(c, z, zg, w.ki0, w.ki1, sw, f);
+        }
+        if (w.ki1 == w.k1) break;
+        k = w.ki1 + 1;
+        end = w.k1;
     }
     f.close();
 }
@@ -510,10 +466,10 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
                                               ColTable &tab)
 {
     const int lane = threadIdx.x & 31, k = kc + lane;
-    const ColEntry e = col_entry(cw, k, 1u);
+    const ColEntry e = col_entry(cw, k);
     const float da = col_plane(cw, k), db = col_plane(cw, k + 1);
-    const bool vx = e.b1 != e.b2;
-    const unsigned in = k >= K0 && k <= K1 ? v_columns(vx, e.cv, cw.nv) : 0u;
+    const bool vx = e.vx;
+    const unsigned in = k >= K0 && k <= K1 ? e.in : 0u;
     const bool is_plain = !vx && in != 0u, is_cross = vx && in == 3u, is_half = vx && (in == 1u || in == 2u);
     const unsigned plain = __ballot_sync(0xffffffffu, is_plain), cross = __ballot_sync(0xffffffffu, is_cross);
     const unsigned half = __ballot_sync(0xffffffffu, is_half), below = (1u << lane) - 1u;
@@ -539,29 +495,13 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
     return h;
 }
 
-// Every slab of one ray per lane, range checked: warps that the walks below
-// do not take (steep rays), and the deterministic transpose.
+// Every slab of one ray per lane, range checked: warps that the walks below do
+// not take (steep rays, and the transpose's values that are not finite).
 template <bool REF, class Sink>
 __device__ __forceinline__ void col_each(const ColWalk &cw, int K0, int K1, const ZRay &z, const ZGrid &zg, Sink &f)
 {
-    ColTable &tab = col_table();
-    const int lane = threadIdx.x & 31;
-    for (int kc = K0 & ~31; kc <= K1; kc += 32) {
-        const ColEntry e = col_entry(cw, kc + lane, 1u);
-        __syncwarp();
-        tab.a[lane] = make_uint4(e.b1, e.b2, __float_as_uint(e.rv), e.cv);
-        tab.d[lane] = make_float2(col_plane(cw, kc + lane), col_plane(cw, kc + lane + 1));
-        __syncwarp();
-        const int n = min(K1 - kc + 1, 32);
-#pragma unroll 1
-        for (int j = max(K0 - kc, 0); j < n; ++j) {
-            const uint4 te = tab.a[j];
-            const float2 d = tab.d[j];
-            ray_slab<REF>(z, zg, z.down ? d.y : d.x, z.down ? d.x : d.y, te.x, te.y, __uint_as_float(te.z), te.w, cw.nv,
-                          f);
-        }
-        f.close();
-    }
+    if (z.live) ray_slabs<REF, true, false, -1>(cw, z, zg, K0, K1, 1u, f);
+    f.close();
 }
 
 // Voxel of biased floor m in the column at the table's address (lo, hi).
@@ -569,14 +509,6 @@ template <typename T = float> __device__ __forceinline__ T *col_voxel(unsigned l
 {
     return reinterpret_cast<T *>(((unsigned long long)hi << 32 | lo) + sizeof(T) * (unsigned)__float_as_int(m));
 }
-
-// Whether the voxel of biased floor m, and the one above it, are in the grid.
-struct ZInside {
-    float lo, hi;           // biased floors 0 and nz
-    __device__ __forceinline__ ZInside(int nz) : lo(kFloorMagic), hi(kFloorMagic + (float)nz) {}
-    __device__ __forceinline__ bool low(float m) const { return m >= lo && m < hi; }
-    __device__ __forceinline__ bool high(float m) const { return m >= lo - 1.f && m < hi - 1.f; }
-};
 
 // The transpose's accumulators: floats, or 64-bit integers of yw * share times
 // a power of two (exact), rounded (the deterministic transpose: integer sums
@@ -629,9 +561,9 @@ __device__ __forceinline__ void col_planes(const ColTable &tab, int j, const uin
 // overlap.  ZCHK: z range checks.
 template <int R, bool REF, bool MIXED, bool ZCHK>
 __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
-                                                GatherSink<> (&f)[R])
+                                                GatherSink (&f)[R])
 {
-    const ZInside in(q.zg.nz);
+    const Inside in(q.zg.nz);
     auto load = [&](const float *p, float m, float &a, float &b) {
         a = !ZCHK || in.low(m) ? __ldg(p) : 0.f;
         b = !ZCHK || in.high(m) ? __ldg(p + 1) : 0.f;
@@ -683,7 +615,7 @@ __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTa
 
 // Forward of the lane's R rays (not steep): sums into f.
 template <int R, bool REF, bool MIXED>
-__device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__restrict__ vol, GatherSink<> (&f)[R])
+__device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__restrict__ vol, GatherSink (&f)[R])
 {
     ColTable &tab = col_table();
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
@@ -710,7 +642,7 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
                                                  const Acc &acc, const float (&y)[R])
 {
     using T = typename Acc::T;
-    const ZInside in(q.zg.nz);
+    const Inside in(q.zg.nz);
     // values l, u of the low and high voxels of rays i.. in one voxel column
     constexpr int S = MERGE == kSingle ? 1 : R;
     auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], T (&l)[S], T (&u)[S]) {

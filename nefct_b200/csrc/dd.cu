@@ -227,7 +227,7 @@ template <bool FWD, DDMode MODE>
 __device__ __forceinline__ void dd_rows(const DDTable &tab, int single, int n, int nz, const float (&rz)[2],
                                         const float (&y)[2], float (&acc)[2])
 {
-    const ZInside in(nz);
+    const Inside in(nz);
     if constexpr (MODE == kWide) {
 #pragma unroll 1
         for (int j = 0; j < n; ++j) {

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_con
     const unsigned sw = (unsigned)(p.g.nx * p.g.ny);
     unsigned su, sv;
     thread_strides(p.g.nx, p.g.ny, w.xdrive, p.fixT != nullptr, su, sv);
-    FixedSink f{w.xdrive && p.fixT ? p.fixT : p.fix, sw, y * w.W, *p.fix_scale};
+    FixedSink f{w.xdrive && p.fixT ? p.fixT : p.fix, y * w.W, *p.fix_scale};
     if (ref_rounding(p.flags)) ray_walk<true>(p.g, w, su, sv, sw, f);
     else ray_walk<false>(p.g, w, su, sv, sw, f);
 }

@@ -154,3 +154,26 @@ def test_two_slices_and_lanes_without_a_ray(cuda, oracle_lib, rows, flags):
     f, b = _both(g, torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda), flags, 3)
     assert_parity(f.cpu().numpy(), ref_f)
     assert_parity(b.cpu().numpy(), ref_b)
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("shape,angle", [((65600, 3, 2), np.pi / 2), ((3, 65600, 2), 0.0)], ids=["wide", "deep"])
+def test_grids_wider_than_65536(cuda, oracle_lib, shape, angle, flags):
+    """Rays that pass the far end of an axis of 65600 voxels, across it (the
+    thread walk: column warps take at most 65535)."""
+    ang = np.array([angle, angle + 5e-4, angle + np.pi, angle + np.pi + 5e-4], np.float32)
+    g = nb.ConeBeam(shape, ang, 1e5, 2e5, 40, 10.0, 3, 0.4, a_shift=6560.0)
+    og = oracle_lib.grid(g.shape, g.center, g.size)
+    args = (g.angles, g.src_iso, g.src_det, g.na, g.da, g.a_shift, g.nb, g.db, g.b_shift)
+    of = oracle_lib.CB_BP if flags else oracle_lib.CB_FWD
+    rng = np.random.default_rng(2)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    ref_f = oracle_lib.cb_forward(og, vol, *args, flags=of)[0]
+    ref_b = oracle_lib.cb_backward(og, y, *args, flags=of)
+    assert 0.3 < (ref_f != 0).mean() < 0.9             # rays on both sides of the end
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    for extra in (0, _lib.NO_TRANSPOSE):
+        assert_parity(ops.cb_forward(v, g, flags | extra).cpu().numpy(), ref_f)
+        assert_parity(ops.cb_backward(s, g, flags | extra).cpu().numpy(), ref_b)
+        assert_parity(ops.cb_backward(s, g, flags | extra | _lib.DETERMINISTIC).cpu().numpy(), ref_b)
