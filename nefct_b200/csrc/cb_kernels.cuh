@@ -195,7 +195,7 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
             h[i] = row(i, r[i]);
             has |= (unsigned)h[i] << i;
         }
-        if (!col_rays<R>(g, r, h, flags, q)) {
+        if (!col_rays<R, true>(g, r, h, flags, q)) {
 #pragma unroll
             for (int i = 0; i < R; ++i)
                 if (h[i]) store(i, 0.f);
@@ -241,7 +241,7 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
     ColRays<R> q;
 #pragma unroll
     for (int i = 0; i < R; ++i) has[i] = has[i] && y[i] != 0.f;
-    if (!col_rays<R>(g, r, has, flags, q)) return;
+    if (!col_rays<R, false>(g, r, has, flags, q)) return;
     float yw[R];
     bool finite = true;
 #pragma unroll

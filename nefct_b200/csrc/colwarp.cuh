@@ -170,34 +170,44 @@ __device__ __forceinline__ float z_pos(const ZRay &z, const ZGrid &zg, float d)
     return __fadd_rn(q, zg.nz2);
 }
 
-// z split of a slab of a ray that is not steep: biased floor and low share.
+// Position at plane offset d.
+template <bool REF> __device__ __forceinline__ float z_at(const ZRay &z, const ZGrid &zg, float d)
+{
+    return REF ? z_pos(z, zg, d) : __fmaf_rn(z.kz, d, z.z0);
+}
+
+// z split of a slab of a ray that is not steep: biased floor and low share.  q,
+// qh: positions at its lower and upper plane (qh: REF only).
 // (The grid has at most 2^20 rows and slabs, and such a ray moves at most one
 // row per slab: positions stay below 2^22, no clamp is needed for the floor.)
-template <bool REF>
-__device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &r)
+template <bool REF> __device__ __forceinline__ void z_share(const ZRay &z, float q, float qh, float &m, float &r)
 {
-    const float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
     m = __fadd_rd(q, kFloorMagic);
     if (REF) {
         const float c = __fadd_rn(m, 1.f - kFloorMagic);
-        r = __saturatef(__fmul_rn(__fadd_rn(c, -q), rcp_approx(__fadd_rn(z_pos(z, zg, hi), -q))));
+        r = __saturatef(__fmul_rn(__fadd_rn(c, -q), rcp_approx(__fadd_rn(qh, -q))));
     } else {
         r = __saturatef(__fmaf_rn(__fadd_rn(__fadd_rn(m, -kFloorMagic), -q), z.ikz, z.ikz));
     }
 }
 
-// z split of any ray's slab: biased floors of its low and high voxel and the low
-// share.  lo, hi: offsets of the lower and upper plane.
+// The same from the offsets of the lower and upper plane.
 template <bool REF>
-__device__ __forceinline__ void z_split(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &mh, float &r)
+__device__ __forceinline__ void z_inner(const ZRay &z, const ZGrid &zg, float lo, float hi, float &m, float &r)
+{
+    z_share<REF>(z, z_at<REF>(z, zg, lo), REF ? z_pos(z, zg, hi) : 0.f, m, r);
+}
+
+// z split of any ray's slab: biased floors of its low and high voxel and the low
+// share.  q, qh: positions at the lower and upper plane (qh: REF or steep only).
+template <bool REF>
+__device__ __forceinline__ void z_split(const ZRay &z, float q, float qh, float &m, float &mh, float &r)
 {
     if (!z.steep) {
-        z_inner<REF>(z, zg, lo, hi, m, r);
+        z_share<REF>(z, q, qh, m, r);
         mh = __fadd_rn(m, 1.f);
         return;
     }
-    float q = REF ? z_pos(z, zg, lo) : __fmaf_rn(z.kz, lo, z.z0);
-    float qh = REF ? z_pos(z, zg, hi) : __fmaf_rn(z.kz, hi, z.z0);
     m = magic_floor<true>(q);
     mh = magic_floor<true>(qh);
     q = fminf(fmaxf(q, -kFloorClamp), kFloorClamp);
@@ -308,7 +318,7 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
 {
     const Inside vin(c.nv), zin(zg.nz);
     float t = __fsub_rn((float)k, c.nu2), da = __fsub_rn(t, c.pu);
-    float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa);
+    float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa), za = z_at<REF>(z, zg, da);
     unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + sw);
     auto slab = [&]() {
         t = __fadd_rn(t, 1.f);
@@ -317,10 +327,10 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
         const float m1 = CHECK ? fminf(ma, mb) : DOWN ? mb : ma, m2 = CHECK ? fmaxf(ma, mb) : DOWN ? ma : mb;
         const bool vx = m1 != m2;
         const float rv = col_ratio(q1, q2, m1, m2);
-        const float lo = z.down ? db : da, hi = z.down ? da : db;
+        const float zb = z_at<REF>(z, zg, db), zl = z.down ? zb : za, zh = z.down ? za : zb;
         float m, mh, r;
-        if constexpr (CHECK) z_split<REF>(z, zg, lo, hi, m, mh, r);
-        else z_inner<REF>(z, zg, lo, hi, m, r);
+        if constexpr (CHECK) z_split<REF>(z, zl, zh, m, mh, r);
+        else z_share<REF>(z, zl, zh, m, r);
         const unsigned z1 = base + (unsigned)__float_as_int(m) * sw;
         const unsigned up = CHECK ? (unsigned)(__float_as_int(mh) - __float_as_int(m)) * sw : sw;
         const unsigned v1 = z1 + (unsigned)__float_as_int(m1) * c.sv, v2 = z1 + (unsigned)__float_as_int(m2) * c.sv;
@@ -339,6 +349,7 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
         da = db;
         qa = qb;
         ma = mb;
+        za = zb;
     };
     while (k <= end) {
         const int last = min(k | 31, end);
@@ -396,8 +407,10 @@ template <int R> struct ColRays {
 };
 
 // Rays r (the whole warp calls it; has: the lane has the ray and it takes
-// part); false when no ray of the warp contributes.
-template <int R>
+// part); false when no ray of the warp contributes.  UPPER: slabs without range
+// checks touch a low voxel's upper neighbour whether it has a share or not (the
+// forward's loads; the transpose's reductions skip it).
+template <int R, bool UPPER>
 __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&r)[R][6], const bool (&has)[R],
                                          uint32_t flags, ColRays<R> &q)
 {
@@ -419,8 +432,8 @@ __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&
             any = true;
             k0 = min(k0, w.k0);
             k1 = max(k1, w.k1);
-            zi0 = max(zi0, w.zi0);
-            zi1 = min(zi1, w.zi1);
+            zi0 = max(zi0, UPPER ? w.zu0 : w.zi0);
+            zi1 = min(zi1, UPPER ? w.zu1 : w.zi1);
             up = up || !q.z[i].down;
             down = down || q.z[i].down;
             steep = steep || q.z[i].steep;

@@ -106,7 +106,8 @@ template <typename T> struct Walk {
     T W, Wmid;           // contribution weights (Wmid: three-voxel middle slot, Q5)
     int nu, nv, k0, k1;  // slab count, transverse extent, inclusive slab range
     int ki0, ki1;        // interior slabs: every candidate voxel is inside the grid
-    int zi0, zi1;        // slabs whose low z voxel and its upper neighbour are inside the grid
+    int zi0, zi1;        // slabs whose z voxels (those with a share) are inside the grid
+    int zu0, zu1;        // slabs whose low z voxel and its upper neighbour are inside the grid
     bool xdrive, vdiv;
 };
 
@@ -180,9 +181,12 @@ __device__ __forceinline__ bool setup_walk(const GridDev<T> &g, const T *r, uint
     w.ki0 = 0; w.ki1 = w.nu - 1;
     const T kvv = w.vdiv ? w.kv / w.dv : w.kv, v0 = (w.vdiv ? w.pv / w.dv : w.pv) + w.nv2;
     clip_axis<T>(v0, kvv, w.nv, w.nv, w.pu, w.nu2, w.nu, w.k0, w.k1, w.ki0, w.ki1);
-    // (top row nz - 1: such a slab reads its low voxel's upper neighbour too)
     w.zi0 = 0; w.zi1 = w.nu - 1;
-    clip_axis<T>(w.z0, w.kz, g.nz, g.nz - 1, w.pu, w.nu2, w.nu, w.k0, w.k1, w.zi0, w.zi1);
+    clip_axis<T>(w.z0, w.kz, g.nz, g.nz, w.pu, w.nu2, w.nu, w.k0, w.k1, w.zi0, w.zi1);
+    // (top row nz - 1: slabs that read their low voxel's upper neighbour whether it
+    // has a share or not)
+    w.zu0 = 0; w.zu1 = w.nu - 1;
+    clip_axis<T>(w.z0, w.kz, g.nz, g.nz - 1, w.pu, w.nu2, w.nu, w.k0, w.k1, w.zu0, w.zu1);
     w.k0 = max(w.k0, 0);
     w.k1 = min(w.k1, w.nu - 1);
     w.ki0 = max(max(w.ki0, w.zi0), w.k0);
