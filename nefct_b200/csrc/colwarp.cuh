@@ -88,10 +88,13 @@ template <int DIV = -1> __device__ __forceinline__ float col_vpos(const ColWalk 
     return __fadd_rn(q, c.nv2);
 }
 
-// Crossing ratio of a slab with v positions q1 <= q2 and biased floors m1, m2.
+// Crossing ratio of a slab with v positions q1 <= q2 and biased floors m1, m2; at
+// most 1 (the approximate reciprocal can pass it by an ulp, and would give a
+// share to a voxel that the ray does not touch, outside the grid at its faces).
 __device__ __forceinline__ float col_ratio(float q1, float q2, float m1, float m2)
 {
-    return m1 != m2 ? FP<float>::ratio(__fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1), __fadd_rn(q2, -q1)) : 1.f;
+    const float num = __fadd_rn(__fadd_rn(m2, -kFloorMagic), -q1);
+    return m1 != m2 ? __saturatef(__fmul_rn(num, rcp_approx(__fadd_rn(q2, -q1)))) : 1.f;
 }
 
 // Whether a voxel of biased floor m, and the one above it, are among n.

@@ -177,3 +177,43 @@ def test_grids_wider_than_65536(cuda, oracle_lib, shape, angle, flags):
         assert_parity(ops.cb_forward(v, g, flags | extra).cpu().numpy(), ref_f)
         assert_parity(ops.cb_backward(s, g, flags | extra).cpu().numpy(), ref_b)
         assert_parity(ops.cb_backward(s, g, flags | extra | _lib.DETERMINISTIC).cpu().numpy(), ref_b)
+
+
+@pytest.mark.parametrize("walk", [0, 3], ids=["thread", "columns"])
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT, _lib.NO_TRANSPOSE, _lib.DETERMINISTIC],
+                         ids=["default", "reference-rounding", "direct", "deterministic"])
+@pytest.mark.parametrize("nz", [1, 2])
+def test_nothing_outside_the_buffers_is_touched(cuda, nz, flags, walk):
+    """Volume, sinogram and workspace between NaN (inputs) or a mark (outputs):
+    rays in the grid's last slice touch no voxel above it, whatever the rounding
+    of their crossing ratios."""
+    import ctypes as C
+    g = nb.ConeBeam((200, 200, nz), np.linspace(0, 2 * np.pi, 90, endpoint=False), 300.0, 600.0, 310, 1.0, 1, 1.0,
+                    z_offsets=np.full(90, 0.5 * nz - 0.5))
+    pad, s, lib = 1 << 17, g.struct(), _lib.load()
+    stream = torch.cuda.current_stream(cuda).cuda_stream
+    wn = lib.nefct_cb_workspace_bytes(C.byref(s), flags)
+    assert wn % 4 == 0
+
+    def inside(n, fill):
+        t = torch.full((n + 2 * pad,), fill, device=cuda)
+        return t, t[pad:pad + n]
+
+    vol_all, vol = inside(200 * 200 * nz, np.nan)
+    ws_all, ws = inside(max(wn // 4, 1), np.nan)
+    out_all, out = inside(90 * 310, 7.0)
+    vol.copy_(torch.rand(vol.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)))
+    back_all, back = inside(vol.numel(), 7.0)
+    y = torch.rand(out.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(5))
+    saved = autotune.current()
+    try:
+        autotune.apply(saved["rows"], saved["order"], walk)
+        _lib.check(lib.nefct_cb_forward(C.byref(s), vol.data_ptr(), out.data_ptr(), flags, ws.data_ptr(), wn, stream))
+        assert torch.isfinite(out).all() and out.any()
+        ws_all.fill_(7.0)
+        _lib.check(lib.nefct_cb_backward(C.byref(s), y.data_ptr(), back.data_ptr(), flags, ws.data_ptr(), wn, stream))
+    finally:
+        autotune.apply(saved["rows"], saved["order"], saved["walk"])
+    assert torch.isfinite(back).all() and back.any()
+    for t in (ws_all, out_all, back_all):
+        assert (t[:pad] == 7.0).all() and (t[-pad:] == 7.0).all()
