@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(256) batch_zcopy_kernel(const __grid_constant_
 }
 
 // One persistent launch serves the tiles [begin, end).
-template <bool FWD>
+template <bool FWD, bool REF>
 __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ BatchArgs a)
 {
     __shared__ long long s_item;
@@ -177,11 +177,11 @@ __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ Batc
         cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, ib, r);
         const size_t id = ((size_t)iv * P.nb + ib) * P.na + ia;
         if (FWD) {
-            P.sino[id] = ray_forward<float, false>(P.g, r, P.flags, P.vol, P.volT);
+            P.sino[id] = ray_forward<float, REF>(P.g, r, P.flags, P.vol, P.volT);
         } else {
             const float y = P.grad[id];
             if (y == 0.f) continue;
-            ray_backward<float, false>(P.g, r, P.flags, y, P.back, P.volT);
+            ray_backward<float, REF>(P.g, r, P.flags, y, P.back, P.volT);
         }
     }
 }
@@ -321,15 +321,17 @@ static nefct_status batch_launch(BatchPlan *b, bool fwd, cudaStream_t s)
     const dim3 blk(32, b->rows);
     BatchArgs &a = *b->args;
     a.begin = 0; a.end = total; a.counter = counter;
+    const bool ref = ref_rounding(b->flags);
     if (b->colwarp) {
-        const bool ref = ref_rounding(b->flags);
         if (fwd && ref) batch_colwarp_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
         else if (fwd) batch_colwarp_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
         else if (ref) batch_colwarp_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
         else batch_colwarp_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
     } else {
-        if (fwd) batch_kernel<true><<<b->grid_blocks, blk, 0, s>>>(a);
-        else batch_kernel<false><<<b->grid_blocks, blk, 0, s>>>(a);
+        if (fwd && ref) batch_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
+        else if (fwd) batch_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
+        else if (ref) batch_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
+        else batch_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
     }
     NEFCT_CHECK_LAUNCH("batch_kernel");
     if (!fwd && b->colwarp) {
@@ -472,7 +474,9 @@ nefct_status nefct_cb_batch_bind(nefct_cb_batch *b, void *workspace, size_t byte
     NEFCT_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int lo = 1 << 30;
     const bool ref = ref_rounding(b->flags);
-    const void *kernels[2] = {(const void *)batch_kernel<true>, (const void *)batch_kernel<false>};
+    const void *kernels[2] = {
+        ref ? (const void *)batch_kernel<true, true> : (const void *)batch_kernel<true, false>,
+        ref ? (const void *)batch_kernel<false, true> : (const void *)batch_kernel<false, false>};
     const void *colwarp_kernels[2] = {
         ref ? (const void *)batch_colwarp_kernel<true, true> : (const void *)batch_colwarp_kernel<true, false>,
         ref ? (const void *)batch_colwarp_kernel<false, true> : (const void *)batch_colwarp_kernel<false, false>};

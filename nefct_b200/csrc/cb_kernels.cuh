@@ -87,8 +87,8 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
     const ZRay z = z_ray(w, zg, true);
-    if (ref_rounding(flags)) ray_slabs<true, true, false, -1>(c, z, zg, w.k0, w.k1, sw, f);
-    else ray_slabs<false, true, false, -1>(c, z, zg, w.k0, w.k1, sw, f);
+    if (ref_rounding(flags)) ray_slabs<true, true, false, -1, true>(c, z, zg, w.k0, w.k1, sw, f);
+    else ray_slabs<false, true, false, -1, true>(c, z, zg, w.k0, w.k1, sw, f);
     f.close();
     return f.whole * w.W;
 }
@@ -102,9 +102,9 @@ __device__ __forceinline__ void thread_strides(int nx, int ny, bool xdrive, bool
 }
 
 // Forward value of one ray: gathers x-driven rays from the y-fastest copy
-// volT when there is one, everything else from the x-fastest volume.  DIV
-// (double only): the voxels are not cubic.
-template <typename T, bool DIV, bool EXACT = false>
+// volT when there is one (COPY: there is), everything else from the x-fastest
+// volume.  VAR: float: the reference's rounding; double: the voxels are not cubic.
+template <typename T, bool VAR, bool EXACT = false, bool COPY = true>
 __device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32_t flags, const T *vol, const T *volT)
 {
     if (EXACT) return exact_forward(g, r, flags, vol, volT);
@@ -112,25 +112,24 @@ __device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32
     if (!setup_walk(g, r, flags, w)) return (T)0;
     const int sw = g.nx * g.ny;
     if constexpr (std::is_same<T, float>::value) {
-        const float *const v = w.xdrive && volT ? volT : vol;
+        const float *const v = COPY && w.xdrive ? volT : vol;
         unsigned su, sv;
-        thread_strides(g.nx, g.ny, w.xdrive, volT != nullptr, su, sv);
+        thread_strides(g.nx, g.ny, w.xdrive, COPY, su, sv);
         GatherSink f(v);
-        if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
-        else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
+        ray_walk<VAR, COPY>(g, w, su, sv, (unsigned)sw, f);
         const float sum = f.whole;
         if (!isfinite(sum)) return ray_resum(g, r[0], r[1], r[2], r[3], r[4], r[5], flags, v, su, sv, (unsigned)sw);
         return sum * w.W;
     } else {
-        if (!w.xdrive) return gather_walk<T, DIV, true, false>(w, g, vol, g.nx, 1, sw);
-        if (volT) return gather_walk<T, DIV, true, false>(w, g, volT, g.ny, 1, sw);
-        return gather_walk<T, DIV, false, false>(w, g, vol, 1, g.nx, sw);
+        if (!w.xdrive) return gather_walk<T, VAR, true, false>(w, g, vol, g.nx, 1, sw);
+        if (volT) return gather_walk<T, VAR, true, false>(w, g, volT, g.ny, 1, sw);
+        return gather_walk<T, VAR, false, false>(w, g, vol, 1, g.nx, sw);
     }
 }
 
 // Transpose contribution of one ray with value y: x-driven rays reduce into
 // the y-fastest accumulator outT when there is one.
-template <typename T, bool DIV, bool EXACT = false>
+template <typename T, bool VAR, bool EXACT = false>
 __device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, uint32_t flags, T y, T *out, T *outT)
 {
     if (EXACT) {
@@ -144,16 +143,15 @@ __device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, ui
         unsigned su, sv;
         thread_strides(g.nx, g.ny, w.xdrive, outT != nullptr, su, sv);
         ScatterSink f{w.xdrive && outT ? outT : out, y * w.W};
-        if (ref_rounding(flags)) ray_walk<true>(g, w, su, sv, (unsigned)sw, f);
-        else ray_walk<false>(g, w, su, sv, (unsigned)sw, f);
+        ray_walk<VAR, true>(g, w, su, sv, (unsigned)sw, f);
     } else {
-        if (!w.xdrive) scatter_walk<T, DIV, true, false>(w, g, out, g.nx, 1, sw, y);
-        else if (outT) scatter_walk<T, DIV, true, false>(w, g, outT, g.ny, 1, sw, y);
-        else scatter_walk<T, DIV, false, false>(w, g, out, 1, g.nx, sw, y);
+        if (!w.xdrive) scatter_walk<T, VAR, true, false>(w, g, out, g.nx, 1, sw, y);
+        else if (outT) scatter_walk<T, VAR, true, false>(w, g, outT, g.ny, 1, sw, y);
+        else scatter_walk<T, VAR, false, false>(w, g, out, 1, g.nx, sw, y);
     }
 }
 
-template <typename T, bool DIV, bool EXACT = false>
+template <typename T, bool VAR, bool EXACT = false, bool COPY = true>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 && !EXACT ? 4 : 1) cb_forward_kernel(const __grid_constant__ CBParams<T> p)
 {
     int ia, ib, iv;
@@ -161,11 +159,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 && !EXACT ? 4 : 1) cb_forw
     if (ia >= p.na || ib >= p.nb) return;
     T r[6];
     cb_ray(p, ia, ib, iv, r);
-    const T acc = ray_forward<T, DIV, EXACT>(p.g, r, p.flags, p.vol, p.volT);
+    const T acc = ray_forward<T, VAR, EXACT, COPY>(p.g, r, p.flags, p.vol, p.volT);
     p.out[(size_t)(p.v0 + iv) * p.na * p.nb + (size_t)ib * p.na + ia] = acc;
 }
 
-template <typename T, bool DIV, bool EXACT = false>
+template <typename T, bool VAR, bool EXACT = false>
 __global__ void __launch_bounds__(256) cb_backward_kernel(const __grid_constant__ CBParams<T> p)
 {
     int ia, ib, iv;
@@ -175,7 +173,7 @@ __global__ void __launch_bounds__(256) cb_backward_kernel(const __grid_constant_
     if (y == (T)0) return;
     T r[6];
     cb_ray(p, ia, ib, iv, r);
-    ray_backward<T, DIV, EXACT>(p.g, r, p.flags, y, p.out, p.outT);
+    ray_backward<T, VAR, EXACT>(p.g, r, p.flags, y, p.out, p.outT);
 }
 
 // Forward of R rows per lane of one detector column (the whole warp calls
@@ -409,15 +407,18 @@ static inline cudaError_t cb_launch(CBParams<T> &p, int na, int nb, int nvc, uin
 {
     dim3 grid, block;
     cb_shape(p, na, nb, nvc, grid, block);
-    // (the float walk has no division path)
-    const bool exact = (flags & NEFCT_EXACT) != 0, div = sizeof(T) == 8 && !cubic(p.g);
+    const bool exact = (flags & NEFCT_EXACT) != 0;
+    const bool var = sizeof(T) == 4 ? ref_rounding(flags) : !cubic(p.g);
     if constexpr (FWD) {
         if (exact) cb_forward_kernel<T, false, true><<<grid, block, 0, s>>>(p);
-        else if (div) cb_forward_kernel<T, sizeof(T) == 8><<<grid, block, 0, s>>>(p);
+        else if (p.volT == nullptr && sizeof(T) == 4) {
+            if (var) cb_forward_kernel<T, true, false, sizeof(T) != 4><<<grid, block, 0, s>>>(p);
+            else cb_forward_kernel<T, false, false, sizeof(T) != 4><<<grid, block, 0, s>>>(p);
+        } else if (var) cb_forward_kernel<T, true><<<grid, block, 0, s>>>(p);
         else cb_forward_kernel<T, false><<<grid, block, 0, s>>>(p);
     } else {
         if (exact) cb_backward_kernel<T, false, true><<<grid, block, 0, s>>>(p);
-        else if (div) cb_backward_kernel<T, sizeof(T) == 8><<<grid, block, 0, s>>>(p);
+        else if (var) cb_backward_kernel<T, true><<<grid, block, 0, s>>>(p);
         else cb_backward_kernel<T, false><<<grid, block, 0, s>>>(p);
     }
     return cudaGetLastError();

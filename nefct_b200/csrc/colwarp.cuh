@@ -231,11 +231,19 @@ __device__ __forceinline__ void z_split(const ZRay &z, float q, float qh, float 
 // and a single column in the grid.
 enum SlabKind { kPlain, kCross, kHalf };
 
+// The voxels of a slab of one ray, their shares, and whether it crosses a v plane.
+struct RaySlab {
+    unsigned p[3];
+    float w[3];
+    bool vx;
+};
+
 // Forward: sums of value * share, by kind of slab and by aligned block of 32
 // slabs (close() ends a block), so that the total does not depend on which
 // rays walk together; sums of partial sums also round less than one running
 // sum.
 struct GatherSink {
+    static constexpr bool kGather = true;
     const float *__restrict__ vol;
     float sum[3], whole;
 
@@ -253,15 +261,23 @@ struct GatherSink {
         else if (kind == kCross) sum[1] = s;
         else sum[2] = s;
     }
-    // (of the last two, those without a share, most of them, are not read)
-    __device__ __forceinline__ void inner(bool vx, const unsigned (&p)[3], const float (&w)[3])
+    // G slabs: all loads first, so that they overlap (of the last two voxels of a
+    // slab, those without a share, most of them, are not read)
+    template <int G> __device__ __forceinline__ void inner(const RaySlab (&s)[G])
     {
-        const float v0 = __ldg(vol + p[0]);
-        const float v1 = w[1] != 0.f ? __ldg(vol + p[1]) : 0.f;
-        const float v2 = w[2] != 0.f ? __ldg(vol + p[2]) : 0.f;
-        const float v = __fmaf_rn(v2, w[2], __fmaf_rn(v1, w[1], __fmaf_rn(v0, w[0], vx ? sum[1] : sum[0])));
-        if (vx) sum[1] = v;
-        else sum[0] = v;
+        float v[G][3];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            v[g][0] = __ldg(vol + s[g].p[0]);
+            v[g][1] = s[g].w[1] != 0.f ? __ldg(vol + s[g].p[1]) : 0.f;
+            v[g][2] = s[g].w[2] != 0.f ? __ldg(vol + s[g].p[2]) : 0.f;
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const float *const w = s[g].w;
+            if (s[g].vx) sum[1] = __fmaf_rn(v[g][2], w[2], __fmaf_rn(v[g][1], w[1], __fmaf_rn(v[g][0], w[0], sum[1])));
+            else sum[0] = __fmaf_rn(v[g][1], w[1], __fmaf_rn(v[g][0], w[0], sum[0]));
+        }
     }
     __device__ __forceinline__ void close()
     {
@@ -272,6 +288,7 @@ struct GatherSink {
 
 // Transpose: one reduction of yw * share per voxel with a share.
 struct ScatterSink {
+    static constexpr bool kGather = false;
     float *acc;
     float yw;
 
@@ -281,9 +298,10 @@ struct ScatterSink {
         for (int i = 0; i < 3; ++i)
             if ((ok >> i & 1u) && w[i] != 0.f) atomicAdd(acc + p[i], yw * w[i]);
     }
-    __device__ __forceinline__ void inner(bool, const unsigned (&p)[3], const float (&w)[3]) const
+    template <int G> __device__ __forceinline__ void inner(const RaySlab (&s)[G]) const
     {
-        edge(kPlain, p, 7u, w);
+#pragma unroll
+        for (int g = 0; g < G; ++g) edge(kPlain, s[g].p, 7u, s[g].w);
     }
     __device__ __forceinline__ void close() const {}
 };
@@ -291,6 +309,7 @@ struct ScatterSink {
 // Deterministic transpose: each contribution yw * share, scaled by a power of
 // two (exact) and rounded to a 64-bit integer (siddon.cuh, to_fixed).
 struct FixedSink {
+    static constexpr bool kGather = false;
     unsigned long long *acc;
     float yw, scale;
 
@@ -301,9 +320,10 @@ struct FixedSink {
             if ((ok >> i & 1u) && w[i] != 0.f)
                 atomicAdd(acc + p[i], (unsigned long long)to_fixed((yw * w[i]) * scale));
     }
-    __device__ __forceinline__ void inner(bool, const unsigned (&p)[3], const float (&w)[3]) const
+    template <int G> __device__ __forceinline__ void inner(const RaySlab (&s)[G]) const
     {
-        edge(kPlain, p, 7u, w);
+#pragma unroll
+        for (int g = 0; g < G; ++g) edge(kPlain, s[g].p, 7u, s[g].w);
     }
     __device__ __forceinline__ void close() const {}
 };
@@ -315,7 +335,7 @@ struct FixedSink {
 // crossing is taken as one with rv = 1 (its third voxel has no share).  The
 // high column is the one at the slab's far plane: where dv < 1 it need not be
 // the low one's neighbour.
-template <bool REF, bool CHECK, bool DOWN, int DIV, class Sink>
+template <bool REF, bool CHECK, bool DOWN, int DIV, bool ALIGN, class Sink>
 __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
                                           Sink &f)
 {
@@ -323,7 +343,7 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
     float t = __fsub_rn((float)k, c.nu2), da = __fsub_rn(t, c.pu);
     float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa), za = z_at<REF>(z, zg, da);
     unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + sw);
-    auto slab = [&]() {
+    auto slab = [&](RaySlab &s) {
         t = __fadd_rn(t, 1.f);
         const float db = __fsub_rn(t, c.pu), qb = col_vpos<DIV>(c, db), mb = magic_floor<CHECK>(qb);
         const float q1 = CHECK ? fminf(qa, qb) : DOWN ? qb : qa, q2 = CHECK ? fmaxf(qa, qb) : DOWN ? qa : qb;
@@ -338,15 +358,18 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
         const unsigned up = CHECK ? (unsigned)(__float_as_int(mh) - __float_as_int(m)) * sw : sw;
         const unsigned v1 = z1 + (unsigned)__float_as_int(m1) * c.sv, v2 = z1 + (unsigned)__float_as_int(m2) * c.sv;
         const bool vfirst = rv > r;             // the middle voxel is (v1, z2), else (v2, z1)
-        const unsigned p[3] = {v1, vfirst ? v1 + up : v2, v2 + up};
         const float both = fminf(rv, r), over = __fsub_rn(r, both);      // r's share in the high column
-        const float w[3] = {both, fabsf(__fsub_rn(rv, r)), __fsub_rn(__fsub_rn(1.f, rv), over)};
+        s.p[0] = v1;
+        s.p[1] = vfirst ? v1 + up : v2;
+        s.p[2] = v2 + up;
+        s.w[0] = both;
+        s.w[1] = fabsf(__fsub_rn(rv, r));
+        s.w[2] = __fsub_rn(__fsub_rn(1.f, rv), over);
+        s.vx = vx;
         if constexpr (CHECK) {
             const bool a = vin.low(m1), b = vx && vin.far(m1, m2), l = zin.low(m), h = zin.far(m, mh);
-            f.edge(!vx ? kPlain : a && b ? kCross : kHalf, p,
-                   (unsigned)(a && l) | (unsigned)(vfirst ? a && h : b && l) << 1 | (unsigned)(b && h) << 2, w);
-        } else {
-            f.inner(vx, p, w);
+            f.edge(!vx ? kPlain : a && b ? kCross : kHalf, s.p,
+                   (unsigned)(a && l) | (unsigned)(vfirst ? a && h : b && l) << 1 | (unsigned)(b && h) << 2, s.w);
         }
         base += c.su;
         da = db;
@@ -354,21 +377,71 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
         ma = mb;
         za = zb;
     };
-    while (k <= end) {
-        const int last = min(k | 31, end);
-        if constexpr (CHECK) {
+    RaySlab one[1];
+    auto single = [&]() {
+        slab(one[0]);
+        if constexpr (!CHECK) f.inner(one);
+    };
+    if constexpr (CHECK) {
 #pragma unroll 1
-            for (; k <= last; ++k) slab();
-        } else {
-#pragma unroll 4
-            for (; k <= last; ++k) slab();
+        for (; k <= end; ++k) {
+            single();
+            if ((k & 31) == 31) f.close();
         }
-        if ((last & 31) == 31) f.close();
+    } else if constexpr (ALIGN) {
+        while (k <= end) {
+            const int last = min(k | 31, end);
+            if constexpr (Sink::kGather) {
+#pragma unroll 2
+                for (; k < last; k += 2) {
+                    RaySlab s[2];
+                    slab(s[0]);
+                    slab(s[1]);
+                    f.inner(s);
+                }
+                if (k <= last) { single(); ++k; }
+            } else {
+#pragma unroll 4
+                for (; k <= last; ++k) single();
+            }
+            if ((last & 31) == 31) f.close();
+        }
+    } else {
+        // a single slab up to an even one, then pairs
+        if (k <= end && (k & 1)) {
+            single();
+            if ((k++ & 31) == 31) f.close();
+        }
+#pragma unroll 4
+        for (; k < end; k += 2) {
+            RaySlab s[2];
+            slab(s[0]);
+            slab(s[1]);
+            f.inner(s);
+            if ((k & 31) == 30) f.close();
+        }
+        if (k <= end) {
+            single();
+            if ((k & 31) == 31) f.close();
+        }
     }
 }
 
+// Slabs k..end, all in the grid, of a ray that is not steep.
+template <bool REF, bool ALIGN, class Sink>
+__device__ __forceinline__ void ray_inner(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end,
+                                             unsigned sw, Sink &f)
+{
+    if (c.vdiv) {
+        if (c.kv < 0.f) ray_slabs<REF, false, true, 1, ALIGN>(c, z, zg, k, end, sw, f);
+        else ray_slabs<REF, false, false, 1, ALIGN>(c, z, zg, k, end, sw, f);
+    } else {
+        if (c.kv < 0.f) ray_slabs<REF, false, true, 0, ALIGN>(c, z, zg, k, end, sw, f);
+        else ray_slabs<REF, false, false, 0, ALIGN>(c, z, zg, k, end, sw, f);
+    }
+}
 // The thread walk: the slabs k0..k1 of a ray, of them ki0..ki1 without range checks.
-template <bool REF, class Sink>
+template <bool REF, bool COPY, class Sink>
 __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<float> &w, unsigned su, unsigned sv,
                                          unsigned sw, Sink &f)
 {
@@ -379,15 +452,10 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
     int k = w.k0, end = interior ? w.ki0 - 1 : w.k1;
 #pragma unroll 1
     for (;;) {
-        ray_slabs<REF, true, false, -1>(c, z, zg, k, end, sw, f);
+        ray_slabs<REF, true, false, -1, true>(c, z, zg, k, end, sw, f);
         if (end == w.k1) break;
-        if (c.vdiv) {
-            if (c.kv < 0.f) ray_slabs<REF, false, true, 1>(c, z, zg, w.ki0, w.ki1, sw, f);
-            else ray_slabs<REF, false, false, 1>(c, z, zg, w.ki0, w.ki1, sw, f);
-        } else {
-            if (c.kv < 0.f) ray_slabs<REF, false, true, 0>(c, z, zg, w.ki0, w.ki1, sw, f);
-            else ray_slabs<REF, false, false, 0>(c, z, zg, w.ki0, w.ki1, sw, f);
-        }
+        if (!COPY && sv != 1u) ray_inner<REF, COPY>(c, z, zg, w.ki0, w.ki1, sw, f);
+        else ray_inner<REF, true>(c, z, zg, w.ki0, w.ki1, sw, f);
         if (w.ki1 == w.k1) break;
         k = w.ki1 + 1;
         end = w.k1;
@@ -516,7 +584,7 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
 template <bool REF, class Sink>
 __device__ __forceinline__ void col_each(const ColWalk &cw, int K0, int K1, const ZRay &z, const ZGrid &zg, Sink &f)
 {
-    if (z.live) ray_slabs<REF, true, false, -1>(cw, z, zg, K0, K1, 1u, f);
+    if (z.live) ray_slabs<REF, true, false, -1, true>(cw, z, zg, K0, K1, 1u, f);
     f.close();
 }
 

@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(256) cb_count_kernel(const __grid_constant__ C
 
 // ---------------- deterministic transpose (fixed point) ----------------
 
+template <bool REF>
 __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_constant__ CBParams<float> p)
 {
     int ia, ib, iv;
@@ -51,8 +52,7 @@ __global__ void __launch_bounds__(256) cb_backward_fixed_kernel(const __grid_con
     unsigned su, sv;
     thread_strides(p.g.nx, p.g.ny, w.xdrive, p.fixT != nullptr, su, sv);
     FixedSink f{w.xdrive && p.fixT ? p.fixT : p.fix, y * w.W, *p.fix_scale};
-    if (ref_rounding(p.flags)) ray_walk<true>(p.g, w, su, sv, sw, f);
-    else ray_walk<false>(p.g, w, su, sv, sw, f);
+    ray_walk<REF, true>(p.g, w, su, sv, sw, f);
 }
 
 // vol[z][y][x] = accZ[y][x][z] / scale (the integer sums of the column warps)
@@ -604,7 +604,8 @@ static nefct_status cb_backward_fixed_impl(const nefct_cb_geom *g, const float *
         }
         dim3 grid, block;
         cb_shape(p, g->na, g->nb, nvc, grid, block);
-        cb_backward_fixed_kernel<<<grid, block, 0, s>>>(p);
+        if (ref_rounding(flags)) cb_backward_fixed_kernel<true><<<grid, block, 0, s>>>(p);
+        else cb_backward_fixed_kernel<false><<<grid, block, 0, s>>>(p);
         NEFCT_CHECK_LAUNCH("cb_backward_fixed_kernel");
     }
     if (cw) {
