@@ -200,7 +200,7 @@ __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first
             const int ib = col_row<R, false>(first, threadIdx.x, i, false);
             P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
         };
-        colwarp_forward<R, REF>(P.g, P.flags, P.volT, row, store);
+        colwarp_forward<R, REF, true>(P.g, P.flags, P.volT, row, store);
     } else {
         float r[R][6], y[R];
         bool has[R];

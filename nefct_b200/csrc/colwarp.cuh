@@ -579,15 +579,6 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
     return h;
 }
 
-// Every slab of one ray per lane, range checked: warps that the walks below do
-// not take (steep rays, and the transpose's values that are not finite).
-template <bool REF, class Sink>
-__device__ __forceinline__ void col_each(const ColWalk &cw, int K0, int K1, const ZRay &z, const ZGrid &zg, Sink &f)
-{
-    if (z.live) ray_slabs<REF, true, false, -1, true>(cw, z, zg, K0, K1, 1u, f);
-    f.close();
-}
-
 // Voxel of biased floor m in the column at the table's address (lo, hi).
 template <typename T = float> __device__ __forceinline__ T *col_voxel(unsigned lo, unsigned hi, float m)
 {
@@ -640,27 +631,40 @@ __device__ __forceinline__ void col_planes(const ColTable &tab, int j, const uin
     }
 }
 
+// z split of ray z at a table row (z_split; only STEEP warps have steep rays,
+// the others' high voxel is the low one's upper neighbour: no mh).
+template <bool REF, bool MIXED, bool STEEP>
+__device__ __forceinline__ void col_split(const ColTable &tab, int j, const uint4 &te, const ZRay &z, const ZGrid &zg,
+                                          float &m, float &mh, float &r)
+{
+    float lo, hi;
+    col_planes<MIXED>(tab, j, te, z, lo, hi);
+    if constexpr (STEEP) z_split<REF>(z, z_at<REF>(z, zg, lo), z_at<REF>(z, zg, hi), m, mh, r);
+    else z_inner<REF>(z, zg, lo, hi, m, r);
+}
+
 // Forward of one chunk's table rows.  Each kind of slab is walked in a loop of
 // its own: no branch stands between the loads of consecutive slabs, so they
 // overlap.  ZCHK: z range checks.
-template <int R, bool REF, bool MIXED, bool ZCHK>
+template <int R, bool REF, bool MIXED, bool STEEP, bool ZCHK>
 __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
                                                 GatherSink (&f)[R])
 {
     const Inside in(q.zg.nz);
-    auto load = [&](const float *p, float m, float &a, float &b) {
+    auto load = [&](unsigned lo, unsigned hi, float m, float mh, float &a, float &b) {
+        const float *const p = col_voxel(lo, hi, m);
         a = !ZCHK || in.low(m) ? __ldg(p) : 0.f;
-        b = !ZCHK || in.high(m) ? __ldg(p + 1) : 0.f;
+        if constexpr (STEEP) b = !ZCHK || in.far(m, mh) ? __ldg(col_voxel(lo, hi, mh)) : 0.f;
+        else b = !ZCHK || in.high(m) ? __ldg(p + 1) : 0.f;
     };
 #pragma unroll 4
     for (int j = 0; j < h.cross; ++j) {
         const uint4 te = tab.a[j];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            float lo, hi, m, r, a, b;
-            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
-            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
-            load(col_voxel(te.x, te.y, m), m, a, b);
+            float m, mh, r, a, b;
+            col_split<REF, MIXED, STEEP>(tab, j, te, q.z[i], q.zg, m, mh, r);
+            load(te.x, te.y, m, mh, a, b);
             f[i].sum[0] = __fmaf_rn(b, __fsub_rn(1.f, r), __fmaf_rn(a, r, f[i].sum[0]));
         }
     }
@@ -670,11 +674,10 @@ __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTa
         const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            float lo, hi, m, r, a, b, c, d;
-            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
-            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
-            load(col_voxel(te.x, te.y, m), m, a, b);
-            load(col_voxel(tc.x, tc.y, m), m, c, d);
+            float m, mh, r, a, b, c, d;
+            col_split<REF, MIXED, STEEP>(tab, j, te, q.z[i], q.zg, m, mh, r);
+            load(te.x, te.y, m, mh, a, b);
+            load(tc.x, tc.y, m, mh, c, d);
             const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11);
             const float acc = __fmaf_rn(b, __fsub_rn(rv, w11), __fmaf_rn(a, w11, f[i].sum[1]));
             f[i].sum[1] = __fmaf_rn(d, __fsub_rn(ov, w21), __fmaf_rn(c, w21, acc));
@@ -686,10 +689,9 @@ __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTa
         const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            float lo, hi, m, r, a, b;
-            col_planes<MIXED>(tab, j, te, q.z[i], lo, hi);
-            z_inner<REF>(q.z[i], q.zg, lo, hi, m, r);
-            load(col_voxel(te.x, te.y, m), m, a, b);
+            float m, mh, r, a, b;
+            col_split<REF, MIXED, STEEP>(tab, j, te, q.z[i], q.zg, m, mh, r);
+            load(te.x, te.y, m, mh, a, b);
             const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11);
             const float wl = tc.x ? w21 : w11, wh = tc.x ? __fsub_rn(ov, w21) : __fsub_rn(rv, w11);
             f[i].sum[2] = __fmaf_rn(b, wh, __fmaf_rn(a, wl, f[i].sum[2]));
@@ -697,15 +699,17 @@ __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTa
     }
 }
 
-// Forward of the lane's R rays (not steep): sums into f.
-template <int R, bool REF, bool MIXED>
+// Forward of the lane's R rays: sums into f.
+template <int R, bool REF, bool MIXED, bool STEEP>
 __device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__restrict__ vol, GatherSink (&f)[R])
 {
     ColTable &tab = col_table();
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
         const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, vol, tab);
-        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1) col_gather_rows<R, REF, MIXED, false>(q, tab, h, f);
-        else col_gather_rows<R, REF, MIXED, true>(q, tab, h, f);
+        if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1)
+            col_gather_rows<R, REF, MIXED, STEEP, false>(q, tab, h, f);
+        else
+            col_gather_rows<R, REF, MIXED, STEEP, true>(q, tab, h, f);
 #pragma unroll
         for (int i = 0; i < R; ++i) f[i].close();
     }
@@ -721,7 +725,8 @@ enum Merge { kSingle, kNear, kAny };
 // one's low voxel w, so a slab takes at most three reductions per column
 // instead of two per ray, and the lanes of a warp, R rows apart, rarely hit
 // the same voxel.
-template <int R, bool REF, bool MIXED, Merge MERGE, bool ZCHK, class Acc>
+// STEEP rays do not merge.
+template <int R, bool REF, bool MIXED, bool STEEP, Merge MERGE, bool ZCHK, class Acc>
 __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
                                                  const Acc &acc, const float (&y)[R])
 {
@@ -729,12 +734,13 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
     const Inside in(q.zg.nz);
     // values l, u of the low and high voxels of rays i.. in one voxel column
     constexpr int S = MERGE == kSingle ? 1 : R;
-    auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], T (&l)[S], T (&u)[S]) {
+    static_assert(!STEEP || MERGE == kSingle, "");
+    auto reduce = [&](unsigned lo, unsigned hi, const float (&m)[S], const float (&mh)[S], T (&l)[S], T (&u)[S]) {
         if (ZCHK) {
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 if (!in.low(m[k])) l[k] = (T)0;
-                if (!in.high(m[k])) u[k] = (T)0;
+                if (STEEP ? !in.far(m[k], mh[k]) : !in.high(m[k])) u[k] = (T)0;
             }
         }
         T *const p = col_voxel<T>(lo, hi, m[0]);
@@ -757,7 +763,7 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
             Acc::red(s + 1, same ? (T)0 : u[1]);
         }
         Acc::red(p, l[0]);
-        Acc::red(p + 1, u[0]);
+        Acc::red(STEEP ? col_voxel<T>(lo, hi, mh[0]) : p + 1, u[0]);
     };
 #pragma unroll 1
     for (int j = h.cross; j < h.n; ++j) {
@@ -765,13 +771,12 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         const float rv = __uint_as_float(tc.z), ov = __uint_as_float(tc.w);
 #pragma unroll
         for (int i = 0; i < R; i += S) {
-            float lo, hi, m[S];
+            float m[S], mh[S];
             T l1[S], u1[S], l2[S], u2[S];
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 float r;
-                col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
-                z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
+                col_split<REF, MIXED, STEEP>(tab, j, te, q.z[i + k], q.zg, m[k], mh[k], r);
                 const float w11 = fminf(rv, r), w21 = __fsub_rn(r, w11), yk = y[i + k];
                 l1[k] = acc.value(yk * w11);
                 u1[k] = acc.value(yk * __fsub_rn(rv, w11));
@@ -779,12 +784,12 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
                 u2[k] = acc.value(yk * __fsub_rn(ov, w21));
             }
             if (j < h.half) {
-                reduce(te.x, te.y, m, l1, u1);
-                reduce(tc.x, tc.y, m, l2, u2);
+                reduce(te.x, te.y, m, mh, l1, u1);
+                reduce(tc.x, tc.y, m, mh, l2, u2);
             } else if (tc.x == 0u) {
-                reduce(te.x, te.y, m, l1, u1);
+                reduce(te.x, te.y, m, mh, l1, u1);
             } else {
-                reduce(te.x, te.y, m, l2, u2);
+                reduce(te.x, te.y, m, mh, l2, u2);
             }
         }
     }
@@ -793,33 +798,31 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
         const uint4 te = tab.a[j];
 #pragma unroll
         for (int i = 0; i < R; i += S) {
-            float lo, hi, m[S];
+            float m[S], mh[S];
             T l[S], u[S];
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 float r;
-                col_planes<MIXED>(tab, j, te, q.z[i + k], lo, hi);
-                z_inner<REF>(q.z[i + k], q.zg, lo, hi, m[k], r);
+                col_split<REF, MIXED, STEEP>(tab, j, te, q.z[i + k], q.zg, m[k], mh[k], r);
                 l[k] = acc.value(y[i + k] * r);
                 u[k] = acc.rest(y[i + k], r);
             }
-            reduce(te.x, te.y, m, l, u);
+            reduce(te.x, te.y, m, mh, l, u);
         }
     }
 }
 
-// Transpose of the lane's R rays (not steep; y finite, 0 for a ray that takes
-// no part).
-template <int R, bool REF, bool MIXED, Merge MERGE, class Acc>
+// Transpose of the lane's R rays (y finite, 0 for a ray that takes no part).
+template <int R, bool REF, bool MIXED, bool STEEP, Merge MERGE, class Acc>
 __device__ __forceinline__ void col_scatter(const ColRays<R> &q, const Acc &acc, const float (&y)[R])
 {
     ColTable &tab = col_table();
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
         const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, acc.vol, tab);
         if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1)
-            col_scatter_rows<R, REF, MIXED, MERGE, false>(q, tab, h, acc, y);
+            col_scatter_rows<R, REF, MIXED, STEEP, MERGE, false>(q, tab, h, acc, y);
         else
-            col_scatter_rows<R, REF, MIXED, MERGE, true>(q, tab, h, acc, y);
+            col_scatter_rows<R, REF, MIXED, STEEP, MERGE, true>(q, tab, h, acc, y);
     }
 }
 

@@ -217,3 +217,47 @@ def test_nothing_outside_the_buffers_is_touched(cuda, nz, flags, walk):
     assert torch.isfinite(back).all() and back.any()
     for t in (ws_all, out_all, back_all):
         assert (t[:pad] == 7.0).all() and (t[-pad:] == 7.0).all()
+
+
+# rows, row pitch, z voxel, z offset: one to three rows per lane (forward), one to
+# four that share reductions (transpose), rows falling in z, with rays that move
+# over a voxel in z per slab
+STEEP = [(24, 6.0, 1.0, 0.0), (120, 1.2, 1.0, 0.0), (120, -1.2, 1.0, 2.0), (129, 0.8, 0.7, 0.0), (161, 0.7, 0.8, 1.0),
+         (200, 0.7, 0.5, -1.0)]
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("case", STEEP, ids=[f"{c[0]}x{c[1]}-dz{c[2]}-off{c[3]}" for c in STEEP])
+def test_steep_rays(cuda, oracle_lib, case, flags):
+    """Cone angles beyond 45 degrees (rays that cross a z plane in every slab and
+    two in some), alone and in warps with others that are not steep; one value
+    that is not finite in such a warp."""
+    rows, pitch, vz, off = case
+    g = nb.ConeBeam((20, 18, 60), ANGLES, 25.0, 50.0, 37, 1.0, rows, pitch, size=(20.0, 18.0, 60.0 * vz),
+                    center=(0.3, -0.2, 0.1), z_offsets=np.linspace(off - 0.5, off + 0.5, ANGLES.size))
+    # voxel rows per slab, at least, of each detector row's rays
+    slope = np.abs((np.arange(rows) + 0.5) * pitch - rows * pitch / 2) / 50.0 / vz
+    rng = np.random.default_rng(rows)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    y[2, rows // 2:, 5] = 0
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    hit = slope[(ref_f != 0).any(axis=(0, 2))]
+    assert hit.max() > 1.05 and hit.min() < 0.5
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    f, bw = _both(g, v, s, flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(bw.cpu().numpy(), ref_b)
+    for ft, bt in _thread_walk(g, v, s, flags):
+        assert torch.equal(f, ft)
+        assert_parity(bt.cpu().numpy(), ref_b)
+    fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
+    assert torch.equal(*fixed)
+    assert_parity(fixed[0].cpu().numpy(), ref_b)
+    y[3, np.flatnonzero(ref_f[3, :, 18])[-1], 18] = np.inf
+    ref_i = _oracle(oracle_lib, g, vol, y, flags)[1]
+    out = ops.cb_backward(torch.from_numpy(y).to(cuda), g, flags).cpu().numpy()
+    fine = np.isfinite(ref_i)
+    assert 0 < (~fine).sum() < ref_i.size // 10
+    np.testing.assert_array_equal(np.isfinite(out), fine)
+    assert_parity(np.where(fine, out, 0), np.where(fine, ref_i, 0))
