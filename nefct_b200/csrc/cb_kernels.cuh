@@ -86,9 +86,10 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     GatherSink f(vol);
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
-    const ZRay z = z_ray(w, zg, true);
-    if (ref_rounding(flags)) ray_slabs<true, true, false, -1, true>(c, z, zg, w.k0, w.k1, sw, f);
-    else ray_slabs<false, true, false, -1, true>(c, z, zg, w.k0, w.k1, sw, f);
+    if (ref_rounding(flags))
+        ray_slabs<true, true, false, -1, true>(c, z_ray<true>(w, zg, z_source<true>(w, zg), true), zg, w.k0, w.k1, sw, f);
+    else
+        ray_slabs<false, true, false, -1, true>(c, z_ray<false>(w, zg, z_source<false>(w, zg), true), zg, w.k0, w.k1, sw, f);
     f.close();
     return f.whole * w.W;
 }
@@ -189,7 +190,7 @@ __device__ __noinline__ static float colwarp_gather_steep(const GridDev<float> &
     const float r[1][6] = {{x1, y1, z1, x2, y2, z2}};
     const bool h[1] = {has};
     ColRays<1> q;
-    if (!col_rays<1, true>(g, r, h, flags, q)) return 0.f;
+    if (!col_rays<1, REF, true>(g, r, h, flags, q)) return 0.f;
     GatherSink f[1] = {GatherSink(volZ)};
     col_gather<1, REF, true, true>(q, volZ, f);
     if (!q.z[0].live) return 0.f;
@@ -214,7 +215,7 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
             h[i] = row(i, r[i]);
             has |= (unsigned)h[i] << i;
         }
-        if (!col_rays<R, true>(g, r, h, flags, q)) {
+        if (!col_rays<R, REF, true>(g, r, h, flags, q)) {
 #pragma unroll
             for (int i = 0; i < R; ++i)
                 if (h[i]) store(i, 0.f);
@@ -267,7 +268,7 @@ __device__ __noinline__ static void colwarp_scatter_rare(const GridDev<float> &g
     const float r[1][6] = {{x1, y1, z1, x2, y2, z2}};
     const bool h[1] = {has};
     ColRays<1> q;
-    if (!col_rays<1, false>(g, r, h, flags, q)) return;
+    if (!col_rays<1, REF, false>(g, r, h, flags, q)) return;
     const float yw[1] = {q.z[0].live ? y * q.W[0] : 0.f};
     if (__all_sync(0xffffffffu, isfinite(yw[0]))) {
         col_scatter<1, REF, true, true, kSingle>(q, acc, yw);
@@ -287,7 +288,7 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
     ColRays<R> q;
 #pragma unroll
     for (int i = 0; i < R; ++i) has[i] = has[i] && y[i] != 0.f;
-    if (!col_rays<R, false>(g, r, has, flags, q)) return;
+    if (!col_rays<R, REF, false>(g, r, has, flags, q)) return;
     float yw[R];
     bool finite = true;
 #pragma unroll

@@ -28,9 +28,13 @@
 // is needed while |kz| (z voxels per slab) stays below 1; steeper rays take
 // the general split.
 //  * By default q1 = fma(kz, d, z0) and q2 - q1 = |kz| exactly: one fused
-//    multiply-add, a floor and one saturating multiply-add per ray and slab,
-//    with fewer roundings than the reference's (the error against FP64 is no
-//    larger), the same in the forward and its transpose.
+//    multiply-add, a floor and one saturating multiply-add per ray and slab, the
+//    same in the forward and its transpose.  Positions count from the source's
+//    row, so that z0 is a fraction held to 2^-25: rounded at the size of a row
+//    number its error, constant along the ray, would go into every share divided
+//    by |kz| (rel-L2 against FP64 of 26 x 22 x 24 voxels, thin slices, source
+//    off the middle: 1.33e-6, now 1.24e-6; the reference's operations in float:
+//    1.24e-6).
 //  * REF (calls with NEFCT_TIE_GT, the switches of the reference's own
 //    backprojection): q1 and q2 with the reference's operations in its order.
 //    A nearly level ray (|kz| ~ 1e-3) divides rounding errors of ~1e-5 voxel
@@ -100,7 +104,10 @@ __device__ __forceinline__ float col_ratio(float q1, float q2, float m1, float m
 // Whether a voxel of biased floor m, and the one above it, are among n.
 struct Inside {
     float lo, hi;           // biased floors 0 and n
-    __device__ __forceinline__ Inside(int n) : lo(kFloorMagic), hi(kFloorMagic + (float)n) {}
+    // first: what floor 0 stands for
+    __device__ __forceinline__ Inside(int n, int first = 0)
+        : lo(kFloorMagic - (float)first), hi(kFloorMagic + (float)(n - first)) {}
+    __device__ __forceinline__ Inside(float lo_, float hi_) : lo(lo_), hi(hi_) {}
     __device__ __forceinline__ bool low(float m) const { return m >= lo && m < hi; }
     __device__ __forceinline__ bool high(float m) const { return m >= lo - 1.f && m < hi - 1.f; }
     // the high one of a slab with floors m < mh, admitted from m = -1 on
@@ -125,10 +132,11 @@ __device__ __forceinline__ ColEntry col_entry(const ColWalk &c, int k)
     return e;
 }
 
-// z part of a ray, in voxel rows.
+// z part of a ray, in voxel rows from row zi on (the source's row; REF: row 0).
 struct ZRay {
     float kz, z0, ikz;      // position kz * d + z0 at plane offset d; ikz = 1 / |kz| (at most 1e30)
     float kw, pw;           // REF: position ((pw + kw * d) * rdz) + nz2
+    int zi;
     int down;               // kz < 0: the slab's lower z plane is its exit plane
     bool live, steep;
 };
@@ -148,16 +156,40 @@ __device__ __forceinline__ ZGrid z_grid(const GridDev<float> &g)
     return ZGrid{g.dz, __fdiv_rn(1.f, g.dz), g.nz2, g.dz != 1.f, g.nz};
 }
 
-// (a lane without a ray walks row 0 under either rounding: its indices stay in
-// the grid)
-__device__ __forceinline__ ZRay z_ray(const Walk<float> &w, const ZGrid &zg, bool live)
+// The source's row zi (within 2^20 rows of the grid, so positions stay below
+// 2^21) and its height above it: pw / dz + nz / 2 - zi, exact but for the
+// division's remainder, which is added back.  The same for every ray of a view.
+struct ZSource {
+    int zi;
+    float row, z0;
+};
+template <bool REF> __device__ __forceinline__ ZSource z_source(const Walk<float> &w, const ZGrid &zg)
+{
+    if (REF) return ZSource{0, 0.f, 0.f};
+    ZSource s;
+    s.row = rintf(fminf(fmaxf(w.z0, -1048576.f), 1048576.f));
+    s.zi = (int)s.row;
+    const float q = zg.div ? __fdiv_rn(w.pw, zg.dz) : w.pw;
+    s.z0 = __fsub_rn(q, __fsub_rn(s.row, zg.nz2));
+    if (zg.div) s.z0 = __fadd_rn(s.z0, __fdiv_rn(__fmaf_rn(-q, zg.dz, w.pw), zg.dz));
+    return s;
+}
+
+// (a lane without a ray walks row 0: its indices stay in the grid)
+template <bool REF>
+__device__ __forceinline__ ZRay z_ray(const Walk<float> &w, const ZGrid &zg, const ZSource &s, bool live)
 {
     ZRay z;
     z.live = live;
     z.kz = live ? w.kz : 0.f;
-    z.z0 = live ? w.z0 : 0.5f;
     z.kw = live ? w.kw : 0.f;
     z.pw = live ? w.pw : __fmul_rn(__fsub_rn(0.5f, zg.nz2), zg.dz);
+    z.zi = s.zi;
+    // (a level ray has its height as rounded: along a plane of the grid that decides
+    // which slice it lies in, as in the reference)
+    z.z0 = !live ? __fsub_rn(0.5f, s.row) : z.kz == 0.f ? __fsub_rn(w.z0, s.row) : s.z0;
+    // (the slope's rounding, added back at the grid's middle plane)
+    if (!REF && zg.div && live) z.z0 = __fmaf_rn(-w.pu * zg.rdz, __fmaf_rn(-w.kz, zg.dz, w.kw), z.z0);
     z.ikz = fminf(__fdiv_rn(1.f, fabsf(z.kz)), 1e30f);
     z.down = z.kz < 0.f;
     z.steep = fabsf(z.kz) > kSteep;
@@ -339,10 +371,10 @@ template <bool REF, bool CHECK, bool DOWN, int DIV, bool ALIGN, class Sink>
 __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
                                           Sink &f)
 {
-    const Inside vin(c.nv), zin(zg.nz);
+    const Inside vin(c.nv), zin(zg.nz, z.zi);
     float t = __fsub_rn((float)k, c.nu2), da = __fsub_rn(t, c.pu);
     float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa), za = z_at<REF>(z, zg, da);
-    unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + sw);
+    unsigned base = (unsigned)k * c.su - (unsigned)kFloorMagicBits * (c.sv + sw) + (unsigned)z.zi * sw;
     auto slab = [&](RaySlab &s) {
         t = __fadd_rn(t, 1.f);
         const float db = __fsub_rn(t, c.pu), qb = col_vpos<DIV>(c, db), mb = magic_floor<CHECK>(qb);
@@ -447,7 +479,7 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
 {
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
-    const ZRay z = z_ray(w, zg, true);
+    const ZRay z = z_ray<REF>(w, zg, z_source<REF>(w, zg), true);
     const bool interior = !z.steep && w.ki0 <= w.ki1;
     int k = w.k0, end = interior ? w.ki0 - 1 : w.k1;
 #pragma unroll 1
@@ -465,6 +497,30 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
 
 // ---- column warps ----
 
+// Warp's table of one 32-slab chunk, its slabs grouped by kind (slabs without
+// a v column in the grid are dropped): rows [0, cross) plain, [cross, half)
+// cross, [half, n) half.  a = (address of the low v column -- of the one
+// column in the grid for a half slab -- less one element per floor bias,
+// offsets of the lower and the upper z plane), c = (address of the high v column, or
+// 1 in c.x when a half slab's column is the high one; rv; 1 - rv).  d: the
+// offsets of the slab's entry and exit planes.
+// base, z0, z1: the volume's address, from the row on that the rays' z positions
+// count from, less one element per floor bias, and the biased floors of its
+// first row and of the one past its last (here, not in registers).
+struct ColTable {
+    uint4 a[32], c[32];
+    float2 d[32];
+    unsigned long long base;
+    float z0, z1;
+};
+
+// Column warps are blocks of 32 x (at most 8) threads: one table per warp.
+__device__ __forceinline__ ColTable &col_table()
+{
+    __shared__ ColTable tables[8];
+    return tables[threadIdx.y];
+}
+
 // A column's walk for one warp: the shared v part, the R rays of the lane and
 // the warp's slab ranges.
 template <int R> struct ColRays {
@@ -481,12 +537,13 @@ template <int R> struct ColRays {
 // part); false when no ray of the warp contributes.  UPPER: slabs without range
 // checks touch a low voxel's upper neighbour whether it has a share or not (the
 // forward's loads; the transpose's reductions skip it).
-template <int R, bool UPPER>
+template <int R, bool REF, bool UPPER>
 __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&r)[R][6], const bool (&has)[R],
                                          uint32_t flags, ColRays<R> &q)
 {
     int k0 = INT_MAX, k1 = INT_MIN, zi0 = INT_MIN, zi1 = INT_MAX;
     bool any = false, up = false, down = false, steep = false;
+    ZSource source;
     q.zg = z_grid(g);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -496,8 +553,9 @@ __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&
             // x and y do not depend on the row: every lane has the same v part
             const unsigned xs = (unsigned)g.nz, ys = (unsigned)g.nx * (unsigned)g.nz;
             q.c = col_walk_of(g, w, w.xdrive ? xs : ys, w.xdrive ? ys : xs);
+            source = z_source<REF>(w, q.zg);
         }
-        q.z[i] = z_ray(w, q.zg, live);
+        q.z[i] = z_ray<REF>(w, q.zg, source, live);
         q.W[i] = w.W;
         if (live) {
             any = true;
@@ -521,33 +579,25 @@ __device__ __forceinline__ bool col_rays(const GridDev<float> &g, const float (&
     return true;
 }
 
-// Warp's table of one 32-slab chunk, its slabs grouped by kind (slabs without
-// a v column in the grid are dropped): rows [0, cross) plain, [cross, half)
-// cross, [half, n) half.  a = (address of the low v column -- of the one
-// column in the grid for a half slab -- less one element per floor bias,
-// offsets of the lower and the upper z plane), c = (address of the high v column, or
-// 1 in c.x when a half slab's column is the high one; rv; 1 - rv).  d: the
-// offsets of the slab's entry and exit planes.
-struct ColTable {
-    uint4 a[32], c[32];
-    float2 d[32];
-};
-
 struct ColChunk {
     int cross, half, n;
 };
 
-// Column warps are blocks of 32 x (at most 8) threads: one table per warp.
-__device__ __forceinline__ ColTable &col_table()
+// The table's view-wide part (before the first chunk; whole warps come from
+// collectives, so the last walk's reads are done).
+template <typename T>
+__device__ __forceinline__ void col_table_start(ColTable &tab, const T *vol, int zi, int nz)
 {
-    __shared__ ColTable tables[8];
-    return tables[threadIdx.y];
+    if ((threadIdx.x & 31) == 0) {
+        tab.base = (unsigned long long)(vol + zi) - sizeof(T) * (unsigned)kFloorMagicBits;
+        tab.z0 = kFloorMagic - (float)zi;
+        tab.z1 = kFloorMagic + (float)(nz - zi);
+    }
 }
 
 // Lane j evaluates slab kc + j, if it is one of K0..K1.  T: the volume's elements.
 template <typename T>
-__device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0, int K1, bool falling, const T *vol,
-                                              ColTable &tab)
+__device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0, int K1, bool falling, ColTable &tab)
 {
     const int lane = threadIdx.x & 31, k = kc + lane;
     const ColEntry e = col_entry(cw, k);
@@ -565,10 +615,10 @@ __device__ __forceinline__ ColChunk col_chunk(const ColWalk &cw, int kc, int K0,
                                                                  : h.half + __popc(half & below);
     __syncwarp();                       // the previous chunk's reads are done
     if (is_plain || is_cross || is_half) {
-        const char *const base = reinterpret_cast<const char *>(vol) - sizeof(T) * (unsigned)kFloorMagicBits;
+        const unsigned long long base = tab.base;
         const unsigned i1 = is_half && in == 2u ? e.b2 : e.b1;
-        const unsigned long long p1 = (unsigned long long)(base + sizeof(T) * (i1 + (unsigned)kFloorMagicBits));
-        const unsigned long long p2 = (unsigned long long)(base + sizeof(T) * (e.b2 + (unsigned)kFloorMagicBits));
+        const unsigned long long p1 = base + sizeof(T) * (i1 + (unsigned)kFloorMagicBits);
+        const unsigned long long p2 = base + sizeof(T) * (e.b2 + (unsigned)kFloorMagicBits);
         tab.a[row] = make_uint4((unsigned)p1, (unsigned)(p1 >> 32), __float_as_uint(falling ? db : da),
                                 __float_as_uint(falling ? da : db));
         tab.c[row] = make_uint4(is_half ? in - 1u : (unsigned)p2, (unsigned)(p2 >> 32), __float_as_uint(e.rv),
@@ -650,7 +700,7 @@ template <int R, bool REF, bool MIXED, bool STEEP, bool ZCHK>
 __device__ __forceinline__ void col_gather_rows(const ColRays<R> &q, const ColTable &tab, const ColChunk &h,
                                                 GatherSink (&f)[R])
 {
-    const Inside in(q.zg.nz);
+    const Inside in = REF ? Inside(q.zg.nz) : ZCHK ? Inside(tab.z0, tab.z1) : Inside(0);
     auto load = [&](unsigned lo, unsigned hi, float m, float mh, float &a, float &b) {
         const float *const p = col_voxel(lo, hi, m);
         a = !ZCHK || in.low(m) ? __ldg(p) : 0.f;
@@ -704,8 +754,9 @@ template <int R, bool REF, bool MIXED, bool STEEP>
 __device__ __forceinline__ void col_gather(const ColRays<R> &q, const float *__restrict__ vol, GatherSink (&f)[R])
 {
     ColTable &tab = col_table();
+    col_table_start(tab, vol, q.z[0].zi, q.zg.nz);
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
-        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, vol, tab);
+        const ColChunk h = col_chunk<float>(q.c, kc, q.K0, q.K1, q.falling, tab);
         if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1)
             col_gather_rows<R, REF, MIXED, STEEP, false>(q, tab, h, f);
         else
@@ -731,7 +782,7 @@ __device__ __forceinline__ void col_scatter_rows(const ColRays<R> &q, const ColT
                                                  const Acc &acc, const float (&y)[R])
 {
     using T = typename Acc::T;
-    const Inside in(q.zg.nz);
+    const Inside in = REF ? Inside(q.zg.nz) : ZCHK ? Inside(tab.z0, tab.z1) : Inside(0);
     // values l, u of the low and high voxels of rays i.. in one voxel column
     constexpr int S = MERGE == kSingle ? 1 : R;
     static_assert(!STEEP || MERGE == kSingle, "");
@@ -817,8 +868,9 @@ template <int R, bool REF, bool MIXED, bool STEEP, Merge MERGE, class Acc>
 __device__ __forceinline__ void col_scatter(const ColRays<R> &q, const Acc &acc, const float (&y)[R])
 {
     ColTable &tab = col_table();
+    col_table_start(tab, acc.vol, q.z[0].zi, q.zg.nz);
     for (int kc = q.K0 & ~31; kc <= q.K1; kc += 32) {
-        const ColChunk h = col_chunk(q.c, kc, q.K0, q.K1, q.falling, acc.vol, tab);
+        const ColChunk h = col_chunk<typename Acc::T>(q.c, kc, q.K0, q.K1, q.falling, tab);
         if (max(kc, q.K0) >= q.ZI0 && min(kc + 31, q.K1) <= q.ZI1)
             col_scatter_rows<R, REF, MIXED, STEEP, MERGE, false>(q, tab, h, acc, y);
         else

@@ -261,3 +261,34 @@ def test_steep_rays(cuda, oracle_lib, case, flags):
     assert 0 < (~fine).sum() < ref_i.size // 10
     np.testing.assert_array_equal(np.isfinite(out), fine)
     assert_parity(np.where(fine, out, 0), np.where(fine, ref_i, 0))
+
+
+@pytest.mark.parametrize("nz,vz,off,rows,pitch", [(600, 0.1, 25.0, 65, 0.2), (300, 1.0, 120.3, 33, 0.3),
+                                                  (120, 0.71, 35.0, 33, 0.4)])
+def test_error_against_double_is_no_larger_than_the_reference_walks(cuda, oracle_lib, nz, vz, off, rows, pitch):
+    """Nearly level rays far from row 0, whose shares divide the error of a z
+    position by a small slope: the rel-L2 error against the double walk is at most
+    1.1 times that of the reference's operations in float (0.2 to 0.8 times on a
+    host build of the walk; positions held as row numbers: 1.5 to 1.8 times)."""
+    g = nb.ConeBeam((26, 22, nz), ANGLES, 70.0, 140.0, 37, 1.5, rows, float(np.float32(pitch)),
+                    size=tuple(float(np.float32(s)) for s in (26.0, 24.2, nz * vz)),
+                    center=tuple(float(np.float32(c)) for c in (0.3, -0.2, 0.1)),
+                    z_offsets=np.linspace(off - 0.05, off + 0.05, ANGLES.size, dtype=np.float32))
+    og = oracle_lib.grid(g.shape, g.center, g.size)
+    args = (g.angles, g.src_iso, g.src_det, g.na, g.da, 0.5, g.nb, g.db, 0.5)
+    rng = np.random.default_rng(1)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    f64 = oracle_lib.cb_forward(og, vol, *args, off=g.z_offsets, f64=True)[0]
+    b64 = oracle_lib.cb_backward(og, y, *args, off=g.z_offsets, flags=oracle_lib.CB_FWD, f64=True)
+    f32 = oracle_lib.cb_forward(og, vol, *args, off=g.z_offsets)[0]
+    b32 = oracle_lib.cb_backward(og, y, *args, off=g.z_offsets, flags=oracle_lib.CB_FWD)
+
+    def err(a, ref):
+        return np.linalg.norm(np.asarray(a, np.float64) - ref) / np.linalg.norm(ref)
+
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    for walk in (3, 0):
+        f, b = (t.cpu().numpy() for t in _both(g, v, s, 0, walk))
+        assert err(f, f64) <= 1.1 * err(f32, f64), (err(f, f64), err(f32, f64))
+        assert err(b, b64) <= 1.1 * err(b32, b64), (err(b, b64), err(b32, b64))
