@@ -380,7 +380,10 @@ __global__ void __launch_bounds__(128) dd_colwarp_kernel(const __grid_constant__
     // the source
     const float uA = F::sub(F::sub(0.5f, uhalf), u1), uB = F::sub(F::sub((float)nu - 0.5f, uhalf), u1);
     const bool ahead = uA * u21 > 0.f && uB * u21 > 0.f;
-    const bool pairs = !FWD && ahead && 2.f * dd_abs(hz) * fmaxf(dd_abs(uA), dd_abs(uB)) < 0.999f;
+    // (neighbouring footprints start that far apart, to the rounding of their
+    // positions, which grows with the grid: less than a voxel, or the rows do not merge)
+    const float apart = 1.f - (1e-3f + 1e-6f * ((float)p.nz + 2.f * dd_abs(z1)));
+    const bool pairs = !FWD && ahead && 2.f * dd_abs(hz) * fmaxf(dd_abs(uA), dd_abs(uB)) < apart;
     // the rows: their z slope, length and value
     float rz[2], y[2], len[2], acc[2] = {0.f, 0.f};
     bool has[2], any = false, finite = true;

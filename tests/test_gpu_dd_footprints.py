@@ -57,3 +57,26 @@ def test_values_that_are_not_finite_stay_in_their_footprints(cuda, db):
         assert 0 < int((~fine).sum()) < ref.numel() // 10
         assert torch.equal(torch.isfinite(out), fine)
         assert_parity(torch.where(fine, out, 0.0).cpu().numpy(), torch.where(fine, ref, 0.0).cpu().numpy())
+
+
+def test_pairs_of_rows_in_a_tall_grid(cuda):
+    """10^6 slices and footprints just under a voxel wide: neighbouring rows'
+    positions, rounded at that height, can lie more than a voxel apart.  Pairing
+    the rows the other way round (one more row in front, without a value) moves no
+    contribution.  The rows' places are exact in float, so both calls have the same
+    footprints."""
+    nz, nb_, db = 1_000_000, 4096, 2.0
+
+    def back(rows, y):
+        # row i of the first call is row i + 1 of the second
+        first = 800_000.0 - (rows - nb_) * db
+        g = ops.DDGeometry((6, 2, nz), np.zeros(1, np.float32), 600.0, 1207.2, 6, 1.0, rows, db,
+                           b_offset=first + rows * db / 2)
+        return ops.dd_backward(y, g, _lib.FDK_NO_WEIGHT)
+
+    y = torch.rand((1, nb_, 6), device=cuda, generator=torch.Generator(device=cuda).manual_seed(2))
+    a = back(nb_, y)
+    b = back(nb_ + 1, torch.cat([torch.zeros((1, 1, 6), device=cuda), y], 1))
+    assert float((a != 0).float().sum()) > 1e4
+    # sums of a few products each: a few roundings of 6e-8
+    assert float((a - b).abs().max()) < 1e-6 * float(a.abs().max())
