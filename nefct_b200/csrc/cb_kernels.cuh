@@ -324,7 +324,9 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
         // within a voxel of the first ray, at both ends, by more than the
         // positions' rounding, it is so in every slab
         const float d0 = col_plane(q.c, q.K0), d1 = col_plane(q.c, q.K1 + 1);
-        const float m = 1e-3f + 1e-6f * (fabsf(q.z[0].z0) + fabsf(q.z[0].kz) * (fabsf(q.c.pu) + fabsf(q.c.nu2)));
+        float size = fabsf(q.z[0].z0) + fabsf(q.z[0].kz) * (fabsf(q.c.pu) + fabsf(q.c.nu2));
+        if (REF) size += fabsf(q.z[0].pw) * q.zg.rdz + q.zg.nz2;
+        const float m = 1e-3f + 1e-6f * size;
         bool near = true;
 #pragma unroll
         for (int i = 1; i < R; ++i) {

@@ -292,3 +292,25 @@ def test_error_against_double_is_no_larger_than_the_reference_walks(cuda, oracle
         f, b = (t.cpu().numpy() for t in _both(g, v, s, 0, walk))
         assert err(f, f64) <= 1.1 * err(f32, f64), (err(f, f64), err(f32, f64))
         assert err(b, b64) <= 1.1 * err(b32, b64), (err(b, b64), err(b32, b64))
+
+
+@pytest.mark.parametrize("flags", [0, _lib.TIE_GT], ids=["default", "reference-rounding"])
+def test_pairs_of_rows_in_a_tall_grid(cuda, flags):
+    """65535 slices and neighbouring rows just under a voxel apart, whose
+    positions round by some thousandths of a voxel at that height: pairing the rows
+    the other way round (one more row in front, without a value) moves no
+    contribution.  The rows' places are exact in float in both calls."""
+    nv, rows, db = 1000, 18, 113 / 64
+    off = np.floor(np.random.default_rng(3).random(nv) * 64000) / 2 - 16000 + np.arange(nv) / 1024
+
+    def back(nb_, y):
+        g = nb.ConeBeam((3, 3, 65535), np.linspace(0, 2 * np.pi, nv, endpoint=False), 12.0, 24.0, 8, 0.5, nb_, db,
+                        b_shift=0.5 + nb_ / 2 - (nb_ - rows) - rows / 2, z_offsets=off.astype(np.float32))
+        return ops.cb_backward(y, g, flags)
+
+    y = torch.rand((nv, rows, 8), device=cuda, generator=torch.Generator(device=cuda).manual_seed(2))
+    a = back(rows, y)
+    b = back(rows + 1, torch.cat([torch.zeros((nv, 1, 8), device=cuda), y], 1))
+    assert int((a != 0).sum()) > 10000
+    # sums of up to a few hundred terms in another order
+    assert float((a - b).abs().max()) < 3e-6 * float(a.abs().max())
