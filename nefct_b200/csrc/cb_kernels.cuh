@@ -440,13 +440,19 @@ static inline int col_rows_next(const GridDev<float> &g, const RayGeom<float> &r
 
 // Column warps apply to FP32 slab walks with a workspace; the z-fastest
 // copy's transposes launch ny planes (grid z: at most 65535); grids as wide keep
-// the thread walk too, the only one run at that width.  (NEFCT_DETERMINISTIC
-// changes nothing for the forward; its transpose has kernels of its own.)
-template <typename T> static inline bool cb_use_colwarp(const nefct_grid &g, uint32_t flags, bool forward)
+// the thread walk too, the only one run at that width.  Up to 8 detector rows
+// leave most lanes of a column warp idle: the thread walk takes them (512^2 x 1 to
+// 64, 120 views of 800 columns: 1 row 1.5 -> 0.26 ms forward and 1.7 -> 0.22
+// transpose, 8 rows 1.6 -> 0.7 and 1.9 -> 0.7 to 0.8, 16 rows 1.6 / 1.3 and 1.9 /
+// 1.5; 128^2: 75 -> 48 and 85 -> 46 us, 75 -> 58 and 92 -> 63, 78 / 82 and 93 / 98).
+// (NEFCT_DETERMINISTIC changes nothing for the forward; its transpose has
+// kernels of its own.)  nb: detector rows, where that counts.
+template <typename T>
+static inline bool cb_use_colwarp(const nefct_grid &g, uint32_t flags, bool forward, int nb = 65535)
 {
     return sizeof(T) == sizeof(float) && (tune_get(NEFCT_TUNE_CB_WALK) & (forward ? 1 : 2)) != 0 &&
            !(flags & (NEFCT_EXACT | NEFCT_NO_TRANSPOSE)) && (forward || !(flags & NEFCT_DETERMINISTIC)) &&
-           g.nx < 65533 && g.ny < 65533;
+           g.nx < 65533 && g.ny < 65533 && nb > 8;
 }
 
 // Launches the thread-walk forward (FWD) or transpose kernel for the views

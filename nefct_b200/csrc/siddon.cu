@@ -513,7 +513,7 @@ static nefct_status cb_forward_impl(const nefct_cb_geom *g, const T *vol, T *sin
     p->vol = vol;
     p->out = sino;
     const size_t nvox = (size_t)g->grid.nx * g->grid.ny * g->grid.nz;
-    const bool cw = cb_use_colwarp<T>(g->grid, flags, true);
+    const bool cw = cb_use_colwarp<T>(g->grid, flags, true, g->nb);
     if (!(flags & NEFCT_NO_TRANSPOSE)) {
         if (!ws || wsb < nvox * sizeof(T)) {
             delete p;
@@ -579,7 +579,7 @@ static nefct_status cb_backward_fixed_impl(const nefct_cb_geom *g, const float *
     unsigned long long *accN = (unsigned long long *)(w + 256);
     unsigned long long *accT = tr ? accN + nvox : nullptr;
     // column warps reduce everything into accN in z-fastest order
-    const bool cw = tr && cb_use_colwarp<float>(g->grid, flags & ~NEFCT_DETERMINISTIC, false);
+    const bool cw = tr && cb_use_colwarp<float>(g->grid, flags & ~NEFCT_DETERMINISTIC, false, g->nb);
     NEFCT_CHECK_CUDA(cudaMemsetAsync(w, 0, cw ? 256 + nvox * sizeof(unsigned long long) : need, s));
     const size_t ns = (size_t)g->na * g->nb * g->nv;
     maxabs_kernel<<<(unsigned)std::min<size_t>((ns + 255) / 256, 148 * 16), 256, 0, s>>>(sino, ns, maxbits);
@@ -644,7 +644,7 @@ static nefct_status cb_backward_impl(const nefct_cb_geom *g, const T *sino, T *v
     p->outT = tr ? (T *)ws : nullptr;
     // column warps reduce into the z-fastest workspace only; the fold then
     // writes every voxel of vol
-    const bool cw = cb_use_colwarp<T>(g->grid, flags, false);
+    const bool cw = cb_use_colwarp<T>(g->grid, flags, false, g->nb);
     cudaError_t e = cw ? cudaSuccess : cudaMemsetAsync(vol, 0, nvox * sizeof(T), s);
     if (e == cudaSuccess && tr) e = cudaMemsetAsync(ws, 0, nvox * sizeof(T), s);
     if (e != cudaSuccess) { delete p; return cuda_fail(e, "cudaMemsetAsync"); }
@@ -812,7 +812,7 @@ static nefct_status cb_forward_static_impl(const nefct_cb_geom *g, const float *
     // the walk nefct_cb_forward takes for these flags and the current
     // launch tuning, over the same kind of volume copy, so the two give the
     // same bits
-    const bool cw = cb_use_colwarp<float>(g->grid, flags, true);
+    const bool cw = cb_use_colwarp<float>(g->grid, flags, true, g->nb);
     float *scratch = nullptr;
     if (tr) {
         st = static_scratch_address(&scratch);

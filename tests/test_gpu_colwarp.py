@@ -182,13 +182,14 @@ def test_grids_wider_than_65536(cuda, oracle_lib, shape, angle, flags):
 @pytest.mark.parametrize("walk", [0, 3], ids=["thread", "columns"])
 @pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT, _lib.NO_TRANSPOSE, _lib.DETERMINISTIC],
                          ids=["default", "reference-rounding", "direct", "deterministic"])
+@pytest.mark.parametrize("rows", [1, 9])
 @pytest.mark.parametrize("nz", [1, 2])
-def test_nothing_outside_the_buffers_is_touched(cuda, nz, flags, walk):
+def test_nothing_outside_the_buffers_is_touched(cuda, nz, rows, flags, walk):
     """Volume, sinogram and workspace between NaN (inputs) or a mark (outputs):
     rays in the grid's last slice touch no voxel above it, whatever the rounding
     of their crossing ratios."""
     import ctypes as C
-    g = nb.ConeBeam((200, 200, nz), np.linspace(0, 2 * np.pi, 90, endpoint=False), 300.0, 600.0, 310, 1.0, 1, 1.0,
+    g = nb.ConeBeam((200, 200, nz), np.linspace(0, 2 * np.pi, 90, endpoint=False), 300.0, 600.0, 310, 1.0, rows, 0.05,
                     z_offsets=np.full(90, 0.5 * nz - 0.5))
     pad, s, lib = 1 << 17, g.struct(), _lib.load()
     stream = torch.cuda.current_stream(cuda).cuda_stream
@@ -201,7 +202,7 @@ def test_nothing_outside_the_buffers_is_touched(cuda, nz, flags, walk):
 
     vol_all, vol = inside(200 * 200 * nz, np.nan)
     ws_all, ws = inside(max(wn // 4, 1), np.nan)
-    out_all, out = inside(90 * 310, 7.0)
+    out_all, out = inside(90 * 310 * rows, 7.0)
     vol.copy_(torch.rand(vol.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)))
     back_all, back = inside(vol.numel(), 7.0)
     y = torch.rand(out.shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(5))
@@ -314,3 +315,26 @@ def test_pairs_of_rows_in_a_tall_grid(cuda, flags):
     assert int((a != 0).sum()) > 10000
     # sums of up to a few hundred terms in another order
     assert float((a - b).abs().max()) < 3e-6 * float(a.abs().max())
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("rows", [7, 8, 9])
+def test_few_detector_rows(cuda, oracle_lib, rows, flags):
+    """Both sides of the line below which the thread walk takes the rows, alone and
+    in a batch plan (column warps at any number of rows)."""
+    from nefct_b200.batch import BatchProjector
+    g = _geom(rows, 1.2, 1.0, 1.0)
+    rng = np.random.default_rng(rows)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    f, b = _both(g, v, s, flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(b.cpu().numpy(), ref_b)
+    plan = BatchProjector([g], [v], grads=[s], flags=flags, strategy="persistent")
+    plan.step()
+    assert torch.equal(plan.sinos[0], f)
+    assert_parity(plan.backs[0].cpu().numpy(), ref_b)
+    fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
+    assert torch.equal(*fixed)
