@@ -114,17 +114,18 @@ __device__ __forceinline__ void warp_reduce(T *gimg, bool valid, int base, T (&v
     }
 }
 
-// Voxels along z per thread of the adjoint (2 is 5 % slower on smooth fields and
-// 2 % faster on white noise, 8 the reverse).
-static constexpr int kWarpZ = 4;
+// Voxels along z per thread of the adjoint: 4 takes 5 to 8 % off smooth fields
+// (192^3 / 384^3: 44 / 290 us) and adds as much where no corner is shared (247 /
+// 1916 us), which 1 voxel and no merging take in 235 / 1860.
+static constexpr int kWarpZ = 2;
 
 // What bounds it: the reductions, which the L2 takes sector by sector (1.9e11/s).
 // Where the field is smooth, neighbours in z have base corners one above the
 // other and neighbours in x one beside the other: a thread adds the upper four
 // taps of a voxel to the lower four of the next, and a lane takes over its
-// neighbour's (warp_reduce), which leaves 2 to 3 reductions of a voxel's 8.
-// 192^3 / 512^3, smooth field: 71 / 1160 -> 46 / 668 us; white noise of +-3 voxels,
-// where nothing is shared: 237 / 4420 -> 250 / 4570 us.
+// neighbour's (warp_reduce), which leaves 2 to 4 reductions of a voxel's 8.
+// 192^3 / 384^3, smooth field: 69 / 491 -> 46 / 315 us; white noise of +-3 voxels,
+// where nothing is shared: 235 / 1860 -> 237 / 1869 us.
 template <typename T>
 __global__ void __launch_bounds__(256) warp_adjoint_kernel(const T *__restrict__ gout, const T *__restrict__ mx,
                                                            const T *__restrict__ my, const T *__restrict__ mz,
