@@ -30,8 +30,8 @@
 //    voxel above while 2h < 1 (wider footprints loop over their voxels).
 //  * The backward sums the shares of two neighbouring rows in registers before
 //    it reduces them.
-// The double build (checks) walks thread by thread of the same layout over the
-// x-fastest volume.  Per-view cos/sin/offset ride in the kernel parameters.
+// The double build (checks) evaluates every footprint per row, two rows per lane,
+// over the x-fastest volume.  Per-view cos/sin/offset ride in the kernel parameters.
 #include <math.h>
 #include <algorithm>
 
@@ -103,25 +103,39 @@ __device__ __forceinline__ double dd_rcp(double x) { return __drcp_rn(x); }
 __device__ __forceinline__ int dd_floor(float x) { return (int)floorf(x); }
 __device__ __forceinline__ int dd_floor(double x) { return (int)floor(x); }
 
-// The double build: one warp walks 32 rows (bins) of one detector column at
-// one view over the slabs of the column's driving axis.
-// FWD false: each lane reduces value * weight into the voxels of its bin's
-// footprint (the reference's kernel); FWD true: each lane sums voxel * weight
+// The double build: one warp walks 32 R rows (bins) of one detector column at
+// one view, R per lane (rows l, l + 32, ...), over the slabs of the column's
+// driving axis; a slab's transverse part is evaluated once for the R rows
+// (128^3, 24 views of 256 x 192, R = 1 / 2 / 4: forward 1.73 / 1.23 / 1.32 ms,
+// backward 1.54 / 1.44 / 1.48).
+// FWD false: each lane reduces value * weight into the voxels of its bins'
+// footprints (the reference's kernel); FWD true: each lane sums voxel * weight
 // over the same voxels with the same weights (the exact transpose) into its
-// bin.  With p.fdk false the weight lacks the FDK factor SAD^2 / (SAD + x cos +
+// bins.  With p.fdk false the weight lacks the FDK factor SAD^2 / (SAD + x cos +
 // y sin)^2.
+static constexpr int kDDRows = 2;
+
 template <bool FWD>
 __global__ void __launch_bounds__(128) dd_kernel(const __grid_constant__ DDParams<double> p)
 {
     using T = double;
     using F = FP<T>;
+    constexpr int R = kDDRows;
     const int ia = blockIdx.x * blockDim.y + threadIdx.y;
-    const int ib = blockIdx.y * 32 + threadIdx.x;
+    const int row = blockIdx.y * 32 * R + threadIdx.x;
     const int iv = blockIdx.z;
-    if (ia >= p.na || ib >= p.nb) return;
-    const size_t bin = ((size_t)(p.v0 + iv) * p.nb + ib) * p.na + ia;
-    const T value = FWD ? (T)0 : p.src[bin];
-    if (!FWD && value == (T)0) return;
+    if (ia >= p.na) return;
+    const size_t bin = ((size_t)(p.v0 + iv) * p.nb + row) * p.na + ia, next = (size_t)32 * p.na;
+    T value[R];
+    bool live[R], any = false;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        live[i] = row + 32 * i < p.nb;
+        value[i] = FWD || !live[i] ? (T)0 : p.src[bin + i * next];
+        live[i] = live[i] && (FWD || value[i] != (T)0);
+        any = any || live[i];
+    }
+    if (!any) return;
 
     const T cphi = p.tab.cs[iv], sphi = p.tab.sn[iv], off = p.tab.off[iv];
     const T x1 = F::mul(-p.sad, cphi), y1 = F::mul(-p.sad, sphi), z1 = off;
@@ -146,13 +160,19 @@ __global__ void __launch_bounds__(128) dd_kernel(const __grid_constant__ DDParam
     // the reference divides inside the slab loop; the quotients do not depend on the slab
     const T r0 = F::div(vl, ul), r1 = F::div(vl, ur), r2 = F::div(vr, ul), r3 = F::div(vr, ur);
     const T hdb = F::div(p.db, (T)2);
-    const T z2 = F::add(dd_center(ib, p.db, p.bi, p.nb), off), z21 = F::sub(z2, z1);
-    const T len = F::sqrt(F::add(F::add(F::mul(x21, x21), F::mul(y21, y21)), F::mul(z21, z21)));
-    const T rzl = F::div(F::sub(z21, hdb), u21), rzr = F::div(F::add(z21, hdb), u21), len_au = F::div(len, dd_abs(u21));
+    T rzl[R], rzr[R], len_au[R], acc[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const T z2 = F::add(dd_center(row + 32 * i, p.db, p.bi, p.nb), off), z21 = F::sub(z2, z1);
+        const T len = F::sqrt(F::add(F::add(F::mul(x21, x21), F::mul(y21, y21)), F::mul(z21, z21)));
+        rzl[i] = F::div(F::sub(z21, hdb), u21);
+        rzr[i] = F::div(F::add(z21, hdb), u21);
+        len_au[i] = F::div(len, dd_abs(u21));
+        acc[i] = (T)0;
+    }
     const T vhalf = (T)(nvt / 2), zhalf = (T)(p.nz / 2), uhalf = F::div((T)nu, (T)2);
     const T sad2 = F::mul(p.sad, p.sad);
     const T xhalf = (T)(p.nx / 2), yhalf = (T)(p.ny / 2);
-    T acc = (T)0;
     for (int iu = 0; iu < nu; ++iu) {
         const T uc = F::sub(F::sub(F::add((T)iu, (T)0.5), uhalf), u1);
         const T c0 = F::add(F::add(F::mul(r0, uc), v1), vhalf);
@@ -163,11 +183,19 @@ __global__ void __launch_bounds__(128) dd_kernel(const __grid_constant__ DDParam
         const T vi2 = dd_max(dd_max(c0, c1), dd_max(c2, c3));
         const int va = max(0, dd_floor(vi1)), vb = min(nvt - 1, dd_floor(vi2));
         if (va > vb) continue;                      // footprint outside the grid
-        const T czl = F::add(F::add(F::mul(rzl, uc), z1), zhalf);
-        const T czr = F::add(F::add(F::mul(rzr, uc), z1), zhalf);
-        const T zi1 = dd_min(czl, czr), zi2 = dd_max(czl, czr);
-        const int za = max(0, dd_floor(zi1)), zb = min(p.nz - 1, dd_floor(zi2));
-        const T izspan = dd_rcp(F::sub(zi2, zi1)), ivspan = dd_rcp(F::sub(vi2, vi1));
+        const T ivspan = dd_rcp(F::sub(vi2, vi1));
+        T zi1[R], zi2[R], izspan[R];
+        int za[R], zb[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const T czl = F::add(F::add(F::mul(rzl[i], uc), z1), zhalf);
+            const T czr = F::add(F::add(F::mul(rzr[i], uc), z1), zhalf);
+            zi1[i] = dd_min(czl, czr);
+            zi2[i] = dd_max(czl, czr);
+            za[i] = max(0, dd_floor(zi1[i]));
+            zb[i] = live[i] ? min(p.nz - 1, dd_floor(zi2[i])) : -1;
+            izspan[i] = dd_rcp(F::sub(zi2[i], zi1[i]));
+        }
         for (int iv2 = va; iv2 <= vb; ++iv2) {
             const T wv = F::mul(F::sub(dd_min((T)iv2 + (T)1, vi2), dd_max((T)iv2, vi1)), ivspan);
             const int ix = xdrive ? iu : iv2, iy = xdrive ? iv2 : iu;
@@ -180,16 +208,23 @@ __global__ void __launch_bounds__(128) dd_kernel(const __grid_constant__ DDParam
                 fw = F::mul(F::mul(sad2, iden), iden);
             }
             const size_t col = (size_t)iy * p.sy + (size_t)ix * p.sx;
-            // (value *) wv * (len / |u21|) * fw per voxel of the column, times wz
-            const T cw = F::mul(F::mul(FWD ? wv : F::mul(value, wv), len_au), fw);
-            for (int iz = za; iz <= zb; ++iz) {
-                const T wz = F::mul(F::sub(dd_min((T)iz + (T)1, zi2), dd_max((T)iz, zi1)), izspan);
-                if (FWD) acc = F::add(acc, F::mul(__ldg(p.src + col + (size_t)iz * p.sz), F::mul(cw, wz)));
-                else atomicAdd(p.dst + col + (size_t)iz * p.sz, F::mul(cw, wz));
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                // (value *) wv * (len / |u21|) * fw per voxel of the column, times wz
+                const T cw = F::mul(F::mul(FWD ? wv : F::mul(value[i], wv), len_au[i]), fw);
+                for (int iz = za[i]; iz <= zb[i]; ++iz) {
+                    const T wz = F::mul(F::sub(dd_min((T)iz + (T)1, zi2[i]), dd_max((T)iz, zi1[i])), izspan[i]);
+                    if (FWD) acc[i] = F::add(acc[i], F::mul(__ldg(p.src + col + (size_t)iz * p.sz), F::mul(cw, wz)));
+                    else atomicAdd(p.dst + col + (size_t)iz * p.sz, F::mul(cw, wz));
+                }
             }
         }
     }
-    if (FWD) p.dst[bin] = acc;
+    if (FWD) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (live[i]) p.dst[bin + i * next] = acc[i];
+    }
 }
 
 // ---- float: column warps ----
@@ -569,7 +604,7 @@ static nefct_status dd_impl(const nefct_dd_geom *g, const T *src, T *dst, uint32
             p->tab.sn[i] = (T)sin(a);
             p->tab.off[i] = g->z_offsets ? (T)g->z_offsets[v0 + i] : (T)0;
         }
-        const int rows = f32 ? 64 : 32;
+        const int rows = f32 ? 64 : 32 * kDDRows;
         dim3 grid((g->na + cols - 1) / cols, (g->nb + rows - 1) / rows, nvc), block(32, cols);
         if constexpr (std::is_same<T, float>::value) {
             if (forward) dd_colwarp_kernel<true><<<grid, block, 0, s>>>(*p);
