@@ -108,10 +108,14 @@ def _pixel_backproject(cyl):
     return op
 
 
-# Line lists at least this long are walked in lor_order (a key pass and a
-# sort, ~1 ms for 16 Mi lines, against a 6-8x slower walk in list order); the
-# results keep the lines' order, so the ops behave exactly as in list order
-# (the backprojection up to the summation order of its float reductions).
+# The forward walks line lists at least this long in lor_order (a key pass and a
+# sort, 0.14 / 0.30 / 0.91 ms for 1 / 4 / 16 Mi lines); the results keep the lines'
+# order and bits.  Through 256^3, list order against order and walk: lines of a
+# 300 mm ring, of which half miss the grid or graze it, 0.66 / 2.5 / 9.9 ms against
+# 0.54 / 1.8 / 7.0; of a ring just around the grid, all of a length, 0.82 / 2.9 /
+# 11.7 against 0.97 / 3.3 / 12.5; 0.5 Mi lines 0.36 against 0.35 and 0.44 against
+# 0.58.  The backprojection takes list order: 0.66 / 2.5 / 9.5 ms against 0.72 / 2.4
+# / 9.9, and 1.2 / 4.5 / 17.8 against 1.4 / 5.0 / 19.8.
 _LOR_AUTO_ORDER = 1 << 20
 
 
@@ -133,8 +137,7 @@ def _backprojection(image, lors, lors_value, grid, center, size):
     g = _host3(grid, int)
     lors = lors.contiguous()
     c, s = _host3(center, float), _host3(size, float)
-    vol = ops.lor_backward(lors, lors_value.contiguous(), g, c, s, _lib.LOR_REF_BACKPROJECT,
-                           order=_lor_walk_order(lors, g, c, s))
+    vol = ops.lor_backward(lors, lors_value.contiguous(), g, c, s, _lib.LOR_REF_BACKPROJECT)
     return vol.view(image.shape)
 
 

@@ -196,7 +196,10 @@ def _check_order(order, n, device):
 def lor_order(lors: torch.Tensor, shape, center=(0.0, 0.0, 0.0), size=None) -> torch.Tensor:
     """Walk order for a large unsorted line list: an int32 permutation that
     groups nearly parallel neighbouring lines (pass it as ``order`` to
-    lor_forward / lor_backward; compute it once per list)."""
+    lor_forward / lor_backward; compute it once per list).  It pays where the
+    lines' lengths in the grid differ (forward 1.6 times, backward 1.1 times
+    faster for a ring twice as wide as the grid), and costs up to 6 % in the
+    backward where they do not."""
     if lors.dim() != 2 or lors.shape[0] != 6:
         raise NefctError(_lib.ERR_INVALID, "lors must be [6, n]")
     _check_tensor(lors, tuple(lors.shape), "lors")
