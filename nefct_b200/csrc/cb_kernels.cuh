@@ -87,9 +87,9 @@ __device__ __noinline__ static float ray_resum(const GridDev<float> &g, float x1
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
     if (ref_rounding(flags))
-        ray_slabs<true, true, false, -1, true>(c, z_ray<true>(w, zg, z_source<true>(w, zg), true), zg, w.k0, w.k1, sw, f);
+        ray_slabs<true, true, false, -1, true, false>(c, z_ray<true>(w, zg, z_source<true>(w, zg), true), zg, w.k0, w.k1, sw, f);
     else
-        ray_slabs<false, true, false, -1, true>(c, z_ray<false>(w, zg, z_source<false>(w, zg), true), zg, w.k0, w.k1, sw, f);
+        ray_slabs<false, true, false, -1, true, false>(c, z_ray<false>(w, zg, z_source<false>(w, zg), true), zg, w.k0, w.k1, sw, f);
     f.close();
     return f.whole * w.W;
 }
@@ -274,7 +274,7 @@ __device__ __noinline__ static void colwarp_scatter_rare(const GridDev<float> &g
         col_scatter<1, REF, true, true, kSingle>(q, acc, yw);
     } else if (q.z[0].live) {
         auto f = ray_sink(acc, yw[0]);
-        ray_slabs<REF, true, false, -1, true>(q.c, q.z[0], q.zg, q.K0, q.K1, 1u, f);
+        ray_slabs<REF, true, false, -1, true, false>(q.c, q.z[0], q.zg, q.K0, q.K1, 1u, f);
     }
 }
 

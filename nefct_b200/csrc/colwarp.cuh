@@ -362,15 +362,16 @@ struct FixedSink {
 
 // Slabs k..end of one ray alone (any strides), with a column warp's operations
 // per slab, so with its bits; v positions and floors are carried from plane to
-// plane.  CHECK: range checks, any slope; else every voxel is in the grid and
-// the ray is not steep, DOWN: v falls along the walk.  A slab without a v
+// plane.  CHECK: range checks, any slope; else every voxel is in the grid, and the
+// ray is STEEP or DOWN says whether v falls along the walk.  A slab without a v
 // crossing is taken as one with rv = 1 (its third voxel has no share).  The
 // high column is the one at the slab's far plane: where dv < 1 it need not be
 // the low one's neighbour.
-template <bool REF, bool CHECK, bool DOWN, int DIV, bool ALIGN, class Sink>
+template <bool REF, bool CHECK, bool DOWN, int DIV, bool ALIGN, bool STEEP, class Sink>
 __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
                                           Sink &f)
 {
+    constexpr bool ANY = CHECK || STEEP;
     const Inside vin(c.nv), zin(zg.nz, z.zi);
     float t = __fsub_rn((float)k, c.nu2), da = __fsub_rn(t, c.pu);
     float qa = col_vpos<DIV>(c, da), ma = magic_floor<CHECK>(qa), za = z_at<REF>(z, zg, da);
@@ -378,16 +379,16 @@ __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const
     auto slab = [&](RaySlab &s) {
         t = __fadd_rn(t, 1.f);
         const float db = __fsub_rn(t, c.pu), qb = col_vpos<DIV>(c, db), mb = magic_floor<CHECK>(qb);
-        const float q1 = CHECK ? fminf(qa, qb) : DOWN ? qb : qa, q2 = CHECK ? fmaxf(qa, qb) : DOWN ? qa : qb;
-        const float m1 = CHECK ? fminf(ma, mb) : DOWN ? mb : ma, m2 = CHECK ? fmaxf(ma, mb) : DOWN ? ma : mb;
+        const float q1 = ANY ? fminf(qa, qb) : DOWN ? qb : qa, q2 = ANY ? fmaxf(qa, qb) : DOWN ? qa : qb;
+        const float m1 = ANY ? fminf(ma, mb) : DOWN ? mb : ma, m2 = ANY ? fmaxf(ma, mb) : DOWN ? ma : mb;
         const bool vx = m1 != m2;
         const float rv = col_ratio(q1, q2, m1, m2);
         const float zb = z_at<REF>(z, zg, db), zl = z.down ? zb : za, zh = z.down ? za : zb;
         float m, mh, r;
-        if constexpr (CHECK) z_split<REF>(z, zl, zh, m, mh, r);
+        if constexpr (ANY) z_split<REF>(z, zl, zh, m, mh, r);
         else z_share<REF>(z, zl, zh, m, r);
         const unsigned z1 = base + (unsigned)__float_as_int(m) * sw;
-        const unsigned up = CHECK ? (unsigned)(__float_as_int(mh) - __float_as_int(m)) * sw : sw;
+        const unsigned up = ANY ? (unsigned)(__float_as_int(mh) - __float_as_int(m)) * sw : sw;
         const unsigned v1 = z1 + (unsigned)__float_as_int(m1) * c.sv, v2 = z1 + (unsigned)__float_as_int(m2) * c.sv;
         const bool vfirst = rv > r;             // the middle voxel is (v1, z2), else (v2, z1)
         const float both = fminf(rv, r), over = __fsub_rn(r, both);      // r's share in the high column
@@ -465,11 +466,11 @@ __device__ __forceinline__ void ray_inner(const ColWalk &c, const ZRay &z, const
                                              unsigned sw, Sink &f)
 {
     if (c.vdiv) {
-        if (c.kv < 0.f) ray_slabs<REF, false, true, 1, ALIGN>(c, z, zg, k, end, sw, f);
-        else ray_slabs<REF, false, false, 1, ALIGN>(c, z, zg, k, end, sw, f);
+        if (c.kv < 0.f) ray_slabs<REF, false, true, 1, ALIGN, false>(c, z, zg, k, end, sw, f);
+        else ray_slabs<REF, false, false, 1, ALIGN, false>(c, z, zg, k, end, sw, f);
     } else {
-        if (c.kv < 0.f) ray_slabs<REF, false, true, 0, ALIGN>(c, z, zg, k, end, sw, f);
-        else ray_slabs<REF, false, false, 0, ALIGN>(c, z, zg, k, end, sw, f);
+        if (c.kv < 0.f) ray_slabs<REF, false, true, 0, ALIGN, false>(c, z, zg, k, end, sw, f);
+        else ray_slabs<REF, false, false, 0, ALIGN, false>(c, z, zg, k, end, sw, f);
     }
 }
 // The thread walk: the slabs k0..k1 of a ray, of them ki0..ki1 without range checks.
@@ -480,13 +481,14 @@ __device__ __forceinline__ void ray_walk(const GridDev<float> &g, const Walk<flo
     const ColWalk c = col_walk_of(g, w, su, sv);
     const ZGrid zg = z_grid(g);
     const ZRay z = z_ray<REF>(w, zg, z_source<REF>(w, zg), true);
-    const bool interior = !z.steep && w.ki0 <= w.ki1;
+    const bool interior = w.ki0 <= w.ki1;
     int k = w.k0, end = interior ? w.ki0 - 1 : w.k1;
 #pragma unroll 1
     for (;;) {
-        ray_slabs<REF, true, false, -1, true>(c, z, zg, k, end, sw, f);
+        ray_slabs<REF, true, false, -1, true, false>(c, z, zg, k, end, sw, f);
         if (end == w.k1) break;
-        if (!COPY && sv != 1u) ray_inner<REF, COPY>(c, z, zg, w.ki0, w.ki1, sw, f);
+        if (z.steep) ray_slabs<REF, false, false, -1, true, true>(c, z, zg, w.ki0, w.ki1, sw, f);
+        else if (!COPY && sv != 1u) ray_inner<REF, COPY>(c, z, zg, w.ki0, w.ki1, sw, f);
         else ray_inner<REF, true>(c, z, zg, w.ki0, w.ki1, sw, f);
         if (w.ki1 == w.k1) break;
         k = w.ki1 + 1;
