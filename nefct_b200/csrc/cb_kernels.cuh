@@ -122,9 +122,9 @@ __device__ __forceinline__ T ray_forward(const GridDev<T> &g, const T *r, uint32
         if (!isfinite(sum)) return ray_resum(g, r[0], r[1], r[2], r[3], r[4], r[5], flags, v, su, sv, (unsigned)sw);
         return sum * w.W;
     } else {
-        if (!w.xdrive) return gather_walk<T, VAR, true, false>(w, g, vol, g.nx, 1, sw);
-        if (volT) return gather_walk<T, VAR, true, false>(w, g, volT, g.ny, 1, sw);
-        return gather_walk<T, VAR, false, false>(w, g, vol, 1, g.nx, sw);
+        if (!w.xdrive) return gather_walk<T, VAR, true>(w, g, vol, g.nx, 1, sw);
+        if (volT) return gather_walk<T, VAR, true>(w, g, volT, g.ny, 1, sw);
+        return gather_walk<T, VAR, false>(w, g, vol, 1, g.nx, sw);
     }
 }
 
@@ -146,9 +146,9 @@ __device__ __forceinline__ void ray_backward(const GridDev<T> &g, const T *r, ui
         ScatterSink f{w.xdrive && outT ? outT : out, y * w.W};
         ray_walk<VAR, true>(g, w, su, sv, (unsigned)sw, f);
     } else {
-        if (!w.xdrive) scatter_walk<T, VAR, true, false>(w, g, out, g.nx, 1, sw, y);
-        else if (outT) scatter_walk<T, VAR, true, false>(w, g, outT, g.ny, 1, sw, y);
-        else scatter_walk<T, VAR, false, false>(w, g, out, 1, g.nx, sw, y);
+        if (!w.xdrive) scatter_walk<T, VAR, true>(w, g, out, g.nx, 1, sw, y);
+        else if (outT) scatter_walk<T, VAR, true>(w, g, outT, g.ny, 1, sw, y);
+        else scatter_walk<T, VAR, false>(w, g, out, 1, g.nx, sw, y);
     }
 }
 

@@ -32,9 +32,9 @@
 //    same in the forward and its transpose.  Positions count from the source's
 //    row, so that z0 is a fraction held to 2^-25: rounded at the size of a row
 //    number its error, constant along the ray, would go into every share divided
-//    by |kz| (rel-L2 against FP64 of 26 x 22 x 24 voxels, thin slices, source
-//    off the middle: 1.33e-6, now 1.24e-6; the reference's operations in float:
-//    1.24e-6).
+//    by |kz| (rel-L2 of the forward against FP64, 600 slices of 0.1 voxel, nearly
+//    level rays: 1.5e-5, so 3.3e-6, the reference's operations in float 8.7e-6; 24
+//    cubic ones: 1.00e-6, 9.4e-7, 9.8e-7).
 //  * REF (calls with NEFCT_TIE_GT, the switches of the reference's own
 //    backprojection): q1 and q2 with the reference's operations in its order.
 //    A nearly level ray (|kz| ~ 1e-3) divides rounding errors of ~1e-5 voxel
@@ -366,7 +366,14 @@ struct FixedSink {
 // ray is STEEP or DOWN says whether v falls along the walk.  A slab without a v
 // crossing is taken as one with rv = 1 (its third voxel has no share).  The
 // high column is the one at the slab's far plane: where dv < 1 it need not be
-// the low one's neighbour.
+// the low one's neighbour.  ALIGN: the lanes of a warp close their blocks of 32
+// slabs together; where the gathers stride along v (x-driven rays without the
+// y-fastest copy) lanes in step read one x column of rows 4 nx bytes apart, whose
+// sectors share banks, so there each keeps its own phase.
+// Bound by issue (76 % with the copy) and the gathers' latency; 256^3, 48 views of
+// 512 x 384: forward 3.56 ms with the y-fastest copy (one slab at a time 3.85), 4.19
+// without (in step 4.83), transpose 3.98 and 8.02; with the reference's rounding
+// 3.86, 4.39, 4.30 and 8.04.
 template <bool REF, bool CHECK, bool DOWN, int DIV, bool ALIGN, bool STEEP, class Sink>
 __device__ __forceinline__ void ray_slabs(const ColWalk &c, const ZRay &z, const ZGrid &zg, int k, int end, unsigned sw,
                                           Sink &f)

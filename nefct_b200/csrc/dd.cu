@@ -13,9 +13,10 @@
 //    span of the bin's lower/upper z edges (:125-139);
 //  * every voxel inside both footprints gets value * (overlap fraction in v)
 //    * (overlap fraction in z) / |u21| * |p2 - p1| * SAD^2 / (SAD + x cos +
-//    y sin)^2 (:141-154).  The footprints are evaluated with the reference's
-//    operations; the weights divide by multiplying with approximate
-//    reciprocals and group the per-column factors (a few ulp per weight).
+//    y sin)^2 (:141-154).  The transverse footprint is evaluated with the
+//    reference's operations (in double the z footprint too); the weights divide
+//    by multiplying with approximate reciprocals and group the per-column
+//    factors (a few ulp per weight).
 //
 // GPU structure (not the reference's), float: one warp walks the rows of one
 // detector column at one view, several per lane, over a z-fastest volume copy

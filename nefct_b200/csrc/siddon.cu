@@ -139,7 +139,7 @@ struct LorParams {
 // kernels under 64 registers and a warp's lines of different signs together
 // (the variants took 100 to 116 registers, so half the warps to hide the
 // gathers' latency with, and ran one after the other).  256^3, 4 Mi ring lines
-// in walk order: forward 4.11 -> 2.99 ms, bound by the gathers' requests (12
+// in walk order: forward 4.11 -> 2.99 ms, bound by the gathers' requests (19
 // sectors each), backward 4.64 -> 4.68 ms, by the L2's rate of scattered
 // reductions (1.9e11/s); in list order 22.8 -> 2.95 and 15.8 -> 4.47 ms.  A
 // y-fastest copy for one of the driving axes, either way round, is slower:
@@ -164,8 +164,8 @@ struct LineWalk {
 
     __device__ __forceinline__ LineWalk(const GridDev<float> &g, const Walk<float> &w)
         : pv(w.pv), kv(w.kv), dv(w.dv), nv2(w.nv2), pw(w.pw), kw(w.kw), dz(g.dz), nz2(g.nz2), pu(w.pu),
-          su(w.xdrive ? 1u : (unsigned)g.nx), sv(w.xdrive ? (unsigned)g.nx : 1u), sw((unsigned)g.nx * (unsigned)g.ny), nv(w.nv), nz(g.nz), vdown(w.kv < 0.f), zdown(w.kw < 0.f), vdiv(w.vdiv),
-          zdiv(g.dz != 1.f)
+          su(w.xdrive ? 1u : (unsigned)g.nx), sv(w.xdrive ? (unsigned)g.nx : 1u), sw((unsigned)g.nx * (unsigned)g.ny),
+          nv(w.nv), nz(g.nz), vdown(w.kv < 0.f), zdown(w.kw < 0.f), vdiv(w.vdiv), zdiv(g.dz != 1.f)
     {
         t = __fsub_rn((float)w.k0, w.nu2);
         base = (unsigned)w.k0 * su - (unsigned)kFloorMagicBits * (sv + sw);

@@ -26,8 +26,10 @@
 //    (rounding-level difference from the per-contribution products);
 //  * slabs whose candidate voxels are all inside the grid skip the range
 //    checks (interior range computed with the clip).
-// This walk serves the double builds, the LOR pair and the intersection
-// count; the float cone-beam kernels split slabs as colwarp.cuh does.
+// This walk serves the double builds and the intersection count (and its
+// set-up every walk); the float cone-beam kernels split slabs as colwarp.cuh
+// does, the LOR pair as LineWalk in siddon.cu, with the operations above and the
+// slope signs at run time.
 #pragma once
 
 #include "common.cuh"
@@ -410,36 +412,35 @@ __device__ __forceinline__ void with_walker(const Walk<T> &w, const GridDev<T> &
     }
 }
 
-// Weighted sum of the volume along the ray (forward):
-//   sum over contributions of v * r, times W (and Wmid for Q5 middles).
-template <typename T, bool DIV, bool SV1, bool Q5>
+// Weighted sum of the volume along the ray (forward): v * r over its
+// contributions, times W.
+template <typename T, bool DIV, bool SV1>
 __device__ __forceinline__ T gather_walk(const Walk<T> &w, const GridDev<T> &g, const T *__restrict__ base, int su,
                                          int sv, int sw)
 {
-    T acc = (T)0, accm = (T)0;
+    T acc = (T)0;
     auto f = [&](const SlabSlots<T> &s) {
         const T v0 = s.ok[0] ? __ldg(base + s.idx[0]) : (T)0;
         const T v1 = s.ok[1] ? __ldg(base + s.idx[1]) : (T)0;
         const T v2 = s.ok[2] ? __ldg(base + s.idx[2]) : (T)0;
         acc += v0 * s.r[0];
-        if (Q5 && s.mid3) accm += v1 * s.r[1];
-        else acc += v1 * s.r[1];
+        acc += v1 * s.r[1];
         acc += v2 * s.r[2];
     };
     with_walker<T, DIV, SV1>(w, g, su, sv, sw, [&](auto &it) { walk_all(it, w.k0, w.k1, w.ki0, w.ki1, f); });
-    return Q5 ? acc * w.W + accm * w.Wmid : acc * w.W;
+    return acc * w.W;
 }
 
 // Scatters value * weight along the ray (transpose); reductions do not wait
 // for their result.
-template <typename T, bool DIV, bool SV1, bool Q5>
+template <typename T, bool DIV, bool SV1>
 __device__ __forceinline__ void scatter_walk(const Walk<T> &w, const GridDev<T> &g, T *base, int su, int sv, int sw,
                                              T value)
 {
-    const T yw = value * w.W, ym = value * w.Wmid;
+    const T yw = value * w.W;
     auto f = [&](const SlabSlots<T> &s) {
         if (s.ok[0]) atomicAdd(base + s.idx[0], yw * s.r[0]);
-        if (s.ok[1]) atomicAdd(base + s.idx[1], ((Q5 && s.mid3) ? ym : yw) * s.r[1]);
+        if (s.ok[1]) atomicAdd(base + s.idx[1], yw * s.r[1]);
         if (s.ok[2]) atomicAdd(base + s.idx[2], yw * s.r[2]);
     };
     with_walker<T, DIV, SV1>(w, g, su, sv, sw, [&](auto &it) { walk_all(it, w.k0, w.k1, w.ki0, w.ki1, f); });
