@@ -683,10 +683,8 @@ __global__ void __launch_bounds__(128, 8) fdk_bp_kernel(const __grid_constant__ 
     float zabs = 0.f;
 #pragma unroll
     for (int k = 0; k < kZ; ++k) zabs = fmaxf(zabs, fabsf(zc[k]));
-    // (the rows inside the detector are addressed with 32-bit row pitches; longer
-    // rows take the path with the row test)
+    const float bhi = (float)(p.nb + 1), brow = (float)(p.nb - 1);
     const unsigned pitch = (unsigned)p.na * (unsigned)(QUAD ? sizeof(float4) : sizeof(float));   // bytes per row
-    const float bhi = (float)(p.nb + 1), brow = p.na < 1 << 28 ? (float)(p.nb - 1) : 0.f;
     for (int v = 0; v < p.nvc; ++v) {
         BpColumn c;
         bp_column(p, p.cs[v], p.sn[v], xc, yc, c);
@@ -1035,10 +1033,12 @@ nefct_status nefct_fdk_backproject_ws(const nefct_cb_geom *g, const float *filte
     if (st) return st;
     if (!filtered || !vol) return fail(NEFCT_ERR_INVALID, "filtered and vol must be non-NULL");
     if (flags & ~NEFCT_FDK_NO_WEIGHT) return fail(NEFCT_ERR_INVALID, "unknown flag bits 0x%x", flags);
-    const bool quad = ws != nullptr;
-    if (quad && ws_bytes < nefct_fdk_workspace_bytes(g))
+    if (ws && ws_bytes < nefct_fdk_workspace_bytes(g))
         return fail(NEFCT_ERR_WORKSPACE, "needs %zu workspace bytes, got %zu", nefct_fdk_workspace_bytes(g), ws_bytes);
-    if (quad && ((uintptr_t)ws & 15)) return fail(NEFCT_ERR_INVALID, "workspace must be 16-byte aligned");
+    if (ws && ((uintptr_t)ws & 15)) return fail(NEFCT_ERR_INVALID, "workspace must be 16-byte aligned");
+    // (the kernel's row pitches are 32-bit numbers of bytes: longer rows of quads
+    // are not made; rows of floats fit, with fewer than 2^31 cells)
+    const bool quad = ws != nullptr && g->na < 1 << 28;
     // a detector of one row or column has no cell with four taps (Q11): every
     // voxel is dropped
     if (g->na < 2 || g->nb < 2) {
