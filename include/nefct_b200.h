@@ -51,10 +51,10 @@ const char *nefct_last_error(void);
  *   NEFCT_TUNE_CB_ORDER  0: row bands outermost (default; keeps the volume
  *                        slab of the rows in flight in L2), 1: views outermost
  *   NEFCT_TUNE_CB_WALK   bit 0 forward, bit 1 transpose: column warps (FP32
- *                        slab walk with a workspace) -- each warp walks up to
- *                        128 rows of one detector column, which share their
- *                        transverse walk, over a z-fastest copy of the volume,
- *                        and NEFCT_TUNE_CB_ROWS counts columns per CTA; a
+ *                        slab walk with a workspace, more than 8 detector
+ *                        rows) -- each warp walks up to 128 rows of one
+ *                        detector column, which share their transverse walk,
+ *                        over a z-fastest copy of the volume, and NEFCT_TUNE_CB_ROWS counts columns per CTA; a
  *                        clear bit: one thread per ray.  Default 3 */
 #define NEFCT_TUNE_CB_ROWS  0
 #define NEFCT_TUNE_CB_ORDER 1
@@ -289,7 +289,8 @@ nefct_status nefct_fdk_filter(const nefct_cb_geom *g, const float *sino, float *
  * cell of the flat detector's first or last (where Q11 keeps or drops it on
  * a rounding) is
  * decided with the reference's own operations, so the same voxels are kept;
- * elsewhere the weights differ from the reference's by a few ulp. */
+ * elsewhere the weights differ from the reference's by a few ulp.  A detector
+ * of one row or one column has no cell with four taps: the volume is 0. */
 #define NEFCT_FDK_NO_WEIGHT 0x100u
 nefct_status nefct_fdk_backproject(const nefct_cb_geom *g, const float *filtered, float *vol, uint32_t flags,
                                    void *stream);
@@ -298,7 +299,8 @@ nefct_status nefct_fdk_backproject(const nefct_cb_geom *g, const float *filtered
  * is first repacked into tap quads (the four bilinear taps of every detector
  * cell side by side) so a voxel reads its taps with one 16-byte load.  Same
  * arithmetic, bit-identical result.  The workspace holds one chunk: up to
- * 128 views, about 400 MB at most (16 bytes per detector cell and view).
+ * 128 views, about 400 MB at most (16 bytes per detector cell and view); from
+ * 2^28 columns on it is not used.
  * No counterpart in the reference. */
 size_t nefct_fdk_workspace_bytes(const nefct_cb_geom *g);
 nefct_status nefct_fdk_backproject_ws(const nefct_cb_geom *g, const float *filtered, float *vol, uint32_t flags,
