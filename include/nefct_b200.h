@@ -54,8 +54,9 @@ const char *nefct_last_error(void);
  *                        slab walk with a workspace, more than 8 detector
  *                        rows) -- each warp walks up to 128 rows of one
  *                        detector column, which share their transverse walk,
- *                        over a z-fastest copy of the volume, and NEFCT_TUNE_CB_ROWS counts columns per CTA; a
- *                        clear bit: one thread per ray.  Default 3 */
+ *                        over a z-fastest copy of the volume, and
+ *                        NEFCT_TUNE_CB_ROWS counts columns per CTA; a clear
+ *                        bit: one thread per ray.  Default 3 */
 #define NEFCT_TUNE_CB_ROWS  0
 #define NEFCT_TUNE_CB_ORDER 1
 #define NEFCT_TUNE_CB_WALK  2

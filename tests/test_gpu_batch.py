@@ -189,3 +189,31 @@ def test_batch_row_tiles(cuda, flags, pitch):
             assert torch.equal(s, ops.cb_forward(v, g, flags))
             # the same shares in another order of addition
             assert_parity(b.cpu().numpy(), ops.cb_backward(y, g, flags).cpu().numpy(), rel=1e-6, mabs=1e-5)
+
+
+@pytest.mark.parametrize("flags", [0, nb._lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("walk", [0, 3], ids=["thread", "columns"])
+def test_batch_steep_rays(cuda, walk, flags):
+    """Cone angles beyond 45 degrees in a plan (whose kernel calls a function for
+    the warps with steep rays), beside an ordinary problem; a value that is not
+    finite stays on its ray."""
+    ang = np.linspace(0.1, 6.0, 7)
+    geoms = [nb.ConeBeam((20, 18, 60), ang, 25.0, 50.0, 37, 1.0, rows, pitch, size=(20.0, 18.0, 60.0 * dz))
+             for rows, pitch, dz in ((24, 6.0, 1.0), (120, 1.2, 1.0), (129, -0.8, 0.7))]
+    geoms.append(nb.ConeBeam((20, 18, 22), ang, 70.0, 140.0, 21, 2.0, 40, 1.1))
+    rng = np.random.default_rng(2)
+    vols = [torch.from_numpy(rng.random(g.vol_shape, dtype=np.float32)).to(cuda) for g in geoms]
+    grads = [torch.from_numpy(rng.random(g.sino_shape, dtype=np.float32)).to(cuda) for g in geoms]
+    vols[1][31, 9, 12] = float("inf")
+    grads[1][2, 60, 18] = float("inf")
+    with _walk(walk):
+        bp = BatchProjector(geoms, vols, grads=grads, flags=flags, strategy="persistent")
+        bp.step()
+        torch.cuda.synchronize()
+        for i, (g, v, y, s, b) in enumerate(zip(geoms, vols, grads, bp.sinos, bp.backs)):
+            assert torch.equal(s, ops.cb_forward(v, g, flags))
+            ref = ops.cb_backward(y, g, flags)
+            fine = torch.isfinite(ref)
+            assert torch.equal(torch.isfinite(b), fine) and bool(fine.all()) == (i != 1)
+            assert_parity(torch.where(fine, b, 0.0).cpu().numpy(), torch.where(fine, ref, 0.0).cpu().numpy(),
+                          rel=1e-6, mabs=1e-5)
