@@ -81,6 +81,7 @@ struct BatchPlan {
     std::vector<std::vector<float>> angles, offsets;
     int strategy = NEFCT_BATCH_PER_PROBLEM;
     bool colwarp = false;                  // column warps (fixed at plan time)
+    bool steep = false;                    // some problem may have steep rays
     std::vector<int> order;                // plan order -> caller index
     std::vector<BatchDesc> desc;           // plan order (device pointers filled at bind)
     std::vector<long long> t0;             // tile offsets, n + 1
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(256) batch_kernel(const __grid_constant__ Batc
 }
 
 // One warp's rows of column ia at view iv, from row `first` on: R rows per lane.
-template <bool FWD, bool REF, int R>
+template <bool FWD, bool REF, bool STEEP, int R>
 __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first, int iv)
 {
     if (FWD) {
@@ -200,7 +201,7 @@ __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first
             const int ib = col_row<R, false>(first, threadIdx.x, i, false);
             P.sino[((size_t)iv * P.nb + ib) * P.na + ia] = v;
         };
-        colwarp_forward<R, REF, true>(P.g, P.flags, P.volT, row, store);
+        colwarp_forward<R, REF, (STEEP ? kSteepCall : kNoSteep)>(P.g, P.flags, P.volT, row, store);
     } else {
         float r[R][6], y[R];
         bool has[R];
@@ -212,8 +213,8 @@ __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first
             y[i] = has[i] ? P.grad[((size_t)iv * P.nb + ib) * P.na + ia] : 0.f;
             cb_ray(P.rg, P.cs[iv], P.sn[iv], P.off[iv], ia, has[i] ? ib : 0, r[i]);
         }
-        if (R > 1 && P.near) colwarp_backward<R, REF, (R > 1)>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
-        else colwarp_backward<R, REF, false>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
+        if (R > 1 && P.near) colwarp_backward<R, REF, (R > 1), STEEP>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
+        else colwarp_backward<R, REF, false, STEEP>(P.g, r, has, P.flags, y, FloatAcc{P.volT});
     }
 }
 
@@ -221,7 +222,7 @@ __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first
 // one warp per column.  Bounded to 64 registers (4 CTAs of 256 threads per
 // SM) like the single-problem kernels: the dynamically indexed problem
 // descriptor then spills up to 200 bytes outside the slab loops.
-template <bool FWD, bool REF>
+template <bool FWD, bool REF, bool STEEP>
 __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_constant__ BatchArgs a)
 {
     __shared__ long long s_item;
@@ -242,9 +243,18 @@ __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_cons
         if (ia >= P.na) continue;         // uniform across the warp
         // 32 rows or fewer left: one row per lane (28 problems of 16^3 to 64^3 with 24
         // to 128 rows, both directions: 0.837 -> 0.796 ms)
-        if (P.nb - rt * 64 > 32) batch_rows<FWD, REF, 2>(P, ia, rt * 64, iv);
-        else batch_rows<FWD, REF, 1>(P, ia, rt * 64, iv);
+        if (P.nb - rt * 64 > 32) batch_rows<FWD, REF, STEEP, 2>(P, ia, rt * 64, iv);
+        else batch_rows<FWD, REF, STEEP, 1>(P, ia, rt * 64, iv);
     }
+}
+
+using BatchKernel = void (*)(const BatchArgs);
+static BatchKernel batch_colwarp(bool fwd, bool ref, bool steep)
+{
+    if (steep) return fwd ? (ref ? batch_colwarp_kernel<true, true, true> : batch_colwarp_kernel<true, false, true>)
+                          : (ref ? batch_colwarp_kernel<false, true, true> : batch_colwarp_kernel<false, false, true>);
+    return fwd ? (ref ? batch_colwarp_kernel<true, true, false> : batch_colwarp_kernel<true, false, false>)
+               : (ref ? batch_colwarp_kernel<false, true, false> : batch_colwarp_kernel<false, false, false>);
 }
 
 // Per-problem strategy: the single-problem kernels launched once per problem
@@ -323,10 +333,8 @@ static nefct_status batch_launch(BatchPlan *b, bool fwd, cudaStream_t s)
     a.begin = 0; a.end = total; a.counter = counter;
     const bool ref = ref_rounding(b->flags);
     if (b->colwarp) {
-        if (fwd && ref) batch_colwarp_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
-        else if (fwd) batch_colwarp_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
-        else if (ref) batch_colwarp_kernel<false, true><<<b->grid_blocks, blk, 0, s>>>(a);
-        else batch_colwarp_kernel<false, false><<<b->grid_blocks, blk, 0, s>>>(a);
+        const auto kernel = batch_colwarp(fwd, ref, b->steep);
+        kernel<<<b->grid_blocks, blk, 0, s>>>(a);
     } else {
         if (fwd && ref) batch_kernel<true, true><<<b->grid_blocks, blk, 0, s>>>(a);
         else if (fwd) batch_kernel<true, false><<<b->grid_blocks, blk, 0, s>>>(a);
@@ -415,6 +423,7 @@ nefct_status nefct_cb_batch_plan(const nefct_cb_problem *problems, int32_t n, ui
         D.tiles_a = b->colwarp ? (g.na + b->rows - 1) / b->rows : (g.na + 31) / 32;
         D.tiles_b = b->colwarp ? (g.nb + 63) / 64 : (g.nb + b->rows - 1) / b->rows;
         D.near = col_rows_next(D.g, D.rg, D.nb) > 1;
+        b->steep = b->steep || cb_may_be_steep(D.g, D.rg, D.nb);
         D.flags = flags;
         b->t0[k + 1] = b->t0[k] + (long long)D.tiles_a * D.tiles_b * g.nv;
         b->c0[k + 1] = b->c0[k] + (long long)((g.grid.nx + 31) / 32) * ((g.grid.nz + 31) / 32) * g.grid.ny;
@@ -477,9 +486,8 @@ nefct_status nefct_cb_batch_bind(nefct_cb_batch *b, void *workspace, size_t byte
     const void *kernels[2] = {
         ref ? (const void *)batch_kernel<true, true> : (const void *)batch_kernel<true, false>,
         ref ? (const void *)batch_kernel<false, true> : (const void *)batch_kernel<false, false>};
-    const void *colwarp_kernels[2] = {
-        ref ? (const void *)batch_colwarp_kernel<true, true> : (const void *)batch_colwarp_kernel<true, false>,
-        ref ? (const void *)batch_colwarp_kernel<false, true> : (const void *)batch_colwarp_kernel<false, false>};
+    const void *colwarp_kernels[2] = {(const void *)batch_colwarp(true, ref, b->steep),
+                                      (const void *)batch_colwarp(false, ref, b->steep)};
     for (const void *k : b->colwarp ? colwarp_kernels : kernels) {
         NEFCT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * b->rows, 0));
         lo = std::min(lo, per_sm);

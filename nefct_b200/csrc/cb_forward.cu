@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(256, 4) cb_colwarp_forward_kernel(const __grid
         const int ib = col_row<R, false>(first, threadIdx.x, i, false);
         p.out[(size_t)(p.v0 + iv) * p.na * p.nb + (size_t)ib * p.na + ia] = v;
     };
-    colwarp_forward<R, REF, false>(p.g, p.flags, p.volT, row, store);
+    colwarp_forward<R, REF, kSteepInline>(p.g, p.flags, p.volT, row, store);
 }
 
 template <bool REF>

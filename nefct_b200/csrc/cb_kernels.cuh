@@ -177,6 +177,10 @@ __global__ void __launch_bounds__(256) cb_backward_kernel(const __grid_constant_
     ray_backward<T, VAR, EXACT>(p.g, r, p.flags, y, p.out, p.outT);
 }
 
+// What a kernel does with steep rays: there are none (cb_may_be_steep); they are
+// walked in line; by a call.
+enum Steep { kNoSteep, kSteepInline, kSteepCall };
+
 // Forward of one row per lane (the whole warp calls it) of a warp with steep
 // rays, not inlined: for the batch kernel, whose walk it would cost registers
 // (64^3 to 384^3 problems: 7.68 against 9.47 ms; the single-problem kernels are
@@ -200,8 +204,8 @@ __device__ __noinline__ static float colwarp_gather_steep(const GridDev<float> &
 
 // Forward of R rows per lane of one detector column (the whole warp calls
 // it) over the z-fastest copy volZ.  row(i, r): the lane's i-th ray (false: it
-// has none); store(i, v): takes its value.  CALL: steep rays by a call.
-template <int R, bool REF, bool CALL, class Row, class Store>
+// has none); store(i, v): takes its value.
+template <int R, bool REF, Steep STEEP, class Row, class Store>
 __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_t flags, const float *__restrict__ volZ,
                                                 Row row, Store store)
 {
@@ -222,7 +226,7 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
             return;
         }
     }
-    if (CALL && q.steep) {
+    if (STEEP == kSteepCall && q.steep) {
 #pragma unroll 1
         for (int i = 0; i < R; ++i) {
             float r[6];
@@ -235,7 +239,7 @@ __device__ __forceinline__ void colwarp_forward(const GridDev<float> &g, uint32_
     GatherSink f[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) f[i] = GatherSink(volZ);
-    if (!CALL && q.steep) col_gather<R, REF, true, true>(q, volZ, f);
+    if (STEEP == kSteepInline && q.steep) col_gather<R, REF, true, true>(q, volZ, f);
     else if (q.rising && q.falling) col_gather<R, REF, true, false>(q, volZ, f);
     else col_gather<R, REF, false, false>(q, volZ, f);
 #pragma unroll
@@ -259,7 +263,8 @@ __device__ __forceinline__ FixedSink ray_sink(const FixedAcc &a, float yw) { ret
 // Transpose of one row per lane (the whole warp calls it) of the warps that the
 // walk below does not take: with steep rays, or with a value that is not finite
 // (then every slab range checked and no voxel without a share touched).  Not
-// inlined: its registers would cost the walk below 1 % more.
+// inlined, and only in the kernels for scans that may have steep rays: the call
+// costs the walk below 1 to 2 %, in line it would cost 1 % more.
 template <bool REF, class Acc>
 __device__ __noinline__ static void colwarp_scatter_rare(const GridDev<float> &g, float x1, float y1, float z1, float x2,
                                                          float y2, float z2, bool has, uint32_t flags, float y,
@@ -280,8 +285,8 @@ __device__ __noinline__ static void colwarp_scatter_rare(const GridDev<float> &g
 
 // Transpose of R rows per lane of one detector column: y[i] times the ray's
 // weights into the z-fastest accumulator acc.  NEXT: the rows are neighbours
-// in z order and merge their reductions.
-template <int R, bool REF, bool NEXT, class Acc>
+// in z order and merge their reductions.  STEEP: there may be steep rays.
+template <int R, bool REF, bool NEXT, bool STEEP, class Acc>
 __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const float (&r)[R][6], bool (&has)[R],
                                                  uint32_t flags, const float (&y)[R], const Acc &acc)
 {
@@ -296,10 +301,22 @@ __device__ __forceinline__ void colwarp_backward(const GridDev<float> &g, const 
         yw[i] = q.z[i].live ? y[i] * q.W[i] : 0.f;
         finite = finite && isfinite(yw[i]);
     }
-    if (q.steep || !__all_sync(0xffffffffu, finite)) {
+    const bool plain = __all_sync(0xffffffffu, finite);
+    if constexpr (STEEP) {
+        if (q.steep || !plain) {
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                colwarp_scatter_rare<REF>(g, r[i][0], r[i][1], r[i][2], r[i][3], r[i][4], r[i][5], has[i], flags, y[i],
+                                          acc);
+            return;
+        }
+    } else if (!plain) {
 #pragma unroll
         for (int i = 0; i < R; ++i)
-            colwarp_scatter_rare<REF>(g, r[i][0], r[i][1], r[i][2], r[i][3], r[i][4], r[i][5], has[i], flags, y[i], acc);
+            if (q.z[i].live) {
+                auto f = ray_sink(acc, yw[i]);
+                ray_slabs<REF, true, false, -1, true, false>(q.c, q.z[i], q.zg, q.K0, q.K1, 1u, f);
+            }
         return;
     }
     const bool mixed = q.rising && q.falling;
@@ -436,6 +453,18 @@ static inline int col_rows_next(const GridDev<float> &g, const RayGeom<float> &r
     const int most = std::min(4.0, 1.0 + 0.98 / (pitch * (rg.src_iso + rad)));
     static constexpr int cost[5] = {0, 67, 100, 145, 185};
     return cb_rows_per_lane(nb, 2, most, cost);
+}
+
+// Whether a scan may have steep rays (kSteep): |kz| <= sqrt(2) max |b| / src_det
+// in units of the z and x pitch, since a ray runs at least src_det in x and y, of
+// it 1 / sqrt(2) along its driving axis.  The transposes and the batch kernels
+// without them are about 1 % faster (256^3, 48 views, transpose 2.008 against 2.031
+// ms; 7 problems of 16^3 to 64^3, 84.9 + 94.8 against 86.1 + 95.5 us).
+static inline bool cb_may_be_steep(const GridDev<float> &g, const RayGeom<float> &rg, int nb)
+{
+    if (!(rg.src_det > 0.f)) return true;
+    const double b0 = (double)rg.bi * rg.db - rg.half_b, b1 = (nb - 1 + (double)rg.bi) * rg.db - rg.half_b;
+    return !(sqrt(2.0) * std::max(fabs(b0), fabs(b1)) / rg.src_det / g.dz < 0.98);
 }
 
 // Column warps apply to FP32 slab walks with a workspace; the z-fastest

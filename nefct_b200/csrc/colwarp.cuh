@@ -185,11 +185,14 @@ __device__ __forceinline__ ZRay z_ray(const Walk<float> &w, const ZGrid &zg, con
     z.kw = live ? w.kw : 0.f;
     z.pw = live ? w.pw : __fmul_rn(__fsub_rn(0.5f, zg.nz2), zg.dz);
     z.zi = s.zi;
-    // (a level ray has its height as rounded: along a plane of the grid that decides
-    // which slice it lies in, as in the reference)
-    z.z0 = !live ? __fsub_rn(0.5f, s.row) : z.kz == 0.f ? __fsub_rn(w.z0, s.row) : s.z0;
-    // (the slope's rounding, added back at the grid's middle plane)
-    if (!REF && zg.div && live) z.z0 = __fmaf_rn(-w.pu * zg.rdz, __fmaf_rn(-w.kz, zg.dz, w.kw), z.z0);
+    z.z0 = 0.f;
+    if (!REF) {
+        // (a level ray has its height as rounded: along a plane of the grid that
+        // decides which slice it lies in, as in the reference)
+        z.z0 = !live ? __fsub_rn(0.5f, s.row) : z.kz == 0.f ? __fsub_rn(w.z0, s.row) : s.z0;
+        // (the slope's rounding, added back at the grid's middle plane)
+        if (zg.div && live) z.z0 = __fmaf_rn(-w.pu * zg.rdz, __fmaf_rn(-w.kz, zg.dz, w.kw), z.z0);
+    }
     z.ikz = fminf(__fdiv_rn(1.f, fabsf(z.kz)), 1e30f);
     z.down = z.kz < 0.f;
     z.steep = fabsf(z.kz) > kSteep;

@@ -338,3 +338,25 @@ def test_few_detector_rows(cuda, oracle_lib, rows, flags):
     assert_parity(plan.backs[0].cpu().numpy(), ref_b)
     fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
     assert torch.equal(*fixed)
+
+
+@pytest.mark.parametrize("flags", [0, _lib.REF_BACKPROJECT], ids=["default", "reference-rounding"])
+@pytest.mark.parametrize("bound", [0.97, 0.99, 1.3])
+def test_both_sides_of_the_steep_line(cuda, oracle_lib, bound, flags):
+    """Transposes are launched without the code for steep rays while sqrt(2) max |b|
+    / src_det stays under 0.98 voxel rows per slab; views along the diagonals have
+    rays that come close to that bound."""
+    rows, vz = 58, 0.8
+    pitch = bound * vz * 50.0 / np.sqrt(2.0) / (rows / 2 - 0.5)
+    ang = np.array([np.pi / 4, 3 * np.pi / 4 + 0.01, 4.0, 5.49], np.float32)
+    g = nb.ConeBeam((20, 18, 60), ang, 25.0, 50.0, 37, 0.7, rows, float(np.float32(pitch)), size=(20.0, 18.0, 60.0 * vz))
+    rng = np.random.default_rng(4)
+    vol = rng.random(g.vol_shape, dtype=np.float32)
+    y = rng.random(g.sino_shape, dtype=np.float32)
+    ref_f, ref_b = _oracle(oracle_lib, g, vol, y, flags)
+    v, s = torch.from_numpy(vol).to(cuda), torch.from_numpy(y).to(cuda)
+    f, b = _both(g, v, s, flags, 3)
+    assert_parity(f.cpu().numpy(), ref_f)
+    assert_parity(b.cpu().numpy(), ref_b)
+    fixed = [ops.cb_backward(s, g, flags | _lib.DETERMINISTIC | extra) for extra in (0, _lib.NO_TRANSPOSE)]
+    assert torch.equal(*fixed)
