@@ -171,7 +171,7 @@ template <bool REF> __device__ __forceinline__ ZSource z_source(const Walk<float
     s.zi = (int)s.row;
     const float q = zg.div ? __fdiv_rn(w.pw, zg.dz) : w.pw;
     s.z0 = __fsub_rn(q, __fsub_rn(s.row, zg.nz2));
-    if (zg.div) s.z0 = __fadd_rn(s.z0, __fdiv_rn(__fmaf_rn(-q, zg.dz, w.pw), zg.dz));
+    if (zg.div) s.z0 = __fmaf_rn(__fmaf_rn(-q, zg.dz, w.pw), zg.rdz, s.z0);
     return s;
 }
 
