@@ -221,7 +221,7 @@ __device__ __forceinline__ void batch_rows(const BatchDesc &P, int ia, int first
 // Column-warp variant: a tile is blockDim.y columns x 64 rows of one view,
 // one warp per column.  Bounded to 64 registers (4 CTAs of 256 threads per
 // SM) like the single-problem kernels: the dynamically indexed problem
-// descriptor then spills up to 200 bytes outside the slab loops.
+// descriptor then spills up to 250 bytes (360 with steep rays) outside the slab loops.
 template <bool FWD, bool REF, bool STEEP>
 __global__ void __launch_bounds__(256, 4) batch_colwarp_kernel(const __grid_constant__ BatchArgs a)
 {

@@ -373,7 +373,7 @@ struct FixedSink {
 // slabs together; where the gathers stride along v (x-driven rays without the
 // y-fastest copy) lanes in step read one x column of rows 4 nx bytes apart, whose
 // sectors share banks, so there each keeps its own phase.
-// Bound by issue (76 % with the copy) and the gathers' latency; 256^3, 48 views of
+// Bound by issue (82 % with the copy) and the gathers' latency; 256^3, 48 views of
 // 512 x 384: forward 3.56 ms with the y-fastest copy (one slab at a time 3.85), 4.19
 // without (in step 4.83), transpose 3.98 and 8.02; with the reference's rounding
 // 3.86, 4.39, 4.30 and 8.04.
